@@ -56,7 +56,7 @@ struct Fmm {
     float *otab = nullptr;   // rotation-based M2M / L2L tables (oct_layout)
     void *arena = nullptr;
     size_t arena_bytes = 0;
-    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ
+    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue
     unsigned long long *h_counts = nullptr;
     // caller particles followed by their source-only symmetry images
     double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr, *eoff = nullptr;
@@ -1116,264 +1116,307 @@ __device__ __forceinline__ void kahan_add(float &s, float &e, float v) {
     s = t;
 }
 
-// Near field of one leaf box per warp.  The box's non-empty near boxes, then
-// its far-direct boxes (interaction-list entries cheaper as pairs, from
-// build_lists_box), are compacted into shared memory with a running count of
-// their sources; the sources are then streamed 32 at a time across box
-// boundaries (each lane walks forward to the box of its staged source), so the
-// pair loop runs without per-box padding or per-box overhead.  Sources are
-// staged as negated coordinates in structure-of-arrays rows, so one 64-bit
-// load gives two consecutive sources and each pair operation is a packed
-// FP32x2 instruction (FADD2 / FFMA2 / FMUL2) over two sources; the reciprocal
-// square roots stay scalar.  Targets: two per lane while more than 48 remain,
-// then one per lane; a chunk of nt < 32 targets gives each target a group of g
-// lanes (a power of two, nt * g <= 32) that split the staged sources.  Each
-// 32-source chunk's FP32 partial sum is added with Kahan compensation.  The
-// result is stored (each particle of a box with targets once; boxes without
-// targets are left as they are).  CLAMP: floor r^2 at kMinR2, needed only when
-// eps^2 < kMinR2 (a zero-distance pair without softening).  UQ: every particle
-// of the tree carries the same charge Q (box_relative_kernel found no other),
-// so the pair weight is r^-3 alone, the sums are scaled by the target's own
-// charge (= Q) at the end, and padding sources sit far away (r^-3 underflows
-// to zero) instead of carrying zero charge.
+// Near field, one CTA per work item (a leaf box, or a share of its target
+// chunks).  The box's non-empty near boxes, then its far-direct boxes
+// (interaction-list entries cheaper as pairs, from build_lists_box), are
+// compacted into shared memory with a running count of their sources; the
+// sources are then streamed kSrcTile at a time across box boundaries (each
+// thread walks forward to the boxes of its staged sources), so the pair loop
+// runs without per-box padding or per-box overhead.  Sources are staged as
+// negated coordinates in structure-of-arrays rows, so one 64-bit load gives
+// two consecutive sources and each pair operation is a packed FP32x2
+// instruction (FADD2 / FFMA2 / FMUL2) over two sources; the reciprocal square
+// roots stay scalar.
+//
+// Split: a chunk of nt <= 2 kP2PThreads targets takes h = ceil(nt / 2) threads,
+// two targets each, and s = kP2PThreads / h such groups (32 at most) that share
+// the staged sources run by run, so the lanes stay busy whatever the box
+// holds (h s / kP2PThreads, ~0.9 on average) and a box with many targets and
+// sources occupies four warps instead of one.  Up to 64 sources per group are
+// summed in FP32 (32 per half of the packed pair), then added with Kahan
+// compensation; the groups' sums are added in group order at the end, so the
+// result does not depend on scheduling.  FP32-pipe bound: 11 FMA-pipe operations and one reciprocal
+// square root per pair.
+//
+// The result is stored (each particle of a box with targets once; boxes
+// without targets are left as they are).  CLAMP: floor r^2 at kMinR2, needed
+// only when eps^2 < kMinR2 (a zero-distance pair without softening).  UQ:
+// every particle of the tree carries the same charge Q (box_relative_kernel
+// found no other), so the pair weight is r^-3 alone, the sums are scaled by
+// the target's own charge (= Q) at the end, and padding sources sit far away
+// (r^-3 underflows to zero) instead of carrying zero charge.
 constexpr int kFarDirectCap = 128;  // far-direct source boxes per leaf box
+constexpr int kP2PThreads = 128;
+constexpr int kSrcTile = 2 * kP2PThreads;  // sources staged per round, two per thread
 // source boxes a leaf box's near field can take: its near boxes and its far-direct ones
 template <int WS>
 constexpr int p2p_nsp() { return ((2 * WS + 1) * (2 * WS + 1) * (2 * WS + 1) + 31) / 32 * 32 + kFarDirectCap; }
 
+template <int WS>
+struct P2PShared {
+    float st[2][4][kSrcTile];      // staged sources (double buffer): -x, -y, -z, charge
+    float4 raw[2][kSrcTile];       // the next sources as copied (double buffer; each thread its own)
+    float4 nb_off[p2p_nsp<WS>()];  // source box centre - target box centre (exact in FP32)
+    int2 nb_rng[p2p_nsp<WS>()];    // (first source, running source count at the box's end)
+    int scan[2][kP2PThreads / 32], nz[2][kP2PThreads / 32];  // per warp and list: sources, non-empty boxes
+    int item;
+};
+
+// Chunks a box's nt targets are cut into.  A chunk's time per source is that
+// of staging it (~60 issue slots per 256 sources and warp) plus 44 FMA-pipe
+// clocks per two sources and group step, 1 / s of them per group: c chunks cost
+// c (1 + 96 / s).  The least of four successive counts is taken, from `parts`
+// on (so that a tree of few boxes gives every CTA slot work) unless a chunk
+// would fall below 16 targets.
+__device__ __forceinline__ int p2p_chunks(int nt, int parts) {
+    if (nt <= 0) return 0;
+    const int c0 = max((nt + 2 * kP2PThreads - 1) / (2 * kP2PThreads), min(parts, (nt + 15) / 16));
+    const int c1 = max(c0, min(c0 + 3, (nt + 7) / 8));
+    int best = c0;
+    float cost = FLT_MAX;
+    for (int c = c0; c <= c1; c++) {
+        const int h = ((nt + c - 1) / c + 1) >> 1, s = min(32, kP2PThreads / h);
+        const float t = (float)c * (1.f + 96.f / (float)s);
+        if (t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
+}
 
 template <int WS, bool CLAMP, bool UQ>
 __device__ __forceinline__ void
-p2p_body(int nbox, const int *__restrict__ nbd, const int *__restrict__ bpid, const int *__restrict__ start,
+p2p_item(P2PShared<WS> &sh, int b, int part, int parts, const int *__restrict__ bpid, const int *__restrict__ start,
          const int4 *__restrict__ coord, const int *__restrict__ nbr, const double *__restrict__ qm,
          const double *__restrict__ roots, int level, float eps2, double *__restrict__ ax, double *__restrict__ ay,
-         double *__restrict__ az, unsigned long long *__restrict__ counts, const int *__restrict__ has_tgt,
-         const float4 *__restrict__ rel, const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap,
-         float (*st)[4][32], float4 (*raw)[2][32], int2 (*nb_rng)[p2p_nsp<WS>()],
-         float4 (*nb_off)[p2p_nsp<WS>()]) {
+         double *__restrict__ az, unsigned long long *__restrict__ counts, const float4 *__restrict__ rel,
+         const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap) {
     constexpr int NS1 = 2 * WS + 1, NS = NS1 * NS1 * NS1;
+    static_assert(NS <= kP2PThreads && kFarDirectCap <= kP2PThreads, "a list is compacted in one round");
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = start[b], nt_all = start[b + 1] - t0;
+    const int nchunk = p2p_chunks(nt_all, parts);
+    if (part >= nchunk) return;
     const float4 pad = UQ ? make_float4(1e18f, 0.f, 0.f, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float2 E2 = make_float2(eps2, eps2);
-    unsigned long long pairs = 0;
-    const unsigned lt_mask = (1u << (threadIdx.x & 31)) - 1u;
-    SV_WARP_BOXES(kWarps) {
-    if (!has_tgt[b]) continue;
-    // a power of two: k * hf is exact
     const float hf = (float)(box_root(roots, bpid, b)[3] / (double)(1 << level));
     const int4 cb = coord[b];
     int nnz = 0, total = 0;
-    // the non-empty boxes of a list (count warp-uniform; -1 entries skipped)
-    // appended with their running source count and their offset
-    auto add_boxes = [&](const int *list, int count) {
-        for (int s0 = 0; s0 < count; s0 += 32) {
-            const int s = s0 + lane;
-            int Q = -1, j0 = 0, cnt = 0;
-            if (s < count) {
-                Q = list[s];
-                if (Q >= 0) {
-                    j0 = start[Q];
-                    cnt = start[Q + 1] - j0;
-                }
+    // the non-empty boxes of a list (-1 entries skipped) appended with their
+    // running source count and their offset: one entry per thread, scanned
+    // over the CTA
+    auto add_boxes = [&](const int *list, int count, int round) {
+        int Q = -1, j0 = 0, cnt = 0;
+        if (tid < count) {
+            Q = list[tid];
+            if (Q >= 0) {
+                j0 = start[Q];
+                cnt = start[Q + 1] - j0;
             }
-            const bool f = cnt > 0;
-            const unsigned bal = __ballot_sync(0xffffffffu, f);
-            int inc = cnt;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
+        }
+        const bool f = cnt > 0;
+        const unsigned bal = __ballot_sync(0xffffffffu, f);
+        int inc = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) sh.scan[round][wid] = inc;
+        if (lane == 0) sh.nz[round][wid] = __popc(bal);
+        __syncthreads();
+        int pos = nnz + __popc(bal & ((1u << lane) - 1u)), run = total + inc;
+#pragma unroll
+        for (int w = 0; w < kP2PThreads / 32; w++) {
+            if (w < wid) {
+                pos += sh.nz[round][w];
+                run += sh.scan[round][w];
             }
-            if (f) {
-                const int pos = nnz + __popc(bal & lt_mask);
-                const int4 cq = coord[Q];
-                nb_rng[wid][pos] = make_int2(j0, total + inc);
-                nb_off[wid][pos] = make_float4((float)(cq.x - cb.x) * hf, (float)(cq.y - cb.y) * hf,
-                                               (float)(cq.z - cb.z) * hf, 0.f);
-            }
-            nnz += __popc(bal);
-            total += __shfl_sync(0xffffffffu, inc, 31);
+            nnz += sh.nz[round][w];
+            total += sh.scan[round][w];
+        }
+        if (f) {
+            const int4 cq = coord[Q];
+            sh.nb_rng[pos] = make_int2(j0, run);
+            sh.nb_off[pos] = make_float4((float)(cq.x - cb.x) * hf, (float)(cq.y - cb.y) * hf,
+                                         (float)(cq.z - cb.z) * hf, 0.f);
         }
     };
-    add_boxes(nbr + (size_t)b * NS, NS);
-    if (fd) add_boxes(fd + (size_t)b * fd_cap, fd_cnt[b]);
-    __syncwarp();
-    const int t0 = start[b], t1 = start[b + 1];
-    // Sources are staged one 32-source chunk ahead: the lane's source of the
-    // next chunk is copied into raw[buf] (cp.async) while the current chunk's
-    // pairs run.  kb / kbeg: the lane's current source box and its first
-    // running index (lanes walk forward through the compacted boxes); kn: the
-    // box slot of the copied source, -1 past the end.
-    int kb = 0, kbeg = 0, kn = -1;
-    auto prefetch = [&](int c0, int buf) {
-        const int j = c0 + lane;
-        kn = -1;
-        if (j < total) {
-            int2 rg = nb_rng[wid][kb];
-            while (rg.y <= j) {
-                kbeg = rg.y;
-                rg = nb_rng[wid][++kb];
-            }
-            cp_async16(&raw[wid][buf][lane], rel + rg.x + (j - kbeg));
-            kn = kb;
-        }
-        cp_async_commit();
-    };
-    // the copied chunk, moved to its target-box offset, into the staging rows
-    auto stage = [&](int buf) {
-        cp_async_wait_all();
-        float4 v = pad;
-        if (kn >= 0) {
-            const float4 r = raw[wid][buf][lane];
-            const float4 o = nb_off[wid][kn];
-            v = make_float4(r.x + o.x, r.y + o.y, r.z + o.z, r.w);
-        }
-        st[wid][0][lane] = -v.x;
-        st[wid][1][lane] = -v.y;
-        st[wid][2][lane] = -v.z;
-        if (!UQ) st[wid][3][lane] = v.w;
-    };
-    int tb = t0;
-    // two targets per lane while more than 48 remain: each staged source
-    // (one shared-memory load) then feeds two pairs.  33-48 targets cost less
-    // as one full pass of 32 and a pass that splits the sources of the
-    // remaining 1-16 targets over 2-32 lanes each.
-    for (; t1 - tb > 48; tb += 64) {
-        const int ia = tb + lane, ib = tb + 32 + lane;
-        const bool vb = ib < t1;
-        const float4 ta = rel[ia], tbv = rel[vb ? ib : ia];
-        if (lane == 0) pairs += (unsigned long long)total * (unsigned long long)min(64, t1 - tb);
+    add_boxes(nbr + (size_t)b * NS, NS, 0);
+    if (fd) add_boxes(fd + (size_t)b * fd_cap, fd_cnt[b], 1);
+    __syncthreads();
+    const int csize = (nt_all + nchunk - 1) / nchunk;
+    for (int ch = part; ch < nchunk; ch += parts) {
+        const int tb = t0 + ch * csize, nt = min(csize, t0 + nt_all - tb);
+        const int h = (nt + 1) >> 1, s = min(32, kP2PThreads / h);
+        // each group's run of a tile: 32 consecutive sources, fewer when more than
+        // eight groups share the staging rows
+        const int run = s <= 8 ? 32 : (s <= 16 ? 16 : 8), tile = s * run;
+        const int grp = tid / h, lt = tid - grp * h;
+        const bool active = grp < s;
+        const int ia = tb + lt, ib = ia + h;
+        const bool vb = active && lt + h < nt;
+        const float4 ta = rel[active ? ia : tb], tbv = rel[vb ? ib : tb];
+        if (tid == 0) atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)nt);
         const float2 AX = make_float2(ta.x, ta.x), AY = make_float2(ta.y, ta.y), AZ = make_float2(ta.z, ta.z);
         const float2 BX = make_float2(tbv.x, tbv.x), BY = make_float2(tbv.y, tbv.y), BZ = make_float2(tbv.z, tbv.z);
         float sax = 0.f, say = 0.f, saz = 0.f, eax = 0.f, eay = 0.f, eaz = 0.f;
         float sbx = 0.f, sby = 0.f, sbz = 0.f, ebx = 0.f, eby = 0.f, ebz = 0.f;
-        kb = kbeg = 0;
-        prefetch(0, 0);
-        for (int c0 = 0, buf = 0; c0 < total; c0 += 32, buf ^= 1) {
-            stage(buf);
-            if (c0 + 32 < total) prefetch(c0 + 32, buf ^ 1);
-            __syncwarp();
-            float2 gax = make_float2(0.f, 0.f), gay = gax, gaz = gax, gbx = gax, gby = gax, gbz = gax;
-#pragma unroll 4
-            for (int k = 0; k < 32; k += 2) {
-                const float2 X = ld2(st[wid][0], k), Y = ld2(st[wid][1], k), Z = ld2(st[wid][2], k);
-                const float2 Q = UQ ? make_float2(1.f, 1.f) : ld2(st[wid][3], k);
-                pair2<CLAMP, UQ>(X, Y, Z, Q, AX, AY, AZ, E2, gax, gay, gaz);
-                pair2<CLAMP, UQ>(X, Y, Z, Q, BX, BY, BZ, E2, gbx, gby, gbz);
+        // Sources are staged one tile ahead: the thread's two sources of the
+        // next tile are copied into raw[buf] (cp.async) while the current
+        // tile's pairs run.  kb / kbeg: the thread's current source box and its
+        // first running index; kn: the box slots of the copied sources, -1 past
+        // the end.
+        int kb = 0, kbeg = 0, kn0 = -1, kn1 = -1;
+        auto copy_one = [&](int j, int end, float4 *dst) {
+            if (j >= end) return -1;
+            int2 rg = sh.nb_rng[kb];
+            while (rg.y <= j) {
+                kbeg = rg.y;
+                rg = sh.nb_rng[++kb];
             }
-            const float fax = gax.x + gax.y, fay = gay.x + gay.y, faz = gaz.x + gaz.y;
-            const float fbx = gbx.x + gbx.y, fby = gby.x + gby.y, fbz = gbz.x + gbz.y;
-            __syncwarp();
-            kahan_add(sax, eax, fax);
-            kahan_add(say, eay, fay);
-            kahan_add(saz, eaz, faz);
-            kahan_add(sbx, ebx, fbx);
-            kahan_add(sby, eby, fby);
-            kahan_add(sbz, ebz, fbz);
-        }
-        {
-            const double c = UQ ? qm[ia] * (double)ta.w : qm[ia];
-            ax[ia] = (double)(sax - eax) * c;
-            ay[ia] = (double)(say - eay) * c;
-            az[ia] = (double)(saz - eaz) * c;
-        }
-        if (vb) {
-            const double c = UQ ? qm[ib] * (double)tbv.w : qm[ib];
-            ax[ib] = (double)(sbx - ebx) * c;
-            ay[ib] = (double)(sby - eby) * c;
-            az[ib] = (double)(sbz - ebz) * c;
-        }
-    }
-    for (; tb < t1; tb += 32) {
-        const int nt = min(32, t1 - tb);
-        int lg = 0;
-        while ((nt << (lg + 1)) <= 32) lg++;
-        const int g = 1 << lg;
-        const int tloc = lane >> lg, sub = lane & (g - 1);
-        const bool valid = tloc < nt;
-        const int i = tb + (valid ? tloc : 0);
-        const float4 ti = rel[i];
-        const float2 TX = make_float2(ti.x, ti.x), TY = make_float2(ti.y, ti.y), TZ = make_float2(ti.z, ti.z);
-        if (lane == 0) pairs += (unsigned long long)total * (unsigned long long)nt;
-        float sx = 0.f, sy = 0.f, sz = 0.f, ex = 0.f, ey = 0.f, ez = 0.f;
-        kb = kbeg = 0;
-        prefetch(0, 0);
-        for (int c0 = 0, buf = 0; c0 < total; c0 += 32, buf ^= 1) {
-            stage(buf);
-            if (c0 + 32 < total) prefetch(c0 + 32, buf ^ 1);
-            __syncwarp();
-            // g lanes per target, each taking pairs of consecutive sources 2 sub + 2 g i
-            // (g = 1: every lane a target and all 32 staged sources; padding adds nothing)
-            float2 gx = make_float2(0.f, 0.f), gy = gx, gz = gx;
-#pragma unroll 4
-            for (int k = 2 * sub; k < 32; k += 2 * g) {
-                const float2 X = ld2(st[wid][0], k), Y = ld2(st[wid][1], k), Z = ld2(st[wid][2], k);
-                const float2 Q = UQ ? make_float2(1.f, 1.f) : ld2(st[wid][3], k);
-                pair2<CLAMP, UQ>(X, Y, Z, Q, TX, TY, TZ, E2, gx, gy, gz);
+            cp_async16(dst, rel + rg.x + (j - kbeg));
+            return kb;
+        };
+        auto prefetch = [&](int c0, int buf) {
+            const int c1 = min(total, c0 + tile);
+            kn0 = copy_one(c0 + tid, c1, &sh.raw[buf][tid]);
+            kn1 = copy_one(c0 + kP2PThreads + tid, c1, &sh.raw[buf][kP2PThreads + tid]);
+            cp_async_commit();
+        };
+        // the copied tile, moved to its target-box offset, into the staging rows
+        auto stage_one = [&](int kn, int k, int buf) {
+            float4 v = pad;
+            if (kn >= 0) {
+                const float4 r = sh.raw[buf][k];
+                const float4 o = sh.nb_off[kn];
+                v = make_float4(r.x + o.x, r.y + o.y, r.z + o.z, r.w);
             }
-            const float fx = gx.x + gx.y, fy = gy.x + gy.y, fz = gz.x + gz.y;
-            __syncwarp();
-            float y = fx - ex, t = sx + y;
-            ex = (t - sx) - y;
-            sx = t;
-            y = fy - ey;
-            t = sy + y;
-            ey = (t - sy) - y;
-            sy = t;
-            y = fz - ez;
-            t = sz + y;
-            ez = (t - sz) - y;
-            sz = t;
+            sh.st[buf][0][k] = -v.x;
+            sh.st[buf][1][k] = -v.y;
+            sh.st[buf][2][k] = -v.z;
+            if (!UQ) sh.st[buf][3][k] = v.w;
+        };
+        prefetch(0, 0);
+        float2 gax = make_float2(0.f, 0.f), gay = gax, gaz = gax, gbx = gax, gby = gax, gbz = gax;
+        for (int c0 = 0, buf = 0; c0 < total; c0 += tile, buf ^= 1) {
+            cp_async_wait_all();
+            stage_one(kn0, tid, buf);
+            if (tile > kP2PThreads) stage_one(kn1, kP2PThreads + tid, buf);
+            // one barrier per tile: a thread writes st[buf] again two tiles later, after
+            // the barrier of the tile between, which every reader of st[buf] reached
+            __syncthreads();
+            if (c0 + tile < total) prefetch(c0 + tile, buf ^ 1);
+            if (active) {
+                const float *sx = &sh.st[buf][0][grp * run];
+                const float *se = sx + run;
+#pragma unroll 1
+                for (; sx < se; sx += 8) {
+#pragma unroll
+                    for (int k = 0; k < 8; k += 2) {
+                        const float2 X = ld2(sx, k), Y = ld2(sx + kSrcTile, k), Z = ld2(sx + 2 * kSrcTile, k);
+                        const float2 Q = UQ ? make_float2(1.f, 1.f) : ld2(sx + 3 * kSrcTile, k);
+                        pair2<CLAMP, UQ>(X, Y, Z, Q, AX, AY, AZ, E2, gax, gay, gaz);
+                        pair2<CLAMP, UQ>(X, Y, Z, Q, BX, BY, BZ, E2, gbx, gby, gbz);
+                    }
+                }
+                // at most 64 sources' FP32 sums (two tiles) per compensated addition
+                if (buf || c0 + tile >= total) {
+                    kahan_add(sax, eax, gax.x + gax.y);
+                    kahan_add(say, eay, gay.x + gay.y);
+                    kahan_add(saz, eaz, gaz.x + gaz.y);
+                    kahan_add(sbx, ebx, gbx.x + gbx.y);
+                    kahan_add(sby, eby, gby.x + gby.y);
+                    kahan_add(sbz, ebz, gbz.x + gbz.y);
+                    gax = gay = gaz = gbx = gby = gbz = make_float2(0.f, 0.f);
+                }
+            }
         }
-        sx -= ex;
-        sy -= ey;
-        sz -= ez;
-        // combine the g lanes of each target
-        for (int o = g >> 1; o > 0; o >>= 1) {
-            sx += __shfl_xor_sync(0xffffffffu, sx, o);
-            sy += __shfl_xor_sync(0xffffffffu, sy, o);
-            sz += __shfl_xor_sync(0xffffffffu, sz, o);
+        // the groups' sums, through shared memory (the staging rows are free
+        // after the barrier): six rows of kP2PThreads
+        float(*red)[kP2PThreads] = reinterpret_cast<float(*)[kP2PThreads]>(&sh.st[0][0][0]);
+        __syncthreads();
+        if (grp > 0 && active) {
+            red[0][tid] = sax - eax;
+            red[1][tid] = say - eay;
+            red[2][tid] = saz - eaz;
+            red[3][tid] = sbx - ebx;
+            red[4][tid] = sby - eby;
+            red[5][tid] = sbz - ebz;
         }
-        if (valid && sub == 0) {
-            const double c = UQ ? qm[i] * (double)ti.w : qm[i];
-            ax[i] = (double)sx * c;
-            ay[i] = (double)sy * c;
-            az[i] = (double)sz * c;
+        __syncthreads();
+        if (grp == 0) {
+            for (int g = 1; g < s; g++) {
+                const int t = g * h + lt;
+                kahan_add(sax, eax, red[0][t]);
+                kahan_add(say, eay, red[1][t]);
+                kahan_add(saz, eaz, red[2][t]);
+                kahan_add(sbx, ebx, red[3][t]);
+                kahan_add(sby, eby, red[4][t]);
+                kahan_add(sbz, ebz, red[5][t]);
+            }
+            const double ca = UQ ? qm[ia] * (double)ta.w : qm[ia];
+            ax[ia] = (double)(sax - eax) * ca;
+            ay[ia] = (double)(say - eay) * ca;
+            az[ia] = (double)(saz - eaz) * ca;
+            if (vb) {
+                const double c = UQ ? qm[ib] * (double)tbv.w : qm[ib];
+                ax[ib] = (double)(sbx - ebx) * c;
+                ay[ib] = (double)(sby - eby) * c;
+                az[ib] = (double)(sbz - ebz) * c;
+            }
         }
+        __syncthreads();  // the staging rows and lists are reused
     }
-    __syncwarp();
-    }
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(&counts[1], pairs);
 }
 
-// counts[2] != 0: box_relative_kernel met two different charges
+// Items are (box, part): part p of `parts` takes the box's target chunks p,
+// p + parts, ...  A single tree launches one CTA per item; a forest (box count
+// on the device) launches resident CTAs that pull items from *queue.
+// counts[2] != 0: box_relative_kernel met two different charges.
 template <int WS, bool CLAMP>
-__global__ void __launch_bounds__(kWarps * 32, 6)
-p2p_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ bpid, const int *__restrict__ start,
-           const int4 *__restrict__ coord, const int *__restrict__ nbr, const double *__restrict__ qm,
-           const double *__restrict__ roots, int level, float eps2, double *__restrict__ ax, double *__restrict__ ay,
-           double *__restrict__ az, unsigned long long *__restrict__ counts, const int *__restrict__ has_tgt,
-           const float4 *__restrict__ rel, const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap) {
-    __shared__ __align__(16) float src[kWarps][4][32];  // staged sources: -x, -y, -z, charge
-    __shared__ int2 nb_rng[kWarps][p2p_nsp<WS>()];    // (first source, running source count at the box's end)
-    __shared__ float4 nb_off[kWarps][p2p_nsp<WS>()];  // source box centre - target box centre (exact in FP32)
-    __shared__ float4 raw[kWarps][2][32];             // next chunk's sources as copied (double buffer)
-    if (counts[2] == 0)
-        p2p_body<WS, CLAMP, true>(nbox, nbd, bpid, start, coord, nbr, qm, roots, level, eps2, ax, ay, az, counts,
-                                  has_tgt, rel, fd, fd_cnt, fd_cap, src, raw, nb_rng, nb_off);
-    else
-        p2p_body<WS, CLAMP, false>(nbox, nbd, bpid, start, coord, nbr, qm, roots, level, eps2, ax, ay, az, counts,
-                                   has_tgt, rel, fd, fd_cnt, fd_cap, src, raw, nb_rng, nb_off);
+__global__ void __launch_bounds__(kP2PThreads, 6)
+p2p_kernel(int nbox, const int *__restrict__ nbd, int parts, int *__restrict__ queue, const int *__restrict__ bpid,
+           const int *__restrict__ start, const int4 *__restrict__ coord, const int *__restrict__ nbr,
+           const double *__restrict__ qm, const double *__restrict__ roots, int level, float eps2,
+           double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
+           unsigned long long *__restrict__ counts, const int *__restrict__ has_tgt, const float4 *__restrict__ rel,
+           const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap) {
+    __shared__ __align__(16) P2PShared<WS> sh;
+    const int items = level_boxes(nbox, nbd) * parts;
+    const bool uq = counts[2] == 0;
+    int it = blockIdx.x;
+    while (true) {
+        if (queue) {
+            __syncthreads();
+            if (threadIdx.x == 0) sh.item = atomicAdd(queue, 1);
+            __syncthreads();
+            it = sh.item;
+        }
+        if (it >= items) return;
+        const int b = it / parts, part = it - b * parts;
+        if (has_tgt[b]) {
+            if (uq)
+                p2p_item<WS, CLAMP, true>(sh, b, part, parts, bpid, start, coord, nbr, qm, roots, level, eps2, ax, ay,
+                                          az, counts, rel, fd, fd_cnt, fd_cap);
+            else
+                p2p_item<WS, CLAMP, false>(sh, b, part, parts, bpid, start, coord, nbr, qm, roots, level, eps2, ax,
+                                           ay, az, counts, rel, fd, fd_cnt, fd_cap);
+        }
+        if (!queue) return;
+    }
 }
 
 // P2P launch: well-separation and whether r^2 needs the kMinR2 floor
-inline void launch_p2p(int ws, float eps2, int grid, cudaStream_t st, int nbox, const int *nbd, const int *bpid,
-                       const int *start, const int4 *coord, const int *nbr, const double *qm, const double *roots,
-                       int level, double *ax, double *ay, double *az, unsigned long long *counts,
+inline void launch_p2p(int ws, float eps2, int grid, cudaStream_t st, int nbox, const int *nbd, int parts, int *queue,
+                       const int *bpid, const int *start, const int4 *coord, const int *nbr, const double *qm,
+                       const double *roots, int level, double *ax, double *ay, double *az, unsigned long long *counts,
                        const int *has_tgt, const float4 *rel, const int *fd = nullptr,
                        const int *fd_cnt = nullptr, int fd_cap = 0) {
     const bool clamp = !(eps2 >= kMinR2);
-#define SV_P2P(W, C) p2p_kernel<W, C><<<grid, kWarps * 32, 0, st>>>(nbox, nbd, bpid, start, coord, nbr, qm, roots, \
-                                                                   level, eps2, ax, ay, az, counts, has_tgt, rel,  \
-                                                                   fd, fd_cnt, fd_cap)
+#define SV_P2P(W, C) p2p_kernel<W, C><<<grid, kP2PThreads, 0, st>>>(nbox, nbd, parts, queue, bpid, start, coord, nbr, \
+                                                                   qm, roots, level, eps2, ax, ay, az, counts,       \
+                                                                   has_tgt, rel, fd, fd_cnt, fd_cap)
     if (ws == 1) {
         if (clamp) SV_P2P(1, true);
         else SV_P2P(1, false);
@@ -1461,7 +1504,7 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         la.lv[L].fd_cnt = (int *)carve((size_t)T.lv[L].nbox * sizeof(int));
     }
     phase_mark(c, 2);
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 3 * sizeof(unsigned long long), c->stream));
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 4 * sizeof(unsigned long long), c->stream));
     // which boxes hold targets (all of them unless symmetry images are present)
     int *tgt[kMortonBits + 1];
     {
@@ -1524,7 +1567,9 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         SV_LAUNCHED(c);
         SV_CK(c, cudaEventRecord(F.ev_rel, F.side));
         if (c->P.profile_phases) SV_CK(c, cudaEventRecord(F.ev_near[0], F.side));
-        launch_p2p(ws, (float)c->P.softening2, div_up(V.nbox, kWarps), F.side, V.nbox, nullptr, nullptr, V.start,
+        // few boxes: their target chunks to several CTAs, two waves of the CTAs that fit at once
+        const int parts = std::max(1, std::min(8, div_up(2 * 6 * device_sms(), V.nbox)));
+        launch_p2p(ws, (float)c->P.softening2, V.nbox * parts, F.side, V.nbox, nullptr, parts, nullptr, nullptr, V.start,
                    V.coord, nbr[L], S.qm, S.root, L, S.ax, S.ay, S.az, F.d_counts, tgt[L], F.rel, la.lv[L].fd,
                    la.lv[L].fd_cnt, kFarDirectCap);
         SV_LAUNCHED(c);
@@ -1700,6 +1745,8 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
 
 
 // ------------------------------------------------------------------ forest --
+constexpr int kForestParts = 2;  // work items per leaf box of the forest's near field
+
 inline int forest_grid(int cap, int per_cta) {
     const int g = div_up(cap > 0 ? cap : 1, per_cta);
     const int gmax = 16 * device_sms();  // grid-stride launches: at most 16 CTAs per SM
@@ -1717,7 +1764,7 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
     Tree &T = *F.ftree;
     int *nbd = fa.d_nbox;
     SV_TRY(tree_build_forest(c, T, f, nbd, fa.d_err));
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 3 * sizeof(unsigned long long), c->stream));
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 4 * sizeof(unsigned long long), c->stream));
     // Two streams, as in run_fmm: target flags, lists and the near field on the
     // second (the forest's slots only: the direct plumes' slots belong to
     // another stream), the upward and downward passes on the main one.
@@ -1760,7 +1807,9 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
         box_relative_kernel<<<g, kWarps * 32, 0, sd>>>(f.cap[L], nbd + L, V.pid, V.start, V.coord, S.x, S.y, S.z,
                                                        S.q, fa.roots, L, F.frel, F.d_counts + 2);
         SV_LAUNCHED(c);
-        launch_p2p(ws, (float)c->P.softening2, g, sd, f.cap[L], nbd + L, V.pid, V.start, V.coord, F.fnbr[L], S.qm,
+        launch_p2p(ws, (float)c->P.softening2, std::min(kForestParts * f.cap[L], 6 * device_sms()), sd, f.cap[L],
+                   nbd + L, kForestParts,
+                   reinterpret_cast<int *>(F.d_counts + 3), V.pid, V.start, V.coord, F.fnbr[L], S.qm,
                    fa.roots, L, S.ax, S.ay, S.az, F.d_counts, F.ftgt[L], F.frel, fd_thresh > 0 ? F.ffd : nullptr,
                    F.ffd_cnt, kFarDirectCap);
         SV_LAUNCHED(c);
@@ -1935,7 +1984,7 @@ static sv_status fmm_state(sv_ctx *c) {
     if (!c->fmm) {
         c->fmm = new Fmm();
         Fmm &F = *c->fmm;
-        SV_CK(c, cudaMalloc(&F.d_counts, 3 * sizeof(unsigned long long)));
+        SV_CK(c, cudaMalloc(&F.d_counts, 4 * sizeof(unsigned long long)));
         SV_CK(c, cudaMallocHost(&F.h_counts, 2 * sizeof(unsigned long long)));
         SV_CK(c, cudaStreamCreateWithFlags(&F.side, cudaStreamNonBlocking));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_fork, cudaEventDisableTiming));
