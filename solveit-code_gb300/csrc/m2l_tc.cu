@@ -27,6 +27,7 @@
 // 8-row x 16-byte core matrices, 128 bytes each, the core matrices of one row
 // group consecutive along K (leading-dimension offset 128 B) and row groups
 // K * 32 bytes apart (stride-dimension offset).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -188,7 +189,7 @@ __device__ __forceinline__ int tc_find_level(const TcArgs &a, int g, int &b) {
 }
 
 // Pass 1 (bucket = false): class histogram.  Pass 3 (bucket = true): rows
-// in class order.  A block takes kClsBoxes consecutive boxes: one thread
+// in class order.  A block takes bpb <= kClsBoxes consecutive boxes: one thread
 // reads each box's header (level, target flag, entry count), a block scan
 // lays the boxes' entries end to end, and the threads then walk the
 // flattened entries (every load independent of the others).  Counts go to a
@@ -200,8 +201,20 @@ __device__ __forceinline__ int tc_find_level(const TcArgs &a, int g, int &b) {
 // fewer of its SM slots (fmm_n1m, 20 steps: 2.36 against 2.40 ms per step).
 constexpr int kClsBoxes = 128;
 
+// Boxes per block: one block per SM, 4 to 128 boxes each.  Plumes resolved in
+// three dimensions have few boxes with hundreds of entries, so a fixed 128 left
+// most SMs idle (131,101 ions in a ball: 792 boxes, 7 blocks, 241 + 501 us for
+// the two passes; 5 boxes per block take the step from 1.67 to 1.42 ms).  A
+// forest's box counts are only bounded here and its boxes sit at the front of
+// each level's range, so its blocks stay small (16 boxes: 24 plumes, 13.2 ->
+// 12.4 ms for two steps).  Two or four blocks per SM measured the same.
+inline int cls_boxes(const TcArgs &a) {
+    const int want = a.total_boxes / device_sms();
+    return std::max(4, std::min(want, a.lv[0].nbd ? 16 : kClsBoxes));
+}
+
 template <bool BUCKET>
-__global__ void __launch_bounds__(kClsBoxes) tc_classes_kernel(TcArgs a, int *__restrict__ ctl,
+__global__ void __launch_bounds__(kClsBoxes) tc_classes_kernel(TcArgs a, int bpb, int *__restrict__ ctl,
                                                                int4 *__restrict__ bucket) {
     __shared__ int hist[kMaxCls];
     __shared__ int base[BUCKET ? kMaxCls : 1];
@@ -211,11 +224,10 @@ __global__ void __launch_bounds__(kClsBoxes) tc_classes_kernel(TcArgs a, int *__
     int *cls_cnt = ctl + kCtl, *cls_off = cls_cnt + a.ncls, *cursor = cls_off + 2 * a.ncls;
     if (BUCKET && ctl[2]) return;  // overflow: the rotation M2L runs instead
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    for (int k = tid; k < a.ncls; k += kClsBoxes) hist[k] = 0;
     // this thread's box
-    const int g = blockIdx.x * kClsBoxes + tid;
+    const int g = blockIdx.x * bpb + tid;
     int n = 0, li = 0, b = 0;
-    if (g < a.total_boxes) {
+    if (tid < bpb && g < a.total_boxes) {
         li = tc_find_level(a, g, b);
         const TcLevel &v = a.lv[li];
         if (b < tc_level_boxes(v) && v.has_tgt[b]) {
@@ -243,9 +255,12 @@ __global__ void __launch_bounds__(kClsBoxes) tc_classes_kernel(TcArgs a, int *__
     if (tid == kClsBoxes - 1) s_off[kClsBoxes] = woff + inc;
     __syncthreads();
     const int total = s_off[kClsBoxes];
+    if (total == 0) return;
+    for (int k = tid; k < a.ncls; k += kClsBoxes) hist[k] = 0;
+    __syncthreads();
     // the box of flattened entry f: the last box whose first entry is <= f
     auto box_of = [&](int f) {
-        int lo = 0, hi = kClsBoxes - 1;
+        int lo = 0, hi = bpb - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (s_off[mid] <= f) lo = mid;
@@ -713,13 +728,13 @@ __global__ void __launch_bounds__(128) m2l_tc_reduce_kernel(TcArgs a, const int 
 template <int P>
 sv_status launch_tc(sv_ctx *c, M2LTc &T, const TcArgs &a, int reduce_warps, cudaStream_t s) {
     static_assert(TcShape<P>::N <= kTmemCols, "accumulator wider than the TMEM allocation");
-    const int blocks = std::max(1, div_up(a.total_boxes, kClsBoxes));
+    const int bpb = cls_boxes(a), blocks = std::max(1, div_up(a.total_boxes, bpb));
     SV_CK(c, cudaMemsetAsync(T.ctl, 0, sizeof(int) * (kCtl + (size_t)a.ncls), s));
-    tc_classes_kernel<false><<<blocks, kClsBoxes, 0, s>>>(a, T.ctl, T.bucket);
+    tc_classes_kernel<false><<<blocks, kClsBoxes, 0, s>>>(a, bpb, T.ctl, T.bucket);
     SV_LAUNCHED(c);
     tc_scan_kernel<<<1, kScanThreads, 0, s>>>(a.ncls, T.cap, T.ctl, T.tiles);
     SV_LAUNCHED(c);
-    tc_classes_kernel<true><<<blocks, kClsBoxes, 0, s>>>(a, T.ctl, T.bucket);
+    tc_classes_kernel<true><<<blocks, kClsBoxes, 0, s>>>(a, bpb, T.ctl, T.bucket);
     SV_LAUNCHED(c);
     TileArgs ta{};
     for (int l = 0; l < a.nlev; l++) ta.M[l] = a.lv[l].M;
