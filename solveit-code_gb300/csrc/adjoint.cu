@@ -389,6 +389,7 @@ sv_status load_state(sv_ctx *c, const double *src) {
 sv_status jtv_add(sv_ctx *c, const double *lax, const double *lay, const double *laz, double *lx, double *ly,
                   double *lz) {
     c->fstatus = c->wstatus;
+    c->S.want_zero = true;
     const sv_status st = sort_state(c, 0, c->n);
     c->fstatus = nullptr;
     SV_TRY(st);
@@ -407,12 +408,7 @@ sv_status jtv_add(sv_ctx *c, const double *lax, const double *lay, const double 
     if (splits < 1) splits = 1;
     const int chunk = div_up(div_up(n, splits), kTile) * kTile;
     splits = div_up(n, chunk);
-    const int atomic_out = splits > 1;
-    if (atomic_out) {
-        SV_CK(c, cudaMemsetAsync(S.ax, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.ay, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.az, 0, sizeof(double) * n, c->stream));
-    }
+    const int atomic_out = splits > 1;  // into the sums the sort cleared
     const dim3 grid(tblocks, splits);
     if (c->P.precision == SV_PREC_FP64)
         jtv_fp64_kernel<<<grid, kTPB, 0, c->stream>>>(S.x, S.y, S.z, S.q, ux, uy, uz, n, chunk, c->P.softening2, S.ax,

@@ -964,6 +964,7 @@ sv_status sv::compute_accel_device(sv_ctx *c, int64_t first, int64_t last) {
         if (outliers) SV_TRY(outliers_detect(c, &st2));  // outliers leave the tree; summed directly below
         auto sort_all = [&](int levels) -> sv_status {
             c->S.want_levels = levels;
+            c->S.want_zero = c->P.method == SV_METHOD_DIRECT;  // its source splits add into the sorted accelerations
             if (outliers) {
                 const ParticleView v{c->x, c->y, c->z, c->q, c->m, st2, c->n, c->n, c->qom};
                 return sort_view(c, v, first, last);

@@ -250,12 +250,7 @@ sv_status direct_accel(sv_ctx *c) {
     if (splits < 1) splits = 1;
     int chunk = div_up(div_up(n, splits), kTile) * kTile;
     splits = div_up(n, chunk);
-    const int atomic_out = splits > 1;
-    if (atomic_out) {
-        SV_CK(c, cudaMemsetAsync(S.ax, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.ay, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.az, 0, sizeof(double) * n, c->stream));
-    }
+    const int atomic_out = splits > 1;  // into the accelerations the sort cleared
     for (int k = 2; k <= 6; k++) phase_mark(c, k);
     dim3 grid(tblocks, splits);
     if (c->P.precision == SV_PREC_FP64) {

@@ -26,24 +26,17 @@ __device__ __forceinline__ bool is_source(int32_t s) { return s == 1 || s == 2; 
 // which made the FP64 fmin / fmax the bound of this reduction.
 __device__ __forceinline__ long long ordered_bits(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
 
-// Per-block min/max of source positions (status 1 or 2), exact.
-__global__ void bbox_partial(const double *__restrict__ x, const double *__restrict__ y,
-                             const double *__restrict__ z, const int32_t *__restrict__ st,
-                             int64_t n, double *__restrict__ out) {
-    const long long lo0 = ordered_bits(__double_as_longlong(1e300)), hi0 = ordered_bits(__double_as_longlong(-1e300));
-    long long mn[3] = {lo0, lo0, lo0}, mx[3] = {hi0, hi0, hi0};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (!is_source(st[i])) continue;
-        const long long p[3] = {ordered_bits(__double_as_longlong(x[i])), ordered_bits(__double_as_longlong(y[i])),
-                                ordered_bits(__double_as_longlong(z[i]))};
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            mn[d] = min(mn[d], p[d]);
-            mx[d] = max(mx[d], p[d]);
-        }
-    }
-    __shared__ long long sh[6][kRedThreads / 32];
+__device__ __forceinline__ bool ordered_nan(long long v) {
+    return (ordered_bits(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
+constexpr double kBig = 1e300;  // bounds of an empty set
+
+// Reduce (mn, mx) over a CTA of NT threads into threads 0..5 of the first
+// warp: the value of axis d's minimum (thread d) or maximum (thread 3 + d).
+template <int NT>
+__device__ __forceinline__ long long block_bounds(long long (&mn)[3], long long (&mx)[3],
+                                                  long long (&sh)[6][NT / 32]) {
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -59,86 +52,103 @@ __global__ void bbox_partial(const double *__restrict__ x, const double *__restr
         }
     }
     __syncthreads();
+    long long v = 0;
     if (threadIdx.x < 6) {
         const int d = threadIdx.x;
-        long long v = d < 3 ? lo0 : hi0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) v = d < 3 ? min(v, sh[d][k]) : max(v, sh[d][k]);
-        out[blockIdx.x * 6 + d] = __longlong_as_double(ordered_bits(v));
+        v = sh[d][0];
+        for (int k = 1; k < NT / 32; k++) v = d < 3 ? min(v, sh[d][k]) : max(v, sh[d][k]);
     }
+    return v;
 }
 
-// Final reduction (kRedThreads threads over the block partials); root =
-// origin (bbox min), cube side S = scale x the smallest power of two > the
-// largest extent, with scale a multiple of 1/8 in [1, 2) (so every box side
-// and every box-centre offset S/2^l * k, |k| < 8, is exact in binary floating
-// point, FP32 included), bbox max, empty flag, and 2^21 / S for the keys.
-__global__ void __launch_bounds__(kRedThreads) bbox_final(const double *__restrict__ part, int nblocks,
-                                                          double *__restrict__ root, double scale) {
-    __shared__ double sh[6];
-    __shared__ double wsh[6][kRedThreads / 32];
-    double v[6] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
-    for (int k = threadIdx.x; k < nblocks; k += blockDim.x)
-        for (int d = 0; d < 6; d++) v[d] = d < 3 ? fmin(v[d], part[k * 6 + d]) : fmax(v[d], part[k * 6 + d]);
-    for (int d = 0; d < 6; d++)
-        for (int o = 16; o > 0; o >>= 1) {
-            const double u = __shfl_xor_sync(0xffffffffu, v[d], o);
-            v[d] = d < 3 ? fmin(v[d], u) : fmax(v[d], u);
-        }
-    if ((threadIdx.x & 31) == 0)
-        for (int d = 0; d < 6; d++) wsh[d][threadIdx.x >> 5] = v[d];
-    __syncthreads();
-    if (threadIdx.x < 6) {
-        const int d = threadIdx.x;
-        double r = d < 3 ? 1e300 : -1e300;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) r = d < 3 ? fmin(r, wsh[d][k]) : fmax(r, wsh[d][k]);
-        sh[d] = r;
+// Root record from the bounds b[6] (min xyz, max xyz): origin (bbox min), cube
+// side S = scale x the smallest power of two > the largest extent, with scale
+// a multiple of 1/8 in [1, 2) (so every box side and every box-centre offset
+// S/2^l * k, |k| < 8, is exact in binary floating point, FP32 included), bbox
+// max, empty flag, and 2^21 / S for the keys.
+__device__ __forceinline__ void write_root(double (&b)[6], double scale, double *__restrict__ root) {
+    double ext = 0.0;
+    const bool empty = b[0] > b[3];
+    for (int d = 0; d < 3; d++) ext = fmax(ext, b[3 + d] - b[d]);
+    if (empty) {
+        for (int d = 0; d < 6; d++) b[d] = 0.0;
+        ext = 0.0;
     }
+    // guard against a zero extent (single particle) and keep the maximum
+    // strictly inside the last cell: S > ext.
+    double S = 1e-12;
+    if (ext > 0.0) {
+        int e;
+        frexp(ext, &e);            // ext = f * 2^e, f in [0.5, 1)
+        S = ldexp(1.0, e) * scale; // >= 2^e > ext
+    }
+    for (int d = 0; d < 3; d++) root[d] = b[d];
+    root[3] = S;
+    for (int d = 0; d < 3; d++) root[4 + d] = b[3 + d];
+    root[7] = empty ? 1.0 : 0.0;
+    root[8] = (double)(1u << kMortonBits) / S;
+}
+
+// Bounds of the source positions (status 1 or 2), exact: per-block minima and
+// maxima, and the last block to finish reduces them and writes the root.  One
+// launch on the integer pipe: a second kernel for the final reduction with
+// FP64 minima took 8.2 us beside the partials' 4.3 (30,011 particles).
+__global__ void __launch_bounds__(kRedThreads)
+bbox_kernel(const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
+            const int32_t *__restrict__ st, int64_t n, long long *__restrict__ part, unsigned *__restrict__ done,
+            double scale, double *__restrict__ root) {
+    const long long lo0 = ordered_bits(__double_as_longlong(kBig)), hi0 = ordered_bits(__double_as_longlong(-kBig));
+    __shared__ long long sh[6][kRedThreads / 32];
+    __shared__ double bounds[6];
+    __shared__ bool last;
+    long long mn[3] = {lo0, lo0, lo0}, mx[3] = {hi0, hi0, hi0};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        if (!is_source(st[i])) continue;
+        const long long p[3] = {ordered_bits(__double_as_longlong(x[i])), ordered_bits(__double_as_longlong(y[i])),
+                                ordered_bits(__double_as_longlong(z[i]))};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            mn[d] = min(mn[d], p[d]);
+            mx[d] = max(mx[d], p[d]);
+        }
+    }
+    const long long v = block_bounds<kRedThreads>(mn, mx, sh);
+    if (threadIdx.x < 6) part[blockIdx.x * 6 + threadIdx.x] = v;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int d = 0; d < 3; d++) {
+        mn[d] = lo0;
+        mx[d] = hi0;
+    }
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += kRedThreads)
+        for (int d = 0; d < 3; d++) {
+            // a block whose bound is not a number is passed over, as fmin and fmax would
+            const long long a = __ldcg(&part[k * 6 + d]), b = __ldcg(&part[k * 6 + 3 + d]);
+            if (!ordered_nan(a)) mn[d] = min(mn[d], a);
+            if (!ordered_nan(b)) mx[d] = max(mx[d], b);
+        }
+    const long long r = block_bounds<kRedThreads>(mn, mx, sh);
+    if (threadIdx.x < 6) bounds[threadIdx.x] = __longlong_as_double(ordered_bits(r));
     __syncthreads();
     if (threadIdx.x == 0) {
-        double ext = 0.0;
-        bool empty = sh[0] > sh[3];
-        for (int d = 0; d < 3; d++) ext = fmax(ext, sh[3 + d] - sh[d]);
-        if (empty) {
-            for (int d = 0; d < 6; d++) sh[d] = 0.0;
-            ext = 0.0;
-        }
-        // guard against a zero extent (single particle) and keep the maximum
-        // strictly inside the last cell: S > ext.
-        double S = 1e-300;
-        if (ext > 0.0) {
-            int e;
-            frexp(ext, &e);            // ext = f * 2^e, f in [0.5, 1)
-            S = ldexp(1.0, e) * scale; // >= 2^e > ext
-        } else {
-            S = 1e-12;
-        }
-        root[0] = sh[0];
-        root[1] = sh[1];
-        root[2] = sh[2];
-        root[3] = S;
-        root[4] = sh[3];
-        root[5] = sh[4];
-        root[6] = sh[5];
-        root[7] = empty ? 1.0 : 0.0;
-        root[8] = (double)(1u << kMortonBits) / S;
+        write_root(bounds, scale, root);
+        *done = 0;
     }
 }
 
 __device__ __forceinline__ uint64_t spread3(uint32_t v) { return morton_spread3(v); }
 
-__global__ void morton_keys(const double *__restrict__ x, const double *__restrict__ y,
-                            const double *__restrict__ z, const int32_t *__restrict__ st,
-                            int64_t n, const double *__restrict__ root,
-                            uint64_t *__restrict__ keys, uint32_t *__restrict__ idx) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    idx[i] = (uint32_t)i;
-    if (!is_source(st[i])) {
-        keys[i] = kInactiveKey;
-        return;
-    }
+// Morton key of a source at (x, y, z); kInactiveKey for anything else.
+__device__ __forceinline__ uint64_t morton_key(double x, double y, double z, int32_t st,
+                                               const double *__restrict__ root) {
+    if (!is_source(st)) return kInactiveKey;
     const double inv = root[8];  // 2^21 / S, exact (S is a power of two)
-    const double p[3] = {x[i] - root[0], y[i] - root[1], z[i] - root[2]};
+    const double p[3] = {x - root[0], y - root[1], z - root[2]};
     uint32_t c[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
@@ -150,27 +160,228 @@ __global__ void morton_keys(const double *__restrict__ x, const double *__restri
         c[d] = (uint32_t)min(max(f, 0), (int)((1u << kMortonBits) - 1));
     }
     // bit order within a level: x lowest, then y, then z
-    keys[i] = spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
+    return spread3(c[0]) | (spread3(c[1]) << 1) | (spread3(c[2]) << 2);
 }
 
-__global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n,
-                              const double *__restrict__ x, const double *__restrict__ y,
-                              const double *__restrict__ z, const double *__restrict__ q,
-                              const double *__restrict__ m, const double *__restrict__ qom,
-                              const int32_t *__restrict__ st, int64_t first, int64_t last, double kconst,
-                              double *__restrict__ xs, double *__restrict__ ys,
-                              double *__restrict__ zs, float *__restrict__ qs,
-                              double *__restrict__ qm) {
+__global__ void morton_keys(const double *__restrict__ x, const double *__restrict__ y,
+                            const double *__restrict__ z, const int32_t *__restrict__ st,
+                            int64_t n, const double *__restrict__ root,
+                            uint64_t *__restrict__ keys, uint32_t *__restrict__ idx) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    idx[i] = (uint32_t)i;
+    keys[i] = morton_key(x[i], y[i], z[i], st[i], root);
+}
+
+// The sorted copy's arrays and what its gather needs.
+struct GatherArgs {
+    const double *x, *y, *z, *q, *m, *qom;
+    const int32_t *st;
+    int64_t first, last;
+    double kconst;
+    double *xs, *ys, *zs;
+    float *qs;
+    double *qm;
+    double *zax, *zay, *zaz;  // sorted accelerations to clear, or null
+};
+
+// source charge of particle i (0: no source), and its K q / m (0: no target)
+__device__ __forceinline__ float sorted_charge(const GatherArgs &a, uint32_t i) {
+    return is_source(a.st[i]) ? (float)a.q[i] : 0.0f;
+}
+__device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
+    const bool tgt = a.st[i] == 1 && (int64_t)i >= a.first && (int64_t)i < a.last && a.m[i] > 0.0;
+    return tgt ? a.kconst * (a.qom ? a.qom[i] : a.q[i] / a.m[i]) : 0.0;
+}
+
+// particle i into sorted slot s
+__device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s, uint32_t i) {
+    a.xs[s] = a.x[i];
+    a.ys[s] = a.y[i];
+    a.zs[s] = a.z[i];
+    a.qs[s] = sorted_charge(a, i);
+    a.qm[s] = sorted_qm(a, i);
+    if (a.zax) a.zax[s] = a.zay[s] = a.zaz[s] = 0.0;
+}
+
+__global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, GatherArgs a) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const uint32_t i = idx[s];
-    xs[s] = x[i];
-    ys[s] = y[i];
-    zs[s] = z[i];
-    const int32_t w = st[i];
-    qs[s] = is_source(w) ? (float)q[i] : 0.0f;
-    const bool tgt = (w == 1) && (int64_t)i >= first && (int64_t)i < last && m[i] > 0.0;
-    qm[s] = tgt ? kconst * (qom ? qom[i] : q[i] / m[i]) : 0.0;
+    if (s < n) gather_one(a, s, idx[s]);
+}
+
+// ------------------------------------------------------------- rank sort --
+// Up to kRankSortMax particles are ordered by two launches instead of CUB's
+// radix passes (one launch per 8 bits of the key, each a launch's latency at
+// these sizes): chunks of CH particles are sorted in shared memory, then every
+// particle's place in the whole order is its place in its own chunk plus its
+// place in every other chunk (binary searches), and it is gathered there
+// directly.  Both steps are stable, so the order is the one a stable radix
+// sort of the same key bits gives.  Latency bound; the searches grow with
+// n^2 / CH.  Serialised times of bounds, keys, order and gather, with CUB's
+// nine passes and now: 256 particles 36 -> 8.8 us, 4,096 97 -> 24, 16,384
+// 104 -> 35, 30,011 103 -> 45.  At 65,536 the searches take 83 us against the
+// 54 of the six passes a tree needs, so the radix passes stay above
+// kRankSortMax.
+constexpr int64_t kRankSortMax = 32768;
+constexpr int64_t kSmallChunkMax = 8192;  // chunks of 256 up to here, of 1024 above
+constexpr int kOneChunk = 1024;           // one CTA sorts a plume of up to this many
+
+// rank of `key` among the run v[0, len) of ascending keys: those below it, or
+// (UPPER) not above it
+template <bool UPPER>
+__device__ __forceinline__ int run_rank(const uint64_t *__restrict__ v, int len, uint64_t key, int sh) {
+    int lo = 0;
+    for (int n = len; n > 0;) {
+        const int half = n >> 1;
+        const uint64_t k = v[lo + half] >> sh;
+        const bool right = UPPER ? k <= key : k < key;
+        lo = right ? lo + half + 1 : lo;
+        n = right ? n - half - 1 : half;
+    }
+    return lo;
+}
+
+// Place of this thread's key in the sorted order of its chunk of CH
+// threads' keys (bits sh and up; equal keys in thread order): by counting
+// within the warp, then by doubling merges in shared memory.
+template <int CH>
+__device__ __forceinline__ int chunk_place(uint64_t key, int sh, uint64_t (*buf)[CH]) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t mine = key >> sh;
+    int r = 0;
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {
+        const uint64_t o = __shfl_sync(0xffffffffu, mine, k);
+        r += (o < mine || (o == mine && k < lane)) ? 1 : 0;
+    }
+    int pos = (threadIdx.x & ~31) + r, cur = 0;
+    for (int run = 32; run < CH; run <<= 1, cur ^= 1) {
+        buf[cur][pos] = mine;
+        __syncthreads();
+        const int start = pos & ~(run - 1), sib = start ^ run;
+        const bool left = start < sib;
+        const int o = left ? run_rank<false>(buf[cur] + sib, run, mine, 0) : run_rank<true>(buf[cur] + sib, run, mine, 0);
+        pos = min(start, sib) + (pos - start) + o;
+        // the next level writes the other buffer; this one is written again after its barrier
+    }
+    return pos;
+}
+
+// n <= CH: bounds, keys, order and gather in one CTA
+template <int CH>
+__global__ void __launch_bounds__(CH)
+sort_one_chunk(int n, int sh, double scale, double *__restrict__ root, uint64_t *__restrict__ keys,
+               uint32_t *__restrict__ idx, GatherArgs a) {
+    __shared__ uint64_t buf[2][CH];
+    __shared__ long long red[6][CH / 32];
+    __shared__ double bounds[6];
+    const int i = threadIdx.x;
+    const long long lo0 = ordered_bits(__double_as_longlong(kBig)), hi0 = ordered_bits(__double_as_longlong(-kBig));
+    long long mn[3] = {lo0, lo0, lo0}, mx[3] = {hi0, hi0, hi0};
+    double p[3] = {0.0, 0.0, 0.0};
+    int32_t st = 0;
+    if (i < n) {
+        st = a.st[i];
+        p[0] = a.x[i];
+        p[1] = a.y[i];
+        p[2] = a.z[i];
+        if (is_source(st))
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const long long v = ordered_bits(__double_as_longlong(p[d]));
+                if (!ordered_nan(v)) mn[d] = mx[d] = v;
+            }
+    }
+    const long long v = block_bounds<CH>(mn, mx, red);
+    if (i < 6) bounds[i] = __longlong_as_double(ordered_bits(v));
+    __syncthreads();
+    if (i == 0) write_root(bounds, scale, root);
+    __syncthreads();
+    const uint64_t key = i < n ? morton_key(p[0], p[1], p[2], st, root) : kInactiveKey;
+    const int pos = chunk_place<CH>(key, sh, buf);  // slots past n: inactive keys behind every particle
+    if (i < n) {
+        keys[pos] = key;
+        idx[pos] = (uint32_t)i;
+        gather_one(a, pos, (uint32_t)i);
+    }
+}
+
+// keys of a chunk of CH consecutive particles, sorted
+template <int CH>
+__global__ void __launch_bounds__(CH)
+sort_chunks(int n, int sh, const double *__restrict__ root, uint64_t *__restrict__ ckeys,
+            uint32_t *__restrict__ cidx, GatherArgs a) {
+    __shared__ uint64_t buf[2][CH];
+    const int base = blockIdx.x * CH, i = base + threadIdx.x;
+    const uint64_t key = i < n ? morton_key(a.x[i], a.y[i], a.z[i], a.st[i], root) : kInactiveKey;
+    const int pos = base + chunk_place<CH>(key, sh, buf);
+    if (i < n) {
+        ckeys[pos] = key;
+        cidx[pos] = (uint32_t)i;
+    }
+}
+
+// Every particle's rank over all chunks, and its gather: kRankLanes lanes per
+// particle, each searching every kRankLanes-th chunk, their counts added; the
+// lanes then move the particle's arrays side by side.  One lane per particle
+// left a few warps per SM waiting for dependent loads (44 against 23 us at
+// 30,011).
+constexpr int kRankLanes = 8;
+template <int CH>
+__global__ void __launch_bounds__(256)
+rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *__restrict__ cidx,
+            uint64_t *__restrict__ keys, uint32_t *__restrict__ idx, GatherArgs a) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int part = t % kRankLanes;
+    const bool live = t / kRankLanes < n;
+    const int s = live ? t / kRankLanes : n - 1;
+    const uint64_t full = ckeys[s], key = full >> sh;
+    const int own = s / CH, whole = n / CH;
+    int rank = part == 0 ? s - own * CH : 0;
+    // whole chunks two at a time, their searches independent of each other:
+    // halving steps over CH keys.  Equal keys of earlier chunks count,
+    // of later ones do not.
+    auto below = [&](uint64_t k, bool eq) { return eq ? k <= key : k < key; };
+    for (int c = part; c < whole; c += 2 * kRankLanes) {
+        int lo[2] = {0, 0};
+        const uint64_t *v[2];
+        bool before[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int cc = min(c + u * kRankLanes, whole - 1);
+            v[u] = ckeys + (size_t)cc * CH;
+            before[u] = cc < own;
+        }
+#pragma unroll
+        for (int half = CH / 2; half > 0; half >>= 1)
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                if (below(v[u][lo[u] + half - 1] >> sh, before[u])) lo[u] += half;
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            // CH - 1 keys are settled by the halving; the last one by itself
+            if (below(v[u][lo[u]] >> sh, before[u])) lo[u]++;
+            if (c + u * kRankLanes < whole && c + u * kRankLanes != own) rank += lo[u];
+        }
+    }
+    // the short last chunk comes after this particle's own
+    if (part == whole % kRankLanes && whole * CH < n && whole != own)
+        rank += run_rank<false>(ckeys + (size_t)whole * CH, n - whole * CH, key, sh);
+#pragma unroll
+    for (int o = kRankLanes / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    if (!live) return;
+    const uint32_t i = cidx[s];
+    switch (part) {
+    case 0: a.xs[rank] = a.x[i]; break;
+    case 1: a.ys[rank] = a.y[i]; break;
+    case 2: a.zs[rank] = a.z[i]; break;
+    case 3: a.qs[rank] = sorted_charge(a, i); break;
+    case 4: a.qm[rank] = sorted_qm(a, i); break;
+    case 5: keys[rank] = full; break;
+    case 6: idx[rank] = i; break;
+    default:
+        if (a.zax) a.zax[rank] = a.zay[rank] = a.zaz[rank] = 0.0;
+    }
 }
 
 // sorted slots of image copies (index >= n_orig) are sources only and have
@@ -229,8 +440,9 @@ sv_status ensure_sorted_capacity(sv_ctx *c, int64_t n) {
     S.cub_bytes = bytes;
     SV_CK(c, cudaMalloc(&S.cub_tmp, bytes));
     S.red_blocks = 2 * device_sms();
-    SV_CK(c, cudaMalloc(&S.red, (size_t)S.red_blocks * 6 * sizeof(double)));
+    SV_CK(c, cudaMalloc(&S.red, (size_t)S.red_blocks * 6 * sizeof(long long)));
     SV_CK(c, cudaMalloc(&S.root, 16 * sizeof(double)));
+    SV_CK(c, cudaMemsetAsync(S.root, 0, 16 * sizeof(double), c->stream));  // root[15]: bbox_kernel's block count
     S.cap = cap;
     return SV_OK;
 }
@@ -244,26 +456,57 @@ static double root_scale(const sv_ctx *c) {
 
 sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t last) {
     const int64_t n = v.n;
+    const bool zero = c->S.want_zero;
     SV_TRY(ensure_sorted_capacity(c, n));
     Sorted &S = c->S;
+    S.want_zero = false;
     S.n = n;
     S.n_orig = v.n_orig;
+    // levels 1 .. want_levels occupy bits >= 3 (kMortonBits - want_levels); bit 63 marks inactive keys
+    const int levels = std::max(1, std::min(kMortonBits, S.want_levels));
+    S.want_levels = kMortonBits;
+    S.key_levels = levels;
+    const int sh = 3 * (kMortonBits - levels);
+    GatherArgs ga{v.x, v.y, v.z, v.q, v.m, v.qom, v.status, first, std::min(last, v.n_orig), c->P.k_const,
+                  S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr};
+    if (zero) {
+        ga.zax = S.ax;
+        ga.zay = S.ay;
+        ga.zaz = S.az;
+    }
+    if (n <= kOneChunk) {
+        if (n <= 256)
+            sort_one_chunk<256><<<1, 256, 0, c->stream>>>((int)n, sh, root_scale(c), S.root, S.keys, S.idx, ga);
+        else
+            sort_one_chunk<kOneChunk><<<1, kOneChunk, 0, c->stream>>>((int)n, sh, root_scale(c), S.root, S.keys, S.idx,
+                                                                      ga);
+        SV_LAUNCHED(c);
+        return SV_OK;
+    }
     const int nb = div_up(n, 256);
-    bbox_partial<<<S.red_blocks, kRedThreads, 0, c->stream>>>(v.x, v.y, v.z, v.status, n, S.red);
+    bbox_kernel<<<std::min(nb, S.red_blocks), kRedThreads, 0, c->stream>>>(
+        v.x, v.y, v.z, v.status, n, S.red, reinterpret_cast<unsigned *>(S.root + 15), root_scale(c), S.root);
     SV_LAUNCHED(c);
-    bbox_final<<<1, kRedThreads, 0, c->stream>>>(S.red, S.red_blocks, S.root, root_scale(c));
-    SV_LAUNCHED(c);
+    if (n <= kRankSortMax) {
+        const int rgrid = div_up(n * kRankLanes, 256);
+        if (n <= kSmallChunkMax) {
+            sort_chunks<256><<<div_up(n, 256), 256, 0, c->stream>>>((int)n, sh, S.root, S.keys_alt, S.idx_alt, ga);
+            SV_LAUNCHED(c);
+            rank_gather<256><<<rgrid, 256, 0, c->stream>>>((int)n, sh, S.keys_alt, S.idx_alt, S.keys, S.idx, ga);
+        } else {
+            sort_chunks<1024><<<div_up(n, 1024), 1024, 0, c->stream>>>((int)n, sh, S.root, S.keys_alt, S.idx_alt, ga);
+            SV_LAUNCHED(c);
+            rank_gather<1024><<<rgrid, 256, 0, c->stream>>>((int)n, sh, S.keys_alt, S.idx_alt, S.keys, S.idx, ga);
+        }
+        SV_LAUNCHED(c);
+        return SV_OK;
+    }
     morton_keys<<<nb, 256, 0, c->stream>>>(v.x, v.y, v.z, v.status, n, S.root, S.keys, S.idx);
     SV_LAUNCHED(c);
     cub::DoubleBuffer<uint64_t> kb(S.keys, S.keys_alt);
     cub::DoubleBuffer<uint32_t> vb(S.idx, S.idx_alt);
     size_t bytes = S.cub_bytes;
-    // levels 1 .. want_levels occupy bits >= 3 (kMortonBits - want_levels); bit 63 marks inactive keys
-    const int levels = std::max(1, std::min(kMortonBits, S.want_levels));
-    S.want_levels = kMortonBits;
-    S.key_levels = levels;
-    SV_CK(c, cub::DeviceRadixSort::SortPairs(S.cub_tmp, bytes, kb, vb, (int)n, 3 * (kMortonBits - levels),
-                                             3 * kMortonBits + 1, c->stream));
+    SV_CK(c, cub::DeviceRadixSort::SortPairs(S.cub_tmp, bytes, kb, vb, (int)n, sh, 3 * kMortonBits + 1, c->stream));
     c->launches += 2 * ((3 * levels + 1 + 7) / 8);  // CUB onesweep: histogram + passes
     if (kb.Current() != S.keys) {
         std::swap(S.keys, S.keys_alt);
@@ -271,8 +514,7 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     if (vb.Current() != S.idx) {
         std::swap(S.idx, S.idx_alt);
     }
-    gather_sorted<<<nb, 256, 0, c->stream>>>(S.idx, n, v.x, v.y, v.z, v.q, v.m, v.qom, v.status, first,
-                                             std::min(last, v.n_orig), c->P.k_const, S.x, S.y, S.z, S.q, S.qm);
+    gather_sorted<<<nb, 256, 0, c->stream>>>(S.idx, n, ga);
     SV_LAUNCHED(c);
     return SV_OK;
 }

@@ -39,13 +39,14 @@ struct Sorted {
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
     double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S
-    double *red = nullptr;     // device reduction scratch
+    long long *red = nullptr;  // device reduction scratch
     int red_blocks = 0;
     int64_t cap = 0;
     // Morton levels the next sort must order (a one-shot request, reset to all
     // of them by the sort) and the levels the last sort ordered: an FMM tree
     // needs its keys ordered down to its leaf level only
     int want_levels = kMortonBits, key_levels = kMortonBits;
+    bool want_zero = false;  // the next sort also clears ax, ay, az (a method that adds into them)
     bool resort = false;  // the FMM found its leaf level below key_levels: sort again, fully
     int64_t n = 0;       // sorted entries (caller particles plus any image copies)
     int64_t n_orig = 0;  // caller particles; sorted idx >= n_orig are image copies
