@@ -708,7 +708,7 @@ void sv_destroy(sv_ctx *c) {
     cudaFree(S.x); cudaFree(S.y); cudaFree(S.z); cudaFree(S.q); cudaFree(S.qm);
     cudaFree(S.idx); cudaFree(S.keys); cudaFree(S.keys_alt); cudaFree(S.idx_alt);
     cudaFree(S.ax); cudaFree(S.ay); cudaFree(S.az); cudaFree(S.cub_tmp);
-    cudaFree(S.root); cudaFree(S.red);
+    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl);
     cudaFree(c->d_stage);
     cudaFree(c->d_scalar);
     if (c->h_scalar) cudaFreeHost(c->h_scalar);
@@ -964,7 +964,7 @@ sv_status sv::compute_accel_device(sv_ctx *c, int64_t first, int64_t last) {
         if (outliers) SV_TRY(outliers_detect(c, &st2));  // outliers leave the tree; summed directly below
         auto sort_all = [&](int levels) -> sv_status {
             c->S.want_levels = levels;
-            c->S.want_zero = c->P.method == SV_METHOD_DIRECT;  // its source splits add into the sorted accelerations
+            if (c->P.method == SV_METHOD_DIRECT) direct_sort_wants(c);
             if (outliers) {
                 const ParticleView v{c->x, c->y, c->z, c->q, c->m, st2, c->n, c->n, c->qom};
                 return sort_view(c, v, first, last);

@@ -108,11 +108,6 @@ struct BhImages {
     const double *off;
 };
 
-__device__ __forceinline__ void split_hilo(double v, float &hi, float &lo) {
-    hi = (float)v;
-    lo = (float)(v - (double)hi);
-}
-
 __global__ void particles_hilo(const double *__restrict__ xs, const double *__restrict__ ys,
                                const double *__restrict__ zs, const float *__restrict__ qs, int n,
                                const double *__restrict__ root, float4 *__restrict__ ph, float4 *__restrict__ pl) {

@@ -7,24 +7,44 @@
 // for inbound targets i and sources j with status 1 or 2 (j != i for the plain
 // sum; the symmetric variants keep the self image, which contributes 0).
 //
-// Layout: targets and sources are the Morton-sorted copy (sort.cu).  One CTA
-// owns TPB*TPT consecutive targets and loops over source tiles staged in
-// shared memory; every warp reads the same source at a time (broadcast).
+// Targets and sources are the Morton-sorted copy (sort.cu).
 //
-// MIXED: the CTA takes the FP64 position of its first target as origin; both
-// targets and the staged sources are converted to FP32 offsets from it (one
-// FP64 subtraction per staged source), so close pairs keep full FP32 relative
-// precision even at 50 um from the plume origin.  Pairs run on the FP32 pipe
-// with rsqrtf (MUFU); each tile's partial sums are added into FP64
-// accumulators.  FP64: the same tiling with every operation in FP64; 1/sqrt is
-// a FP32 rsqrt seed refined by two Newton steps in FP64.
-#include <cfloat>
+// MIXED: every unordered pair once.  The particles form blocks of 32 R; a warp
+// holds a block's coordinates and sums in registers (R particles per lane) and
+// takes tiles of 32 particles of another block, one per lane, which travel
+// around the lanes together with their own sums: after 32 steps every pair of
+// the block and the tile has been met once and has added to both sides
+// (F_ji = -F_ij up to the charges).  A pair of interactions then costs 16
+// FP32-pipe operations and one reciprocal square root instead of 24 and two.
+// Coordinates are FP32 offsets from the block's middle particle, formed from the
+// FP32 hi + lo parts that the sort wrote by an exact subtraction and one
+// rounding; where a tile comes within the block's extent, the parts that rounding
+// left out are kept too and added to each difference (six operations more, in a
+// few tiles per block), so that every pair's offset is rounded relative to its own
+// length and not to the block's.  The force error against FP64 is 1.2e-7 to 3e-7
+// (relative L2 over plumes of 256 to 30,011 ions); coordinates rounded relative to
+// a CTA's first target gave 3e-7 to 5.6e-6, set by each plume's closest pairs.
+// The loop has no FP64 instruction (GB300 issues one FP64 warp instruction in 64
+// clocks: conversions and FP64 sums per 256-source tile took 12 to 18 % of the
+// one-sided kernel).  At most 128 sources' (or 256 targets') FP32 sums go to the
+// FP64 accumulators in memory at once.
+//
+// FP64: the same pairing with every operation in FP64, or (symmetry images)
+// one-sided tiles in shared memory; r^-3 is a FP32 rsqrt seed and a third-order
+// correction in FP64.
+//
+// Measured per launch (serialised), against the one-sided kernels they
+// replaced: mixed, 30,011 particles of two charges 381 -> 303 us, 16,384 of one
+// charge 123 -> 99 us, 3,001 with 81 images 652 -> 235 us (144 CTAs before: the
+// images were not split); FP64, 4,096 particles 773 -> 315 us.
+#include <algorithm>
 
 #include "sv_internal.cuh"
 
 namespace sv {
 namespace {
 
+// one-sided FP64 kernel (symmetry images)
 constexpr int kTPB = 128;   // threads per CTA
 constexpr int kTPT = 2;     // targets per thread
 constexpr int kTile = 256;  // sources per shared-memory tile
@@ -61,107 +81,380 @@ __device__ __forceinline__ bool block_has_target(const double *__restrict__ qm, 
     return __syncthreads_or(any) != 0;
 }
 
-__global__ void __launch_bounds__(kTPB)
-direct_mixed_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
-                    const double *__restrict__ zs, const float *__restrict__ qs,
-                    const double *__restrict__ qm, int n, int chunk, float eps2, Images im,
-                    double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                    int atomic_out) {
-    __shared__ __align__(16) float tile[4][kTile];  // staged sources: -x, -y, -z, charge
-    const int t0 = blockIdx.x * (kTPB * kTPT);
-    const int j_begin = blockIdx.y * chunk;
-    const int j_end = min(n, j_begin + chunk);
-    const int o = min(t0, n - 1);
-    const double ox = xs[o], oy = ys[o], oz = zs[o];
-    if (!block_has_target(qm, t0, n)) return;  // whole CTA of non-targets (target subsets)
+// ------------------------------------------------------------------ mixed --
+struct PairArgs {
+    const float4 *ph, *pl;   // sorted positions hi (w: charge) and lo (w: 1 = target)
+    int n, nb;               // particles, blocks of 32 R of them
+    int ct, nch;             // tiles per unit (of the R x images of a block pair), units per block pair
+    float eps2;
+    int kind, images;        // symmetry images, as Images
+    const float4 *off;       // translational offsets: hi (xyz) and lo (xyz) per image
+    double *ax, *ay, *az;    // sums, added into
+    const int *differ;       // nonzero: source charges differ
+};
 
-    float2 TX[kTPT], TY[kTPT], TZ[kTPT];
-    const float2 E2 = make_float2(eps2, eps2);
-    double sx[kTPT], sy[kTPT], sz[kTPT];
+// (hi + lo) - (ohi + olo) as r + res: r the difference rounded once (of the hi
+// parts with its exact rounding error, Knuth, then the small parts), res what
+// that rounding left out
+__device__ __forceinline__ float hilo_diff(float hi, float lo, float ohi, float olo, float &res) {
+    const float s = hi - ohi, bb = s - hi;
+    const float t = ((hi - (s - bb)) - (ohi + bb)) + (lo - olo);
+    const float r = s + t, tt = r - s;
+    res = (s - (r - tt)) + (t - tt);
+    return r;
+}
+
+// a float's value as a double, by its bits (the conversion instruction runs at
+// the FP64 rate); denormals become zero
+__device__ __forceinline__ double widen(float f) {
+    const uint32_t u = __float_as_uint(f), m = u & 0x7fffffffu;
+    uint32_t hi = (m >> 3) + 0x38000000u, lo = u << 29;
+    if (m >= 0x7f800000u) hi |= 0x7ff00000u;
+    if (m < 0x00800000u) hi = lo = 0;
+    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
+}
+
+constexpr int kPairWarps = 4;    // warps (units) per CTA
+constexpr int kMaxTiles = 4;     // tiles per unit: 128 sources per FP32 sum of a target
+constexpr float kFar = 1e18f;    // coordinate of absent particles: r^-3 underflows to zero
+
+// A block's particles in registers (two per packed value) and the travelling
+// particle; the parts of the block's coordinates below FP32 in shared memory.
+template <int R>
+struct PairBlock {
+    float2 X[R / 2], Y[R / 2], Z[R / 2], Q[R / 2];   // coordinates, charges
+    float2 gx[R / 2], gy[R / 2], gz[R / 2];          // sums
+};
+template <int R>
+struct PairLow {
+    float2 x[R / 2][32], y[R / 2][32], z[R / 2][32];
+};
+
+// 32 steps of a travelling tile: negated coordinates (nx, ny, nz), charge q, and
+// with NEAR the parts below FP32 (mx, my, mz); (sx, sy, sz) return the sums on
+// the travelling particle (SYM).
+template <int R, bool UQ, bool CLAMP, bool SYM, bool NEAR>
+__device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low, float2 E2, float nx, float ny,
+                                          float nz, float q, float mx, float my, float mz, float &sx, float &sy,
+                                          float &sz) {
+    constexpr int H = R / 2;
+    const int lane = threadIdx.x & 31, from = (lane + 1) & 31;
+#pragma unroll 1
+    for (int step = 0; step < 32; step++) {
+        const float2 NX = make_float2(nx, nx), NY = make_float2(ny, ny), NZ = make_float2(nz, nz);
+        const float2 QJ = make_float2(q, q);
+        float2 jx, jy, jz;
 #pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int i = t0 + threadIdx.x + k * kTPB;
-        const int ii = min(i, n - 1);
-        const float tx = (float)(xs[ii] - ox), ty = (float)(ys[ii] - oy), tz = (float)(zs[ii] - oz);
-        TX[k] = make_float2(tx, tx);
-        TY[k] = make_float2(ty, ty);
-        TZ[k] = make_float2(tz, tz);
-        sx[k] = sy[k] = sz[k] = 0.0;
+        for (int p = 0; p < H; p++) {
+            float2 dx = __fadd2_rn(b.X[p], NX), dy = __fadd2_rn(b.Y[p], NY), dz = __fadd2_rn(b.Z[p], NZ);
+            if (NEAR) {
+                dx = __fadd2_rn(dx, __fadd2_rn(low.x[p][lane], make_float2(mx, mx)));
+                dy = __fadd2_rn(dy, __fadd2_rn(low.y[p][lane], make_float2(my, my)));
+                dz = __fadd2_rn(dz, __fadd2_rn(low.z[p][lane], make_float2(mz, mz)));
+            }
+            float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, E2)));
+            if (CLAMP) r2 = make_float2(fmaxf(r2.x, kMinR2), fmaxf(r2.y, kMinR2));
+            const float2 inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+            const float2 w = __fmul2_rn(__fmul2_rn(inv, inv), inv);
+            const float2 wi = UQ ? w : __fmul2_rn(QJ, w);
+            b.gx[p] = __ffma2_rn(dx, wi, b.gx[p]);
+            b.gy[p] = __ffma2_rn(dy, wi, b.gy[p]);
+            b.gz[p] = __ffma2_rn(dz, wi, b.gz[p]);
+            if (SYM) {
+                const float2 wj = UQ ? w : __fmul2_rn(b.Q[p], w);
+                jx = p == 0 ? __fmul2_rn(dx, wj) : __ffma2_rn(dx, wj, jx);
+                jy = p == 0 ? __fmul2_rn(dy, wj) : __ffma2_rn(dy, wj, jy);
+                jz = p == 0 ? __fmul2_rn(dz, wj) : __ffma2_rn(dz, wj, jz);
+            }
+        }
+        nx = __shfl_sync(0xffffffffu, nx, from);
+        ny = __shfl_sync(0xffffffffu, ny, from);
+        nz = __shfl_sync(0xffffffffu, nz, from);
+        if (NEAR) {
+            mx = __shfl_sync(0xffffffffu, mx, from);
+            my = __shfl_sync(0xffffffffu, my, from);
+            mz = __shfl_sync(0xffffffffu, mz, from);
+        }
+        if (!UQ) q = __shfl_sync(0xffffffffu, q, from);
+        if (SYM) {
+            sx = __shfl_sync(0xffffffffu, sx - (jx.x + jx.y), from);
+            sy = __shfl_sync(0xffffffffu, sy - (jy.x + jy.y), from);
+            sz = __shfl_sync(0xffffffffu, sz - (jz.x + jz.y), from);
+        }
     }
-    for (int g = 0; g < im.count; g++) {
-        for (int jt = j_begin; jt < j_end; jt += kTile) {
-            __syncthreads();
-            for (int s = threadIdx.x; s < kTile; s += kTPB) {
-                const int j = jt + s;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (j < j_end) {
-                    double px = xs[j], py = ys[j], pz = zs[j];
-                    image_of(im, g, px, py, pz);
-                    v = make_float4((float)(px - ox), (float)(py - oy), (float)(pz - oz), qs[j]);
+}
+
+// One unit: block A (registers) against tiles [k0, k1) of block B.  SYM: both
+// sides' sums (A != B); otherwise the sums of A only (A == B, every ordered
+// pair).  UQ: all charges equal, applied once at the end.
+template <int R, bool UQ, bool CLAMP, bool SYM>
+__device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, int A, int B, int k0, int k1) {
+    const int lane = threadIdx.x & 31;
+    const int i0 = A * 32 * R;
+    const int io = min(i0 + 16 * R, a.n - 1);  // the block's middle particle: offsets half as long as from its first
+    const float4 oh = a.ph[io], ol = a.pl[io];
+    PairBlock<R> b;
+    int tgt = 0;     // bit r: this lane's particle r of the block is a target
+    float ext = 0.f;  // the block's largest offset on any axis
+    __syncwarp();    // the previous unit's reads of `low`
+#pragma unroll
+    for (int p = 0; p < R / 2; p++) {
+        float c[2][7];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = i0 + 32 * (2 * p + u) + lane;
+            if (i < a.n) {
+                const float4 h = a.ph[i], l = a.pl[i];
+                c[u][0] = hilo_diff(h.x, l.x, oh.x, ol.x, c[u][4]);
+                c[u][1] = hilo_diff(h.y, l.y, oh.y, ol.y, c[u][5]);
+                c[u][2] = hilo_diff(h.z, l.z, oh.z, ol.z, c[u][6]);
+                c[u][3] = h.w;
+                tgt |= l.w != 0.f ? 1 << (2 * p + u) : 0;
+                ext = fmaxf(ext, fmaxf(fabsf(c[u][0]), fmaxf(fabsf(c[u][1]), fabsf(c[u][2]))));
+            } else {
+                c[u][0] = -kFar;
+                c[u][1] = c[u][2] = c[u][3] = c[u][4] = c[u][5] = c[u][6] = 0.f;
+            }
+        }
+        b.X[p] = make_float2(c[0][0], c[1][0]);
+        b.Y[p] = make_float2(c[0][1], c[1][1]);
+        b.Z[p] = make_float2(c[0][2], c[1][2]);
+        b.Q[p] = make_float2(c[0][3], c[1][3]);
+        low.x[p][lane] = make_float2(c[0][4], c[1][4]);
+        low.y[p][lane] = make_float2(c[0][5], c[1][5]);
+        low.z[p][lane] = make_float2(c[0][6], c[1][6]);
+        b.gx[p] = b.gy[p] = b.gz[p] = make_float2(0.f, 0.f);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
+    const bool anyA = __any_sync(0xffffffffu, tgt);
+    const float q0 = UQ ? oh.w : 1.f;
+    const float2 E2 = make_float2(a.eps2, a.eps2);
+    for (int k = k0; k < k1; k++) {
+        const int g = k / R, j = B * 32 * R + 32 * (k - g * R) + lane;
+        float nx = -kFar, ny = 0.f, nz = 0.f, q = 0.f, mx = 0.f, my = 0.f, mz = 0.f;  // negated coordinates
+        bool jt = false, near = false;
+        if (j < a.n) {
+            float4 h = a.ph[j], l = a.pl[j];
+            jt = l.w != 0.f;
+            q = h.w;
+            float ohx = oh.x, ohy = oh.y, ohz = oh.z, olx = ol.x, oly = ol.y, olz = ol.z;
+            if (a.kind == 1 && g) {
+                // source rotated by g*pi/2 about z (quadrantRotationFunction, auxiliary_functions.h:55-57)
+                const float hx = h.x, lx = l.x, sgx = g == 3 ? 1.f : -1.f, sgy = g == 1 ? 1.f : -1.f;
+                if (g == 2) {
+                    h.x = -hx; l.x = -lx;
+                    h.y = -h.y; l.y = -l.y;
+                } else {
+                    h.x = sgx * h.y; l.x = sgx * l.y;
+                    h.y = sgy * hx; l.y = sgy * lx;
                 }
-                tile[0][s] = -v.x;
-                tile[1][s] = -v.y;
-                tile[2][s] = -v.z;
-                tile[3][s] = v.w;
+            } else if (a.kind == 2) {
+                // source shifted by the image offset: the origin shifted back
+                const float4 fh = a.off[2 * g], fl = a.off[2 * g + 1];
+                auto back = [](float &hi, float &lo, float fhi, float flo) {
+                    const float s = hi - fhi, bb = s - hi;
+                    const float e = ((hi - (s - bb)) - (fhi + bb)) + (lo - flo);
+                    const float r = s + e;
+                    lo = e - (r - s);
+                    hi = r;
+                };
+                back(ohx, olx, fh.x, fl.x);
+                back(ohy, oly, fh.y, fl.y);
+                back(ohz, olz, fh.z, fl.z);
             }
-            __syncthreads();
-            // two sources per packed FP32x2 operation; r^2 floored at kMinR2
-            // (self pair with eps = 0: d = 0 -> 0 * finite)
-            float2 gx[kTPT], gy[kTPT], gz[kTPT];
-#pragma unroll
-            for (int k = 0; k < kTPT; k++) gx[k] = gy[k] = gz[k] = make_float2(0.f, 0.f);
-#pragma unroll 4
-            for (int s = 0; s < kTile; s += 2) {
-                const float2 X = ld2(tile[0], s), Y = ld2(tile[1], s), Z = ld2(tile[2], s), Q = ld2(tile[3], s);
-#pragma unroll
-                for (int k = 0; k < kTPT; k++) pair2<true, false>(X, Y, Z, Q, TX[k], TY[k], TZ[k], E2, gx[k], gy[k], gz[k]);
+            nx = -hilo_diff(h.x, l.x, ohx, olx, mx);
+            ny = -hilo_diff(h.y, l.y, ohy, oly, my);
+            nz = -hilo_diff(h.z, l.z, ohz, olz, mz);
+            mx = -mx;
+            my = -my;
+            mz = -mz;
+            // within twice the block's extent of its origin (a pair may be closer
+            // than the coordinates' rounding allows for)
+            near = fmaxf(fabsf(nx), fmaxf(fabsf(ny), fabsf(nz))) <= 2.f * ext;
+        }
+        const bool anyB = SYM && __any_sync(0xffffffffu, jt);
+        if (!anyA && !anyB) continue;
+        float sx = 0.f, sy = 0.f, sz = 0.f;  // the travelling particle's sums
+        if (!SYM || __any_sync(0xffffffffu, near))
+            pair_tile<R, UQ, CLAMP, SYM, true>(b, low, E2, nx, ny, nz, q, mx, my, mz, sx, sy, sz);
+        else
+            pair_tile<R, UQ, CLAMP, SYM, false>(b, low, E2, nx, ny, nz, q, mx, my, mz, sx, sy, sz);
+        if (SYM && jt) {
+            if (a.kind == 1 && g) {  // the sum on the unrotated particle: turned back by -g*pi/2
+                const float tx = sx, ty = sy;
+                if (g == 2) {
+                    sx = -tx;
+                    sy = -ty;
+                } else {
+                    sx = g == 1 ? ty : -ty;
+                    sy = g == 1 ? -tx : tx;
+                }
             }
-#pragma unroll
-            for (int k = 0; k < kTPT; k++) {
-                sx[k] += gx[k].x + gx[k].y;
-                sy[k] += gy[k].x + gy[k].y;
-                sz[k] += gz[k].x + gz[k].y;
-            }
+            atomicAdd(&a.ax[j], widen(sx * q0));
+            atomicAdd(&a.ay[j], widen(sy * q0));
+            atomicAdd(&a.az[j], widen(sz * q0));
         }
     }
+    if (!anyA) return;
 #pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int i = t0 + threadIdx.x + k * kTPB;
-        if (i >= n) continue;
-        const double c = qm[i];
-        if (c == 0.0) continue;
-        if (atomic_out) {
-            atomicAdd(&ax[i], sx[k] * c);
-            atomicAdd(&ay[i], sy[k] * c);
-            atomicAdd(&az[i], sz[k] * c);
+    for (int r = 0; r < R; r++) {
+        if (!(tgt >> r & 1)) continue;
+        const int i = i0 + 32 * r + lane;
+        atomicAdd(&a.ax[i], widen((r & 1 ? b.gx[r / 2].y : b.gx[r / 2].x) * q0));
+        atomicAdd(&a.ay[i], widen((r & 1 ? b.gy[r / 2].y : b.gy[r / 2].x) * q0));
+        atomicAdd(&a.az[i], widen((r & 1 ? b.gz[r / 2].y : b.gz[r / 2].x) * q0));
+    }
+}
+
+// Unit (v, d) -> block pair (A, A + d mod nb), d = 0 .. nb / 2 (for even nb the
+// last distance from the first half of the blocks only): every unordered block
+// pair once.
+__device__ __forceinline__ bool unit_blocks(int64_t v, int d, int nb, int nch, int &A, int &B, int &ch) {
+    A = (int)(v / nch);
+    ch = (int)(v - (int64_t)A * nch);
+    if (A >= nb || (2 * (int64_t)d == nb && 2 * (int64_t)A >= nb)) return false;
+    B = (int)(((int64_t)A + d) % nb);
+    return true;
+}
+// grid of nb x nch units per distance, kPairWarps to a CTA; distances in y
+inline dim3 pair_grid(int nb, int nch) {
+    return dim3((unsigned)div_up((int64_t)nb * nch, kPairWarps), (unsigned)std::min(nb / 2 + 1, 65535));
+}
+
+template <int R, bool CLAMP>
+__global__ void __launch_bounds__(32 * kPairWarps, 3) direct_pairs_kernel(PairArgs a) {
+    __shared__ PairLow<R> lows[kPairWarps];
+    PairLow<R> &low = lows[threadIdx.x >> 5];
+    const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    const bool differ = *a.differ != 0;
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;  // also for every larger distance
+        const int k0 = ch * a.ct, k1 = min(k0 + a.ct, R * a.images);
+        if (differ) {
+            if (A != B) pair_unit<R, false, CLAMP, true>(a, low, A, B, k0, k1);
+            else pair_unit<R, false, CLAMP, false>(a, low, A, B, k0, k1);
         } else {
-            ax[i] = sx[k] * c;
-            ay[i] = sy[k] * c;
-            az[i] = sz[k] * c;
+            if (A != B) pair_unit<R, true, CLAMP, true>(a, low, A, B, k0, k1);
+            else pair_unit<R, true, CLAMP, false>(a, low, A, B, k0, k1);
         }
     }
 }
 
-// 1/sqrt(r2) in FP64: FP32 seed, two Newton-Raphson steps y <- y(3 - r2 y^2)/2
-// (each step doubles the number of correct bits: ~23 -> ~46 -> full FP64).
-__device__ __forceinline__ double rsqrt_f64(double r2) {
-    double y = (double)rsqrtf(fmaxf((float)r2, FLT_MIN));
-    double h = 0.5 * r2;
-    y = y * fma(-h * y, y, 1.5);
-    y = y * fma(-h * y, y, 1.5);
-    return y;
+template <int R>
+cudaError_t launch_pairs(PairArgs a, cudaStream_t st) {
+    a.nb = div_up(a.n, 32 * R);
+    // about 16 units per SM sub-partition, of at most kMaxTiles tiles
+    const int64_t per = (int64_t)R * a.images, tiles = ((int64_t)a.nb * (a.nb + 1) / 2) * per;
+    a.ct = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxTiles, tiles / (64 * (int64_t)device_sms())));
+    a.nch = div_up(per, a.ct);
+    const dim3 grid = pair_grid(a.nb, a.nch);
+    if (a.eps2 >= kMinR2) direct_pairs_kernel<R, false><<<grid, 32 * kPairWarps, 0, st>>>(a);
+    else direct_pairs_kernel<R, true><<<grid, 32 * kPairWarps, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
+// R = 8 amortises the travelling particle's shuffles over eight pairs; below
+// 2,048 particles its few units would leave most of the GPU idle
+cudaError_t launch_pairs(const PairArgs &a, cudaStream_t st) {
+    if (a.n <= 0) return cudaSuccess;
+    return a.n < 2048 ? launch_pairs<2>(a, st) : launch_pairs<8>(a, st);
+}
+
+// ------------------------------------------------------------------- FP64 --
+// r2^(-3/2) in FP64: y = FP32 rsqrt of the truncated r2 (relative error e/2,
+// |e| < 4e-7), then y^3 (1 - e')^(-3/2) with e' = 1 - r2 y^2 to second order in
+// e' (the next term is below 2e-19): six FP64 operations, where two Newton steps
+// on 1/r and its cube took nine and two conversions at the FP64 rate.  The
+// conversions go by bits; r2 past the FP32 range gives y = 0, below it the
+// smallest normal seed (a zero distance stays finite).
+__device__ __forceinline__ double inv_cube_f64(double r2) {
+    const int h = max(__double2hiint(r2), 0x38100000);
+    const int f = h >= 0x47f00000 ? 0x7f800000 : (int)(((uint32_t)(h - 0x38000000) << 3) |
+                                                       ((uint32_t)__double2loint(r2) >> 29));
+    const uint32_t u = __float_as_uint(rsqrt_ftz(__int_as_float(f)));
+    const double y = u ? __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29)) : 0.0;
+    const double y2 = y * y, e = fma(-r2, y2, 1.0), y3 = y2 * y;
+    return fma(y3 * e, fma(1.875, e, 1.5), y3);
+}
+
+struct Pair64Args {
+    const double *x, *y, *z, *qm;
+    const float *q;
+    int n, nb;
+    double eps2;
+    double *ax, *ay, *az;
+};
+
+// Every unordered pair once, as the mixed kernel: one particle per lane against
+// a tile of 32 that travels around the lanes with its sums.  FP64-pipe bound (20
+// operations per pair of interactions; shuffles, loads and atomics are free
+// beside them).
+template <bool SYM>
+__device__ __forceinline__ void pair64_unit(const Pair64Args &a, int A, int B) {
+    const int lane = threadIdx.x & 31, i = 32 * A + lane, j = 32 * B + lane;
+    const int ii = min(i, a.n - 1), jj = min(j, a.n - 1);
+    const bool it = i < a.n && a.qm[ii] != 0.0, jt = SYM && j < a.n && a.qm[jj] != 0.0;
+    if (!__any_sync(0xffffffffu, it || jt)) return;
+    const double xi = a.x[ii], yi = a.y[ii], zi = a.z[ii];
+    const double qi = i < a.n ? (double)a.q[ii] : 0.0;  // absent particles carry no charge
+    double xj = a.x[jj], yj = a.y[jj], zj = a.z[jj], qj = j < a.n ? (double)a.q[jj] : 0.0;
+    double fx = 0.0, fy = 0.0, fz = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    const int from = (lane + 1) & 31;
+#pragma unroll 2
+    for (int step = 0; step < 32; step++) {
+        const double dx = xi - xj, dy = yi - yj, dz = zi - zj;
+        const double w = inv_cube_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2))));
+        const double wi = qj * w;
+        fx = fma(dx, wi, fx);
+        fy = fma(dy, wi, fy);
+        fz = fma(dz, wi, fz);
+        if (SYM) {
+            const double wj = -(qi * w);
+            gx = __shfl_sync(0xffffffffu, fma(dx, wj, gx), from);
+            gy = __shfl_sync(0xffffffffu, fma(dy, wj, gy), from);
+            gz = __shfl_sync(0xffffffffu, fma(dz, wj, gz), from);
+        }
+        xj = __shfl_sync(0xffffffffu, xj, from);
+        yj = __shfl_sync(0xffffffffu, yj, from);
+        zj = __shfl_sync(0xffffffffu, zj, from);
+        qj = __shfl_sync(0xffffffffu, qj, from);
+    }
+    if (it) {
+        atomicAdd(&a.ax[i], fx);
+        atomicAdd(&a.ay[i], fy);
+        atomicAdd(&a.az[i], fz);
+    }
+    if (jt) {
+        atomicAdd(&a.ax[j], gx);
+        atomicAdd(&a.ay[j], gy);
+        atomicAdd(&a.az[j], gz);
+    }
+}
+
+__global__ void __launch_bounds__(32 * kPairWarps) direct_pairs64_kernel(Pair64Args a) {
+    const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, 1, A, B, ch)) return;
+        if (A != B) pair64_unit<true>(a, A, B);
+        else pair64_unit<false>(a, A, B);
+    }
+}
+
+// One-sided FP64 sum with symmetry images: kTPB * kTPT targets per CTA against
+// (image, source tile) units [blockIdx.y * per, + per).
 __global__ void __launch_bounds__(kTPB)
 direct_fp64_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
                    const double *__restrict__ zs, const float *__restrict__ qs,
-                   const double *__restrict__ qm, int n, int chunk, double eps2, Images im,
-                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                   int atomic_out) {
+                   const double *__restrict__ qm, int n, int64_t per, double eps2, Images im,
+                   double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az) {
     __shared__ dbl4_t tile[kTile];
     const int t0 = blockIdx.x * (kTPB * kTPT);
-    const int j_begin = blockIdx.y * chunk;
-    const int j_end = min(n, j_begin + chunk);
+    const int ntile = (n + kTile - 1) / kTile;
+    const int64_t u0 = blockIdx.y * per, u1 = min(u0 + per, (int64_t)ntile * im.count);
     double tx[kTPT], ty[kTPT], tz[kTPT], sx[kTPT], sy[kTPT], sz[kTPT];
     if (!block_has_target(qm, t0, n)) return;
 #pragma unroll
@@ -172,94 +465,106 @@ direct_fp64_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
         tz[k] = zs[ii];
         sx[k] = sy[k] = sz[k] = 0.0;
     }
-    for (int g = 0; g < im.count; g++) {
-        for (int jt = j_begin; jt < j_end; jt += kTile) {
-            __syncthreads();
-            for (int s = threadIdx.x; s < kTile; s += kTPB) {
-                const int j = jt + s;
-                dbl4_t v = dbl4(0.0, 0.0, 0.0, 0.0);
-                if (j < j_end) {
-                    double px = xs[j], py = ys[j], pz = zs[j];
-                    image_of(im, g, px, py, pz);
-                    v = dbl4(px, py, pz, (double)qs[j]);
-                } else {
-                    v = dbl4(xs[j_begin] + 1.0, 0.0, 0.0, 0.0);  // far, zero charge
-                }
-                tile[s] = v;
-            }
-            __syncthreads();
+    for (int64_t u = u0; u < u1; u++) {
+        const int g = (int)(u / ntile), jt = (int)(u - (int64_t)g * ntile) * kTile;
+        __syncthreads();
+        for (int s = threadIdx.x; s < kTile; s += kTPB) {
+            const int j = min(jt + s, n - 1);
+            double px = xs[j], py = ys[j], pz = zs[j];
+            image_of(im, g, px, py, pz);
+            tile[s] = dbl4(px, py, pz, jt + s < n ? (double)qs[j] : 0.0);
+        }
+        __syncthreads();
 #pragma unroll 2
-            for (int s = 0; s < kTile; s++) {
-                const dbl4_t v = tile[s];
+        for (int s = 0; s < kTile; s++) {
+            const dbl4_t v = tile[s];
 #pragma unroll
-                for (int k = 0; k < kTPT; k++) {
-                    const double dx = tx[k] - v.x, dy = ty[k] - v.y, dz = tz[k] - v.z;
-                    const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-                    const double inv = rsqrt_f64(r2);
-                    const double w = v.w * inv * inv * inv;
-                    sx[k] = fma(dx, w, sx[k]);
-                    sy[k] = fma(dy, w, sy[k]);
-                    sz[k] = fma(dz, w, sz[k]);
-                }
+            for (int k = 0; k < kTPT; k++) {
+                const double dx = tx[k] - v.x, dy = ty[k] - v.y, dz = tz[k] - v.z;
+                const double w = v.w * inv_cube_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+                sx[k] = fma(dx, w, sx[k]);
+                sy[k] = fma(dy, w, sy[k]);
+                sz[k] = fma(dz, w, sz[k]);
             }
         }
     }
 #pragma unroll
     for (int k = 0; k < kTPT; k++) {
         const int i = t0 + threadIdx.x + k * kTPB;
-        if (i >= n) continue;
-        const double c = qm[i];
-        if (c == 0.0) continue;
-        if (atomic_out) {
-            atomicAdd(&ax[i], sx[k] * c);
-            atomicAdd(&ay[i], sy[k] * c);
-            atomicAdd(&az[i], sz[k] * c);
-        } else {
-            ax[i] = sx[k] * c;
-            ay[i] = sy[k] * c;
-            az[i] = sz[k] * c;
-        }
+        if (i >= n || qm[i] == 0.0) continue;
+        atomicAdd(&ax[i], sx[k]);
+        atomicAdd(&ay[i], sy[k]);
+        atomicAdd(&az[i], sz[k]);
     }
 }
 
 }  // namespace
 
+void direct_sort_wants(sv_ctx *c) {
+    c->S.want_zero = true;
+    c->S.want_hilo = c->P.precision == SV_PREC_MIXED;
+    c->S.hl_abs = c->P.symmetry == SV_SYM_ROTATIONAL;
+}
+
 sv_status direct_accel(sv_ctx *c) {
     const int n = (int)c->S.n;
     Sorted &S = c->S;
     Images im{0, 1, nullptr};
-    double *d_off = nullptr;
+    const float4 *off_hl = nullptr;
+    void *d_off = nullptr;
     if (c->P.symmetry == SV_SYM_ROTATIONAL) {
         im.kind = 1;
         im.count = 4;
     } else if (c->P.symmetry == SV_SYM_TRANSLATIONAL) {
-        static thread_local double h_off[3 * 4096];
-        const int cnt = trans_images(c->P, h_off, 4096);
+        struct Offsets {
+            double m[3 * 4096];     // metres
+            float4 hl[2 * 4096];    // the same as FP32 hi and lo parts
+        };
+        static thread_local Offsets h;
+        const int cnt = trans_images(c->P, h.m, 4096);
         if (cnt <= 0 || cnt > 4096) return set_error(c, SV_ERR_INVALID, "bad translational image set (%d)", cnt);
-        SV_CK(c, cudaMallocAsync(&d_off, sizeof(double) * 3 * cnt, c->stream));
-        SV_CK(c, cudaMemcpyAsync(d_off, h_off, sizeof(double) * 3 * cnt, cudaMemcpyHostToDevice, c->stream));
+        for (int g = 0; g < cnt; g++) {
+            const double *m = h.m + 3 * g;
+            const float hi[3] = {(float)m[0], (float)m[1], (float)m[2]};
+            h.hl[2 * g] = make_float4(hi[0], hi[1], hi[2], 0.f);
+            h.hl[2 * g + 1] = make_float4((float)(m[0] - hi[0]), (float)(m[1] - hi[1]), (float)(m[2] - hi[2]), 0.f);
+        }
+        const size_t bytes = c->P.precision == SV_PREC_FP64 ? sizeof(double) * 3 * cnt : sizeof(float4) * 2 * cnt;
+        SV_CK(c, cudaMallocAsync(&d_off, bytes, c->stream));
+        SV_CK(c, cudaMemcpyAsync(d_off, c->P.precision == SV_PREC_FP64 ? (const void *)h.m : (const void *)h.hl, bytes,
+                                 cudaMemcpyHostToDevice, c->stream));
         im.kind = 2;
         im.count = cnt;
-        im.off = d_off;
+        im.off = (const double *)d_off;
+        off_hl = (const float4 *)d_off;
     }
-    const int tblocks = div_up(n, kTPB * kTPT);
-    // split the source range so that the grid fills the GPU ~8 CTAs per SM deep
-    int splits = div_up(8 * device_sms(), tblocks);
-    const int max_splits = div_up(n, kTile);
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    int chunk = div_up(div_up(n, splits), kTile) * kTile;
-    splits = div_up(n, chunk);
-    const int atomic_out = splits > 1;  // into the accelerations the sort cleared
     for (int k = 2; k <= 6; k++) phase_mark(c, k);
-    dim3 grid(tblocks, splits);
-    if (c->P.precision == SV_PREC_FP64) {
-        direct_fp64_kernel<<<grid, kTPB, 0, c->stream>>>(S.x, S.y, S.z, S.q, S.qm, n, chunk, c->P.softening2,
-                                                         im, S.ax, S.ay, S.az, atomic_out);
+    S.raw = true;
+    if (c->P.precision == SV_PREC_FP64 && im.kind == 0) {
+        const Pair64Args a{S.x, S.y, S.z, S.qm, S.q, n, div_up(n, 32), c->P.softening2, S.ax, S.ay, S.az};
+        direct_pairs64_kernel<<<pair_grid(a.nb, 1), 32 * kPairWarps, 0, c->stream>>>(a);
+    } else if (c->P.precision == SV_PREC_FP64) {
+        // the (image, tile) units split so that the grid fills the GPU ~8 CTAs per SM deep
+        const int tblocks = div_up(n, kTPB * kTPT);
+        const int64_t units = (int64_t)div_up(n, kTile) * im.count;
+        const int64_t splits = std::max<int64_t>(1, std::min<int64_t>({div_up(8 * device_sms(), tblocks), units, 65535}));
+        const int64_t per = (units + splits - 1) / splits;
+        direct_fp64_kernel<<<dim3(tblocks, (unsigned)div_up(units, per)), kTPB, 0, c->stream>>>(
+            S.x, S.y, S.z, S.q, S.qm, n, per, c->P.softening2, im, S.ax, S.ay, S.az);
     } else {
-        direct_mixed_kernel<<<grid, kTPB, 0, c->stream>>>(S.x, S.y, S.z, S.q, S.qm, n, chunk,
-                                                          (float)c->P.softening2, im, S.ax, S.ay, S.az,
-                                                          atomic_out);
+        PairArgs a{};
+        a.ph = S.ph;
+        a.pl = S.pl;
+        a.n = n;
+        a.eps2 = (float)c->P.softening2;
+        a.kind = im.kind;
+        a.images = im.count;
+        a.off = off_hl;
+        a.ax = S.ax;
+        a.ay = S.ay;
+        a.az = S.az;
+        a.differ = reinterpret_cast<const int *>(S.root + 14);
+        SV_CK(c, launch_pairs(a, c->stream));
     }
     SV_LAUNCHED(c);
     if (d_off) SV_CK(c, cudaFreeAsync(d_off, c->stream));
@@ -270,29 +575,19 @@ sv_status direct_accel(sv_ctx *c) {
     return SV_OK;
 }
 
-cudaError_t launch_direct_mixed_sorted(const double *xs, const double *ys, const double *zs, const float *qs,
-                                       const double *qm, int n, float eps2, double *ax, double *ay, double *az,
-                                       cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    const int tblocks = div_up(n, kTPB * kTPT);
-    int splits = div_up(8 * device_sms(), tblocks);
-    const int max_splits = div_up(n, kTile);
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    const int chunk = div_up(div_up(n, splits), kTile) * kTile;
-    splits = div_up(n, chunk);
-    const int atomic_out = splits > 1;
-    cudaError_t e = cudaSuccess;
-    if (atomic_out) {
-        e = cudaMemsetAsync(ax, 0, sizeof(double) * n, stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ay, 0, sizeof(double) * n, stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(az, 0, sizeof(double) * n, stream);
-        if (e != cudaSuccess) return e;
-    }
-    Images im{0, 1, nullptr};
-    direct_mixed_kernel<<<dim3(tblocks, splits), kTPB, 0, stream>>>(xs, ys, zs, qs, qm, n, chunk, eps2, im, ax, ay,
-                                                                    az, atomic_out);
-    return cudaGetLastError();
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, int n, float eps2, double *ax, double *ay,
+                                       double *az, const int *charges_differ, cudaStream_t stream) {
+    PairArgs a{};
+    a.ph = ph;
+    a.pl = pl;
+    a.n = n;
+    a.eps2 = eps2;
+    a.images = 1;
+    a.ax = ax;
+    a.ay = ay;
+    a.az = az;
+    a.differ = charges_differ;
+    return launch_pairs(a, stream);
 }
 
 }  // namespace sv

@@ -112,6 +112,7 @@ __global__ void na_bbox_final(const double *__restrict__ part, int nb, double *_
         root[1] = sh[0] > sh[3] ? 0.0 : sh[1];
         root[2] = sh[0] > sh[3] ? 0.0 : sh[2];
         root[3] = S;
+        reinterpret_cast<int *>(root + 7)[0] = 0;
     }
 }
 
@@ -145,35 +146,44 @@ __global__ void na_keys(const double *__restrict__ x3, const int32_t *__restrict
     keys[i] = na_spread3(c[0]) | (na_spread3(c[1]) << 1) | (na_spread3(c[2]) << 2);
 }
 
+// the sorted particles as the pair kernel takes them (FP32 hi + lo positions
+// relative to the root's origin, source charge, target mark), K q / m, the sums
+// cleared, and a mark when the source charges differ
 __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double *__restrict__ x3,
                           const double *__restrict__ q, const double *__restrict__ m,
-                          const int32_t *__restrict__ st, double kconst, double *__restrict__ xs,
-                          double *__restrict__ ys, double *__restrict__ zs, float *__restrict__ qs,
-                          double *__restrict__ qm) {
+                          const int32_t *__restrict__ st, double kconst, const double *__restrict__ root,
+                          float4 *__restrict__ ph, float4 *__restrict__ pl, double *__restrict__ qm,
+                          double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
+                          int *__restrict__ differ) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = idx[s];
-    xs[s] = x3[3 * i];
-    ys[s] = x3[3 * i + 1];
-    zs[s] = x3[3 * i + 2];
+    float4 h, l;
+    split_hilo(x3[3 * i] - root[0], h.x, l.x);
+    split_hilo(x3[3 * i + 1] - root[1], h.y, l.y);
+    split_hilo(x3[3 * i + 2] - root[2], h.z, l.z);
     const int32_t w = st[i];
-    qs[s] = is_src(w) ? (float)q[i] : 0.0f;
-    qm[s] = (w == 1 && m[i] > 0.0) ? kconst * q[i] / m[i] : 0.0;
+    h.w = is_src(w) ? (float)q[i] : 0.0f;
+    const double k = (w == 1 && m[i] > 0.0) ? kconst * q[i] / m[i] : 0.0;
+    l.w = k != 0.0 ? 1.f : 0.f;
+    ph[s] = h;
+    pl[s] = l;
+    qm[s] = k;
+    ax[s] = ay[s] = az[s] = 0.0;
+    if (h.w != (is_src(st[0]) ? (float)q[0] : 0.0f)) *differ = 1;
 }
 
-// every output entry is written: targets get their acceleration, everything
-// else 0 (entries of the sorted arrays that the kernel did not touch may hold
-// the previous call's values and are never passed on)
+// every output entry is written: targets get their acceleration, everything else 0
 __global__ void na_scatter(const uint32_t *__restrict__ idx, int n, const double *__restrict__ qm,
                            const double *__restrict__ ax, const double *__restrict__ ay,
                            const double *__restrict__ az, double *__restrict__ a3) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = idx[s];
-    const bool t = qm[s] != 0.0;
-    a3[3 * i] = t ? ax[s] : 0.0;
-    a3[3 * i + 1] = t ? ay[s] : 0.0;
-    a3[3 * i + 2] = t ? az[s] : 0.0;
+    const double k = qm[s];
+    a3[3 * i] = k != 0.0 ? ax[s] * k : 0.0;
+    a3[3 * i + 1] = k != 0.0 ? ay[s] * k : 0.0;
+    a3[3 * i + 2] = k != 0.0 ? az[s] * k : 0.0;
 }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -210,17 +220,16 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     uint64_t *keys_alt = (uint64_t *)carve(sizeof(uint64_t) * ni);
     uint32_t *idx = (uint32_t *)carve(sizeof(uint32_t) * ni);
     uint32_t *idx_alt = (uint32_t *)carve(sizeof(uint32_t) * ni);
-    double *xs = (double *)carve(sizeof(double) * ni);
-    double *ys = (double *)carve(sizeof(double) * ni);
-    double *zs = (double *)carve(sizeof(double) * ni);
-    float *qs = (float *)carve(sizeof(float) * ni);
+    float4 *ph = (float4 *)carve(sizeof(float4) * ni);
+    float4 *pl = (float4 *)carve(sizeof(float4) * ni);
     double *qm = (double *)carve(sizeof(double) * ni);
     double *ax = (double *)carve(sizeof(double) * ni);
     double *ay = (double *)carve(sizeof(double) * ni);
     double *az = (double *)carve(sizeof(double) * ni);
     const int red_blocks = 2 * device_sms();
     double *part = (double *)carve(sizeof(double) * 6 * red_blocks);
-    double *root = (double *)carve(sizeof(double) * 8);
+    double *root = (double *)carve(sizeof(double) * 8);  // [7] int: source charges differ
+    int *differ = reinterpret_cast<int *>(root + 7);
     cub::DoubleBuffer<uint64_t> kb(keys, keys_alt);
     cub::DoubleBuffer<uint32_t> vb(idx, idx_alt);
     size_t tmp_bytes = 0;
@@ -237,9 +246,10 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     if (cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, ni, 0, 3 * kMortonBits + 1, s) != cudaSuccess)
         return SV_ERR_CUDA;
     const uint32_t *sidx = vb.Current();
-    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, xs, ys, zs, qs, qm);
+    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, root, ph, pl, qm, ax, ay, az,
+                                  differ);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;
-    if (launch_direct_mixed_sorted(xs, ys, zs, qs, qm, ni, (float)softening2, ax, ay, az, s) != cudaSuccess)
+    if (launch_direct_mixed_sorted(ph, pl, ni, (float)softening2, ax, ay, az, differ, s) != cudaSuccess)
         return SV_ERR_CUDA;
     na_scatter<<<nb, 256, 0, s>>>(sidx, ni, qm, ax, ay, az, a3);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;

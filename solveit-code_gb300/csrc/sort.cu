@@ -137,6 +137,7 @@ bbox_kernel(const double *__restrict__ x, const double *__restrict__ y, const do
     __syncthreads();
     if (threadIdx.x == 0) {
         write_root(bounds, scale, root);
+        reinterpret_cast<int *>(root + 14)[0] = 0;
         *done = 0;
     }
 }
@@ -183,6 +184,10 @@ struct GatherArgs {
     float *qs;
     double *qm;
     double *zax, *zay, *zaz;  // sorted accelerations to clear, or null
+    float4 *ph, *pl;          // FP32 hi + lo positions to write, or null
+    int abs_xy;               // ... relative to the z axis in x and y, not to the root's origin
+    const double *root;
+    int *differ;              // set when a source charge differs from particle 0's (with ph)
 };
 
 // source charge of particle i (0: no source), and its K q / m (0: no target)
@@ -202,6 +207,17 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s, uint3
     a.qs[s] = sorted_charge(a, i);
     a.qm[s] = sorted_qm(a, i);
     if (a.zax) a.zax[s] = a.zay[s] = a.zaz[s] = 0.0;
+    if (a.ph) {
+        float4 h, l;
+        split_hilo(a.x[i] - (a.abs_xy ? 0.0 : a.root[0]), h.x, l.x);
+        split_hilo(a.y[i] - (a.abs_xy ? 0.0 : a.root[1]), h.y, l.y);
+        split_hilo(a.z[i] - a.root[2], h.z, l.z);
+        h.w = a.qs[s];
+        l.w = a.qm[s] != 0.0 ? 1.f : 0.f;
+        a.ph[s] = h;
+        a.pl[s] = l;
+        if (h.w != sorted_charge(a, 0)) *a.differ = 1;
+    }
 }
 
 __global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, GatherArgs a) {
@@ -295,7 +311,10 @@ sort_one_chunk(int n, int sh, double scale, double *__restrict__ root, uint64_t 
     const long long v = block_bounds<CH>(mn, mx, red);
     if (i < 6) bounds[i] = __longlong_as_double(ordered_bits(v));
     __syncthreads();
-    if (i == 0) write_root(bounds, scale, root);
+    if (i == 0) {
+        write_root(bounds, scale, root);
+        reinterpret_cast<int *>(root + 14)[0] = 0;
+    }
     __syncthreads();
     const uint64_t key = i < n ? morton_key(p[0], p[1], p[2], st, root) : kInactiveKey;
     const int pos = chunk_place<CH>(key, sh, buf);  // slots past n: inactive keys behind every particle
@@ -371,12 +390,33 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
     for (int o = kRankLanes / 2; o > 0; o >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, o);
     if (!live) return;
     const uint32_t i = cidx[s];
+    if (part < 3) {
+        const double v = (part == 0 ? a.x : part == 1 ? a.y : a.z)[i];
+        (part == 0 ? a.xs : part == 1 ? a.ys : a.zs)[rank] = v;
+        if (a.ph) {
+            float h, l;
+            split_hilo(v - (a.abs_xy && part < 2 ? 0.0 : a.root[part]), h, l);
+            reinterpret_cast<float *>(a.ph + rank)[part] = h;
+            reinterpret_cast<float *>(a.pl + rank)[part] = l;
+        }
+        return;
+    }
     switch (part) {
-    case 0: a.xs[rank] = a.x[i]; break;
-    case 1: a.ys[rank] = a.y[i]; break;
-    case 2: a.zs[rank] = a.z[i]; break;
-    case 3: a.qs[rank] = sorted_charge(a, i); break;
-    case 4: a.qm[rank] = sorted_qm(a, i); break;
+    case 3: {
+        const float q = sorted_charge(a, i);
+        a.qs[rank] = q;
+        if (a.ph) {
+            a.ph[rank].w = q;
+            if (q != sorted_charge(a, 0)) *a.differ = 1;
+        }
+        break;
+    }
+    case 4: {
+        const double k = sorted_qm(a, i);
+        a.qm[rank] = k;
+        if (a.ph) a.pl[rank].w = k != 0.0 ? 1.f : 0.f;
+        break;
+    }
     case 5: keys[rank] = full; break;
     case 6: idx[rank] = i; break;
     default:
@@ -389,8 +429,8 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
 __global__ void scatter_accel(const uint32_t *__restrict__ idx, int64_t n, int64_t n_orig,
                               const double *__restrict__ axs, const double *__restrict__ ays,
                               const double *__restrict__ azs, const double *__restrict__ far, int64_t fs,
-                              const double *__restrict__ qm, double *__restrict__ ax, double *__restrict__ ay,
-                              double *__restrict__ az) {
+                              const double *__restrict__ qm, int raw, double *__restrict__ ax,
+                              double *__restrict__ ay, double *__restrict__ az) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = idx[s];
@@ -403,6 +443,11 @@ __global__ void scatter_accel(const uint32_t *__restrict__ idx, int64_t n, int64
         ax[i] = axs[s] + far[s];
         ay[i] = ays[s] + far[fs + s];
         az[i] = azs[s] + far[2 * fs + s];
+    } else if (raw) {
+        const double k = qm[s];
+        ax[i] = axs[s] * k;
+        ay[i] = ays[s] * k;
+        az[i] = azs[s] * k;
     } else {
         ax[i] = axs[s];
         ay[i] = ays[s];
@@ -418,7 +463,7 @@ sv_status ensure_sorted_capacity(sv_ctx *c, int64_t n) {
     cudaFree(S.x); cudaFree(S.y); cudaFree(S.z); cudaFree(S.q); cudaFree(S.qm);
     cudaFree(S.idx); cudaFree(S.keys); cudaFree(S.keys_alt); cudaFree(S.idx_alt);
     cudaFree(S.ax); cudaFree(S.ay); cudaFree(S.az); cudaFree(S.cub_tmp);
-    cudaFree(S.root); cudaFree(S.red);
+    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl);
     S = Sorted();
     const int64_t cap = n < 1024 ? 1024 : n;
     SV_CK(c, cudaMalloc(&S.x, cap * sizeof(double)));
@@ -456,10 +501,20 @@ static double root_scale(const sv_ctx *c) {
 
 sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t last) {
     const int64_t n = v.n;
-    const bool zero = c->S.want_zero;
+    const bool zero = c->S.want_zero, hilo = c->S.want_hilo, hl_abs = c->S.hl_abs;
     SV_TRY(ensure_sorted_capacity(c, n));
     Sorted &S = c->S;
-    S.want_zero = false;
+    S.want_zero = S.want_hilo = S.raw = false;
+    S.hl_abs = hl_abs;
+    if (hilo && S.hl_cap < n) {
+        cudaFree(S.ph);
+        cudaFree(S.pl);
+        S.ph = S.pl = nullptr;
+        S.hl_cap = 0;
+        SV_CK(c, cudaMalloc(&S.ph, sizeof(float4) * S.cap));
+        SV_CK(c, cudaMalloc(&S.pl, sizeof(float4) * S.cap));
+        S.hl_cap = S.cap;
+    }
     S.n = n;
     S.n_orig = v.n_orig;
     // levels 1 .. want_levels occupy bits >= 3 (kMortonBits - want_levels); bit 63 marks inactive keys
@@ -468,7 +523,8 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     S.key_levels = levels;
     const int sh = 3 * (kMortonBits - levels);
     GatherArgs ga{v.x, v.y, v.z, v.q, v.m, v.qom, v.status, first, std::min(last, v.n_orig), c->P.k_const,
-                  S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr};
+                  S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr, hilo ? S.ph : nullptr,
+                  hilo ? S.pl : nullptr, hl_abs ? 1 : 0, S.root, reinterpret_cast<int *>(S.root + 14)};
     if (zero) {
         ga.zax = S.ax;
         ga.zay = S.ay;
@@ -527,8 +583,10 @@ sv_status sort_state(sv_ctx *c, int64_t first, int64_t last) {
 sv_status unsort_accel(sv_ctx *c) {
     const int64_t n = c->S.n;
     scatter_accel<<<div_up(n, 256), 256, 0, c->stream>>>(c->S.idx, n, c->S.n_orig, c->S.ax, c->S.ay, c->S.az,
-                                                         c->S.far, c->S.far_stride, c->S.qm, c->ax, c->ay, c->az);
+                                                         c->S.far, c->S.far_stride, c->S.qm, c->S.raw, c->ax, c->ay,
+                                                         c->az);
     c->S.far = nullptr;
+    c->S.raw = false;
     SV_LAUNCHED(c);
     return SV_OK;
 }

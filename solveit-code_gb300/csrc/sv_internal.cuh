@@ -32,13 +32,20 @@ struct Sorted {
     uint64_t *keys = nullptr, *keys_alt = nullptr;
     uint32_t *idx_alt = nullptr;
     double *ax = nullptr, *ay = nullptr, *az = nullptr;  // acceleration, sorted order
+    bool raw = false;  // ax, ay, az lack the factor K q/m (the scatter multiplies; cleared by it)
+    // positions as FP32 hi + lo parts relative to `root`'s origin (hl_abs: to the
+    // z axis in x and y), hi.w the source charge, lo.w 1 for targets; written by
+    // the sort when want_hilo
+    float4 *ph = nullptr, *pl = nullptr;
+    int64_t hl_cap = 0;
     // a second field to add in the scatter (the FMM's far field: x, y, z at
     // far, far + far_stride, far + 2 far_stride), or null; cleared by it
     const double *far = nullptr;
     int64_t far_stride = 0;
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
-    double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S
+    double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S;
+                               // [14] int: 1 when the sorted source charges differ (want_hilo)
     long long *red = nullptr;  // device reduction scratch
     int red_blocks = 0;
     int64_t cap = 0;
@@ -47,6 +54,7 @@ struct Sorted {
     // needs its keys ordered down to its leaf level only
     int want_levels = kMortonBits, key_levels = kMortonBits;
     bool want_zero = false;  // the next sort also clears ax, ay, az (a method that adds into them)
+    bool want_hilo = false, hl_abs = false;  // the next sort also writes ph, pl
     bool resort = false;  // the FMM found its leaf level below key_levels: sort again, fully
     int64_t n = 0;       // sorted entries (caller particles plus any image copies)
     int64_t n_orig = 0;  // caller particles; sorted idx >= n_orig are image copies
@@ -271,12 +279,20 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
 sv_status unsort_accel(sv_ctx *c);
 
 // direct.cu
-sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a*
-// the mixed-precision all-pairs kernel on caller-provided sorted arrays
-// (no symmetry images); launches only, allocates nothing
-cudaError_t launch_direct_mixed_sorted(const double *xs, const double *ys, const double *zs, const float *qs,
-                                       const double *qm, int n, float eps2, double *ax, double *ay, double *az,
-                                       cudaStream_t stream);
+sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; raw sums in mixed precision)
+// what the direct sum of this context needs of its sort (want_zero, want_hilo)
+void direct_sort_wants(sv_ctx *c);
+// the mixed-precision all-pairs sums (no symmetry images) of n sorted
+// particles given as FP32 hi + lo parts (Sorted::ph, pl), without the targets'
+// factor K q / m, added into the cleared ax, ay, az; launches only, allocates nothing
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, int n, float eps2, double *ax, double *ay,
+                                       double *az, const int *charges_differ, cudaStream_t stream);
+
+// a double as FP32 hi + lo parts (48 bits)
+__device__ __forceinline__ void split_hilo(double v, float &hi, float &lo) {
+    hi = (float)v;
+    lo = (float)(v - (double)hi);
+}
 
 // tree.cu / bh.cu / fmm.cu
 sv_status bh_accel(sv_ctx *c);
