@@ -16,13 +16,14 @@
 // with the Jacobian-transpose product of the softened Coulomb sum
 //     (J^T la)_k = sum_j G(x_k - x_j) (q_j u_k - q_k u_j),  u = K q/m la,
 //     G(d) = I / s^3 - 3 d d^T / s^5,  s^2 = |d|^2 + eps^2,
-// a pair kernel with the same tiling and precision modes as the direct sum.
-// The forward pass keeps the state every `checkpoint_every` steps; the
-// backward pass re-runs each segment from its checkpoint, keeping the segment's
-// x_h, and walks it in reverse.
+// a pair kernel that visits every unordered pair once, as the direct sum's: the
+// contribution to j is minus the contribution to k.
+// The forward pass keeps the state every `checkpoint_every` steps and the x_h of
+// its last segment; the backward pass re-runs each other segment from its
+// checkpoint, keeping the segment's x_h, and walks it in reverse.
 #include <cfloat>
 
-#include "sv_internal.cuh"
+#include "pairs.cuh"
 
 namespace sv {
 
@@ -31,9 +32,10 @@ struct Adj {
     double dt = 0, t0 = 0;
     int64_t n = 0, cap = 0;
     int seg_cap = 0;
+    int xh_seg = -1;          // segment whose x_h are in xh (-1: none that still holds)
     double *ck = nullptr;     // nck x 6 x n: x, y, z, vx, vy, vz
     double *xh = nullptr;     // every x 3 x n: x_h of a segment
-    double *lam = nullptr;    // 12 x n: lx(3) lv(3) la(3) tmp(3)
+    double *lam = nullptr;    // lx(3) lv(3) la(3) x n, then 4 n + 2: staging, or u as FP32 hi and lo float4s
     double *fin = nullptr;    // 6 x n: final state, restored after the backward pass
     double *lE = nullptr;     // 4: dL/dE, then max |u| scratch
     bool forward_done = false;
@@ -41,307 +43,416 @@ struct Adj {
 
 namespace {
 
-constexpr int kTPB = 128;
-constexpr int kTPT = 2;
-constexpr int kTile = 128;
-
 __device__ __forceinline__ double clampd(double v, double hi) { return fmin(fmax(v, 0.0), hi); }
 
-// (1)-(4): lv += h2 lx; lh = lx (in place); la = k lv; lE += c la
-__global__ void adj_prep(double *__restrict__ lx, double *__restrict__ ly, double *__restrict__ lz,
-                         double *__restrict__ lvx, double *__restrict__ lvy, double *__restrict__ lvz,
-                         double *__restrict__ lax, double *__restrict__ lay, double *__restrict__ laz,
-                         const double *__restrict__ q, const double *__restrict__ m, const int32_t *__restrict__ st,
-                         const int32_t *__restrict__ wst, const double *__restrict__ t_inj, int64_t n, double ts,
-                         double dt, double eoa, double *__restrict__ lE) {
-    double e0 = 0, e1 = 0, e2 = 0;
+// Start of a reverse step at its mid positions xh (x, y, z of n each): the state's
+// positions and the step's window; (1)-(4): lv += h2 lx; lh = lx (in place); la =
+// k lv; lE += c la; and max |u| of u = K q/m la (non-negative doubles order like
+// their bit patterns)
+struct PrepArgs {
+    const double *xh;
+    double *x, *y, *z;
+    int32_t *wst;
+    const double *lx;       // lx, ly, lz of n each
+    double *lv, *la;        // likewise
+    const double *qom, *t_inj;
+    const int32_t *st;
+    int64_t n;
+    double ts, dt, eoa, kconst;
+    double *lE;
+    unsigned long long *umax;
+};
+
+__global__ void adj_prep(PrepArgs a) {
+    double e0 = 0, e1 = 0, e2 = 0, um = 0;
+    const int64_t n = a.n;
+    const double h = 0.5 * a.dt;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t w = st[i];
-        const double h = 0.5 * dt;
-        const double h2 = (w == 1 || w == 2) ? clampd(ts + dt - t_inj[i], h) : 0.0;
+        a.x[i] = a.xh[i];
+        a.y[i] = a.xh[n + i];
+        a.z[i] = a.xh[2 * n + i];
+        const int32_t w = a.st[i];
+        const double ti = a.t_inj[i];
+        const int32_t ws = ti <= a.ts + h ? w : 0;
+        a.wst[i] = ws;
+        const double h2 = (w == 1 || w == 2) ? clampd(a.ts + a.dt - ti, h) : 0.0;
         // kicked: inbound and injected by the step's mid time (the window of the force)
-        const double k = (wst[i] == 1) ? clampd(ts + dt - t_inj[i], dt) : 0.0;
-        double vx = lvx[i] + h2 * lx[i], vy = lvy[i] + h2 * ly[i], vz = lvz[i] + h2 * lz[i];
-        lvx[i] = vx;
-        lvy[i] = vy;
-        lvz[i] = vz;
-        lax[i] = k * vx;
-        lay[i] = k * vy;
-        laz[i] = k * vz;
-        const double c = (w == 1 && m[i] > 0.0) ? eoa * q[i] / m[i] : 0.0;
+        const double k = ws == 1 ? clampd(a.ts + a.dt - ti, a.dt) : 0.0;
+        const double vx = a.lv[i] + h2 * a.lx[i], vy = a.lv[n + i] + h2 * a.lx[n + i],
+                     vz = a.lv[2 * n + i] + h2 * a.lx[2 * n + i];
+        a.lv[i] = vx;
+        a.lv[n + i] = vy;
+        a.lv[2 * n + i] = vz;
+        a.la[i] = k * vx;
+        a.la[n + i] = k * vy;
+        a.la[2 * n + i] = k * vz;
+        const double c = w == 1 ? a.eoa * a.qom[i] : 0.0;
         e0 += c * k * vx;
         e1 += c * k * vy;
         e2 += c * k * vz;
+        const double u = fabs(a.kconst * a.qom[i] * k) * fmax(fabs(vx), fmax(fabs(vy), fabs(vz)));
+        if (u <= DBL_MAX) um = fmax(um, u);  // a non-finite adjoint propagates through the sum itself
     }
     for (int o = 16; o > 0; o >>= 1) {
         e0 += __shfl_xor_sync(0xffffffffu, e0, o);
         e1 += __shfl_xor_sync(0xffffffffu, e1, o);
         e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+        um = fmax(um, __shfl_xor_sync(0xffffffffu, um, o));
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&lE[0], e0);
-        atomicAdd(&lE[1], e1);
-        atomicAdd(&lE[2], e2);
+        atomicAdd(&a.lE[0], e0);
+        atomicAdd(&a.lE[1], e1);
+        atomicAdd(&a.lE[2], e2);
+        if (um > 0.0) atomicMax(a.umax, (unsigned long long)__double_as_longlong(um));
     }
 }
 
-// u = K q/m la in sorted order (S.qm is K q/m for targets, 0 otherwise), and
-// max |u| (non-negative doubles order like their bit patterns)
+// the power of two that brings max |u| into [1/2, 1) (1 when it is zero), and
+// the exponent it removes
+__device__ __forceinline__ double u_scale(double um, int &ue) {
+    ue = 0;
+    if (um > 0.0) frexp(um, &ue);
+    return ldexp(1.0, -ue);
+}
+
+constexpr double kLen = 1073741824.0;  // 2^30: mixed-precision coordinates are in 2^-30 m (1/s^5 in metres overflows FP32)
+
+// u = K q/m la in sorted order (S.qm is K q/m for targets, 0 otherwise): FP64
+// values, or scaled FP32 hi and lo parts
 __global__ void adj_gather_u(const uint32_t *__restrict__ idx, int n, const double *__restrict__ qm,
-                             const double *__restrict__ lax, const double *__restrict__ lay,
-                             const double *__restrict__ laz, double *__restrict__ ux, double *__restrict__ uy,
-                             double *__restrict__ uz, unsigned long long *__restrict__ umax) {
+                             const double *__restrict__ la, const double *__restrict__ umax,
+                             double *__restrict__ u, float4 *__restrict__ uh, float4 *__restrict__ ul) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    double a = 0.0;
-    if (s < n) {
-        const uint32_t i = idx[s];
-        const double k = qm[s];
-        const double u0 = k * lax[i], u1 = k * lay[i], u2 = k * laz[i];
-        ux[s] = u0;
-        uy[s] = u1;
-        uz[s] = u2;
-        a = fmax(fabs(u0), fmax(fabs(u1), fabs(u2)));
-        if (!(a <= DBL_MAX)) a = 0.0;  // a non-finite adjoint propagates through the sum itself
-    }
-    for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-    if ((threadIdx.x & 31) == 0 && a > 0.0) atomicMax(umax, (unsigned long long)__double_as_longlong(a));
-}
-
-// lh += (J^T la) (sorted result scattered to caller order), then lx = lh, lv += h1 lh
-__global__ void adj_post(const uint32_t *__restrict__ idx, int64_t ns, int64_t n_orig,
-                         const double *__restrict__ jx, const double *__restrict__ jy, const double *__restrict__ jz,
-                         double *__restrict__ lx, double *__restrict__ ly, double *__restrict__ lz) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= ns) return;
+    if (s >= n) return;
     const uint32_t i = idx[s];
-    if ((int64_t)i >= n_orig) return;
-    lx[i] += jx[s];
-    ly[i] += jy[s];
-    lz[i] += jz[s];
+    const double k = qm[s];
+    const double v[3] = {k * la[i], k * la[n + i], k * la[2 * (int64_t)n + i]};
+    if (u) {
+        for (int d = 0; d < 3; d++) u[d * (int64_t)n + s] = v[d];
+        return;
+    }
+    int ue;
+    const double su = u_scale(*umax, ue);
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), l = h;
+    split_hilo(v[0] * su, h.x, l.x);
+    split_hilo(v[1] * su, h.y, l.y);
+    split_hilo(v[2] * su, h.z, l.z);
+    uh[s] = h;
+    ul[s] = l;
 }
 
-__global__ void adj_drift_back(double *__restrict__ lx, double *__restrict__ ly, double *__restrict__ lz,
-                               double *__restrict__ lvx, double *__restrict__ lvy, double *__restrict__ lvz,
-                               const int32_t *__restrict__ st, const double *__restrict__ t_inj, int64_t n, double ts,
-                               double dt) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t w = st[i];
-        const double h = 0.5 * dt;
-        const double h1 = (w == 1 || w == 2) ? clampd(ts + h - t_inj[i], h) : 0.0;
-        lvx[i] += h1 * lx[i];
-        lvy[i] += h1 * ly[i];
-        lvz[i] += h1 * lz[i];
+// End of a reverse step: lh += J^T la (the sorted sums, times their scale), then
+// lx = lh, lv += h1 lh
+__global__ void adj_post(const uint32_t *__restrict__ idx, int64_t n, const double *__restrict__ jx,
+                         const double *__restrict__ jy, const double *__restrict__ jz, int mixed,
+                         unsigned long long *__restrict__ umax, double *__restrict__ lx, double *__restrict__ lv,
+                         const int32_t *__restrict__ st, const double *__restrict__ t_inj, double ts, double dt) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    double back = 1.0;
+    if (mixed) {
+        int ue;
+        (void)u_scale(__longlong_as_double((long long)*umax), ue);
+        back = ldexp(1.0, 90 + ue);
+    }
+    const uint32_t i = idx[s];
+    const double h = 0.5 * dt;
+    const int32_t w = st[i];
+    const double h1 = (w == 1 || w == 2) ? clampd(ts + h - t_inj[i], h) : 0.0;
+    const double j[3] = {jx[s], jy[s], jz[s]};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const double l = lx[d * n + i] + j[d] * back;
+        lx[d * n + i] = l;
+        lv[d * n + i] += h1 * l;
     }
 }
 
-__device__ __forceinline__ double rsqrt_newton(double r2) {
-    double y = (double)rsqrtf(fmaxf((float)r2, FLT_MIN));
-    const double hh = 0.5 * r2;
-    y = y * fma(-hh * y, y, 1.5);
-    y = y * fma(-hh * y, y, 1.5);
-    return y;
-}
-
-struct alignas(32) JSrc64 {
-    double x, y, z, q, ux, uy, uz, pad;
+// ------------------------------------------- Jacobian-transpose pair sums --
+struct JPair64Args {
+    const double *x, *y, *z, *u;  // u: x, y, z of n each
+    const float *q;
+    int n, nb;
+    double eps2;
+    double *ox, *oy, *oz;
 };
 
-// Jacobian-transpose pair sum in FP64 on the Morton-sorted copy.
-__global__ void __launch_bounds__(kTPB)
-jtv_fp64_kernel(const double *__restrict__ xs, const double *__restrict__ ys, const double *__restrict__ zs,
-                const float *__restrict__ qs, const double *__restrict__ ux, const double *__restrict__ uy,
-                const double *__restrict__ uz, int n, int chunk, double eps2, double *__restrict__ ox,
-                double *__restrict__ oy, double *__restrict__ oz, int atomic_out) {
-    __shared__ JSrc64 tile[kTile];
-    const int t0 = blockIdx.x * (kTPB * kTPT);
-    const int j_begin = blockIdx.y * chunk;
-    const int j_end = min(n, j_begin + chunk);
-    double tx[kTPT], ty[kTPT], tz[kTPT], tq[kTPT], tux[kTPT], tuy[kTPT], tuz[kTPT];
-    double sx[kTPT], sy[kTPT], sz[kTPT];
-#pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int ii = min(t0 + (int)threadIdx.x + k * kTPB, n - 1);
-        tx[k] = xs[ii];
-        ty[k] = ys[ii];
-        tz[k] = zs[ii];
-        tq[k] = qs[ii];
-        tux[k] = ux[ii];
-        tuy[k] = uy[ii];
-        tuz[k] = uz[ii];
-        sx[k] = sy[k] = sz[k] = 0.0;
+// FP64: one particle per lane against a tile of 32 that travels around the lanes
+// with its sums (SYM; otherwise every ordered pair of one block).
+template <bool SYM>
+__device__ __forceinline__ void jtv64_unit(const JPair64Args &a, int A, int B) {
+    const int lane = threadIdx.x & 31, i = 32 * A + lane, j = 32 * B + lane;
+    const int64_t n = a.n;
+    const int ii = min(i, a.n - 1), jj = min(j, a.n - 1);
+    const bool li = i < a.n, lj = j < a.n;  // absent particles carry neither charge nor adjoint
+    const double xi = a.x[ii], yi = a.y[ii], zi = a.z[ii], qi = li ? (double)a.q[ii] : 0.0;
+    const double uxi = li ? a.u[ii] : 0.0, uyi = li ? a.u[n + ii] : 0.0, uzi = li ? a.u[2 * n + ii] : 0.0;
+    double xj = a.x[jj], yj = a.y[jj], zj = a.z[jj], qj = lj ? (double)a.q[jj] : 0.0;
+    double uxj = lj ? a.u[jj] : 0.0, uyj = lj ? a.u[n + jj] : 0.0, uzj = lj ? a.u[2 * n + jj] : 0.0;
+    double fx = 0.0, fy = 0.0, fz = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    const int from = (lane + 1) & 31;
+    for (int step = 0; step < 32; step++) {
+        const double dx = xi - xj, dy = yi - yj, dz = zi - zj;
+        const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2)));
+        // 1/s from the FP32 seed, to second order in e = 1 - r2 y^2
+        const double y = rsqrt_seed_f64(r2), e = fma(-r2, y * y, 1.0);
+        const double inv = fma(y * e, fma(0.375, e, 0.5), y);
+        const double inv2 = inv * inv, inv3 = inv * inv2;
+        const double wx = qj * uxi - qi * uxj, wy = qj * uyi - qi * uyj, wz = qj * uzi - qi * uzj;
+        const double dw = -3.0 * (fma(dx, wx, fma(dy, wy, dz * wz)) * inv2) * inv3;
+        const double vx = fma(dw, dx, wx * inv3), vy = fma(dw, dy, wy * inv3), vz = fma(dw, dz, wz * inv3);
+        fx += vx;
+        fy += vy;
+        fz += vz;
+        if (SYM) {
+            gx = __shfl_sync(0xffffffffu, gx - vx, from);
+            gy = __shfl_sync(0xffffffffu, gy - vy, from);
+            gz = __shfl_sync(0xffffffffu, gz - vz, from);
+        }
+        xj = __shfl_sync(0xffffffffu, xj, from);
+        yj = __shfl_sync(0xffffffffu, yj, from);
+        zj = __shfl_sync(0xffffffffu, zj, from);
+        qj = __shfl_sync(0xffffffffu, qj, from);
+        uxj = __shfl_sync(0xffffffffu, uxj, from);
+        uyj = __shfl_sync(0xffffffffu, uyj, from);
+        uzj = __shfl_sync(0xffffffffu, uzj, from);
     }
-    for (int jt = j_begin; jt < j_end; jt += kTile) {
-        __syncthreads();
-        for (int s = threadIdx.x; s < kTile; s += kTPB) {
-            const int j = jt + s;
-            JSrc64 v{};
-            if (j < j_end) {
-                v.x = xs[j];
-                v.y = ys[j];
-                v.z = zs[j];
-                v.q = qs[j];
-                v.ux = ux[j];
-                v.uy = uy[j];
-                v.uz = uz[j];
-            }
-            tile[s] = v;
-        }
-        __syncthreads();
-        const int lim = min(kTile, j_end - jt);
-        for (int s = 0; s < lim; s++) {
-            const JSrc64 v = tile[s];
-#pragma unroll
-            for (int k = 0; k < kTPT; k++) {
-                const double dx = tx[k] - v.x, dy = ty[k] - v.y, dz = tz[k] - v.z;
-                const double r2 = dx * dx + dy * dy + dz * dz + eps2;
-                const double inv = rsqrt_newton(r2);
-                const double inv2 = inv * inv, inv3 = inv * inv2;
-                const double wx = v.q * tux[k] - tq[k] * v.ux;
-                const double wy = v.q * tuy[k] - tq[k] * v.uy;
-                const double wz = v.q * tuz[k] - tq[k] * v.uz;
-                const double dw = 3.0 * ((dx * wx + dy * wy + dz * wz) * inv2) * inv3;
-                sx[k] += wx * inv3 - dw * dx;
-                sy[k] += wy * inv3 - dw * dy;
-                sz[k] += wz * inv3 - dw * dz;
-            }
-        }
+    if (li) {
+        atomicAdd(&a.ox[i], fx);
+        atomicAdd(&a.oy[i], fy);
+        atomicAdd(&a.oz[i], fz);
     }
-#pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int i = t0 + threadIdx.x + k * kTPB;
-        if (i >= n) continue;
-        if (atomic_out) {
-            atomicAdd(&ox[i], sx[k]);
-            atomicAdd(&oy[i], sy[k]);
-            atomicAdd(&oz[i], sz[k]);
-        } else {
-            ox[i] = sx[k];
-            oy[i] = sy[k];
-            oz[i] = sz[k];
-        }
+    if (SYM && lj) {
+        atomicAdd(&a.ox[j], gx);
+        atomicAdd(&a.oy[j], gy);
+        atomicAdd(&a.oz[j], gz);
     }
 }
 
-// Source of the mixed kernel: coordinates and u as FP32 hi/lo pairs.
-struct alignas(16) JSrc32 {
-    float xh, yh, zh, q;
-    float xl, yl, zl, p0;
-    float uxh, uyh, uzh, p1;
-    float uxl, uyl, uzl, p2;
-};
-
-__device__ __forceinline__ void split_hl(double v, float &h, float &l) {
-    h = (float)v;
-    l = (float)(v - (double)h);
+__global__ void __launch_bounds__(32 * kPairWarps) jtv_pairs64_kernel(JPair64Args a) {
+    const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, 1, A, B, ch)) return;
+        if (A != B) jtv64_unit<true>(a, A, B);
+        else jtv64_unit<false>(a, A, B);
+    }
 }
 
-// Jacobian-transpose pair sum, mixed precision.  The adjoint amplifies the
-// error of close pairs over a rollout (a pair at a few softening lengths
-// dominates J), so the pair arithmetic is FP32 on hi/lo splits:
-//   d = (x_k,hi - x_j,hi) + (x_k,lo - x_j,lo)
-// with both coordinates taken relative to the CTA's first target (the hi
-// difference of a close pair is exact by Sterbenz's lemma), and
+// Mixed precision.  The adjoint amplifies the error of close pairs over a rollout
+// (a pair at a few softening lengths dominates J), so the pair arithmetic is FP32
+// on hi/lo splits:
+//   d = x_k - x_j from offsets to the block's middle particle, with the parts
+// below their rounding kept where a tile comes near the block (as the direct
+// sum), and
 //   w = (q_j u_k,hi - q_k u_j,hi) + (q_j u_k,lo - q_k u_j,lo)
 // so a small difference of two large, nearly equal adjoints keeps its digits.
 // Units: coordinates in 2^-30 m (1/s^3 in metres overflows FP32), u scaled by
-// a power of two su from max|u|; both are exact and undone in FP64 at the end.
-// rsqrtf is refined by one Newton step.  Tiles accumulate in FP32, FP64 across
-// tiles.
-__global__ void __launch_bounds__(kTPB)
-jtv_mixed_kernel(const double *__restrict__ xs, const double *__restrict__ ys, const double *__restrict__ zs,
-                 const float *__restrict__ qs, const double *__restrict__ ux, const double *__restrict__ uy,
-                 const double *__restrict__ uz, const double *__restrict__ umax, int n, int chunk, double eps2,
-                 double *__restrict__ ox, double *__restrict__ oy, double *__restrict__ oz, int atomic_out) {
-    __shared__ JSrc32 tile[kTile];
-    const int t0 = blockIdx.x * (kTPB * kTPT);
-    const int j_begin = blockIdx.y * chunk;
-    const int j_end = min(n, j_begin + chunk);
-    const int o = min(t0, n - 1);
-    const double bx = xs[o], by = ys[o], bz = zs[o];
-    const double sc = 1073741824.0;  // 2^30
-    int ue = 0;
-    const double um = *umax;
-    if (um > 0.0) frexp(um, &ue);
-    const double su = ldexp(1.0, -ue);
-    const double back = sc * sc * sc / su;
-    const float e2 = (float)(eps2 * sc * sc);
-    const float min_r2 = (float)(kMinR2 * sc * sc);
-    float txh[kTPT], tyh[kTPT], tzh[kTPT], txl[kTPT], tyl[kTPT], tzl[kTPT], tq[kTPT];
-    float tuxh[kTPT], tuyh[kTPT], tuzh[kTPT], tuxl[kTPT], tuyl[kTPT], tuzl[kTPT];
-    double sx[kTPT], sy[kTPT], sz[kTPT];
+// a power of two from max|u|; both are exact and undone in FP64 at the end.
+// The reciprocal square root is refined by one Newton step.  FP32-pipe bound:
+// 45 operations per pair (39 when all charges are equal), two targets per packed
+// instruction, each pair once: 16,384 particles 532 -> 211 us per launch, 4,096
+// 54 -> 21 us, against the one-sided scalar kernel.
+struct JPairArgs {
+    const float4 *ph, *pl, *uh, *ul;
+    int n, nb, ct, nch;
+    float e2;
+    double *ox, *oy, *oz;
+    const int *differ;
+};
+
+constexpr int kJR = 4, kJH = kJR / 2;  // particles (packed pairs) of the block per lane
+
+struct JBlock {
+    float2 X[kJH], Y[kJH], Z[kJH], Q[kJH], ux[kJH], uy[kJH], uz[kJH], vx[kJH], vy[kJH], vz[kJH];
+    float2 fx[kJH], fy[kJH], fz[kJH];
+};
+struct JLow {
+    float2 x[kJH][32], y[kJH][32], z[kJH][32];
+};
+// the travelling particle: negated coordinates, their parts below FP32, charge,
+// negated u (hi, lo), and its sums
+struct JTravel {
+    float x, y, z, mx, my, mz, q, ux, uy, uz, vx, vy, vz, sx, sy, sz;
+};
+
+__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float turn(float v) { return __shfl_sync(0xffffffffu, v, ((threadIdx.x & 31) + 1) & 31); }
+
+template <bool UQ, bool SYM, bool NEAR>
+__device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, float min_r2, JTravel &t) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int step = 0; step < 32; step++) {
+        float2 jx, jy, jz;
 #pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int ii = min(t0 + (int)threadIdx.x + k * kTPB, n - 1);
-        split_hl((xs[ii] - bx) * sc, txh[k], txl[k]);
-        split_hl((ys[ii] - by) * sc, tyh[k], tyl[k]);
-        split_hl((zs[ii] - bz) * sc, tzh[k], tzl[k]);
-        tq[k] = qs[ii];
-        split_hl(ux[ii] * su, tuxh[k], tuxl[k]);
-        split_hl(uy[ii] * su, tuyh[k], tuyl[k]);
-        split_hl(uz[ii] * su, tuzh[k], tuzl[k]);
-        sx[k] = sy[k] = sz[k] = 0.0;
-    }
-    for (int jt = j_begin; jt < j_end; jt += kTile) {
-        __syncthreads();
-        for (int s = threadIdx.x; s < kTile; s += kTPB) {
-            const int j = jt + s;
-            JSrc32 v{};
-            if (j < j_end) {
-                split_hl((xs[j] - bx) * sc, v.xh, v.xl);
-                split_hl((ys[j] - by) * sc, v.yh, v.yl);
-                split_hl((zs[j] - bz) * sc, v.zh, v.zl);
-                v.q = qs[j];
-                split_hl(ux[j] * su, v.uxh, v.uxl);
-                split_hl(uy[j] * su, v.uyh, v.uyl);
-                split_hl(uz[j] * su, v.uzh, v.uzl);
+        for (int p = 0; p < kJH; p++) {
+            float2 dx = __fadd2_rn(b.X[p], dup(t.x)), dy = __fadd2_rn(b.Y[p], dup(t.y)),
+                   dz = __fadd2_rn(b.Z[p], dup(t.z));
+            if (NEAR) {
+                dx = __fadd2_rn(dx, __fadd2_rn(low.x[p][lane], dup(t.mx)));
+                dy = __fadd2_rn(dy, __fadd2_rn(low.y[p][lane], dup(t.my)));
+                dz = __fadd2_rn(dz, __fadd2_rn(low.z[p][lane], dup(t.mz)));
             }
-            tile[s] = v;
-        }
-        __syncthreads();
-        float fx[kTPT], fy[kTPT], fz[kTPT];
-#pragma unroll
-        for (int k = 0; k < kTPT; k++) fx[k] = fy[k] = fz[k] = 0.0f;
-        const int lim = min(kTile, j_end - jt);
-        for (int s = 0; s < lim; s++) {
-            const JSrc32 v = tile[s];
-#pragma unroll
-            for (int k = 0; k < kTPT; k++) {
-                const float dx = (txh[k] - v.xh) + (txl[k] - v.xl);
-                const float dy = (tyh[k] - v.yh) + (tyl[k] - v.yl);
-                const float dz = (tzh[k] - v.zh) + (tzl[k] - v.zl);
-                float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, e2)));
-                r2 = fmaxf(r2, min_r2);
-                float inv = rsqrtf(r2);
-                inv = inv * fmaf(-0.5f * r2 * inv, inv, 1.5f);
-                const float inv2 = inv * inv, inv3 = inv * inv2;
-                const float wx = fmaf(-tq[k], v.uxh, v.q * tuxh[k]) + fmaf(-tq[k], v.uxl, v.q * tuxl[k]);
-                const float wy = fmaf(-tq[k], v.uyh, v.q * tuyh[k]) + fmaf(-tq[k], v.uyl, v.q * tuyl[k]);
-                const float wz = fmaf(-tq[k], v.uzh, v.q * tuzh[k]) + fmaf(-tq[k], v.uzl, v.q * tuzl[k]);
-                const float dw = 3.0f * (fmaf(dx, wx, fmaf(dy, wy, dz * wz)) * inv2) * inv3;
-                fx[k] = fmaf(-dw, dx, fmaf(wx, inv3, fx[k]));
-                fy[k] = fmaf(-dw, dy, fmaf(wy, inv3, fy[k]));
-                fz[k] = fmaf(-dw, dz, fmaf(wz, inv3, fz[k]));
+            float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, E2)));
+            r2 = make_float2(fmaxf(r2.x, min_r2), fmaxf(r2.y, min_r2));
+            float2 inv = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
+            inv = __fmul2_rn(inv, __ffma2_rn(__fmul2_rn(__fmul2_rn(r2, dup(-0.5f)), inv), inv, dup(1.5f)));
+            const float2 inv2 = __fmul2_rn(inv, inv), inv3 = __fmul2_rn(inv, inv2);
+            // q_j u_k - q_k u_j (the travelling u is negated)
+            auto weight = [&](float2 uh, float2 ul, float th, float tl) {
+                if (UQ) return __fadd2_rn(__fadd2_rn(uh, dup(th)), __fadd2_rn(ul, dup(tl)));
+                return __fadd2_rn(__ffma2_rn(b.Q[p], dup(th), __fmul2_rn(dup(t.q), uh)),
+                                  __ffma2_rn(b.Q[p], dup(tl), __fmul2_rn(dup(t.q), ul)));
+            };
+            const float2 wx = weight(b.ux[p], b.vx[p], t.ux, t.vx), wy = weight(b.uy[p], b.vy[p], t.uy, t.vy),
+                         wz = weight(b.uz[p], b.vz[p], t.uz, t.vz);
+            const float2 dot = __ffma2_rn(dx, wx, __ffma2_rn(dy, wy, __fmul2_rn(dz, wz)));
+            const float2 dw = __fmul2_rn(__fmul2_rn(dot, inv2), __fmul2_rn(inv3, dup(-3.0f)));
+            const float2 vx = __ffma2_rn(dw, dx, __fmul2_rn(wx, inv3)), vy = __ffma2_rn(dw, dy, __fmul2_rn(wy, inv3)),
+                         vz = __ffma2_rn(dw, dz, __fmul2_rn(wz, inv3));
+            b.fx[p] = __fadd2_rn(b.fx[p], vx);
+            b.fy[p] = __fadd2_rn(b.fy[p], vy);
+            b.fz[p] = __fadd2_rn(b.fz[p], vz);
+            if (SYM) {
+                jx = p == 0 ? vx : __fadd2_rn(jx, vx);
+                jy = p == 0 ? vy : __fadd2_rn(jy, vy);
+                jz = p == 0 ? vz : __fadd2_rn(jz, vz);
             }
         }
+        t.x = turn(t.x);
+        t.y = turn(t.y);
+        t.z = turn(t.z);
+        if (NEAR) {
+            t.mx = turn(t.mx);
+            t.my = turn(t.my);
+            t.mz = turn(t.mz);
+        }
+        if (!UQ) t.q = turn(t.q);
+        t.ux = turn(t.ux);
+        t.uy = turn(t.uy);
+        t.uz = turn(t.uz);
+        t.vx = turn(t.vx);
+        t.vy = turn(t.vy);
+        t.vz = turn(t.vz);
+        if (SYM) {
+            t.sx = turn(t.sx - (jx.x + jx.y));
+            t.sy = turn(t.sy - (jy.x + jy.y));
+            t.sz = turn(t.sz - (jz.x + jz.y));
+        }
+    }
+}
+
+template <bool UQ, bool SYM>
+__device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, int B, int k0, int k1) {
+    const int lane = threadIdx.x & 31;
+    const float sc = (float)kLen;
+    const int i0 = A * 32 * kJR, io = min(i0 + 16 * kJR, a.n - 1);
+    const float4 oh = a.ph[io], ol = a.pl[io];
+    JBlock b;
+    float ext = 0.f;
+    __syncwarp();  // the previous unit's reads of `low`
 #pragma unroll
-        for (int k = 0; k < kTPT; k++) {
-            sx[k] += (double)fx[k];
-            sy[k] += (double)fy[k];
-            sz[k] += (double)fz[k];
+    for (int p = 0; p < kJH; p++) {
+        float c[2][13];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int i = i0 + 32 * (2 * p + u) + lane;
+#pragma unroll
+            for (int e = 0; e < 13; e++) c[u][e] = 0.f;
+            c[u][0] = -kFar;
+            if (i < a.n) {
+                const float4 h = a.ph[i], l = a.pl[i], uh = a.uh[i], ul = a.ul[i];
+                c[u][0] = hilo_diff(h.x, l.x, oh.x, ol.x, c[u][4]) * sc;
+                c[u][1] = hilo_diff(h.y, l.y, oh.y, ol.y, c[u][5]) * sc;
+                c[u][2] = hilo_diff(h.z, l.z, oh.z, ol.z, c[u][6]) * sc;
+                c[u][3] = h.w;
+                c[u][7] = uh.x;
+                c[u][8] = uh.y;
+                c[u][9] = uh.z;
+                c[u][10] = ul.x;
+                c[u][11] = ul.y;
+                c[u][12] = ul.z;
+                ext = fmaxf(ext, fmaxf(fabsf(c[u][0]), fmaxf(fabsf(c[u][1]), fabsf(c[u][2]))));
+            }
+        }
+        auto both = [&](int e) { return make_float2(c[0][e], c[1][e]); };
+        b.X[p] = both(0);
+        b.Y[p] = both(1);
+        b.Z[p] = both(2);
+        b.Q[p] = both(3);
+        low.x[p][lane] = make_float2(c[0][4] * sc, c[1][4] * sc);
+        low.y[p][lane] = make_float2(c[0][5] * sc, c[1][5] * sc);
+        low.z[p][lane] = make_float2(c[0][6] * sc, c[1][6] * sc);
+        b.ux[p] = both(7);
+        b.uy[p] = both(8);
+        b.uz[p] = both(9);
+        b.vx[p] = both(10);
+        b.vy[p] = both(11);
+        b.vz[p] = both(12);
+        b.fx[p] = b.fy[p] = b.fz[p] = make_float2(0.f, 0.f);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ext = fmaxf(ext, __shfl_xor_sync(0xffffffffu, ext, o));
+    const float q0 = UQ ? oh.w : 1.f;
+    const float2 E2 = dup(a.e2);
+    const float min_r2 = kMinR2 * sc * sc;
+    for (int k = k0; k < k1; k++) {
+        const int j = B * 32 * kJR + 32 * k + lane;
+        JTravel t{};
+        t.x = -kFar;
+        bool near = false;
+        if (j < a.n) {
+            const float4 h = a.ph[j], l = a.pl[j], uh = a.uh[j], ul = a.ul[j];
+            t.x = -sc * hilo_diff(h.x, l.x, oh.x, ol.x, t.mx);
+            t.y = -sc * hilo_diff(h.y, l.y, oh.y, ol.y, t.my);
+            t.z = -sc * hilo_diff(h.z, l.z, oh.z, ol.z, t.mz);
+            t.mx *= -sc;
+            t.my *= -sc;
+            t.mz *= -sc;
+            t.q = h.w;
+            t.ux = -uh.x;
+            t.uy = -uh.y;
+            t.uz = -uh.z;
+            t.vx = -ul.x;
+            t.vy = -ul.y;
+            t.vz = -ul.z;
+            near = fmaxf(fabsf(t.x), fmaxf(fabsf(t.y), fabsf(t.z))) <= 2.f * ext;
+        }
+        if (!SYM || __any_sync(0xffffffffu, near)) jtv_tile<UQ, SYM, true>(b, low, E2, min_r2, t);
+        else jtv_tile<UQ, SYM, false>(b, low, E2, min_r2, t);
+        if (SYM && j < a.n) {
+            atomicAdd(&a.ox[j], widen(t.sx * q0));
+            atomicAdd(&a.oy[j], widen(t.sy * q0));
+            atomicAdd(&a.oz[j], widen(t.sz * q0));
         }
     }
 #pragma unroll
-    for (int k = 0; k < kTPT; k++) {
-        const int i = t0 + threadIdx.x + k * kTPB;
-        if (i >= n) continue;
-        if (atomic_out) {
-            atomicAdd(&ox[i], sx[k] * back);
-            atomicAdd(&oy[i], sy[k] * back);
-            atomicAdd(&oz[i], sz[k] * back);
+    for (int r = 0; r < kJR; r++) {
+        const int i = i0 + 32 * r + lane;
+        if (i >= a.n) continue;
+        atomicAdd(&a.ox[i], widen((r & 1 ? b.fx[r / 2].y : b.fx[r / 2].x) * q0));
+        atomicAdd(&a.oy[i], widen((r & 1 ? b.fy[r / 2].y : b.fy[r / 2].x) * q0));
+        atomicAdd(&a.oz[i], widen((r & 1 ? b.fz[r / 2].y : b.fz[r / 2].x) * q0));
+    }
+}
+
+__global__ void __launch_bounds__(32 * kPairWarps, 3) jtv_pairs_kernel(JPairArgs a) {
+    __shared__ JLow lows[kPairWarps];
+    JLow &low = lows[threadIdx.x >> 5];
+    const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
+    const bool differ = *a.differ != 0;
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;
+        const int k0 = ch * a.ct, k1 = min(k0 + a.ct, kJR);
+        if (differ) {
+            if (A != B) jtv_unit<false, true>(a, low, A, B, k0, k1);
+            else jtv_unit<false, false>(a, low, A, B, k0, k1);
         } else {
-            ox[i] = sx[k] * back;
-            oy[i] = sy[k] * back;
-            oz[i] = sz[k] * back;
+            if (A != B) jtv_unit<true, true>(a, low, A, B, k0, k1);
+            else jtv_unit<true, false>(a, low, A, B, k0, k1);
         }
     }
 }
@@ -370,59 +481,81 @@ int stream_grid(int64_t n) {
     return (int)(b < 1 ? 1 : (b > 16 * device_sms() ? 16 * device_sms() : b));
 }
 
-sv_status copy_state(sv_ctx *c, double *dst) {
-    const size_t b = sizeof(double) * c->n;
-    double *src[6] = {c->x, c->y, c->z, c->vx, c->vy, c->vz};
-    for (int k = 0; k < 6; k++) SV_CK(c, cudaMemcpyAsync(dst + k * c->n, src[k], b, cudaMemcpyDeviceToDevice, c->stream));
+struct SixArrays {
+    double *a[6];
+};
+// x, y, z, vx, vy, vz to (to = 1) or from a checkpoint of 6 n
+__global__ void copy_state_kernel(SixArrays st, double *__restrict__ ck, int64_t n, int to) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < 6 * n; t += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(t / n);
+        double *p = st.a[k] + (t - k * n);
+        if (to) ck[t] = *p;
+        else *p = ck[t];
+    }
+}
+
+sv_status copy_state(sv_ctx *c, double *ck, bool to) {
+    if (c->n == 0) return SV_OK;
+    copy_state_kernel<<<stream_grid(6 * c->n), 256, 0, c->stream>>>(
+        SixArrays{{c->x, c->y, c->z, c->vx, c->vy, c->vz}}, ck, c->n, to ? 1 : 0);
+    SV_LAUNCHED(c);
     return SV_OK;
 }
 
-sv_status load_state(sv_ctx *c, const double *src) {
-    const size_t b = sizeof(double) * c->n;
-    double *dst[6] = {c->x, c->y, c->z, c->vx, c->vy, c->vz};
-    for (int k = 0; k < 6; k++) SV_CK(c, cudaMemcpyAsync(dst[k], src + k * c->n, b, cudaMemcpyDeviceToDevice, c->stream));
-    return SV_OK;
-}
+// the 4 n + 2 doubles behind the adjoints, on a 16-byte boundary
+double *scratch(const Adj &A) { return A.lam + 9 * A.n + (A.n & 1); }
 
-// J(x)^T la for the positions currently in c->x, over the particles of
-// c->wstatus (the step's window): result added into (lx, ly, lz)
-sv_status jtv_add(sv_ctx *c, const double *lax, const double *lay, const double *laz, double *lx, double *ly,
-                  double *lz) {
+// One reverse step that starts at ts, from its mid positions xh: the adjoints
+// (lx, lv) of the step's end become those of its start.
+sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
+    Adj &A = *c->adj;
+    const int64_t nn = A.n;
+    double *lx = A.lam, *lv = lx + 3 * nn, *la = lv + 3 * nn;
+    unsigned long long *umax = reinterpret_cast<unsigned long long *>(A.lE + 3);
+    SV_CK(c, cudaMemsetAsync(umax, 0, sizeof(*umax), c->stream));
+    adj_prep<<<stream_grid(nn), 256, 0, c->stream>>>(PrepArgs{xh, c->x, c->y, c->z, c->wstatus, lx, lv, la, c->qom,
+                                                              c->t_inj, c->status, nn, ts, A.dt, c->P.e_over_amu,
+                                                              c->P.k_const, A.lE, umax});
+    SV_LAUNCHED(c);
+    // the particles of the step's window in Morton order
+    const bool fp64 = c->P.precision == SV_PREC_FP64;
     c->fstatus = c->wstatus;
     c->S.want_zero = true;
-    const sv_status st = sort_state(c, 0, c->n);
+    c->S.want_hilo = !fp64;
+    c->S.hl_abs = false;
+    const sv_status st = sort_state(c, 0, nn);
     c->fstatus = nullptr;
     SV_TRY(st);
     Sorted &S = c->S;
     const int n = (int)S.n;
-    Adj &A = *c->adj;
-    double *ux = A.lam + 9 * A.n, *uy = ux + A.n, *uz = uy + A.n;  // tmp block
-    unsigned long long *umax = reinterpret_cast<unsigned long long *>(A.lE + 3);
-    SV_CK(c, cudaMemsetAsync(umax, 0, sizeof(*umax), c->stream));
-    adj_gather_u<<<grid_of(n), 256, 0, c->stream>>>(S.idx, n, S.qm, lax, lay, laz, ux, uy, uz, umax);
+    double *u = scratch(A);
+    float4 *uh = reinterpret_cast<float4 *>(u), *ul = uh + nn;
+    adj_gather_u<<<grid_of(n), 256, 0, c->stream>>>(S.idx, n, S.qm, la, A.lE + 3, fp64 ? u : nullptr, uh, ul);
     SV_LAUNCHED(c);
-    const int tblocks = div_up(n, kTPB * kTPT);
-    int splits = div_up(8 * device_sms(), tblocks);
-    const int max_splits = div_up(n, kTile);
-    if (splits > max_splits) splits = max_splits;
-    if (splits < 1) splits = 1;
-    const int chunk = div_up(div_up(n, splits), kTile) * kTile;
-    splits = div_up(n, chunk);
-    const int atomic_out = splits > 1;  // into the sums the sort cleared
-    const dim3 grid(tblocks, splits);
-    if (c->P.precision == SV_PREC_FP64)
-        jtv_fp64_kernel<<<grid, kTPB, 0, c->stream>>>(S.x, S.y, S.z, S.q, ux, uy, uz, n, chunk, c->P.softening2, S.ax,
-                                                      S.ay, S.az, atomic_out);
-    else
-        jtv_mixed_kernel<<<grid, kTPB, 0, c->stream>>>(S.x, S.y, S.z, S.q, ux, uy, uz, A.lE + 3, n, chunk,
-                                                       c->P.softening2, S.ax, S.ay, S.az, atomic_out);
+    if (fp64) {
+        const JPair64Args a{S.x, S.y, S.z, u, S.q, n, div_up(n, 32), c->P.softening2, S.ax, S.ay, S.az};
+        jtv_pairs64_kernel<<<pair_grid(a.nb, 1), 32 * kPairWarps, 0, c->stream>>>(a);
+    } else {
+        JPairArgs a{S.ph, S.pl, uh, ul, n, div_up(n, 32 * kJR), 0, 0, (float)(c->P.softening2 * kLen * kLen),
+                    S.ax, S.ay, S.az, reinterpret_cast<const int *>(S.root + 14)};
+        // about 16 units per SM sub-partition
+        const int64_t tiles = (int64_t)a.nb * (a.nb + 1) / 2 * kJR;
+        a.ct = (int)std::max<int64_t>(1, std::min<int64_t>({kMaxTiles, kJR, tiles / (64 * (int64_t)device_sms())}));
+        a.nch = div_up(kJR, a.ct);
+        jtv_pairs_kernel<<<pair_grid(a.nb, a.nch), 32 * kPairWarps, 0, c->stream>>>(a);
+    }
     SV_LAUNCHED(c);
-    adj_post<<<grid_of(n), 256, 0, c->stream>>>(S.idx, n, S.n_orig, S.ax, S.ay, S.az, lx, ly, lz);
+    adj_post<<<grid_of(n), 256, 0, c->stream>>>(S.idx, n, S.ax, S.ay, S.az, fp64 ? 0 : 1, umax, lx, lv, c->status,
+                                                c->t_inj, ts, A.dt);
     SV_LAUNCHED(c);
     return SV_OK;
 }
 
 }  // namespace
+
+void adjoint_state_changed(sv_ctx *c) {
+    if (c->adj) c->adj->xh_seg = -1;
+}
 
 void adjoint_free(sv_ctx *c) {
     if (!c->adj) return;
@@ -466,7 +599,7 @@ extern "C" sv_status sv_adjoint_forward(sv_ctx *c, int32_t nsteps, double dt, do
         const int64_t cap = n > 1 ? n : 1;
         SV_CK(c, cudaMalloc(&A.ck, sizeof(double) * 6 * cap * nck));
         SV_CK(c, cudaMalloc(&A.xh, sizeof(double) * 3 * cap * seg));
-        SV_CK(c, cudaMalloc(&A.lam, sizeof(double) * 12 * cap));
+        SV_CK(c, cudaMalloc(&A.lam, sizeof(double) * (13 * cap + 2)));
         SV_CK(c, cudaMalloc(&A.fin, sizeof(double) * 6 * cap));
         SV_CK(c, cudaMalloc(&A.lE, sizeof(double) * 4));  // lE[3]: max |u| of a step
         A.cap = cap;
@@ -478,10 +611,15 @@ extern "C" sv_status sv_adjoint_forward(sv_ctx *c, int32_t nsteps, double dt, do
     A.every = checkpoint_every;
     A.dt = dt;
     A.t0 = t0;
+    A.xh_seg = -1;
+    const int last = nsteps > 0 ? (nsteps - 1) / checkpoint_every : 0;
     for (int s = 0; s < nsteps; s++) {
-        if (s % checkpoint_every == 0) SV_TRY(copy_state(c, A.ck + (size_t)(s / checkpoint_every) * 6 * n));
-        SV_TRY(leapfrog_step(c, t0 + dt * s, dt, nullptr));
+        const int k = s / checkpoint_every;
+        if (s % checkpoint_every == 0) SV_TRY(copy_state(c, A.ck + (size_t)k * 6 * n, true));
+        // the last segment's mid positions serve the backward pass as they are
+        SV_TRY(leapfrog_step(c, t0 + dt * s, dt, k == last ? A.xh + (size_t)(s - k * checkpoint_every) * 3 * n : nullptr));
     }
+    if (nsteps > 0) A.xh_seg = last;
     A.forward_done = true;
     return SV_OK;
 }
@@ -495,9 +633,8 @@ extern "C" sv_status sv_adjoint_backward(sv_ctx *c, const double *dl_dx3, const 
     const int64_t n = A.n;
     if (n != c->n) return set_error(c, SV_ERR_STATE, "state changed since sv_adjoint_forward");
     double *lx = A.lam, *ly = lx + n, *lz = ly + n, *lvx = lz + n, *lvy = lvx + n, *lvz = lvy + n;
-    double *lax = lvz + n, *lay = lax + n, *laz = lay + n;
-    // final adjoints from the caller (host, 3n interleaved); staging in the tmp block
-    double *tmp = A.lam + 9 * n;
+    // final adjoints from the caller (host, 3n interleaved); staging behind the adjoints
+    double *tmp = scratch(A);
     SV_CK(c, cudaMemcpyAsync(tmp, dl_dx3, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->stream));
     deinterleave<<<grid_of(n), 256, 0, c->stream>>>(tmp, n, lx, ly, lz);
     SV_LAUNCHED(c);
@@ -505,33 +642,24 @@ extern "C" sv_status sv_adjoint_backward(sv_ctx *c, const double *dl_dx3, const 
     deinterleave<<<grid_of(n), 256, 0, c->stream>>>(tmp, n, lvx, lvy, lvz);
     SV_LAUNCHED(c);
     SV_CK(c, cudaMemsetAsync(A.lE, 0, sizeof(double) * 3, c->stream));
-    SV_TRY(copy_state(c, A.fin));
+    SV_TRY(copy_state(c, A.fin, true));
     const double dt = A.dt;
     for (int k = (A.nsteps - 1) / A.every; k >= 0 && A.nsteps > 0; k--) {
         const int s0 = k * A.every;
         const int s1 = s0 + A.every < A.nsteps ? s0 + A.every : A.nsteps;
-        // recompute the segment from its checkpoint, keeping every x_h
-        SV_TRY(load_state(c, A.ck + (size_t)k * 6 * n));
-        for (int s = s0; s < s1; s++)
-            SV_TRY(leapfrog_step(c, A.t0 + dt * s, dt, A.xh + (size_t)(s - s0) * 3 * n));
-        for (int s = s1 - 1; s >= s0; s--) {
-            const double ts = A.t0 + dt * s;
-            const double *xh = A.xh + (size_t)(s - s0) * 3 * n;
-            SV_CK(c, cudaMemcpyAsync(c->x, xh, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-            SV_CK(c, cudaMemcpyAsync(c->y, xh + n, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-            SV_CK(c, cudaMemcpyAsync(c->z, xh + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->stream));
-            SV_TRY(window_status(c, ts + 0.5 * dt));
-            adj_prep<<<stream_grid(n), 256, 0, c->stream>>>(lx, ly, lz, lvx, lvy, lvz, lax, lay, laz, c->q, c->m,
-                                                            c->status, c->wstatus, c->t_inj, n, ts, dt,
-                                                            c->P.e_over_amu, A.lE);
-            SV_LAUNCHED(c);
-            SV_TRY(jtv_add(c, lax, lay, laz, lx, ly, lz));
-            adj_drift_back<<<stream_grid(n), 256, 0, c->stream>>>(lx, ly, lz, lvx, lvy, lvz, c->status, c->t_inj, n,
-                                                                  ts, dt);
-            SV_LAUNCHED(c);
+        // recompute the segment from its checkpoint, keeping every x_h, unless
+        // they are at hand
+        if (A.xh_seg != k || c->field.nt > 0) {
+            A.xh_seg = -1;
+            SV_TRY(copy_state(c, A.ck + (size_t)k * 6 * n, false));
+            for (int s = s0; s < s1; s++)
+                SV_TRY(leapfrog_step(c, A.t0 + dt * s, dt, A.xh + (size_t)(s - s0) * 3 * n));
+            A.xh_seg = k;
         }
+        for (int s = s1 - 1; s >= s0; s--)
+            SV_TRY(reverse_step(c, A.xh + (size_t)(s - s0) * 3 * n, A.t0 + dt * s));
     }
-    SV_TRY(load_state(c, A.fin));
+    SV_TRY(copy_state(c, A.fin, false));
     if (dl_dx0) {
         interleave<<<grid_of(n), 256, 0, c->stream>>>(lx, ly, lz, n, tmp);
         SV_LAUNCHED(c);

@@ -731,6 +731,7 @@ sv_status sv_set_params(sv_ctx *c, const sv_params *p) {
     if (p->device != c->device) return set_error(c, SV_ERR_INVALID, "device cannot change on a context");
     c->P = *p;
     batch_invalidate(c);
+    adjoint_state_changed(c);
     return SV_OK;
 }
 
@@ -750,6 +751,7 @@ static sv_status upload_state(sv_ctx *c, int64_t n, const double *x3, const doub
     c->n = n;
     c->have_state = true;
     c->have_accel = false;
+    adjoint_state_changed(c);
     c->ev_seq = 0;
     if (c->d_ev_count) SV_CK(c, cudaMemsetAsync(c->d_ev_count, 0, sizeof(unsigned long long), c->stream));
     SV_TRY(field_prepare(c));
@@ -820,6 +822,7 @@ sv_status sv_upload_ref32(sv_ctx *c, int64_t n, const float *pos4, const float *
     c->n = n;
     c->have_state = true;
     c->have_accel = false;
+    adjoint_state_changed(c);
     c->ev_seq = 0;
     if (c->d_ev_count) SV_CK(c, cudaMemsetAsync(c->d_ev_count, 0, sizeof(unsigned long long), c->stream));
     SV_TRY(field_prepare(c));
@@ -857,6 +860,7 @@ sv_status sv_update_state(sv_ctx *c, int64_t n, const double *x3, const double *
                                     (long long)c->n);
     SV_CK(c, cudaSetDevice(c->device));
     c->have_accel = false;
+    adjoint_state_changed(c);
     if (n == 0) return SV_OK;
     const double *mx = (const double *)mapped_host(x3), *mv = (const double *)mapped_host(v3);
     const int32_t *ms = (const int32_t *)mapped_host(status);
@@ -1098,6 +1102,7 @@ sv_status sv_set_boundary(sv_ctx *c, const sv_boundary *b) {
             if (c->P.sym_axes[k] && !(c->P.domain_size[k] > 0.0))
                 return set_error(c, SV_ERR_INVALID, "folding a periodic axis needs domain_size > 0");
     c->B = *b;
+    adjoint_state_changed(c);
     if (c->batch) batch_invalidate(c);
     return SV_OK;
 }

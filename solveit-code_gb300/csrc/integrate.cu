@@ -31,6 +31,7 @@ struct DriftArgs {
     const double *t_inj;
     const int32_t *species;
     int32_t *window;  // status for the force and kick of the step, or null
+    double *save;     // the drifted positions as well (x, y, z of n each), or null
     int64_t n;
     double t_start, h;
     const double *tb;
@@ -116,6 +117,12 @@ __device__ void record_event(const DriftArgs &a, long long seq, int phase, int64
     a.ev_key[slot] = ((unsigned long long)seq << 34) | ((unsigned long long)phase << 32) | (unsigned long long)(uint32_t)i;
 }
 
+__device__ __forceinline__ void save_positions(const DriftArgs &a, int64_t i, double x, double y, double z) {
+    a.save[i] = x;
+    a.save[a.n + i] = y;
+    a.save[2 * a.n + i] = z;
+}
+
 // FULL = false: no crash test, folding or boundary conditions (the common
 // case), compiled without their code so the streaming loop keeps few registers
 template <bool FULL>
@@ -138,6 +145,7 @@ __global__ void drift_kernel(DriftArgs a) {
         const double ti = tinj[i];
         if (!(ti <= T)) {  // not injected by the end of this half step: outside the window
             if (win) win[i] = 0;
+            if (a.save) save_positions(a, i, px[i], py[i], pz[i]);
             continue;
         }
         int32_t w = pst[i];
@@ -149,6 +157,7 @@ __global__ void drift_kernel(DriftArgs a) {
                 pz[i] += pvz[i] * s;
             }
             if (win) win[i] = w;
+            if (a.save) save_positions(a, i, px[i], py[i], pz[i]);
             continue;
         }
         const int32_t w0 = w;
@@ -215,6 +224,7 @@ __global__ void drift_kernel(DriftArgs a) {
         }
         if (w != w0) pst[i] = w;
         if (win) win[i] = w;
+        if (a.save) save_positions(a, i, x, y, z);
     }
 }
 
@@ -258,13 +268,6 @@ __global__ void kick_kernel(double *__restrict__ vx, double *__restrict__ vy, do
         vy[i] += (ay[i] + fy * f) * s;
         vz[i] += (az[i] + fz * f) * s;
     }
-}
-
-__global__ void window_kernel(const int32_t *__restrict__ st, const double *__restrict__ t_inj, int64_t n, double T,
-                              int32_t *__restrict__ out) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = t_inj[i] <= T ? st[i] : 0;
 }
 
 constexpr int kETile = 256;
@@ -356,7 +359,8 @@ void events_free(sv_ctx *c) {
     c->ev_cap = 0;
 }
 
-sv_status drift(sv_ctx *c, double t_start, double h, int32_t *window, const double *tb, long long seq_base) {
+sv_status drift(sv_ctx *c, double t_start, double h, int32_t *window, const double *tb, long long seq_base,
+                double *save) {
     const sv_boundary &B = c->B;
     DriftArgs a{};
     a.x = c->x; a.y = c->y; a.z = c->z;
@@ -365,6 +369,7 @@ sv_status drift(sv_ctx *c, double t_start, double h, int32_t *window, const doub
     a.t_inj = c->t_inj;
     a.species = c->species;
     a.window = window;
+    a.save = save;
     a.n = c->n;
     a.t_start = t_start;
     a.h = h;
@@ -402,25 +407,13 @@ sv_status kick(sv_ctx *c, double t_start, double dt, const int32_t *st, const do
     return SV_OK;
 }
 
-sv_status window_status(sv_ctx *c, double t_window) {
-    window_kernel<<<stream_grid(c->n), 256, 0, c->stream>>>(c->status, c->t_inj, c->n, t_window, c->wstatus);
-    SV_LAUNCHED(c);
-    return SV_OK;
-}
-
 sv_status leapfrog_step(sv_ctx *c, double ts, double dt, double *save_xh) {
     const double h = 0.5 * dt;
     if (c->B.crash != SV_CRASH_NONE || c->B.bc != SV_BC_NONE) SV_TRY(events_reserve(c));
     SV_TRY(field_prepare(c));
     SV_TRY(energy_inject(c, ts + h));
-    SV_TRY(drift(c, ts, h, c->wstatus));
+    SV_TRY(drift(c, ts, h, c->wstatus, nullptr, 0, save_xh));
     SV_TRY(energy_first(c, ts + h));
-    if (save_xh) {
-        const size_t b = sizeof(double) * c->n;
-        SV_CK(c, cudaMemcpyAsync(save_xh, c->x, b, cudaMemcpyDeviceToDevice, c->stream));
-        SV_CK(c, cudaMemcpyAsync(save_xh + c->n, c->y, b, cudaMemcpyDeviceToDevice, c->stream));
-        SV_CK(c, cudaMemcpyAsync(save_xh + 2 * c->n, c->z, b, cudaMemcpyDeviceToDevice, c->stream));
-    }
     c->fstatus = c->wstatus;
     const sv_status s = compute_accel_device(c, 0, c->n);
     c->fstatus = nullptr;

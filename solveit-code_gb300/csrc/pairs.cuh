@@ -1,0 +1,66 @@
+// pairs.cuh -- pieces shared by the kernels that visit every unordered pair of
+// particles once (direct.cu, adjoint.cu): the particles form blocks, a warp holds
+// one block in registers and a tile of 32 particles of another block travels
+// around its lanes with its own sums.
+#pragma once
+
+#include <algorithm>
+
+#include "sv_internal.cuh"
+
+namespace sv {
+
+// (hi + lo) - (ohi + olo) as r + res: r the difference rounded once (of the hi
+// parts with its exact rounding error, Knuth, then the small parts), res what
+// that rounding left out
+__device__ __forceinline__ float hilo_diff(float hi, float lo, float ohi, float olo, float &res) {
+    const float s = hi - ohi, bb = s - hi;
+    const float t = ((hi - (s - bb)) - (ohi + bb)) + (lo - olo);
+    const float r = s + t, tt = r - s;
+    res = (s - (r - tt)) + (t - tt);
+    return r;
+}
+
+// a float's value as a double, by its bits (the conversion instruction runs at
+// the FP64 rate); denormals become zero
+__device__ __forceinline__ double widen(float f) {
+    const uint32_t u = __float_as_uint(f), m = u & 0x7fffffffu;
+    uint32_t hi = (m >> 3) + 0x38000000u, lo = u << 29;
+    if (m >= 0x7f800000u) hi |= 0x7ff00000u;
+    if (m < 0x00800000u) hi = lo = 0;
+    return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
+}
+
+constexpr int kPairWarps = 4;    // warps (units) per CTA
+constexpr int kMaxTiles = 4;     // tiles per unit: 128 sources per FP32 sum of a target
+constexpr float kFar = 1e18f;    // coordinate of absent particles: r^-3 underflows to zero
+
+// 1/sqrt(r2) to FP32 precision as a double (relative error e/2 with |e| < 4e-7,
+// e = 1 - r2 y^2): the FP32 reciprocal square root of the truncated r2, converted
+// by bits on the integer pipe (the conversion instructions run at the FP64
+// rate).  r2 past the FP32 range gives 0, below it the smallest normal seed (a
+// zero distance stays finite).
+__device__ __forceinline__ double rsqrt_seed_f64(double r2) {
+    const int h = max(__double2hiint(r2), 0x38100000);
+    const int f = h >= 0x47f00000 ? 0x7f800000 : (int)(((uint32_t)(h - 0x38000000) << 3) |
+                                                       ((uint32_t)__double2loint(r2) >> 29));
+    const uint32_t u = __float_as_uint(rsqrt_ftz(__int_as_float(f)));
+    return u ? __hiloint2double((int)((u >> 3) + 0x38000000u), (int)(u << 29)) : 0.0;
+}
+
+// Unit (v, d) -> block pair (A, A + d mod nb), d = 0 .. nb / 2 (for even nb the
+// last distance from the first half of the blocks only): every unordered block
+// pair once.
+__device__ __forceinline__ bool unit_blocks(int64_t v, int d, int nb, int nch, int &A, int &B, int &ch) {
+    A = (int)(v / nch);
+    ch = (int)(v - (int64_t)A * nch);
+    if (A >= nb || (2 * (int64_t)d == nb && 2 * (int64_t)A >= nb)) return false;
+    B = (int)(((int64_t)A + d) % nb);
+    return true;
+}
+// grid of nb x nch units per distance, kPairWarps to a CTA; distances in y
+inline dim3 pair_grid(int nb, int nch) {
+    return dim3((unsigned)div_up((int64_t)nb * nch, kPairWarps), (unsigned)std::min(nb / 2 + 1, 65535));
+}
+
+}  // namespace sv

@@ -319,6 +319,8 @@ sv_status compute_accel_device(sv_ctx *c, int64_t first, int64_t last);
 
 // adjoint.cu
 void adjoint_free(sv_ctx *c);
+// the state, its statuses or the parameters were replaced: the mid positions kept by a forward pass no longer hold
+void adjoint_state_changed(sv_ctx *c);
 
 // outliers.cu: detection (status with outliers masked for the tree), the
 // direct sums of every interaction with an outlier, the flags of the last run
@@ -346,8 +348,9 @@ void batch_free(sv_ctx *c);
 // receives the status the following force and kick see (0 outside the
 // window).  With tb (device {t0, dt, k}) t_start is taken relative to
 // tb[0] + tb[1] * tb[2] and the event order from seq_base + 2 * tb[2].
+// save: the drifted positions as well (x, y, z of n each), or null.
 sv_status drift(sv_ctx *c, double t_start, double h, int32_t *window, const double *tb = nullptr,
-                long long seq_base = 0);
+                long long seq_base = 0, double *save = nullptr);
 // Kick over [t_start, t_start + dt] of the particles with st == 1 (st: the
 // windowed status of the step).
 sv_status kick(sv_ctx *c, double t_start, double dt, const int32_t *st, const double *tb = nullptr);
@@ -355,8 +358,6 @@ sv_status kick(sv_ctx *c, double t_start, double dt, const int32_t *st, const do
 sv_status leapfrog_step(sv_ctx *c, double ts, double dt, double *save_xh = nullptr);
 // status as the force sees it (windowed during a leapfrog step)
 inline const int32_t *force_status(const sv_ctx *c) { return c->fstatus ? c->fstatus : c->status; }
-// wstatus[i] = status[i] if t_inj[i] <= t_window else 0 (adjoint re-runs)
-sv_status window_status(sv_ctx *c, double t_window);
 sv_status events_reserve(sv_ctx *c);
 void events_free(sv_ctx *c);
 // field.cu: the per-particle walk caches of the emitter field (grown to n, reset to -1)
