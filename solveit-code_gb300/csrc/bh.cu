@@ -471,19 +471,15 @@ sv_status bh_accel(sv_ctx *c) {
     phase_mark(c, 4);
     phase_mark(c, 5);
     BhImages im{0, 1, nullptr};
-    double *d_off = nullptr;
     if (c->P.symmetry == SV_SYM_ROTATIONAL) {
         im.kind = 1;
         im.count = 4;
     } else if (c->P.symmetry == SV_SYM_TRANSLATIONAL) {
-        static thread_local double h_off[3 * 4096];
-        const int cnt = trans_images(c->P, h_off, 4096);
-        if (cnt <= 0 || cnt > 4096) return set_error(c, SV_ERR_INVALID, "bad translational image set (%d)", cnt);
-        SV_CK(c, cudaMallocAsync(&d_off, sizeof(double) * 3 * cnt, c->stream));
-        SV_CK(c, cudaMemcpyAsync(d_off, h_off, sizeof(double) * 3 * cnt, cudaMemcpyHostToDevice, c->stream));
+        const ImageSet *I = nullptr;
+        SV_TRY(image_set(c, &I));
         im.kind = 2;
-        im.count = cnt;
-        im.off = d_off;
+        im.count = I->count;
+        im.off = I->m;
     }
     SV_CK(c, cudaMemsetAsync(B.d_counts, 0, 2 * sizeof(unsigned long long), c->stream));
     // inactive sorted slots (beyond n_act) are never targets (qm = 0)
@@ -503,7 +499,6 @@ sv_status bh_accel(sv_ctx *c) {
         SV_CK(c, cudaMemsetAsync(S.az + T.n_act, 0, sizeof(double) * (n - T.n_act), c->stream));
     }
     phase_mark(c, 6);
-    if (d_off) SV_CK(c, cudaFreeAsync(d_off, c->stream));
     // the counts reach the host with the stream; bh_counts reads them
     SV_CK(c, cudaMemcpyAsync(B.h_counts, B.d_counts, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              c->stream));

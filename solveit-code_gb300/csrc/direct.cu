@@ -465,32 +465,16 @@ sv_status direct_accel(sv_ctx *c) {
     Sorted &S = c->S;
     Images im{0, 1, nullptr};
     const float4 *off_hl = nullptr;
-    void *d_off = nullptr;
     if (c->P.symmetry == SV_SYM_ROTATIONAL) {
         im.kind = 1;
         im.count = 4;
     } else if (c->P.symmetry == SV_SYM_TRANSLATIONAL) {
-        struct Offsets {
-            double m[3 * 4096];     // metres
-            float4 hl[2 * 4096];    // the same as FP32 hi and lo parts
-        };
-        static thread_local Offsets h;
-        const int cnt = trans_images(c->P, h.m, 4096);
-        if (cnt <= 0 || cnt > 4096) return set_error(c, SV_ERR_INVALID, "bad translational image set (%d)", cnt);
-        for (int g = 0; g < cnt; g++) {
-            const double *m = h.m + 3 * g;
-            const float hi[3] = {(float)m[0], (float)m[1], (float)m[2]};
-            h.hl[2 * g] = make_float4(hi[0], hi[1], hi[2], 0.f);
-            h.hl[2 * g + 1] = make_float4((float)(m[0] - hi[0]), (float)(m[1] - hi[1]), (float)(m[2] - hi[2]), 0.f);
-        }
-        const size_t bytes = c->P.precision == SV_PREC_FP64 ? sizeof(double) * 3 * cnt : sizeof(float4) * 2 * cnt;
-        SV_CK(c, cudaMallocAsync(&d_off, bytes, c->stream));
-        SV_CK(c, cudaMemcpyAsync(d_off, c->P.precision == SV_PREC_FP64 ? (const void *)h.m : (const void *)h.hl, bytes,
-                                 cudaMemcpyHostToDevice, c->stream));
+        const ImageSet *I = nullptr;
+        SV_TRY(image_set(c, &I));
         im.kind = 2;
-        im.count = cnt;
-        im.off = (const double *)d_off;
-        off_hl = (const float4 *)d_off;
+        im.count = I->count;
+        im.off = I->m;
+        off_hl = I->hl;
     }
     for (int k = 2; k <= 6; k++) phase_mark(c, k);
     S.raw = true;
@@ -521,7 +505,6 @@ sv_status direct_accel(sv_ctx *c) {
         SV_CK(c, launch_pairs(a, c->stream));
     }
     SV_LAUNCHED(c);
-    if (d_off) SV_CK(c, cudaFreeAsync(d_off, c->stream));
     const double pairs = (double)n * (double)n * (double)im.count;
     c->stats.pair_interactions = pairs;
     c->stats.cell_interactions = 0;

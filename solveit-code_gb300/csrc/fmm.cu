@@ -59,10 +59,9 @@ struct Fmm {
     unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue
     unsigned long long *h_counts = nullptr;
     // caller particles followed by their source-only symmetry images
-    double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr, *eoff = nullptr;
+    double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr;
     int32_t *est = nullptr;
     int64_t ecap = 0;
-    int eoff_cap = 0;
     int *has_tgt = nullptr;  // per box of every level: box holds a target
     int64_t tgt_cap = 0;
     float4 *rel = nullptr;   // particle offset from its leaf box centre (FP32) + charge
@@ -1959,7 +1958,7 @@ void fmm_free(sv_ctx *c) {
     cudaFree(F.cls_theta); cudaFree(F.cls_phase); cudaFree(F.cls_rho2); cudaFree(F.dmat);
     cudaFree(F.zc); cudaFree(F.nrm); cudaFree(F.otab); cudaFree(F.arena); cudaFree(F.d_counts);
     cudaFree(F.ex); cudaFree(F.ey); cudaFree(F.ez); cudaFree(F.eq); cudaFree(F.em); cudaFree(F.est);
-    cudaFree(F.eoff); cudaFree(F.has_tgt); cudaFree(F.rel); cudaFree(F.far);
+    cudaFree(F.has_tgt); cudaFree(F.rel); cudaFree(F.far);
     cudaFree(F.farena); cudaFree(F.frel);
     m2l_tc_free(F.tc);
     if (F.ftree) {
@@ -2003,24 +2002,16 @@ sv_status fmm_sort_images(sv_ctx *c, int64_t first, int64_t last) {
     Fmm &F = *c->fmm;
     const int64_t n = c->n;
     int kind = 0, nimg = 1;
-    std::vector<double> off;
+    const double *off = nullptr;
     if (c->P.symmetry == SV_SYM_ROTATIONAL) {
         kind = 1;
         nimg = 4;
     } else if (c->P.symmetry == SV_SYM_TRANSLATIONAL) {
+        const ImageSet *I = nullptr;
+        SV_TRY(image_set(c, &I));
         kind = 2;
-        std::vector<double> h(3 * 4096);
-        nimg = trans_images(c->P, h.data(), 4096);
-        if (nimg <= 0 || nimg > 4096) return set_error(c, SV_ERR_INVALID, "bad translational image set (%d)", nimg);
-        // the zero offset (the particles themselves) goes first
-        off.reserve(3 * nimg);
-        int zero = -1;
-        for (int g = 0; g < nimg; g++)
-            if (h[3 * g] == 0.0 && h[3 * g + 1] == 0.0 && h[3 * g + 2] == 0.0) zero = g;
-        if (zero < 0) return set_error(c, SV_ERR_INVALID, "image set without the zero offset");
-        off.insert(off.end(), {0.0, 0.0, 0.0});
-        for (int g = 0; g < nimg; g++)
-            if (g != zero) off.insert(off.end(), {h[3 * g], h[3 * g + 1], h[3 * g + 2]});
+        nimg = I->count;
+        off = I->zero_first;
     }
     const int64_t ne = n * nimg;
     if (ne > (int64_t)INT32_MAX) return set_error(c, SV_ERR_CAPACITY, "%lld particles with images", (long long)ne);
@@ -2036,19 +2027,8 @@ sv_status fmm_sort_images(sv_ctx *c, int64_t first, int64_t last) {
         SV_CK(c, cudaMalloc(&F.est, sizeof(int32_t) * ne));
         F.ecap = ne;
     }
-    if (kind == 2) {
-        if (F.eoff_cap < nimg) {
-            cudaFree(F.eoff);
-            F.eoff = nullptr;
-            SV_CK(c, cudaMalloc(&F.eoff, sizeof(double) * 3 * nimg));
-            F.eoff_cap = nimg;
-        }
-        SV_CK(c, cudaMemcpyAsync(F.eoff, off.data(), sizeof(double) * 3 * nimg, cudaMemcpyHostToDevice, c->stream));
-        // the host vector must outlive the copy
-        SV_CK(c, cudaStreamSynchronize(c->stream));
-    }
     expand_images_kernel<<<div_up(ne, 256), 256, 0, c->stream>>>(c->x, c->y, c->z, c->q, c->m, force_status(c), n, kind,
-                                                                 nimg, F.eoff, F.ex, F.ey, F.ez, F.eq, F.em, F.est);
+                                                                 nimg, off, F.ex, F.ey, F.ez, F.eq, F.em, F.est);
     SV_LAUNCHED(c);
     const ParticleView v{F.ex, F.ey, F.ez, F.eq, F.em, F.est, ne, n};
     return sort_view(c, v, first, last);

@@ -199,21 +199,23 @@ __device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
     return tgt ? a.kconst * (a.qom ? a.qom[i] : a.q[i] / a.m[i]) : 0.0;
 }
 
-// particle i into sorted slot s
+// particle i into sorted slot s (every load before the first store)
 __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s, uint32_t i) {
-    a.xs[s] = a.x[i];
-    a.ys[s] = a.y[i];
-    a.zs[s] = a.z[i];
-    a.qs[s] = sorted_charge(a, i);
-    a.qm[s] = sorted_qm(a, i);
+    const double x = a.x[i], y = a.y[i], z = a.z[i], k = sorted_qm(a, i);
+    const float q = sorted_charge(a, i);
+    a.xs[s] = x;
+    a.ys[s] = y;
+    a.zs[s] = z;
+    a.qs[s] = q;
+    a.qm[s] = k;
     if (a.zax) a.zax[s] = a.zay[s] = a.zaz[s] = 0.0;
     if (a.ph) {
         float4 h, l;
-        split_hilo(a.x[i] - (a.abs_xy ? 0.0 : a.root[0]), h.x, l.x);
-        split_hilo(a.y[i] - (a.abs_xy ? 0.0 : a.root[1]), h.y, l.y);
-        split_hilo(a.z[i] - a.root[2], h.z, l.z);
-        h.w = a.qs[s];
-        l.w = a.qm[s] != 0.0 ? 1.f : 0.f;
+        split_hilo(x - (a.abs_xy ? 0.0 : a.root[0]), h.x, l.x);
+        split_hilo(y - (a.abs_xy ? 0.0 : a.root[1]), h.y, l.y);
+        split_hilo(z - a.root[2], h.z, l.z);
+        h.w = q;
+        l.w = k != 0.0 ? 1.f : 0.f;
         a.ph[s] = h;
         a.pl[s] = l;
         if (h.w != sorted_charge(a, 0)) *a.differ = 1;

@@ -91,6 +91,19 @@ struct SubTable {
     double bt[kMaxSubLevels] = {};
 };
 
+// The translational image offsets of a context's parameters on the device, kept
+// while the parameters they follow from do (listing and sorting them on the host
+// and copying them took ~100 us per evaluation at 81 images).
+constexpr int kMaxImages = 4096;
+struct ImageSet {
+    int count = 0, levels = 0, axes[3] = {};
+    double domain[3] = {};
+    double *buf = nullptr;
+    const double *m = nullptr;           // 3 per image: metres, in the reference's summation order
+    const float4 *hl = nullptr;          // the same as FP32 hi and lo parts, two per image
+    const double *zero_first = nullptr;  // metres, the zero offset first
+};
+
 // energy bookkeeping of the reference's integrator (sv_set_energy, energy.cu)
 struct EnergyBook {
     int on = 0, init_steps = 0, steps = 0, interval = 1;
@@ -169,8 +182,11 @@ struct sv_ctx {
     // their join events, the last one the fork from the context's stream
     cudaStream_t cps[4] = {};
     cudaEvent_t cpe[5] = {};
-    double *h_accel = nullptr;    // page-locked host copy of the acceleration (sv_add_accel_ref32)
-    int64_t h_accel_cap = 0;      // doubles
+    // page-locked, mapped staging of small uploads; the event marks its last read
+    void *h_stage = nullptr;
+    size_t h_stage_bytes = 0;
+    cudaEvent_t h_stage_read = nullptr;
+    sv::ImageSet images{};        // translational images of the current parameters
     double *d_scalar = nullptr;   // device scratch for small reductions
     double *h_scalar = nullptr;   // pinned mirror
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
@@ -383,6 +399,9 @@ void energy_rearm(sv_ctx *c);
 
 // image offsets (metres) of the translational lattice, in summation order
 int trans_images(const sv_params &P, double *out, int max_out);
+// the context's image set for its parameters, on the device
+sv_status image_set(sv_ctx *c, const ImageSet **out);
+void images_free(sv_ctx *c);
 
 // constant memory copies per context are not used: parameters travel as
 // kernel arguments so that several contexts can share a device.
