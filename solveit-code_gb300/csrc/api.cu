@@ -1092,6 +1092,7 @@ sv_status sv::compute_accel_device(sv_ctx *c, int64_t first, int64_t last) {
         auto sort_all = [&](int levels) -> sv_status {
             c->S.want_levels = levels;
             if (c->P.method == SV_METHOD_DIRECT) direct_sort_wants(c);
+            else if (c->P.method == SV_METHOD_BARNES_HUT) bh_sort_wants(c);
             if (outliers) {
                 const ParticleView v{c->x, c->y, c->z, c->q, c->m, st2, c->n, c->n, c->qom};
                 return sort_view(c, v, first, last);

@@ -17,28 +17,27 @@
 //   * the octree is tree.cu's level structure built down to single-particle
 //     boxes; a box is a leaf of the walk when it holds <= leaf_size particles
 //     (the reference stops at one particle per leaf);
-//   * cell properties are reduced bottom-up, one kernel per level, in FP64;
+//   * cell properties are reduced bottom-up in FP64 in one launch: a CTA per box
+//     of a middle level takes its whole subtree, and the last one to finish the
+//     levels above;
 //   * node centres and particle positions are stored as FP32 (hi, lo) pairs
 //     relative to the root origin, so (target - centre) is formed as
 //     (t_hi - c_hi) + (t_lo - c_lo): FP64-like differences with FP32
 //     arithmetic only (the walk has no FP64 instruction);
-//   * the walk is warp-cooperative and stackless, over the tree threaded the
-//     way the reference threads its cells (nextSibling, cell.h:33-35,
-//     cell.cpp:171-172): every cell keeps a skip link to the next cell of
-//     the depth-first order outside its own subtree (its next sibling, else
-//     its parent's skip link).  A warp owns 32 Morton-consecutive targets
-//     and walks one cell at a time; each lane keeps one bit per level, set
-//     when it rejected the current ancestor at that level, so a lane takes
-//     part at a cell when it rejected the cell's parent.  Taking part, it
-//     applies its own acceptance test and adds the monopole when it
-//     accepts; when some lane rejects, the warp goes down to the first child
-//     (or, at a leaf, the rejecting lanes sum the leaf's particles
-//     directly), else it follows the skip link.  Each target gets exactly
-//     the cells its own walk would accept, the warp visits a cell at most
-//     once, and no stack bounds the depth.
+//   * the walk is warp-cooperative over batches of cells: a warp owns TPW
+//     Morton-consecutive targets and keeps a stack of (cell, mask of the targets
+//     that rejected its parent).  It takes up to 32 cells off the stack at a time,
+//     a lane loading each (one memory latency for 32 cells), then tests them one
+//     after the other (32 / TPW at a time) from shared memory with a target per
+//     lane: a target that accepts adds the monopole, the others' mask goes with
+//     the cell's children onto the stack, or with the particles of a leaf into a
+//     direct sum.  Each target gets exactly the cells its own walk would accept.
+//     The stack is bounded: near its end the warp takes one cell at a time, which
+//     adds at most seven entries per level.
+#include <algorithm>
 #include <cfloat>
 
-#include "sv_internal.cuh"
+#include "pairs.cuh"
 #include "tree.cuh"
 
 namespace sv {
@@ -46,9 +45,7 @@ namespace sv {
 struct Bh {
     void *arena = nullptr;
     size_t arena_bytes = 0;
-    float4 *ph = nullptr, *pl = nullptr;  // particle hi (xyz, q) and lo (xyz, 0)
-    int64_t pcap = 0;
-    unsigned long long *d_counts = nullptr;  // [0] accepted cells, [1] direct pairs
+    unsigned long long *d_counts = nullptr;  // [0] accepted cells, [1] direct pairs, [2] finished subtrees
     unsigned long long *h_counts = nullptr;
     int level_hint = -1;  // deepest level of the last tree
 };
@@ -56,50 +53,166 @@ struct Bh {
 namespace {
 
 constexpr int kBhWarps = 4;
-constexpr int kBhHalfWarps = 32;  // warps per SM below which the walk takes 16 targets per warp
 
-struct BhLevels {
-    const float4 *nh[kMortonBits + 1];  // centre hi (xyz) + net charge
-    const float4 *nl[kMortonBits + 1];  // centre lo (xyz) + delta
-    const int *child0[kMortonBits + 1];
-    const int *start[kMortonBits + 1];
-    const int *skip[kMortonBits + 1];   // next cell of the depth-first order outside the subtree, or kEnd
-    int deepest;
-    int leaf_size;
+// A cell of the walk: centre hi (xyz) and net charge, centre lo (xyz) and delta =
+// |centre - geometric centre|, and (first particle, particle count, first child,
+// children | level << 8); cells of all levels in one array, level by level.
+struct Cells {
+    float4 *hi, *lo;
+    int4 *link;
 };
 
-// a cell as (level << 24) | box, and the end of the walk
-constexpr int kEnd = -1;
-__host__ __device__ __forceinline__ int cell_id(int l, int b) { return (l << 24) | b; }
-
-// Skip links of every cell of levels 0..D, one thread per cell: its next
-// sibling (same parent), else the first ancestor's next sibling, else kEnd.
-struct SkipArgs {
-    const int *parent[kMortonBits + 1];
-    int *skip[kMortonBits + 1];
-    int nbox[kMortonBits + 1];
-    int first[kMortonBits + 2];  // first global cell of each level; first[D + 1] = all cells
-    int D;
+// Cell properties, level by level (reductions in FP64).
+struct PropLevel {
+    int nbox, first;   // boxes, and the level's first cell in Cells
+    const int *start, *child0;
+    const int4 *coord;
+    double *Q, *U;
+    double3 *coc;
+};
+struct PropArgs {
+    int deepest, top;  // top: the level with a CTA per box
+    PropLevel lv[kMortonBits + 1];
+    Cells cells;
+    const double *xs, *ys, *zs, *root;
+    const float *qs;
+    unsigned long long *done;
 };
 
-__global__ void skip_links_kernel(SkipArgs a) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= a.first[a.D + 1]) return;
-    int l = 0;
-    while (l < a.D && g >= a.first[l + 1]) l++;
-    const int b0 = g - a.first[l];
-    int lv = l, b = b0, out = kEnd;
-    for (;;) {
-        const bool sib = b + 1 < a.nbox[lv] && (lv == 0 || a.parent[lv][b + 1] == a.parent[lv][b]);
-        if (sib) {
-            out = cell_id(lv, b + 1);
-            break;
+// Properties of box b of level l (computeCellProperties :337-390): from its
+// particles at the deepest level, else from its children (:358-388): centre =
+// sum_c coc_c |Q_c| / sum_c U_c, the geometric centre when U = 0.
+__device__ __forceinline__ void props_box(const PropArgs &a, int l, int b) {
+    const PropLevel &V = a.lv[l];
+    const double side = a.root[3] / (double)(1ll << l);
+    const int s0 = V.start[b], s1 = V.start[b + 1];
+    double q = 0, u = 0, tx = 0, ty = 0, tz = 0;
+    int c0 = 0, c1 = 0;
+    if (l == a.deepest) {
+        // four particles' loads in flight at a time (as the children below)
+        for (int j = s0; j < s1; j += 4) {
+            float qj[4];
+            double x[4], y[4], z[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int jj = min(j + k, s1 - 1);
+                qj[k] = a.qs[jj];
+                x[k] = a.xs[jj];
+                y[k] = a.ys[jj];
+                z[k] = a.zs[jj];
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (j + k >= s1) break;
+                const double qd = widen(qj[k]), aq = fabs(qd);
+                q += qd;
+                u += aq;
+                tx += aq * (x[k] - a.root[0]);
+                ty += aq * (y[k] - a.root[1]);
+                tz += aq * (z[k] - a.root[2]);
+            }
         }
-        if (lv == 0) break;
-        b = a.parent[lv][b];
-        lv--;
+    } else {
+        const PropLevel &C = a.lv[l + 1];
+        c0 = V.child0[b];
+        c1 = V.child0[b + 1];
+        for (int c = c0; c < c1; c += 4) {
+            double qc[4], uc[4], x[4], y[4], z[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int cc = min(c + k, c1 - 1);
+                qc[k] = __ldcg(&C.Q[cc]);
+                uc[k] = __ldcg(&C.U[cc]);
+                const double *p = reinterpret_cast<const double *>(C.coc + cc);
+                x[k] = __ldcg(p);
+                y[k] = __ldcg(p + 1);
+                z[k] = __ldcg(p + 2);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (c + k >= c1) break;
+                const double w = fabs(qc[k]);
+                q += qc[k];
+                u += uc[k];
+                tx += x[k] * w;
+                ty += y[k] * w;
+                tz += z[k] * w;
+            }
+        }
     }
-    a.skip[l][b0] = out;
+    const int4 cb = V.coord[b];
+    // box coordinates are below 2^21: exact in FP32
+    const double gx = widen((float)cb.x + 0.5f) * side, gy = widen((float)cb.y + 0.5f) * side,
+                 gz = widen((float)cb.z + 0.5f) * side;
+    double cx = gx, cy = gy, cz = gz;
+    if (u != 0.0) {
+        // 1 / u = y^2 / (1 - e) with e = 1 - u y^2, |e| < 4e-7, to third order
+        double r;
+        if (u > 1e-30 && u < 1e30) {
+            const double y = rsqrt_seed_f64(u), y2 = y * y, e = fma(-u, y2, 1.0);
+            r = fma(y2, fma(e, e, e), y2);
+        } else {
+            r = 1.0 / u;
+        }
+        cx = tx * r;
+        cy = ty * r;
+        cz = tz * r;
+    }
+    V.Q[b] = q;
+    V.U[b] = u;
+    V.coc[b] = make_double3(cx, cy, cz);
+    const double dx = cx - gx, dy = cy - gy, dz = cz - gz;
+    const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    // sqrt to beyond the FP32 it is stored in: d2 y (1 + (1 - d2 y^2) / 2)
+    const double y = rsqrt_seed_f64(d2), dy0 = d2 * y;
+    float4 h, lo;
+    split_hilo_bits(cx, h.x, lo.x);
+    split_hilo_bits(cy, h.y, lo.y);
+    split_hilo_bits(cz, h.z, lo.z);
+    h.w = (float)q;
+    lo.w = (float)fma(dy0, 0.5 * fma(-dy0, y, 1.0), dy0);
+    const int g = V.first + b;
+    a.cells.hi[g] = h;
+    a.cells.lo[g] = lo;
+    a.cells.link[g] = make_int4(s0, s1 - s0, l < a.deepest ? a.lv[l + 1].first + c0 : 0, (c1 - c0) | (l << 8));
+}
+
+// One CTA per box of level `top`: the boxes of its subtree are contiguous at every
+// level; deepest level first, then up to the box itself.  The last CTA to finish
+// takes the levels above.  One launch for all levels, over as many SMs as the
+// middle level has boxes: one launch per fine level and a single CTA for every
+// level of up to 1,024 boxes took 85 us at 65,536 ions, this 67.
+constexpr int kPropThreads = 128;
+constexpr int kPropTop = 256;  // the middle level: the deepest of up to this many boxes
+__global__ void __launch_bounds__(kPropThreads) props_kernel(PropArgs a) {
+    __shared__ int lo[kMortonBits + 1], hi[kMortonBits + 1];
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        int x = blockIdx.x, y = x + 1;
+        for (int l = a.top;; l++) {
+            lo[l] = x;
+            hi[l] = y;
+            if (l == a.deepest) break;
+            x = a.lv[l].child0[x];
+            y = a.lv[l].child0[y];
+        }
+    }
+    __syncthreads();
+    for (int l = a.deepest; l >= a.top; l--) {
+        for (int b = lo[l] + threadIdx.x; b < hi[l]; b += kPropThreads) props_box(a, l, b);
+        __syncthreads();
+    }
+    if (a.top == 0) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.done, 1ull) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int l = a.top - 1; l >= 0; l--) {
+        for (int b = threadIdx.x; b < a.lv[l].nbox; b += kPropThreads) props_box(a, l, b);
+        __syncthreads();
+    }
 }
 
 struct BhImages {
@@ -108,249 +221,211 @@ struct BhImages {
     const double *off;
 };
 
-__global__ void particles_hilo(const double *__restrict__ xs, const double *__restrict__ ys,
-                               const double *__restrict__ zs, const float *__restrict__ qs, int n,
-                               const double *__restrict__ root, float4 *__restrict__ ph, float4 *__restrict__ pl) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float hx, lx, hy, ly, hz, lz;
-    split_hilo(xs[i] - root[0], hx, lx);
-    split_hilo(ys[i] - root[1], hy, ly);
-    split_hilo(zs[i] - root[2], hz, lz);
-    ph[i] = make_float4(hx, hy, hz, qs[i]);
-    pl[i] = make_float4(lx, ly, lz, 0.f);
-}
-
-// deepest level: properties straight from the particles of each box
-__global__ void props_from_particles(int nbox, const int *__restrict__ start, const int4 *__restrict__ coord,
-                                     const double *__restrict__ xs, const double *__restrict__ ys,
-                                     const double *__restrict__ zs, const float *__restrict__ qs,
-                                     const double *__restrict__ root, int level, double *__restrict__ Q,
-                                     double *__restrict__ U, double3 *__restrict__ coc, float4 *__restrict__ nh,
-                                     float4 *__restrict__ nl) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nbox) return;
-    const double side = root[3] / (double)(1ll << level);
-    double q = 0, u = 0, cx = 0, cy = 0, cz = 0;
-    for (int j = start[b]; j < start[b + 1]; j++) {
-        const double qj = qs[j], aq = fabs(qj);
-        q += qj;
-        u += aq;
-        cx += aq * (xs[j] - root[0]);
-        cy += aq * (ys[j] - root[1]);
-        cz += aq * (zs[j] - root[2]);
-    }
-    const int4 c = coord[b];
-    const double gx = (c.x + 0.5) * side, gy = (c.y + 0.5) * side, gz = (c.z + 0.5) * side;
-    if (u != 0.0) {
-        cx /= u;
-        cy /= u;
-        cz /= u;
-    } else {
-        cx = gx;
-        cy = gy;
-        cz = gz;
-    }
-    Q[b] = q;
-    U[b] = u;
-    coc[b] = make_double3(cx, cy, cz);
-    const double dx = cx - gx, dy = cy - gy, dz = cz - gz;
-    float hx, lx, hy, ly, hz, lz;
-    split_hilo(cx, hx, lx);
-    split_hilo(cy, hy, ly);
-    split_hilo(cz, hz, lz);
-    nh[b] = make_float4(hx, hy, hz, (float)q);
-    nl[b] = make_float4(lx, ly, lz, (float)sqrt(dx * dx + dy * dy + dz * dz));
-}
-
-// coarser levels from their children (computeCellProperties :358-388):
-// centre = sum_c coc_c |Q_c| / sum_c U_c, geometric centre when U = 0
-struct PropLevel {
-    int nbox;
-    const int *child0;
-    const int4 *coord;
-    double *Q, *U;
-    double3 *coc;
-    float4 *nh, *nl;
+struct WalkArgs {
+    Cells cells;
+    int deepest, leaf_size;
+    const float4 *ph, *pl;   // sorted particles hi (xyz, charge) and lo (xyz, 1 = target)
+    const double *xs, *ys, *zs, *qm;
+    int n;
+    const double *root;
+    float theta, eps2;
+    BhImages im;
+    double *ax, *ay, *az;    // stored (one image), or added into (more)
+    unsigned long long *counts;
 };
 
-__device__ __forceinline__ void props_box(int b, int level, const double *__restrict__ root, const PropLevel &C,
-                                          const PropLevel &V) {
-    const double side = root[3] / (double)(1ll << level);
-    double q = 0, u = 0, tx = 0, ty = 0, tz = 0;
-    for (int c = V.child0[b]; c < V.child0[b + 1]; c++) {
-        const double qc = C.Q[c], w = fabs(qc);
-        q += qc;
-        u += C.U[c];
-        const double3 p = C.coc[c];
-        tx += p.x * w;
-        ty += p.y * w;
-        tz += p.z * w;
-    }
-    const int4 cb = V.coord[b];
-    const double gx = (cb.x + 0.5) * side, gy = (cb.y + 0.5) * side, gz = (cb.z + 0.5) * side;
-    double cx = gx, cy = gy, cz = gz;
-    if (u != 0.0) {
-        cx = tx / u;
-        cy = ty / u;
-        cz = tz / u;
-    }
-    V.Q[b] = q;
-    V.U[b] = u;
-    V.coc[b] = make_double3(cx, cy, cz);
-    const double dx = cx - gx, dy = cy - gy, dz = cz - gz;
-    float hx, lx, hy, ly, hz, lz;
-    split_hilo(cx, hx, lx);
-    split_hilo(cy, hy, ly);
-    split_hilo(cz, hz, lz);
-    V.nh[b] = make_float4(hx, hy, hz, (float)q);
-    V.nl[b] = make_float4(lx, ly, lz, (float)sqrt(dx * dx + dy * dy + dz * dz));
-}
+constexpr int kStack = 512;                      // entries per warp
+constexpr int kStackTail = 7 * kMortonBits + 8;  // room that one cell at a time can need
 
-// one level from the level below it, one thread per box
-__global__ void props_from_children(int level, const double *__restrict__ root, PropLevel C, PropLevel V) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < V.nbox) props_box(b, level, root, C, V);
-}
-
-// Levels top .. 0 in one CTA, level by level (coarse levels have few boxes,
-// and one launch per level made each of them a launch's latency).
-struct PropLevels {
-    PropLevel lv[kMortonBits + 1];
+struct WalkShared {
+    uint2 stack[kStack];      // cell, targets (bit per target)
+    float4 hi[32], lo[32];    // the batch's cells, or 32 particles of its opened leaves
+    float side[32];
+    uint32_t mask[32];
+    int idx[32];              // particles: sorted slot
+    int leaf_at[32];          // first particle slot of each opened leaf of the batch
+    int2 leaf[32];            // its particle range
+    uint32_t leaf_mask[32];
 };
-__global__ void props_coarse_levels(int top, const double *__restrict__ root, PropLevels P) {
-    for (int l = top; l >= 0; l--) {
-        for (int b = threadIdx.x; b < P.lv[l].nbox; b += blockDim.x) props_box(b, l, root, P.lv[l + 1], P.lv[l]);
-        __syncthreads();
-    }
+
+// 1/sqrt(x), refined by one Newton step (the hardware's approximation alone is
+// off by up to two units in the last place)
+__device__ __forceinline__ float rsqrt_refined(float x) {
+    const float y = rsqrt_ftz(x);
+    const float r = y * fmaf(-0.5f * x * y, y, 1.5f);
+    return y > 0.f && y <= FLT_MAX ? r : y;  // x beyond FP32, or zero
 }
 
-// TPW targets per warp: 32, or 16 with the two half-warps sharing each
-// target (both take the same acceptance decisions, the lower half adds the
-// accepted cells, the halves split each opened leaf's particles and add their
-// sums at the end): twice the warps for a small plume, each walking the union
-// of fewer targets' cells.
+// TPW targets per warp; with fewer than 32, 32 / TPW groups of lanes share the
+// targets and take different cells and particles.  blockIdx.y: the symmetry image.
 template <int TPW>
-__global__ void __launch_bounds__(kBhWarps * 32)
-bh_walk_kernel(BhLevels T, const float4 *__restrict__ ph, const float4 *__restrict__ pl,
-               const double *__restrict__ xs, const double *__restrict__ ys, const double *__restrict__ zs,
-               const double *__restrict__ qm, int n, const double *__restrict__ root, float theta, float eps2,
-               BhImages im, double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-               unsigned long long *__restrict__ counts) {
-    // cell side of every level, from the root cube on the device
-    __shared__ float side[kMortonBits + 1];
-    if (threadIdx.x <= T.deepest) side[threadIdx.x] = (float)(root[3] / (double)(1ll << threadIdx.x));
+__global__ void __launch_bounds__(kBhWarps * 32) bh_walk_kernel(WalkArgs a) {
+    constexpr int G = 32 / TPW;
+    constexpr uint32_t kAll = TPW == 32 ? 0xffffffffu : (1u << TPW) - 1u;
+    __shared__ float side[kMortonBits + 1];  // cell side of every level, from the root cube on the device
+    __shared__ WalkShared sh_all[kBhWarps];
+    if (threadIdx.x <= a.deepest) side[threadIdx.x] = (float)(a.root[3] / (double)(1ll << threadIdx.x));
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int half = lane / TPW;  // 0, or 1 for the upper half-warp when TPW = 16
-    const int i = (blockIdx.x * kBhWarps + wid) * TPW + lane % TPW;
-    const bool live = i < n && qm[i] != 0.0;
-    const unsigned live_mask = __ballot_sync(0xffffffffu, live);
+    WalkShared &sh = sh_all[wid];
+    const int tl = lane % TPW, grp = lane / TPW;
+    const int i = (blockIdx.x * kBhWarps + wid) * TPW + tl;
+    const bool live = i < a.n && a.qm[i] != 0.0;
+    const uint32_t live_mask = __ballot_sync(0xffffffffu, live) & kAll;
     if (live_mask == 0) return;
-    const int ii = i < n ? i : n - 1;
-    const double px = xs[ii], py = ys[ii], pz = zs[ii];
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    unsigned long long n_cells = 0, n_pairs = 0;
-    for (int g = 0; g < im.count; g++) {
-        // target position in this image's frame, and the force rotation back
-        double tx = px, ty = py, tz = pz;
-        int cb = 1, sb = 0;
-        bool self_excl = true;
-        if (im.kind == 1) {
-            // quadrant g: target rotated by -g*pi/2, force rotated by +g*pi/2
-            const int cf = (g == 0) ? 1 : (g == 2 ? -1 : 0);
-            const int sf = (g == 1) ? -1 : (g == 3 ? 1 : 0);
-            tx = cf * px - sf * py;
-            ty = sf * px + cf * py;
-            cb = cf;
-            sb = -sf;
-            self_excl = g == 0;
-        } else if (im.kind == 2) {
-            tx = px - im.off[3 * g];
-            ty = py - im.off[3 * g + 1];
-            tz = pz - im.off[3 * g + 2];
-            self_excl = im.off[3 * g] == 0.0 && im.off[3 * g + 1] == 0.0 && im.off[3 * g + 2] == 0.0;
+    const int ii = i < a.n ? i : a.n - 1;
+    // target position in this image's frame, and the force rotation back
+    const int g = blockIdx.y;
+    double tx = a.xs[ii], ty = a.ys[ii], tz = a.zs[ii];
+    int cb = 1, sb = 0;
+    bool self_excl = true;
+    if (a.im.kind == 1) {
+        // quadrant g: target rotated by -g*pi/2, force rotated by +g*pi/2
+        const int cf = (g == 0) ? 1 : (g == 2 ? -1 : 0);
+        const int sf = (g == 1) ? -1 : (g == 3 ? 1 : 0);
+        const double px = tx, py = ty;
+        tx = cf * px - sf * py;
+        ty = sf * px + cf * py;
+        cb = cf;
+        sb = -sf;
+        self_excl = g == 0;
+    } else if (a.im.kind == 2) {
+        const double *off = a.im.off + 3 * g;
+        tx -= off[0];
+        ty -= off[1];
+        tz -= off[2];
+        self_excl = off[0] == 0.0 && off[1] == 0.0 && off[2] == 0.0;
+    }
+    float thx, tlx, thy, tly, thz, tlz;
+    split_hilo(tx - a.root[0], thx, tlx);
+    split_hilo(ty - a.root[1], thy, tly);
+    split_hilo(tz - a.root[2], thz, tlz);
+    const int self = self_excl ? i : -1;
+    float fx = 0.f, fy = 0.f, fz = 0.f;
+    unsigned n_cells = 0, n_pairs = 0;
+    if (lane == 0) sh.stack[0] = make_uint2(0u, live_mask);
+    int size = 1;
+    __syncwarp();
+    while (size > 0) {
+        // as many cells as the stack has room for their children
+        const int room = (kStack - kStackTail - size) / 7;
+        const int nb = min(min(32, size), max(1, room));
+        size -= nb;
+        uint32_t rej = 0;
+        int4 link = make_int4(0, 0, 0, 0);
+        if (lane < nb) {
+            const uint2 e = sh.stack[size + lane];
+            link = a.cells.link[e.x];
+            sh.hi[lane] = a.cells.hi[e.x];
+            sh.lo[lane] = a.cells.lo[e.x];
+            sh.side[lane] = side[link.w >> 8];
+            sh.mask[lane] = e.y;
         }
-        float thx, tlx, thy, tly, thz, tlz;
-        split_hilo(tx - root[0], thx, tlx);
-        split_hilo(ty - root[1], thy, tly);
-        split_hilo(tz - root[2], thz, tlz);
-        float fx = 0.f, fy = 0.f, fz = 0.f;
-        unsigned want = 0;  // bit l: this lane rejected the current cell's ancestor at level l
-        int node = cell_id(0, 0);
-        while (node != kEnd) {
-            const int lvl = node >> 24, b = node & 0xffffff;
-            // taking part: the root for every live target, else the lanes that rejected the parent
-            const bool mine = lvl == 0 ? live : ((want >> (lvl - 1)) & 1u) != 0;
-            // everything the cell's visit may need, loaded together: one memory
-            // latency per cell instead of a chain of three
-            const float4 h = T.nh[lvl][b], lo = T.nl[lvl][b];
-            const int s0 = T.start[lvl][b], s1 = T.start[lvl][b + 1];
-            const int child = lvl < T.deepest ? T.child0[lvl][b] : 0, skip = T.skip[lvl][b];
-            bool deeper = false, rej = false;
-            if (__any_sync(0xffffffffu, mine)) {
-                const float dx = (thx - h.x) + (tlx - lo.x), dy = (thy - h.y) + (tly - lo.y),
-                            dz = (thz - h.z) + (tlz - lo.z);
-                const float d = sqrtf(fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2))));
-                const bool acc = mine && theta * (d - lo.w) > side[lvl];
-                if (acc && half == 0) {
-                    const float f = h.w / (d * d * d);
-                    fx = fmaf(f, dx, fx);
-                    fy = fmaf(f, dy, fy);
-                    fz = fmaf(f, dz, fz);
-                    n_cells++;
+        __syncwarp();
+        for (int k0 = 0; k0 < nb; k0 += G) {
+            const int k = G == 1 ? k0 : min(k0 + grp, nb - 1);
+            const float4 h = sh.hi[k], lo = sh.lo[k];
+            const bool mine = (sh.mask[k] >> tl & 1u) && (G == 1 || k0 + grp < nb);
+            const float dx = (thx - h.x) + (tlx - lo.x), dy = (thy - h.y) + (tly - lo.y),
+                        dz = (thz - h.z) + (tlz - lo.z);
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, a.eps2)));
+            const float inv = rsqrt_refined(r2);
+            const bool acc = mine && a.theta * (r2 * inv - lo.w) > sh.side[k];
+            if (acc) {
+                const float f = h.w * (inv * inv * inv);
+                fx = fmaf(f, dx, fx);
+                fy = fmaf(f, dy, fy);
+                fz = fmaf(f, dz, fz);
+                n_cells++;
+            }
+            const uint32_t bal = __ballot_sync(0xffffffffu, mine && !acc);
+            if (lane >= k0 && lane < k0 + G) rej = (bal >> ((lane - k0) * TPW)) & kAll;
+        }
+        // rejected cells: an internal one's children onto the stack
+        const int level = link.w >> 8;
+        const bool leaf = rej != 0 && (level == a.deepest || link.y <= a.leaf_size);
+        const int nch = rej != 0 && !leaf ? link.w & 0xff : 0;
+        int inc = nch;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        for (int c = 0; c < nch; c++) sh.stack[size + inc - nch + c] = make_uint2((uint32_t)(link.z + c), rej);
+        size += __shfl_sync(0xffffffffu, inc, 31);
+        // the leaves' particles, laid end to end, 32 at a time
+        const uint32_t leaves = __ballot_sync(0xffffffffu, leaf);
+        if (leaves) {
+            int pinc = leaf ? link.y : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, pinc, o);
+                if (lane >= o) pinc += t;
+            }
+            const int total = __shfl_sync(0xffffffffu, pinc, 31), nleaf = __popc(leaves);
+            if (leaf) {
+                const int r = __popc(leaves & ((1u << lane) - 1u));
+                sh.leaf_at[r] = pinc - link.y;
+                sh.leaf[r] = make_int2(link.x, link.y);
+                sh.leaf_mask[r] = rej;
+            }
+            __syncwarp();
+            int at = 0;  // the lane's current leaf: lanes walk forward
+            for (int p0 = 0; p0 < total; p0 += 32) {
+                const int p = p0 + lane, np = min(32, total - p0);
+                if (p < total) {
+                    while (at + 1 < nleaf && sh.leaf_at[at + 1] <= p) at++;
+                    const int j = sh.leaf[at].x + (p - sh.leaf_at[at]);
+                    sh.hi[lane] = a.ph[j];
+                    sh.lo[lane] = a.pl[j];
+                    sh.idx[lane] = j;
+                    sh.mask[lane] = sh.leaf_mask[at];
                 }
-                rej = mine && !acc;
-                if (__any_sync(0xffffffffu, rej)) {
-                    const bool leaf = lvl == T.deepest || (s1 - s0) <= T.leaf_size;
-                    if (leaf) {
-#pragma unroll 4
-                        for (int j = s0 + half; j < s1; j += 32 / TPW) {
-                            const float4 qh = ph[j], ql = pl[j];
-                            if (rej && !(self_excl && j == i)) {
-                                const float ex = (thx - qh.x) + (tlx - ql.x), ey = (thy - qh.y) + (tly - ql.y),
-                                            ez = (thz - qh.z) + (tlz - ql.z);
-                                const float dd = sqrtf(fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, eps2))));
-                                const float f = qh.w / (dd * dd * dd);
-                                fx = fmaf(f, ex, fx);
-                                fy = fmaf(f, ey, fy);
-                                fz = fmaf(f, ez, fz);
-                                n_pairs++;
-                            }
-                        }
-                    } else {
-                        deeper = true;  // warp-uniform: the cell is internal and some lane rejected it
+                __syncwarp();
+#pragma unroll 2
+                for (int k0 = 0; k0 < np; k0 += G) {
+                    const int k = G == 1 ? k0 : min(k0 + grp, np - 1);
+                    if ((sh.mask[k] >> tl & 1u) && sh.idx[k] != self && (G == 1 || k0 + grp < np)) {
+                        const float4 qh = sh.hi[k], ql = sh.lo[k];
+                        const float ex = (thx - qh.x) + (tlx - ql.x), ey = (thy - qh.y) + (tly - ql.y),
+                                    ez = (thz - qh.z) + (tlz - ql.z);
+                        const float inv = rsqrt_refined(fmaf(ex, ex, fmaf(ey, ey, fmaf(ez, ez, a.eps2))));
+                        const float f = qh.w * (inv * inv * inv);
+                        fx = fmaf(f, ex, fx);
+                        fy = fmaf(f, ey, fy);
+                        fz = fmaf(f, ez, fz);
+                        n_pairs++;
                     }
                 }
+                __syncwarp();
             }
-            // bit lvl: this lane goes below this cell (it rejected an internal cell)
-            want = (deeper && rej) ? (want | (1u << lvl)) : (want & ~(1u << lvl));
-            node = deeper ? cell_id(lvl + 1, child) : skip;
         }
-        sx += (float)cb * fx - (float)sb * fy;
-        sy += (float)sb * fx + (float)cb * fy;
-        sz += fz;
+        __syncwarp();
     }
-    if (TPW == 16) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, 16);
-        sy += __shfl_xor_sync(0xffffffffu, sy, 16);
-        sz += __shfl_xor_sync(0xffffffffu, sz, 16);
+    float sx = (float)cb * fx - (float)sb * fy, sy = (float)sb * fx + (float)cb * fy, sz = fz;
+#pragma unroll
+    for (int o = 16; o >= TPW; o >>= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        sz += __shfl_xor_sync(0xffffffffu, sz, o);
     }
-    if (half == 0 && live) {
-        const double c = qm[i];
-        ax[i] = (double)sx * c;
-        ay[i] = (double)sy * c;
-        az[i] = (double)sz * c;
-    } else if (half == 0 && i < n) {
-        ax[i] = ay[i] = az[i] = 0.0;
+    if (grp == 0 && live) {
+        const double c = a.qm[i];
+        if (a.im.count == 1) {
+            a.ax[i] = (double)sx * c;
+            a.ay[i] = (double)sy * c;
+            a.az[i] = (double)sz * c;
+        } else {
+            atomicAdd(&a.ax[i], (double)sx * c);
+            atomicAdd(&a.ay[i], (double)sy * c);
+            atomicAdd(&a.az[i], (double)sz * c);
+        }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        n_cells += __shfl_xor_sync(0xffffffffu, n_cells, o);
-        n_pairs += __shfl_xor_sync(0xffffffffu, n_pairs, o);
-    }
+    n_cells = __reduce_add_sync(0xffffffffu, n_cells);
+    n_pairs = __reduce_add_sync(0xffffffffu, n_pairs);
     if (lane == 0) {
-        atomicAdd(&counts[0], n_cells);
-        atomicAdd(&counts[1], n_pairs);
+        atomicAdd(&a.counts[0], (unsigned long long)n_cells);
+        atomicAdd(&a.counts[1], (unsigned long long)n_pairs);
     }
 }
 
@@ -361,7 +436,7 @@ sv_status bh_accel(sv_ctx *c) {
         return set_error(c, SV_ERR_UNSUPPORTED, "Barnes-Hut runs in mixed precision only");
     if (!c->bh) {
         c->bh = new Bh();
-        SV_CK(c, cudaMalloc(&c->bh->d_counts, 2 * sizeof(unsigned long long)));
+        SV_CK(c, cudaMalloc(&c->bh->d_counts, 3 * sizeof(unsigned long long)));
         SV_CK(c, cudaMallocHost(&c->bh->h_counts, 2 * sizeof(unsigned long long)));
     }
     Bh &B = *c->bh;
@@ -379,22 +454,24 @@ sv_status bh_accel(sv_ctx *c) {
     }
     phase_mark(c, 2);
     phase_mark(c, 3);
+    SV_CK(c, cudaMemsetAsync(B.d_counts, 0, 3 * sizeof(unsigned long long), c->stream));
     if (T.n_act == 0) {
-        SV_CK(c, cudaMemsetAsync(S.ax, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.ay, 0, sizeof(double) * n, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.az, 0, sizeof(double) * n, c->stream));
+        // no source: nothing acts on anything (the scatter writes zeros for non-targets, and targets are sources)
+        SV_CK(c, cudaMemcpyAsync(B.h_counts, B.d_counts, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                 c->stream));
         return SV_OK;
     }
     const int D = T.deepest;
     B.level_hint = D;
-    // storage: per level Q, U (double), coc (double3), nh, nl (float4), skip links (int)
+    // storage: cells of every level, then per level Q, U (double), coc (double3)
     auto rounded = [](size_t sz) { return (sz + 255) & ~(size_t)255; };
-    size_t bytes = 0;
+    size_t cells = 0, bytes = 0;
     for (int l = 0; l <= D; l++) {
         const size_t nb = T.lv[l].nbox;
-        bytes += 2 * rounded(nb * sizeof(double)) + rounded(nb * sizeof(double3)) + 2 * rounded(nb * sizeof(float4)) +
-                 rounded(nb * sizeof(int));
+        cells += nb;
+        bytes += 2 * rounded(nb * sizeof(double)) + rounded(nb * sizeof(double3));
     }
+    bytes += 3 * rounded(cells * sizeof(float4));
     if (B.arena_bytes < bytes) {
         cudaFree(B.arena);
         B.arena = nullptr;
@@ -403,71 +480,34 @@ sv_status bh_accel(sv_ctx *c) {
         SV_CK(c, cudaMalloc(&B.arena, want));
         B.arena_bytes = want;
     }
-    if (B.pcap < n) {
-        cudaFree(B.ph);
-        cudaFree(B.pl);
-        B.ph = B.pl = nullptr;
-        SV_CK(c, cudaMalloc(&B.ph, sizeof(float4) * n));
-        SV_CK(c, cudaMalloc(&B.pl, sizeof(float4) * n));
-        B.pcap = n;
-    }
     char *p = (char *)B.arena;
     auto carve = [&](size_t sz) {
         char *r = p;
         p += rounded(sz);
         return (void *)r;
     };
-    double *Q[kMortonBits + 1], *U[kMortonBits + 1];
-    double3 *coc[kMortonBits + 1];
-    BhLevels L{};
-    SkipArgs sk{};
-    sk.D = D;
+    PropArgs pa{};
+    pa.deepest = D;
+    pa.cells.hi = (float4 *)carve(cells * sizeof(float4));
+    pa.cells.lo = (float4 *)carve(cells * sizeof(float4));
+    pa.cells.link = (int4 *)carve(cells * sizeof(int4));
+    int first = 0;
     for (int l = 0; l <= D; l++) {
         const size_t nb = T.lv[l].nbox;
-        Q[l] = (double *)carve(nb * sizeof(double));
-        U[l] = (double *)carve(nb * sizeof(double));
-        coc[l] = (double3 *)carve(nb * sizeof(double3));
-        L.nh[l] = (const float4 *)carve(nb * sizeof(float4));
-        L.nl[l] = (const float4 *)carve(nb * sizeof(float4));
-        L.child0[l] = T.lv[l].child0;
-        L.start[l] = T.lv[l].start;
-        sk.skip[l] = (int *)carve(nb * sizeof(int));
-        L.skip[l] = sk.skip[l];
-        sk.parent[l] = T.lv[l].parent;
-        sk.nbox[l] = (int)nb;
-        sk.first[l + 1] = sk.first[l] + (int)nb;
+        double *Q = (double *)carve(nb * sizeof(double)), *U = (double *)carve(nb * sizeof(double));
+        pa.lv[l] = PropLevel{(int)nb, first, T.lv[l].start, T.lv[l].child0, T.lv[l].coord, Q, U,
+                             (double3 *)carve(nb * sizeof(double3))};
+        first += (int)nb;
+        if (l == 0 || nb <= kPropTop) pa.top = l;
     }
-    skip_links_kernel<<<div_up(sk.first[D + 1], 256), 256, 0, c->stream>>>(sk);
+    pa.xs = S.x;
+    pa.ys = S.y;
+    pa.zs = S.z;
+    pa.qs = S.q;
+    pa.root = S.root;
+    pa.done = B.d_counts + 2;
+    props_kernel<<<pa.lv[pa.top].nbox, kPropThreads, 0, c->stream>>>(pa);
     SV_LAUNCHED(c);
-    L.deepest = D;
-    L.leaf_size = c->P.leaf_size;
-    particles_hilo<<<div_up(T.n_act, 256), 256, 0, c->stream>>>(S.x, S.y, S.z, S.q, T.n_act, S.root, B.ph, B.pl);
-    SV_LAUNCHED(c);
-    {
-        const Level &V = T.lv[D];
-        props_from_particles<<<div_up(V.nbox, 128), 128, 0, c->stream>>>(
-            V.nbox, V.start, V.coord, S.x, S.y, S.z, S.q, S.root, D, Q[D], U[D], coc[D], (float4 *)L.nh[D],
-            (float4 *)L.nl[D]);
-        SV_LAUNCHED(c);
-    }
-    {
-        PropLevels pl{};
-        for (int l = 0; l <= D; l++)
-            pl.lv[l] = PropLevel{T.lv[l].nbox, T.lv[l].child0, T.lv[l].coord, Q[l], U[l], coc[l],
-                                 (float4 *)L.nh[l], (float4 *)L.nl[l]};
-        // the coarse levels (every level above holding at most kCoarseBoxes boxes) in one launch
-        constexpr int kCoarseBoxes = 1024;
-        int top = -1;
-        while (top + 1 < D && T.lv[top + 1].nbox <= kCoarseBoxes) top++;
-        for (int l = D - 1; l > top; l--) {
-            props_from_children<<<div_up(T.lv[l].nbox, 128), 128, 0, c->stream>>>(l, S.root, pl.lv[l + 1], pl.lv[l]);
-            SV_LAUNCHED(c);
-        }
-        if (top >= 0) {
-            props_coarse_levels<<<1, kCoarseBoxes, 0, c->stream>>>(top, S.root, pl);
-            SV_LAUNCHED(c);
-        }
-    }
     phase_mark(c, 4);
     phase_mark(c, 5);
     BhImages im{0, 1, nullptr};
@@ -481,23 +521,21 @@ sv_status bh_accel(sv_ctx *c) {
         im.count = I->count;
         im.off = I->m;
     }
-    SV_CK(c, cudaMemsetAsync(B.d_counts, 0, 2 * sizeof(unsigned long long), c->stream));
+    // Targets per warp: 32 from 32 such warps per SM on, 16 from 8, else 8 (more
+    // warps, each walking the union of fewer targets' cells).  us per evaluation
+    // with 32 / 16 / 8: 1,500 ions 230 / 191 / 168, 16,000 277 / 239 / 213, 65,536
+    // 392 / 374 / 374, 300,000 751 / 777 / 827.
     // inactive sorted slots (beyond n_act) are never targets (qm = 0)
-    // half-warp targets while 32 per warp would leave fewer than kBhHalfWarps warps per SM
-    if (div_up(n, 32) < kBhHalfWarps * device_sms())
-        bh_walk_kernel<16><<<div_up(n, 16 * kBhWarps), 32 * kBhWarps, 0, c->stream>>>(
-            L, B.ph, B.pl, S.x, S.y, S.z, S.qm, T.n_act, S.root, c->P.theta, (float)c->P.softening2, im, S.ax, S.ay,
-            S.az, B.d_counts);
-    else
-        bh_walk_kernel<32><<<div_up(n, 32 * kBhWarps), 32 * kBhWarps, 0, c->stream>>>(
-            L, B.ph, B.pl, S.x, S.y, S.z, S.qm, T.n_act, S.root, c->P.theta, (float)c->P.softening2, im, S.ax, S.ay,
-            S.az, B.d_counts);
+    const WalkArgs wa{pa.cells, D, c->P.leaf_size, S.ph, S.pl, S.x, S.y, S.z, S.qm, T.n_act, S.root, c->P.theta,
+                      (float)c->P.softening2, im, S.ax, S.ay, S.az, B.d_counts};
+    auto walk = [&](auto kernel, int tpw) {
+        kernel<<<dim3(div_up(T.n_act, tpw * kBhWarps), im.count), 32 * kBhWarps, 0, c->stream>>>(wa);
+    };
+    const int64_t warps = (int64_t)div_up(T.n_act, 32) * im.count;
+    if (warps >= 32 * (int64_t)device_sms()) walk(bh_walk_kernel<32>, 32);
+    else if (warps >= 8 * (int64_t)device_sms()) walk(bh_walk_kernel<16>, 16);
+    else walk(bh_walk_kernel<8>, 8);
     SV_LAUNCHED(c);
-    if (T.n_act < n) {
-        SV_CK(c, cudaMemsetAsync(S.ax + T.n_act, 0, sizeof(double) * (n - T.n_act), c->stream));
-        SV_CK(c, cudaMemsetAsync(S.ay + T.n_act, 0, sizeof(double) * (n - T.n_act), c->stream));
-        SV_CK(c, cudaMemsetAsync(S.az + T.n_act, 0, sizeof(double) * (n - T.n_act), c->stream));
-    }
     phase_mark(c, 6);
     // the counts reach the host with the stream; bh_counts reads them
     SV_CK(c, cudaMemcpyAsync(B.h_counts, B.d_counts, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
@@ -506,6 +544,12 @@ sv_status bh_accel(sv_ctx *c) {
     c->stats.boxes = 0;
     for (int l = 0; l <= D; l++) c->stats.boxes += T.lv[l].nbox;
     return SV_OK;
+}
+
+void bh_sort_wants(sv_ctx *c) {
+    c->S.want_hilo = true;
+    c->S.hl_abs = false;
+    c->S.want_zero = c->P.symmetry != SV_SYM_NONE;  // the images' forces are added up
 }
 
 int bh_sort_levels(const sv_ctx *c) {
@@ -528,8 +572,6 @@ void bh_free(sv_ctx *c) {
     if (!c->bh) return;
     Bh &B = *c->bh;
     cudaFree(B.arena);
-    cudaFree(B.ph);
-    cudaFree(B.pl);
     cudaFree(B.d_counts);
     cudaFreeHost(B.h_counts);
     delete c->bh;

@@ -31,6 +31,18 @@ __device__ __forceinline__ double widen(float f) {
     return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
 
+// v as FP32 hi (truncated, by bits) + lo parts: one FP64 subtraction and one
+// conversion instead of four operations at the FP64 rate
+__device__ __forceinline__ void split_hilo_bits(double v, float &hi, float &lo) {
+    const uint32_t vh = (uint32_t)__double2hiint(v), m = vh & 0x7fffffffu;
+    if (m < 0x38100000u || m >= 0x47f00000u) {  // outside FP32's normal range
+        split_hilo(v, hi, lo);
+        return;
+    }
+    hi = __uint_as_float((vh & 0x80000000u) | ((m - 0x38000000u) << 3) | ((uint32_t)__double2loint(v) >> 29));
+    lo = (float)(v - widen(hi));
+}
+
 constexpr int kPairWarps = 4;    // warps (units) per CTA
 constexpr int kMaxTiles = 4;     // tiles per unit: 128 sources per FP32 sum of a target
 constexpr float kFar = 1e18f;    // coordinate of absent particles: r^-3 underflows to zero

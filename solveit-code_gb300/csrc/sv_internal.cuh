@@ -317,6 +317,7 @@ sv_status bh_accel(sv_ctx *c);
 sv_status sampled_error_range(sv_ctx *c, int64_t first, int64_t count, int k_max, double *err);
 // Morton levels the Barnes-Hut's next sort needs (its last tree's depth + 2, or all)
 int bh_sort_levels(const sv_ctx *c);
+void bh_sort_wants(sv_ctx *c);  // what the walk needs of its sort (want_hilo, want_zero)
 // the last Barnes-Hut evaluation's cell and pair interaction counts (waits for the stream)
 sv_status bh_counts(sv_ctx *c, double *cells, double *pairs);
 sv_status fmm_accel(sv_ctx *c);
