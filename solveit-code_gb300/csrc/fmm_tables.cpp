@@ -14,9 +14,13 @@
 // formula has to be matched.
 #include "fmm_tables.h"
 
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <complex>
 #include <map>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 namespace sv {
@@ -88,6 +92,13 @@ std::vector<std::vector<cd>> yrot(int p, double a, double *max_imag) {
     for (int n = 0; n < p; n++) G[n].assign((2 * n + 1) * (2 * n + 1), cd(0, 0));
     std::vector<double> P0, P1;
     const double ca = std::cos(a), sa = std::sin(a);
+    // Y_n^m at the two points of a quadrature node, index n^2 + n + m: each is
+    // evaluated once per node and not once per matrix entry
+    std::vector<cd> Y0(p * p), Y1(p * p);
+    auto fill = [p](std::vector<cd> &Y, const std::vector<double> &P, double phi) {
+        for (int n = 0; n < p; n++)
+            for (int m = -n; m <= n; m++) Y[n * n + n + m] = ynm(n, m, P, p, phi);
+    };
     for (size_t it = 0; it < gx.size(); it++) {
         const double ct = gx[it], st = std::sqrt(std::max(0.0, 1 - ct * ct));
         legendre(p, ct, P0);
@@ -101,12 +112,19 @@ std::vector<std::vector<cd>> yrot(int p, double a, double *max_imag) {
             const double vct = std::max(-1.0, std::min(1.0, vz / vr));
             const double vph = std::atan2(vy, vx);
             legendre(p, vct, P1);
+            fill(Y0, P0, ph);
+            fill(Y1, P1, vph);
             for (int n = 0; n < p; n++) {
                 const double f = w * (2 * n + 1) / (4 * M_PI);
                 for (int m = -n; m <= n; m++) {
-                    const cd fv = ynm(n, m, P1, p, vph);
+                    // f Y1 conj(Y0), in real arithmetic (the complex product's
+                    // special-case handling costs more than the product)
+                    const cd fv = f * Y1[n * n + n + m];
+                    const double a = fv.real(), b = fv.imag();
                     for (int mp = -n; mp <= n; mp++) {
-                        G[n][(mp + n) * (2 * n + 1) + (m + n)] += f * fv * std::conj(ynm(n, mp, P0, p, ph));
+                        const cd y = Y0[n * n + n + mp];
+                        const double c = y.real(), d = -y.imag();
+                        G[n][(mp + n) * (2 * n + 1) + (m + n)] += cd(a * c - b * d, a * d + b * c);
                     }
                 }
             }
@@ -117,6 +135,56 @@ std::vector<std::vector<cd>> yrot(int p, double a, double *max_imag) {
         for (auto &v : g) mi = std::max(mi, std::fabs(v.imag()));
     *max_imag = mi;
     return G;
+}
+
+struct RotPair {
+    std::vector<std::vector<cd>> f, b;  // f(u) -> f(Ry(theta) u'), f(Ry(-theta) u')
+    double imag = 0;                    // largest imaginary part left by the quadrature
+};
+
+// f(0) .. f(n - 1), independent of each other, over a few threads (the first
+// evaluation with an order and separation waits for its tables)
+// false when a call threw (out of memory)
+template <typename F>
+bool over_threads(size_t n, F &&f) {
+    const size_t nt = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), n});
+    std::atomic<bool> failed{false};
+    auto share = [&](size_t first) {
+        try {
+            for (size_t k = first; k < n; k += nt) f(k);
+        } catch (...) {
+            failed = true;
+        }
+    };
+    std::thread pool[8];
+    size_t started = 1;
+    try {
+        for (; started < nt; started++) pool[started] = std::thread(share, started);
+    } catch (const std::system_error &) {
+        // no more threads: the remaining shares run here
+    }
+    for (size_t k = started; k < nt; k++) share(k);
+    if (nt > 0) share(0);
+    for (size_t k = 1; k < started; k++) pool[k].join();
+    return !failed;
+}
+
+// Both y-rotations of every angle.
+bool rotations(int p, const std::vector<double> &thetas, std::vector<RotPair> &out, std::string &err) {
+    out.resize(thetas.size());
+    const bool ok = over_threads(thetas.size(), [&](size_t k) {
+        double m1 = 0, m2 = 0;
+        out[k].f = yrot(p, thetas[k], &m1);
+        out[k].b = yrot(p, -thetas[k], &m2);
+        out[k].imag = std::max(m1, m2);
+    });
+    if (!ok) err = "out of memory";
+    for (const RotPair &r : out)
+        if (ok && r.imag > 1e-9) {
+            err = "y-rotation matrix is not real";
+            return false;
+        }
+    return ok;
 }
 
 // fold a real (2n+1)^2 rotation block into E ((n+1) rows) and O (n rows) of
@@ -202,16 +270,12 @@ bool build_fmm_tables(int p, int ws, FmmTables &T, std::string &err) {
             }
     T.ntheta = (int)thetas.size();
     T.dmat.assign((size_t)T.ntheta * T.dsz, 0.f);
+    std::vector<RotPair> rot;
+    if (!rotations(p, thetas, rot, err)) return false;
     for (int ti = 0; ti < T.ntheta; ti++) {
-        double mi1 = 0, mi2 = 0;
         // forward rotation Ry(-theta) acts on coefficients as f(u) -> f(Ry(theta) u'),
         // the backward one Ry(theta) as f(u) -> f(Ry(-theta) u')
-        auto Gf = yrot(p, thetas[ti], &mi1);
-        auto Gb = yrot(p, -thetas[ti], &mi2);
-        if (mi1 > 1e-9 || mi2 > 1e-9) {
-            err = "y-rotation matrix is not real";
-            return false;
-        }
+        const auto &Gf = rot[ti].f, &Gb = rot[ti].b;
         float *base = &T.dmat[(size_t)ti * T.dsz];
         for (int n = 0; n < p; n++) {
             fold(Gf[n], n, T.stride, base + dmat_offset_e(n, p), base + T.esz + dmat_offset_o(n, p));
@@ -294,73 +358,78 @@ bool build_m2l_dense(int p, int ws, std::vector<double> &K, std::string &err) {
         for (int j = k; j < p; j++)
             for (int n = k; n < p; n++)
                 zc[((size_t)k * p + j) * p + n] = ((j + k) & 1 ? -1.0 : 1.0) * fact(j + n) / (N(n, k) * N(j, k));
-    std::map<long long, std::pair<std::vector<std::vector<cd>>, std::vector<std::vector<cd>>>> rot;
-    // real index of (n, m, part): n^2 for Re(c_n^0); n^2 + 2m - 1 / n^2 + 2m for Re / Im(c_n^m)
-    auto ri = [](int n, int m, int im) { return m == 0 ? n * n : n * n + 2 * m - 1 + im; };
-    std::vector<cd> A(p * p), B(p * p), Cz(p * p), Rr(p * p);  // [n][m], m = 0..n
+    std::map<long long, int> theta_index;
+    std::vector<double> thetas;
     for (int dx = -range; dx <= range; dx++)
         for (int dy = -range; dy <= range; dy++)
             for (int dz = -range; dz <= range; dz++) {
                 if (!fmm_m2l_class(dx, dy, dz, ws)) continue;
-                const int id = ((dx + range) * side + (dy + range)) * side + (dz + range);
-                const double r = std::sqrt((double)(dx * dx + dy * dy + dz * dz));
-                const double th = std::acos(dz / r), ph = std::atan2((double)dy, (double)dx);
-                const long long key = std::llround(th * 1e12);
-                if (!rot.count(key)) {
-                    double mi1 = 0, mi2 = 0;
-                    auto gf = yrot(p, th, &mi1);
-                    auto gb = yrot(p, -th, &mi2);
-                    if (mi1 > 1e-9 || mi2 > 1e-9) {
-                        err = "y-rotation matrix is not real";
-                        return false;
-                    }
-                    rot[key] = {gf, gb};
-                }
-                const auto &Gf = rot[key].first, &Gb = rot[key].second;
-                // a real y-rotation of degree n on coefficients m = 0..n of a
-                // real-symmetric expansion (c_n^-m = conj c_n^m)
-                auto yrot_apply = [&](const std::vector<std::vector<cd>> &G, const std::vector<cd> &in,
-                                      std::vector<cd> &out) {
-                    for (int n = 0; n < p; n++) {
-                        const int w = 2 * n + 1;
-                        auto g = [&](int mp, int m) { return G[n][(mp + n) * w + (m + n)].real(); };
-                        for (int mp = 0; mp <= n; mp++) {
-                            double re = g(mp, 0) * in[n * p].real(), im = 0.0;
-                            for (int m = 1; m <= n; m++) {
-                                re += (g(mp, m) + g(mp, -m)) * in[n * p + m].real();
-                                if (mp > 0) im += (g(mp, m) - g(mp, -m)) * in[n * p + m].imag();
-                            }
-                            out[n * p + mp] = cd(re, im);
-                        }
-                    }
-                };
-                for (int n0 = 0; n0 < p; n0++)
-                    for (int m0 = 0; m0 <= n0; m0++)
-                        for (int part = 0; part < (m0 == 0 ? 1 : 2); part++) {
-                            std::fill(A.begin(), A.end(), cd(0, 0));
-                            // unit input, then the phase e^{i m phi}
-                            A[n0 * p + m0] = (part == 0 ? cd(1, 0) : cd(0, 1)) * std::polar(1.0, m0 * ph);
-                            yrot_apply(Gf, A, B);
-                            // translation along z: C_j^k = sum_n C[k][j][n] r^-(j+n+1) B_n^k
-                            std::fill(Cz.begin(), Cz.end(), cd(0, 0));
-                            for (int k = 0; k < p; k++)
-                                for (int j = k; j < p; j++) {
-                                    cd acc(0, 0);
-                                    for (int n = k; n < p; n++)
-                                        acc += zc[((size_t)k * p + j) * p + n] * std::pow(r, -(j + n + 1)) * B[n * p + k];
-                                    Cz[j * p + k] = acc;
-                                }
-                            yrot_apply(Gb, Cz, Rr);
-                            const int kin = ri(n0, m0, part);
-                            for (int j = 0; j < p; j++)
-                                for (int k = 0; k <= j; k++) {
-                                    const cd v = Rr[j * p + k] * std::polar(1.0, -k * ph);
-                                    K[((size_t)id * R + ri(j, k, 0)) * R + kin] = v.real();
-                                    if (k > 0) K[((size_t)id * R + ri(j, k, 1)) * R + kin] = v.imag();
-                                }
-                        }
+                const double th = std::acos(dz / std::sqrt((double)(dx * dx + dy * dy + dz * dz)));
+                if (theta_index.emplace(std::llround(th * 1e12), (int)thetas.size()).second) thetas.push_back(th);
             }
-    return true;
+    std::vector<RotPair> rot;
+    if (!rotations(p, thetas, rot, err)) return false;
+    // real index of (n, m, part): n^2 for Re(c_n^0); n^2 + 2m - 1 / n^2 + 2m for Re / Im(c_n^m)
+    auto ri = [](int n, int m, int im) { return m == 0 ? n * n : n * n + 2 * m - 1 + im; };
+    const bool ok = over_threads(ncls, [&](size_t cls) {
+        const int dx = (int)cls / (side * side) - range, dy = (int)cls / side % side - range,
+                  dz = (int)cls % side - range;
+        if (!fmm_m2l_class(dx, dy, dz, ws)) return;
+        std::vector<cd> A(p * p), B(p * p), Cz(p * p), Rr(p * p);  // [n][m], m = 0..n
+        std::vector<double> rpow(2 * p);  // r^-q
+        std::vector<cd> phase(p);         // e^{-i k phi}
+        const int id = ((dx + range) * side + (dy + range)) * side + (dz + range);
+        const double r = std::sqrt((double)(dx * dx + dy * dy + dz * dz));
+        const double th = std::acos(dz / r), ph = std::atan2((double)dy, (double)dx);
+        const RotPair &G = rot[theta_index.at(std::llround(th * 1e12))];
+        const auto &Gf = G.f, &Gb = G.b;
+        for (int q = 0; q < 2 * p; q++) rpow[q] = std::pow(r, -q);
+        for (int k = 0; k < p; k++) phase[k] = std::polar(1.0, -k * ph);
+        // a real y-rotation of degree n on coefficients m = 0..n of a
+        // real-symmetric expansion (c_n^-m = conj c_n^m)
+        auto yrot_apply = [&](const std::vector<std::vector<cd>> &G, const std::vector<cd> &in,
+                              std::vector<cd> &out) {
+            for (int n = 0; n < p; n++) {
+                const int w = 2 * n + 1;
+                auto g = [&](int mp, int m) { return G[n][(mp + n) * w + (m + n)].real(); };
+                for (int mp = 0; mp <= n; mp++) {
+                    double re = g(mp, 0) * in[n * p].real(), im = 0.0;
+                    for (int m = 1; m <= n; m++) {
+                        re += (g(mp, m) + g(mp, -m)) * in[n * p + m].real();
+                        if (mp > 0) im += (g(mp, m) - g(mp, -m)) * in[n * p + m].imag();
+                    }
+                    out[n * p + mp] = cd(re, im);
+                }
+            }
+        };
+        for (int n0 = 0; n0 < p; n0++)
+            for (int m0 = 0; m0 <= n0; m0++)
+                for (int part = 0; part < (m0 == 0 ? 1 : 2); part++) {
+                    std::fill(A.begin(), A.end(), cd(0, 0));
+                    // unit input, then the phase e^{i m phi}
+                    A[n0 * p + m0] = (part == 0 ? cd(1, 0) : cd(0, 1)) * std::polar(1.0, m0 * ph);
+                    yrot_apply(Gf, A, B);
+                    // translation along z: C_j^k = sum_n C[k][j][n] r^-(j+n+1) B_n^k
+                    std::fill(Cz.begin(), Cz.end(), cd(0, 0));
+                    for (int k = 0; k < p; k++)
+                        for (int j = k; j < p; j++) {
+                            cd acc(0, 0);
+                            for (int n = k; n < p; n++)
+                                acc += zc[((size_t)k * p + j) * p + n] * rpow[j + n + 1] * B[n * p + k];
+                            Cz[j * p + k] = acc;
+                        }
+                    yrot_apply(Gb, Cz, Rr);
+                    const int kin = ri(n0, m0, part);
+                    for (int j = 0; j < p; j++)
+                        for (int k = 0; k <= j; k++) {
+                            const cd v = Rr[j * p + k] * phase[k];
+                            K[((size_t)id * R + ri(j, k, 0)) * R + kin] = v.real();
+                            if (k > 0) K[((size_t)id * R + ri(j, k, 1)) * R + kin] = v.imag();
+                        }
+                }
+    });
+    if (!ok) err = "out of memory";
+    return ok;
 }
 
 }  // namespace sv
