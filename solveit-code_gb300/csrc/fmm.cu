@@ -56,7 +56,8 @@ struct Fmm {
     float *otab = nullptr;   // rotation-based M2M / L2L tables (oct_layout)
     void *arena = nullptr;
     size_t arena_bytes = 0;
-    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue
+    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue,
+                                             // [4] finished target-flag CTAs
     unsigned long long *h_counts = nullptr;
     // caller particles followed by their source-only symmetry images
     double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr;
@@ -82,8 +83,7 @@ struct Fmm {
     // the near field runs on its own stream beside the upward and downward passes
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_lists = nullptr, ev_join = nullptr, ev_near[2] = {};
-    cudaEvent_t ev_rel = nullptr;  // the second stream's leaf offsets (F.rel) are written
-    cudaEvent_t ev_m2l_lists = nullptr;  // single plume: near, interaction and far-direct lists built (second stream)
+    cudaEvent_t ev_rel = nullptr;  // single plume: the second stream's lists, leaf offsets (F.rel) and leaf flags are written
     M2LTc tc;                // the M2L on the tensor cores (m2l_tc.cu)
 };
 
@@ -390,8 +390,9 @@ __global__ void expand_images_kernel(const double *__restrict__ x, const double 
     est[t] = g == 0 ? w : ((w == 1 || w == 2) ? 2 : w);
 }
 
-// box holds at least one target (K q/m != 0): leaf level from particles,
-// coarser levels from children
+// box holds at least one target (K q/m != 0).  Forest: leaf level from particles,
+// coarser levels from children, a launch each (its box counts are only known on
+// the device, and its launches are cheap graph nodes)
 __global__ void leaf_targets_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ start,
                                     const double *__restrict__ qm, int *__restrict__ flag) {
     const int nb = level_boxes(nbox, nbd);
@@ -409,6 +410,58 @@ __global__ void parent_targets_kernel(int nbox, const int *__restrict__ nbd, con
         int f = 0;
         for (int c = child0[b]; c < child0[b + 1] && !f; c++) f = cflag[c];
         flag[b] = f;
+    }
+}
+
+// Single tree: the levels above the leaves in one launch (the leaf flags come
+// with the leaf offsets).  A CTA takes the subtree of one box of level `top`; the
+// last CTA to finish takes the levels above.  (Letting every leaf climb and mark
+// its ancestors had all of them write the same few flags: 184 us for 10,121
+// leaves.)
+struct TargetArgs {
+    int L, top;
+    int nbox[kMortonBits + 1];
+    const int *child0[kMortonBits + 1];
+    int *flag[kMortonBits + 1];
+    unsigned *done;                   // zero before; CTAs that have finished
+};
+constexpr int kFlagThreads = 256;
+constexpr int kFlagTop = 8;  // the middle level: the deepest of up to this many boxes per SM
+
+__device__ __forceinline__ void target_flag(const TargetArgs &a, int l, int b) {
+    int f = 0;
+    for (int c = a.child0[l][b]; c < a.child0[l][b + 1] && !f; c++) f = __ldcg(&a.flag[l + 1][c]);
+    a.flag[l][b] = f;
+}
+
+__global__ void __launch_bounds__(kFlagThreads) target_flags_kernel(TargetArgs a) {
+    __shared__ int lo[kMortonBits + 1], hi[kMortonBits + 1];
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        int x = blockIdx.x, y = x + 1;
+        for (int l = a.top;; l++) {
+            lo[l] = x;
+            hi[l] = y;
+            if (l == a.L) break;
+            x = a.child0[l][x];
+            y = a.child0[l][y];
+        }
+    }
+    __syncthreads();
+    for (int l = a.L - 1; l >= a.top; l--) {
+        __syncthreads();
+        for (int b = lo[l] + threadIdx.x; b < hi[l]; b += kFlagThreads) target_flag(a, l, b);
+    }
+    if (a.top == 0) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int l = a.top - 1; l >= 0; l--) {
+        for (int b = threadIdx.x; b < a.nbox[l]; b += kFlagThreads) target_flag(a, l, b);
+        __syncthreads();
     }
 }
 
@@ -615,7 +668,8 @@ struct OctOff {
 };
 
 // One output (j, k) of a z-shift by a fixed distance: sum_n Z[k][j][n] B[k][n]
-template <int P>
+// (SH: the table is in shared memory)
+template <int P, bool SH>
 __device__ __forceinline__ float2 zshift_row(const float *__restrict__ zt, const float2 *Bk, int j, int k) {
     constexpr int RS = rot_rs<P>();
     const float4 *Z = reinterpret_cast<const float4 *>(zt + ((size_t)k * P + j) * RS);
@@ -623,7 +677,7 @@ __device__ __forceinline__ float2 zshift_row(const float *__restrict__ zt, const
     float re = 0.f, im = 0.f;
 #pragma unroll
     for (int q = 0; q < RS / 4; q++) {
-        const float4 z = __ldg(Z + q);
+        const float4 z = SH ? Z[q] : __ldg(Z + q);
         const float4 b0 = B4[2 * q], b1 = B4[2 * q + 1];
         re = fmaf(z.x, b0.x, fmaf(z.y, b0.z, fmaf(z.z, b1.x, fmaf(z.w, b1.z, re))));
         im = fmaf(z.x, b0.y, fmaf(z.y, b0.w, fmaf(z.z, b1.y, fmaf(z.w, b1.w, im))));
@@ -632,12 +686,12 @@ __device__ __forceinline__ float2 zshift_row(const float *__restrict__ zt, const
 }
 
 // Rotation-based translation of one coefficient vector (GR normalisation,
-// compact layout) along an octant direction: phase e^{i m phi}, y-rotation
+// compact layout; `in` holds the lane's slots) along an octant direction: phase e^{i m phi}, y-rotation
 // that takes the direction to +z, fixed z-shift Z, back-rotation, phase
 // e^{-i m phi}; the result is added into the lane's accumulators.  A and B are
 // the warp's degree-major / order-major rows, zero outside (n, m <= n).
-template <int P>
-__device__ __forceinline__ void oct_translate(const float2 *__restrict__ in, const float2 *__restrict__ ph,
+template <int P, bool SH>
+__device__ __forceinline__ void oct_translate(const float2 (&in)[2], const float2 *__restrict__ ph,
                                               const float *__restrict__ D, const float *__restrict__ Z, float2 *A,
                                               float2 *B, const int *cn, const int *cm, const int *cs,
                                               const bool *has, float2 *acc) {
@@ -645,13 +699,13 @@ __device__ __forceinline__ void oct_translate(const float2 *__restrict__ in, con
     constexpr int ESZ = RS * P * (P + 1) / 2, OSZ = RS * P * (P - 1) / 2;
 #pragma unroll
     for (int t = 0; t < 2; t++)
-        if (has[t]) A[cn[t] * SR + cm[t]] = cmul(in[cs[t]], ph[cm[t]]);
+        if (has[t]) A[cn[t] * SR + cm[t]] = cmul(in[t], ph[cm[t]]);
     __syncwarp();
     if (has[0]) B[cm[0] * SR + cn[0]] = rot_row<P, G0>(D, 0, ESZ, A, cn[0], cm[0]);
     if (has[1]) B[cm[1] * SR + cn[1]] = rot_row<P, G1>(D, 0, ESZ, A, cn[1], cm[1]);
     __syncwarp();
-    if (has[0]) A[cn[0] * SR + cm[0]] = zshift_row<P>(Z, B, cn[0], cm[0]);
-    if (has[1]) A[cn[1] * SR + cm[1]] = zshift_row<P>(Z, B, cn[1], cm[1]);
+    if (has[0]) A[cn[0] * SR + cm[0]] = zshift_row<P, SH>(Z, B, cn[0], cm[0]);
+    if (has[1]) A[cn[1] * SR + cm[1]] = zshift_row<P, SH>(Z, B, cn[1], cm[1]);
     __syncwarp();
     if (has[0]) acc[0] = cadd(acc[0], cmul(rot_row<P, G0>(D, ESZ + OSZ, 2 * ESZ + OSZ, A, cn[0], cm[0]), cconj(ph[cm[0]])));
     if (has[1]) acc[1] = cadd(acc[1], cmul(rot_row<P, G1>(D, ESZ + OSZ, 2 * ESZ + OSZ, A, cn[1], cm[1]), cconj(ph[cm[1]])));
@@ -672,15 +726,37 @@ __device__ __forceinline__ void coef_slots(int lane, int *cn, int *cm, int *cs, 
     has[1] = lane < EXTRA;
 }
 
-// M2M: one warp per parent box; each child's multipole translated to the
-// parent centre by rotation (O(p^3) per child instead of the O(p^4) direct
-// R-convolution), child -> parent box units folded into the z-shift table.
+// the lane's slots of a box's coefficients; through L2 (another warp of this
+// launch may have written them)
+template <int P>
+__device__ __forceinline__ void load_slots(const float2 *src, const int *cs, const bool *has, float2 (&v)[2]) {
+#pragma unroll
+    for (int t = 0; t < 2; t++) v[t] = has[t] ? __ldcg(src + cs[t]) : make_float2(0.f, 0.f);
+}
+
+// M2M of one child: its multipole translated to the parent's centre by rotation
+// (O(p^3) per child instead of the O(p^4) direct R-convolution), child -> parent
+// box units folded into the z-shift table, added to acc.
+template <int P, bool SH>
+__device__ __forceinline__ void m2m_child(int ch, const int4 *__restrict__ ccoord, const float2 *Mc, const float *otab,
+                                          float2 *A, float2 *B, const int *cn, const int *cm, const int *cs,
+                                          const bool *has, float2 *acc) {
+    using O = OctOff<P>;
+    const int4 cc = ccoord[ch];
+    const int oc = (cc.x & 1) | ((cc.y & 1) << 1) | ((cc.z & 1) << 2);
+    const int th = (int)otab[O::th_m2m + oc];
+    float2 in[2];
+    load_slots<P>(Mc + (size_t)ch * ncoef(P), cs, has, in);
+    oct_translate<P, SH>(in, reinterpret_cast<const float2 *>(otab + O::ph_m2m) + oc * P,
+                         otab + O::rot + th * O::DSZ, otab + O::zm2m, A, B, cn, cm, cs, has, acc);
+}
+
+// one level, one warp per parent box
 template <int P>
 __global__ void __launch_bounds__(kWarps * 32)
 m2m_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ child0, const int4 *__restrict__ ccoord,
-           const float2 *__restrict__ Mc, float2 *__restrict__ Mp, const float *__restrict__ otab) {
-    constexpr int NC = ncoef(P), SR = sh_rs<P>();
-    using O = OctOff<P>;
+           const float2 *Mc, float2 *Mp, const float *__restrict__ otab) {
+    constexpr int SR = sh_rs<P>();
     __shared__ __align__(16) float2 A[kWarps][P * SR], B[kWarps][P * SR];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int t = lane; t < P * SR; t += 32) A[wid][t] = B[wid][t] = make_float2(0.f, 0.f);
@@ -692,15 +768,81 @@ m2m_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ child0
     for (int b = blockIdx.x * kWarps + wid; b < nb; b += gridDim.x * kWarps) {
         float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         const int ch1 = child0[b + 1];
-        for (int ch = child0[b]; ch < ch1; ch++) {
-            const int4 cc = ccoord[ch];
-            const int oc = (cc.x & 1) | ((cc.y & 1) << 1) | ((cc.z & 1) << 2);
-            const int th = (int)otab[O::th_m2m + oc];
-            oct_translate<P>(Mc + (size_t)ch * NC, reinterpret_cast<const float2 *>(otab + O::ph_m2m) + oc * P,
-                             otab + O::rot + th * O::DSZ, otab + O::zm2m, A[wid], B[wid], cn, cm, cs, has, acc);
+        for (int ch = child0[b]; ch < ch1; ch++)
+            m2m_child<P, false>(ch, ccoord, Mc, otab, A[wid], B[wid], cn, cm, cs, has, acc);
+        if (has[0]) Mp[(size_t)b * ncoef(P) + cs[0]] = acc[0];
+        if (has[1]) Mp[(size_t)b * ncoef(P) + cs[1]] = acc[1];
+    }
+}
+
+// The coarse levels of a single tree in one launch: one CTA, level by level with
+// barriers between them, the translation tables in shared memory.  A level with
+// few boxes is a chain of dependent table loads in one warp per parent, and a
+// launch of its own: 20,011 ions in a column, the five levels' ten launches took
+// 102 us serialised, these two and the rest 80.  M2M: a warp per child (levels whose children
+// number at most kCoarseBoxes), the translated multipoles kept in `tmp` and added
+// per parent in child order.
+constexpr int kCoarseBoxes = 64, kCoarseWarps = 16;
+struct CoarseM2M {
+    int top, last;  // levels top, top - 1, ..., last
+    const float *otab;
+    int nbox[kMortonBits + 1];
+    const int *child0[kMortonBits + 1];
+    const int4 *coord[kMortonBits + 1];
+    float2 *M[kMortonBits + 1], *tmp[kMortonBits + 1];
+};
+template <int P>
+constexpr int oct_size() { return OctOff<P>::th_l2l + 8; }
+// rows A and B of every warp, then the tables
+template <int P>
+constexpr size_t coarse_smem() {
+    return (size_t)kCoarseWarps * 2 * P * sh_rs<P>() * sizeof(float2) + (oct_size<P>() + 3) / 4 * 16;
+}
+template <int P, typename K>
+cudaError_t dyn_smem(K kernel) {
+    if (coarse_smem<P>() <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coarse_smem<P>());
+}
+// the warp's zeroed rows and the CTA's copy of the tables
+template <int P>
+__device__ __forceinline__ const float *coarse_setup(const float *__restrict__ otab, float2 *ab, float2 *&A, float2 *&B) {
+    constexpr int SR = sh_rs<P>();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    A = ab + 2 * wid * (P * SR);
+    B = A + P * SR;
+    for (int t = lane; t < P * SR; t += 32) A[t] = B[t] = make_float2(0.f, 0.f);
+    float *tab = reinterpret_cast<float *>(ab + 2 * kCoarseWarps * (P * SR));
+    for (int t = threadIdx.x; t < oct_size<P>(); t += blockDim.x) tab[t] = otab[t];
+    __syncthreads();
+    return tab;
+}
+template <int P>
+__global__ void __launch_bounds__(kCoarseWarps * 32) m2m_coarse_kernel(CoarseM2M a) {
+    constexpr int NC = ncoef(P);
+    extern __shared__ __align__(16) float2 ab[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float2 *A, *B;
+    const float *tab = coarse_setup<P>(a.otab, ab, A, B);
+    int cn[2], cm[2], cs[2];
+    bool has[2];
+    coef_slots<P>(lane, cn, cm, cs, has);
+    for (int l = a.top; l >= a.last; l--) {
+        float2 *tmp = a.tmp[l + 1];
+        for (int ch = wid; ch < a.nbox[l + 1]; ch += kCoarseWarps) {
+            float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            m2m_child<P, true>(ch, a.coord[l + 1], a.M[l + 1], tab, A, B, cn, cm, cs, has, acc);
+            if (has[0]) tmp[(size_t)ch * NC + cs[0]] = acc[0];
+            if (has[1]) tmp[(size_t)ch * NC + cs[1]] = acc[1];
         }
-        if (has[0]) Mp[(size_t)b * NC + cs[0]] = acc[0];
-        if (has[1]) Mp[(size_t)b * NC + cs[1]] = acc[1];
+        __syncthreads();
+        for (int t = threadIdx.x; t < a.nbox[l] * NC; t += blockDim.x) {
+            const int b = t / NC, k = t - b * NC;
+            const int c0 = a.child0[l][b], c1 = a.child0[l][b + 1];
+            float2 acc = make_float2(0.f, 0.f);
+            for (int ch = c0; ch < c1; ch++) acc = cadd(acc, __ldcg(&tmp[(size_t)ch * NC + k]));
+            a.M[l][t] = acc;
+        }
+        __syncthreads();
     }
 }
 
@@ -823,10 +965,37 @@ __global__ void __launch_bounds__(m2l_warps<P>() * 32, m2l_min_ctas<P>()) m2l_ke
 // L = (sum of the level's M2L partials, in chunk order) + L2L(parent's L),
 // the L2L by rotation (O(p^3)), parent -> child box units folded into the
 // z-shift table
+// SH: the coarse kernel (tables in shared memory, the partials summed in a.L)
+template <int P, bool SH>
+__device__ __forceinline__ void l2l_box(const L2LArgs &a, const float *otab, int b, float2 *A, float2 *B, const int *cn, const int *cm,
+                                        const int *cs, const bool *has) {
+    constexpr int NC = ncoef(P);
+    using O = OctOff<P>;
+    float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+        if (has[t]) {
+            if (SH) acc[t] = __ldcg(&a.L[(size_t)b * NC + cs[t]]);
+            else
+                for (int ch = 0; ch < a.chunks; ch++)
+                    acc[t] = cadd(acc[t], a.part[((size_t)b * a.chunks + ch) * NC + cs[t]]);
+        }
+    if (a.has_parent) {
+        const int4 cb = a.coord[b];
+        const int oc = (cb.x & 1) | ((cb.y & 1) << 1) | ((cb.z & 1) << 2);
+        const int th = (int)otab[O::th_l2l + oc];
+        float2 in[2];
+        load_slots<P>(a.Lp + (size_t)a.parent[b] * NC, cs, has, in);
+        oct_translate<P, SH>(in, reinterpret_cast<const float2 *>(otab + O::ph_l2l) + oc * P,
+                             otab + O::rot + th * O::DSZ, otab + O::zl2l, A, B, cn, cm, cs, has, acc);
+    }
+    if (has[0]) a.L[(size_t)b * NC + cs[0]] = acc[0];
+    if (has[1]) a.L[(size_t)b * NC + cs[1]] = acc[1];
+}
+
 template <int P>
 __global__ void __launch_bounds__(kWarps * 32) l2l_kernel(L2LArgs a) {
-    constexpr int NC = ncoef(P), SR = sh_rs<P>();
-    using O = OctOff<P>;
+    constexpr int SR = sh_rs<P>();
     __shared__ __align__(16) float2 A[kWarps][P * SR], B[kWarps][P * SR];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int t = lane; t < P * SR; t += 32) A[wid][t] = B[wid][t] = make_float2(0.f, 0.f);
@@ -835,24 +1004,50 @@ __global__ void __launch_bounds__(kWarps * 32) l2l_kernel(L2LArgs a) {
     bool has[2];
     coef_slots<P>(lane, cn, cm, cs, has);
     const int nb = level_boxes(a.nbox, a.nbd);
-    for (int b = blockIdx.x * kWarps + wid; b < nb; b += gridDim.x * kWarps) {
-        if (!a.has_tgt[b]) continue;
-        float2 acc[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    for (int b = blockIdx.x * kWarps + wid; b < nb; b += gridDim.x * kWarps)
+        if (a.has_tgt[b]) l2l_box<P, false>(a, a.otab, b, A[wid], B[wid], cn, cm, cs, has);
+}
+
+// the coarse levels first .. last in one CTA, as m2m_coarse_kernel
+struct CoarseL2L {
+    int first, last;
+    L2LArgs lv[kMortonBits + 1];
+};
+template <int P>
+__global__ void __launch_bounds__(kCoarseWarps * 32) l2l_coarse_kernel(CoarseL2L a) {
+    constexpr int NC = ncoef(P);
+    extern __shared__ __align__(16) float2 ab[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float2 *A, *B;
+    const float *tab = coarse_setup<P>(a.lv[a.first].otab, ab, A, B);
+    int cn[2], cm[2], cs[2];
+    bool has[2];
+    coef_slots<P>(lane, cn, cm, cs, has);
+    // every level's M2L partials first (their loads depend on nothing), in chunk order
+    for (int l = a.first; l <= a.last; l++) {
+        const L2LArgs &v = a.lv[l];
+        for (int t = threadIdx.x; t < v.nbox * NC; t += blockDim.x) {
+            const int b = t / NC, k = t - b * NC;
+            if (!v.has_tgt[b]) continue;
+            const float2 *p = v.part + (size_t)b * v.chunks * NC + k;
+            float2 acc = make_float2(0.f, 0.f);
+            for (int c0 = 0; c0 < v.chunks; c0 += 8) {
+                float2 x[8];
 #pragma unroll
-        for (int t = 0; t < 2; t++)
-            if (has[t])
-                for (int ch = 0; ch < a.chunks; ch++)
-                    acc[t] = cadd(acc[t], a.part[((size_t)b * a.chunks + ch) * NC + cs[t]]);
-        if (a.has_parent) {
-            const int4 cb = a.coord[b];
-            const int oc = (cb.x & 1) | ((cb.y & 1) << 1) | ((cb.z & 1) << 2);
-            const int th = (int)a.otab[O::th_l2l + oc];
-            oct_translate<P>(a.Lp + (size_t)a.parent[b] * NC,
-                             reinterpret_cast<const float2 *>(a.otab + O::ph_l2l) + oc * P,
-                             a.otab + O::rot + th * O::DSZ, a.otab + O::zl2l, A[wid], B[wid], cn, cm, cs, has, acc);
+                for (int u = 0; u < 8; u++) x[u] = p[(size_t)min(c0 + u, v.chunks - 1) * NC];
+#pragma unroll
+                for (int u = 0; u < 8; u++)
+                    if (c0 + u < v.chunks) acc = cadd(acc, x[u]);
+            }
+            v.L[t] = acc;
         }
-        if (has[0]) a.L[(size_t)b * NC + cs[0]] = acc[0];
-        if (has[1]) a.L[(size_t)b * NC + cs[1]] = acc[1];
+    }
+    __syncthreads();
+    for (int l = a.first; l <= a.last; l++) {
+        if (!a.lv[l].has_parent) continue;
+        for (int b = wid; b < a.lv[l].nbox; b += kCoarseWarps)
+            if (a.lv[l].has_tgt[b]) l2l_box<P, true>(a.lv[l], tab, b, A, B, cn, cm, cs, has);
+        __syncthreads();
     }
 }
 
@@ -1076,13 +1271,14 @@ __global__ void __launch_bounds__(kWarps * 32) m2p_kernel(TreecodeArgs a) {
 // (one FP64 subtraction per particle) with its charge: the P2P kernel then
 // forms source offsets from the target box centre as offset + k*h in FP32.
 // A charge other than qs[0] sets *mixed (zeroed beforehand), which keeps the
-// P2P kernel on its per-source charge path.
+// P2P kernel on its per-source charge path.  With flag, the box's target flag.
 __global__ void __launch_bounds__(kWarps * 32)
 box_relative_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ bpid,
                     const int *__restrict__ start, const int4 *__restrict__ coord, const double *__restrict__ xs,
                     const double *__restrict__ ys, const double *__restrict__ zs, const float *__restrict__ qs,
                     const double *__restrict__ roots, int level, float4 *__restrict__ rel,
-                    unsigned long long *__restrict__ mixed) {
+                    unsigned long long *__restrict__ mixed, const double *__restrict__ qm = nullptr,
+                    int *__restrict__ flag = nullptr) {
     const float q0 = qs[0];
     bool diff = false;
     SV_WARP_BOXES(kWarps) {
@@ -1090,10 +1286,16 @@ box_relative_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict
     const double h = root[3] / (double)(1 << level);
     const int4 cb = coord[b];
     const double cx = root[0] + (cb.x + 0.5) * h, cy = root[1] + (cb.y + 0.5) * h, cz = root[2] + (cb.z + 0.5) * h;
+    bool tgt = false;
     for (int j = start[b] + lane; j < start[b + 1]; j += 32) {
         const float q = qs[j];
         diff |= q != q0;
         rel[j] = make_float4((float)(xs[j] - cx), (float)(ys[j] - cy), (float)(zs[j] - cz), q);
+        if (flag) tgt |= qm[j] != 0.0;
+    }
+    if (flag) {
+        const bool any = __any_sync(0xffffffffu, tgt);
+        if (lane == 0) flag[b] = any;
     }
     }
     if (__any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) *mixed = 1ull;
@@ -1476,6 +1678,24 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         cnt[l] = (int *)carve(nb * sizeof(int));
         part[l] = chunks[l] > 1 ? (float2 *)carve(nb * chunks[l] * NC * sizeof(float2)) : Lv[l];
     }
+    // which boxes hold targets (all of them unless symmetry images are present)
+    int *tgt[kMortonBits + 1];
+    {
+        int64_t tot = 0;
+        for (int l = 0; l <= L; l++) tot += T.lv[l].nbox;
+        if (F.tgt_cap < tot) {
+            cudaFree(F.has_tgt);
+            F.has_tgt = nullptr;
+            const int64_t want = tot + tot / 2;  // headroom: a growing tree reallocates rarely
+            SV_CK(c, cudaMalloc(&F.has_tgt, sizeof(int) * want));
+            F.tgt_cap = want;
+        }
+        int64_t o = 0;
+        for (int l = 0; l <= L; l++) {
+            tgt[l] = F.has_tgt + o;
+            o += T.lv[l].nbox;
+        }
+    }
     // every level's lists in two launches (near lists, then interaction lists)
     ListArgs la{};
     la.nlev = L + 1;
@@ -1503,25 +1723,7 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         la.lv[L].fd_cnt = (int *)carve((size_t)T.lv[L].nbox * sizeof(int));
     }
     phase_mark(c, 2);
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 4 * sizeof(unsigned long long), c->stream));
-    // which boxes hold targets (all of them unless symmetry images are present)
-    int *tgt[kMortonBits + 1];
-    {
-        int64_t tot = 0;
-        for (int l = 0; l <= L; l++) tot += T.lv[l].nbox;
-        if (F.tgt_cap < tot) {
-            cudaFree(F.has_tgt);
-            F.has_tgt = nullptr;
-            const int64_t want = tot + tot / 2;  // headroom: a growing tree reallocates rarely
-            SV_CK(c, cudaMalloc(&F.has_tgt, sizeof(int) * want));
-            F.tgt_cap = want;
-        }
-        int64_t o = 0;
-        for (int l = 0; l <= L; l++) {
-            tgt[l] = F.has_tgt + o;
-            o += T.lv[l].nbox;
-        }
-    }
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 5 * sizeof(unsigned long long), c->stream));
     if (F.rel_cap < c->S.n) {
         cudaFree(F.rel);
         cudaFree(F.far);
@@ -1532,22 +1734,19 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         F.rel_cap = c->S.n;
     }
     double *fx = F.far, *fy = F.far + F.rel_cap, *fz = F.far + 2 * F.rel_cap;
-    // Two streams from here on.  The second takes the leaf level's target
-    // flags, then the near and interaction lists of every level in two
+    // Two streams from here on.  The second takes the near and interaction
+    // lists of every level in two
     // launches (boxes found by binary search over each level's Morton codes),
     // then runs the near field (P2P), which needs only the sorted particles,
-    // the leaf boxes and their near lists, and writes the accelerations.  The
-    // main stream derives the coarser target flags and runs the upward pass,
-    // then M2L / L2L and the far field (L2P or the treecode's M2P, into their
+    // the leaf boxes, their target flags and near lists, and writes the
+    // accelerations.  The main stream runs the
+    // upward pass, then M2L / L2L and the far field (L2P or the treecode's M2P, into their
     // own arrays) beside the near field, then waits for it; the scatter to the
     // caller's order adds the two.
     SV_CK(c, cudaEventRecord(F.ev_fork, c->stream));
     SV_CK(c, cudaStreamWaitEvent(F.side, F.ev_fork, 0));
     {
         const Level &V = T.lv[L];
-        leaf_targets_kernel<<<div_up(V.nbox, 256), 256, 0, F.side>>>(V.nbox, nullptr, V.start, S.qm, tgt[L]);
-        SV_LAUNCHED(c);
-        SV_CK(c, cudaEventRecord(F.ev_lists, F.side));
         box_codes_kernel<<<div_up(la.total, 256), 256, 0, F.side>>>(la);
         SV_LAUNCHED(c);
         const int64_t slots = (int64_t)la.total * ns;
@@ -1560,9 +1759,10 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
             else m2l_lists_kernel<2><<<g, kWarps * 32, 0, F.side>>>(la, cap, F.d_counts);
             SV_LAUNCHED(c);
         }
-        SV_CK(c, cudaEventRecord(F.ev_m2l_lists, F.side));
+        SV_CK(c, cudaEventRecord(F.ev_lists, F.side));
         box_relative_kernel<<<div_up(V.nbox, kWarps), kWarps * 32, 0, F.side>>>(
-            V.nbox, nullptr, nullptr, V.start, V.coord, S.x, S.y, S.z, S.q, S.root, L, F.rel, F.d_counts + 2);
+            V.nbox, nullptr, nullptr, V.start, V.coord, S.x, S.y, S.z, S.q, S.root, L, F.rel, F.d_counts + 2, S.qm,
+            tgt[L]);
         SV_LAUNCHED(c);
         SV_CK(c, cudaEventRecord(F.ev_rel, F.side));
         if (c->P.profile_phases) SV_CK(c, cudaEventRecord(F.ev_near[0], F.side));
@@ -1579,28 +1779,58 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         }
         SV_CK(c, cudaEventRecord(F.ev_join, F.side));
     }
-    // coarser target flags from the leaf flags
-    SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_lists, 0));
-    for (int l = L - 1; l >= 0; l--) {
-        parent_targets_kernel<<<div_up(T.lv[l].nbox, 256), 256, 0, c->stream>>>(T.lv[l].nbox, nullptr,
-                                                                                T.lv[l].child0, tgt[l + 1], tgt[l]);
-        SV_LAUNCHED(c);
-    }
     phase_mark(c, 3);
-    // upward pass
+    // Upward pass.  Where its blocks fill the SMs it starts after the lists: beside
+    // them it would hold the SMs that the lists, and the near field behind them
+    // (the longest kernel of an evaluation), are waiting for.  131,101 ions in a
+    // ball, 728 leaf boxes: 3,820 against 3,896 us for three steps; 20,011 ions,
+    // 272 boxes: 420 against 405 us, so fewer boxes start at once.
+    if (T.lv[L].nbox >= kWarps * device_sms()) SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_lists, 0));
     {
         const Level &V = T.lv[L];
         p2m_kernel<P><<<div_up(V.nbox, p2m_warps<P>()), p2m_warps<P>() * 32, 0, c->stream>>>(
             V.nbox, nullptr, nullptr, V.start, V.coord, S.x, S.y, S.z, S.q, S.root, L, F.nrm, Mv[L]);
         SV_LAUNCHED(c);
     }
-    for (int l = L - 1; l >= 2; l--) {
+    // levels 2 .. coarse and their children have few boxes: one launch for all of them
+    int coarse = 1;
+    while (coarse + 1 < L && T.lv[coarse + 2].nbox <= kCoarseBoxes) coarse++;
+    if (coarse == 2) coarse = 1;  // one level gains nothing from one CTA
+    for (int l = L - 1; l > coarse; l--) {
         const Level &V = T.lv[l];
         m2m_kernel<P><<<div_up(V.nbox, kWarps), kWarps * 32, 0, c->stream>>>(
             V.nbox, nullptr, V.child0, T.lv[l + 1].coord, Mv[l + 1], Mv[l], F.otab);
         SV_LAUNCHED(c);
     }
-    SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_m2l_lists, 0));
+    if (coarse >= 2) {
+        CoarseM2M cm{};
+        cm.top = coarse;
+        cm.last = 2;
+        cm.otab = F.otab;
+        for (int l = 2; l <= coarse + 1; l++) {
+            cm.nbox[l] = T.lv[l].nbox;
+            cm.child0[l] = T.lv[l].child0;
+            cm.coord[l] = T.lv[l].coord;
+            cm.M[l] = Mv[l];
+            cm.tmp[l] = Lv[l];  // free until the downward pass
+        }
+        SV_CK(c, (dyn_smem<P>(m2m_coarse_kernel<P>)));
+        m2m_coarse_kernel<P><<<1, kCoarseWarps * 32, coarse_smem<P>(), c->stream>>>(cm);
+        SV_LAUNCHED(c);
+    }
+    // the second stream's lists, leaf offsets and leaf flags; then the coarser flags
+    SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_rel, 0));
+    TargetArgs tf{};
+    tf.L = L;
+    tf.done = reinterpret_cast<unsigned *>(F.d_counts + 4);
+    for (int l = 0; l <= L; l++) {
+        tf.nbox[l] = T.lv[l].nbox;
+        tf.child0[l] = T.lv[l].child0;
+        tf.flag[l] = tgt[l];
+        if (l == 0 || (l < L && T.lv[l].nbox <= kFlagTop * device_sms())) tf.top = l;
+    }
+    target_flags_kernel<<<T.lv[tf.top].nbox, kFlagThreads, 0, c->stream>>>(tf);
+    SV_LAUNCHED(c);
     phase_mark(c, 4);
     const bool treecode = c->P.fmm_type == SV_FMM_TREECODE || c->P.fmm_type == SV_FMM_TREECODE_OUTLIERS;
     // downward pass: M2L of all levels in one launch, then L2L level by level
@@ -1672,9 +1902,16 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         }
         m2l_kernel<P><<<div_up(warps, m2l_warps<P>()), m2l_warps<P>() * 32, 0, c->stream>>>(a);
         SV_LAUNCHED(c);
+        CoarseL2L cl{};
+        // the same for the locals: a warp per box
+        int lcoarse = 1;
+        while (lcoarse + 1 <= L && T.lv[lcoarse + 1].nbox <= kCoarseBoxes) lcoarse++;
+        if (lcoarse == 2) lcoarse = 1;  // one level gains nothing from one CTA
+        cl.first = 2;
+        cl.last = lcoarse;
         for (int l = 2; l <= L; l++) {
             const Level &V = T.lv[l];
-            L2LArgs b{};
+            L2LArgs &b = cl.lv[l];
             b.nbox = V.nbox;
             b.chunks = chunks[l];
             b.has_parent = l > 2;
@@ -1686,7 +1923,14 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
             b.part = part[l];
             b.L = Lv[l];
             b.otab = F.otab;
-            l2l_kernel<P><<<div_up(V.nbox, kWarps), kWarps * 32, 0, c->stream>>>(b);
+        }
+        if (lcoarse >= 2) {
+            SV_CK(c, (dyn_smem<P>(l2l_coarse_kernel<P>)));
+            l2l_coarse_kernel<P><<<1, kCoarseWarps * 32, coarse_smem<P>(), c->stream>>>(cl);
+            SV_LAUNCHED(c);
+        }
+        for (int l = std::max(2, lcoarse + 1); l <= L; l++) {
+            l2l_kernel<P><<<div_up(T.lv[l].nbox, kWarps), kWarps * 32, 0, c->stream>>>(cl.lv[l]);
             SV_LAUNCHED(c);
         }
     }
@@ -1725,7 +1969,6 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
             SV_LAUNCHED(c);
             S.far = F.far;
         } else if (L >= 2) {
-            SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_rel, 0));  // the leaf offsets of the second stream
             l2p_kernel<P><<<div_up(V.nbox, kWarps), kWarps * 32, 0, c->stream>>>(
                 V.nbox, nullptr, nullptr, V.start, F.rel, S.qm, S.root, L, F.nrm, Lv[L], fx, fy, fz, tgt[L], 0);
             SV_LAUNCHED(c);
@@ -1763,7 +2006,7 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
     Tree &T = *F.ftree;
     int *nbd = fa.d_nbox;
     SV_TRY(tree_build_forest(c, T, f, nbd, fa.d_err));
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 4 * sizeof(unsigned long long), c->stream));
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 5 * sizeof(unsigned long long), c->stream));
     // Two streams, as in run_fmm: target flags, lists and the near field on the
     // second (the forest's slots only: the direct plumes' slots belong to
     // another stream), the upward and downward passes on the main one.
@@ -1970,7 +2213,6 @@ void fmm_free(sv_ctx *c) {
     if (F.ev_fork) cudaEventDestroy(F.ev_fork);
     if (F.ev_join) cudaEventDestroy(F.ev_join);
     if (F.ev_lists) cudaEventDestroy(F.ev_lists);
-    if (F.ev_m2l_lists) cudaEventDestroy(F.ev_m2l_lists);
     if (F.ev_rel) cudaEventDestroy(F.ev_rel);
     for (cudaEvent_t e : F.ev_near)
         if (e) cudaEventDestroy(e);
@@ -1983,13 +2225,12 @@ static sv_status fmm_state(sv_ctx *c) {
     if (!c->fmm) {
         c->fmm = new Fmm();
         Fmm &F = *c->fmm;
-        SV_CK(c, cudaMalloc(&F.d_counts, 4 * sizeof(unsigned long long)));
+        SV_CK(c, cudaMalloc(&F.d_counts, 5 * sizeof(unsigned long long)));
         SV_CK(c, cudaMallocHost(&F.h_counts, 2 * sizeof(unsigned long long)));
         SV_CK(c, cudaStreamCreateWithFlags(&F.side, cudaStreamNonBlocking));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_fork, cudaEventDisableTiming));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_join, cudaEventDisableTiming));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_lists, cudaEventDisableTiming));
-        SV_CK(c, cudaEventCreateWithFlags(&F.ev_m2l_lists, cudaEventDisableTiming));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_rel, cudaEventDisableTiming));
         SV_CK(c, cudaEventCreate(&F.ev_near[0]));
         SV_CK(c, cudaEventCreate(&F.ev_near[1]));
