@@ -343,48 +343,58 @@ struct Pair64Args {
 };
 
 // Every unordered pair once, as the mixed kernel: one particle per lane against
-// a tile of 32 that travels around the lanes with its sums.  FP64-pipe bound (20
-// operations per pair of interactions; shuffles, loads and atomics are free
-// beside them).
+// a tile of 32 that travels around the lanes with its sums.  FP64-pipe bound: 20
+// operations per pair of interactions, 18 where the charges of both tiles are equal
+// (UQ) and are applied once after the tile; shuffles, loads and atomics are free
+// beside them.
+template <bool UQ, bool SYM>
+__device__ __forceinline__ void pair64_tile(double xi, double yi, double zi, double qi, double xj, double yj,
+                                            double zj, double qj, double eps2, double (&f)[3], double (&g)[3]) {
+    const int from = ((threadIdx.x & 31) + 1) & 31;
+#pragma unroll 2
+    for (int step = 0; step < 32; step++) {
+        const double dx = xi - xj, dy = yi - yj, dz = zi - zj;
+        const double w = inv_cube_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+        const double wi = UQ ? w : qj * w;
+        f[0] = fma(dx, wi, f[0]);
+        f[1] = fma(dy, wi, f[1]);
+        f[2] = fma(dz, wi, f[2]);
+        if (SYM) {
+            const double wj = UQ ? -w : -(qi * w);
+            g[0] = __shfl_sync(0xffffffffu, fma(dx, wj, g[0]), from);
+            g[1] = __shfl_sync(0xffffffffu, fma(dy, wj, g[1]), from);
+            g[2] = __shfl_sync(0xffffffffu, fma(dz, wj, g[2]), from);
+        }
+        xj = __shfl_sync(0xffffffffu, xj, from);
+        yj = __shfl_sync(0xffffffffu, yj, from);
+        zj = __shfl_sync(0xffffffffu, zj, from);
+        if (!UQ) qj = __shfl_sync(0xffffffffu, qj, from);
+    }
+}
+
 template <bool SYM>
 __device__ __forceinline__ void pair64_unit(const Pair64Args &a, int A, int B) {
     const int lane = threadIdx.x & 31, i = 32 * A + lane, j = 32 * B + lane;
     const int ii = min(i, a.n - 1), jj = min(j, a.n - 1);
     const bool it = i < a.n && a.qm[ii] != 0.0, jt = SYM && j < a.n && a.qm[jj] != 0.0;
     if (!__any_sync(0xffffffffu, it || jt)) return;
-    const double xi = a.x[ii], yi = a.y[ii], zi = a.z[ii];
-    const double qi = i < a.n ? (double)a.q[ii] : 0.0;  // absent particles carry no charge
-    double xj = a.x[jj], yj = a.y[jj], zj = a.z[jj], qj = j < a.n ? (double)a.q[jj] : 0.0;
-    double fx = 0.0, fy = 0.0, fz = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-    const int from = (lane + 1) & 31;
-#pragma unroll 2
-    for (int step = 0; step < 32; step++) {
-        const double dx = xi - xj, dy = yi - yj, dz = zi - zj;
-        const double w = inv_cube_f64(fma(dx, dx, fma(dy, dy, fma(dz, dz, a.eps2))));
-        const double wi = qj * w;
-        fx = fma(dx, wi, fx);
-        fy = fma(dy, wi, fy);
-        fz = fma(dz, wi, fz);
-        if (SYM) {
-            const double wj = -(qi * w);
-            gx = __shfl_sync(0xffffffffu, fma(dx, wj, gx), from);
-            gy = __shfl_sync(0xffffffffu, fma(dy, wj, gy), from);
-            gz = __shfl_sync(0xffffffffu, fma(dz, wj, gz), from);
-        }
-        xj = __shfl_sync(0xffffffffu, xj, from);
-        yj = __shfl_sync(0xffffffffu, yj, from);
-        zj = __shfl_sync(0xffffffffu, zj, from);
-        qj = __shfl_sync(0xffffffffu, qj, from);
-    }
+    // absent particles carry no charge
+    const double qi = i < a.n ? (double)a.q[ii] : 0.0, qj = j < a.n ? (double)a.q[jj] : 0.0;
+    const double q0 = __shfl_sync(0xffffffffu, qi, 0);
+    const bool equal = __all_sync(0xffffffffu, qi == q0 && qj == q0);
+    double f[3] = {0.0, 0.0, 0.0}, g[3] = {0.0, 0.0, 0.0};
+    if (equal) pair64_tile<true, SYM>(a.x[ii], a.y[ii], a.z[ii], qi, a.x[jj], a.y[jj], a.z[jj], qj, a.eps2, f, g);
+    else pair64_tile<false, SYM>(a.x[ii], a.y[ii], a.z[ii], qi, a.x[jj], a.y[jj], a.z[jj], qj, a.eps2, f, g);
+    const double k = equal ? q0 : 1.0;
     if (it) {
-        atomicAdd(&a.ax[i], fx);
-        atomicAdd(&a.ay[i], fy);
-        atomicAdd(&a.az[i], fz);
+        atomicAdd(&a.ax[i], f[0] * k);
+        atomicAdd(&a.ay[i], f[1] * k);
+        atomicAdd(&a.az[i], f[2] * k);
     }
     if (jt) {
-        atomicAdd(&a.ax[j], gx);
-        atomicAdd(&a.ay[j], gy);
-        atomicAdd(&a.az[j], gz);
+        atomicAdd(&a.ax[j], g[0] * k);
+        atomicAdd(&a.ay[j], g[1] * k);
+        atomicAdd(&a.az[j], g[2] * k);
     }
 }
 

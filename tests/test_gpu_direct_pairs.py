@@ -72,3 +72,15 @@ def test_images(sym, n, prec):
         kw = dict(symmetry=sv.SYM_TRANSLATIONAL, sym_axes=(1, 1, 0), sym_levels=1, domain_size=(2e-6, 2e-6, 0.0))
     a = accel(st, softening2=EPS20, precision=prec, **kw)
     assert rel_l2(a, ref, st["status"]) < BOUND[prec]
+
+
+@pytest.mark.parametrize("n", [64, 97, 1024])
+def test_fp64_tiles_of_equal_charges(n):
+    """Charges that differ between regions only: pairs of tiles with one charge take the
+    sum without them, pairs of tiles with two do not; source-only and ignored particles mixed in."""
+    st = state(n, False, 90 + n)
+    st["q"] = np.where(st["x"] < np.median(st["x"]), 2.0, -1.0)
+    st["status"][5::17] = 2
+    st["status"][7::19] = 0
+    a = accel(st, softening2=EPS20, precision=sv.FP64)
+    assert rel_l2(a, O.direct_f64(st, EPS20), st["status"]) < BOUND[sv.FP64]
