@@ -60,3 +60,30 @@ def test_forest_near_field_alone():
         n = st["q"].size
         assert rel_l2(a[o:o + n], O.direct_f64(st, EPS20), st["status"]) < 1e-5
         o += n
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("ws", [1, 2])
+@pytest.mark.parametrize("n", [1, 40, 129, 700, 3001])
+def test_images_leave_the_targets_lanes(n, ws, mixed):
+    """Boxes of image copies and targets together: the targets alone are gathered (one or
+    several rounds of 128 particles, one or several chunks), the images and source-only
+    particles pull.  The cube sits on the rotation axis, so that every box holds all four
+    quadrants' copies."""
+    st = cube(max(n, 2), 900 + n)
+    st["x"][:, :2] -= 2.0 ** -24
+    if n == 1:
+        st["status"][1:] = 2
+    if mixed:
+        rng = np.random.default_rng(n)
+        st["q"] = rng.choice([1.0, 2.0, -1.0], st["q"].size)
+        st["status"][1:] = rng.choice(np.array([1, 2], np.int32), st["q"].size - 1, p=[0.5, 0.5])
+    ref = O.direct_f64(st, EPS20, sym=1)
+    with sv.ForceMethod(softening2=EPS20, method=sv.FMM, symmetry=sv.SYM_ROTATIONAL, fmm_order=4, fmm_ws=ws,
+                        fmm_root_scale=1.875, fmm_leaf_target=4096) as fm:
+        fm.upload(st)
+        a = fm.accel()
+        s = fm.stats()
+    assert s.cell_interactions == 0
+    assert rel_l2(a, ref, st["status"]) < 2e-6
+    assert not np.any(a[st["status"] != 1])
