@@ -45,7 +45,7 @@ namespace sv {
 constexpr int kBatchBits = 18;       // Morton bits per axis below the plume id
 constexpr int kPidShift = 3 * kBatchBits;
 constexpr int kMaxPlumes = 512;      // plume ids use bits 54..62; bit 63 stays clear
-constexpr int kChunk = 8192;         // view slots per bounding-box partial
+constexpr int kChunk = 1024;         // view slots per bounding-box partial, four per thread
 constexpr int kBLevels = kMortonBits + 1;
 
 struct DirectItem {
@@ -62,11 +62,11 @@ struct Batch {
     int64_t nv = 0, nf = 0;           // view slots; FMM slots (the first nf)
     uint32_t *vsrc = nullptr;         // view slot -> caller particle
     uint32_t *vtag = nullptr;         // view slot -> plume id * 4 + image
-    double *roots = nullptr;          // [8 * np]
+    double *roots = nullptr;          // [8 * np] root records, [np] Morton cells per unit of length
     int *delta = nullptr;             // [np] cube enlargement exponents of the last evaluation
     std::vector<int> h_delta;
     int *d_hist = nullptr;            // [nfp * kBLevels] split-level histogram per FMM plume
-    int *d_vbeg = nullptr;            // [np + 1] first view slot per plume id
+    int *d_vbeg = nullptr;            // [np + 1] first view slot per plume id, [np] its slots per particle
     int nchunks = 0;
     int *chunk_beg = nullptr;         // [nchunks + 1]
     int *pid_chunk = nullptr;         // [np + 1]
@@ -133,29 +133,43 @@ __device__ __forceinline__ void slot_pos(uint32_t i, uint32_t tag, const double 
     }
 }
 
-__global__ void bbox_chunks_kernel(const int *__restrict__ chunk_beg, const uint32_t *__restrict__ vsrc,
-                                   const uint32_t *__restrict__ vtag, const double *__restrict__ x,
-                                   const double *__restrict__ y, const double *__restrict__ z,
-                                   const int32_t *__restrict__ st, double *__restrict__ red) {
+// Bounds of each chunk's sources, as ordered integers (no FP64 operation).  A
+// chain of dependent loads per slot (slot -> particle -> position): four slots
+// per thread in 1,284 CTAs where 31 per thread in 173 took 86 us (24 plumes,
+// 1,313,906 slots).
+constexpr int kBoundThreads = 256;
+__global__ void __launch_bounds__(kBoundThreads)
+bbox_chunks_kernel(const int *__restrict__ chunk_beg, const uint32_t *__restrict__ vsrc,
+                   const uint32_t *__restrict__ vtag, const double *__restrict__ x, const double *__restrict__ y,
+                   const double *__restrict__ z, const int32_t *__restrict__ st, double *__restrict__ red) {
+    constexpr int PER = kChunk / kBoundThreads, W = kBoundThreads / 32;
     const int b0 = chunk_beg[blockIdx.x], b1 = chunk_beg[blockIdx.x + 1];
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int v = b0 + threadIdx.x; v < b1; v += blockDim.x) {
-        const uint32_t i = vsrc[v];
-        if (!is_src(st[i])) continue;
+    const long long lo0 = ordered_bits(__double_as_longlong(1e300)), hi0 = ordered_bits(__double_as_longlong(-1e300));
+    long long mn[3] = {lo0, lo0, lo0}, mx[3] = {hi0, hi0, hi0};
+    uint32_t src[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) src[k] = vsrc[min(b0 + (int)threadIdx.x + k * kBoundThreads, b1 - 1)];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const uint32_t i = src[k];
+        const int v = b0 + threadIdx.x + k * kBoundThreads;
+        if (v >= b1 || !is_src(st[i])) continue;
         double p[3] = {x[i], y[i], z[i]};
         rot_image((int)(vtag[v] & 3u), p[0], p[1]);
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            mn[d] = fmin(mn[d], p[d]);
-            mx[d] = fmax(mx[d], p[d]);
+            const long long o = ordered_bits(__double_as_longlong(p[d]));
+            if (ordered_nan(o)) continue;
+            mn[d] = min(mn[d], o);
+            mx[d] = max(mx[d], o);
         }
     }
-    __shared__ double sh[6][8];
+    __shared__ long long sh[6][W];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         for (int o = 16; o > 0; o >>= 1) {
-            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+            mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+            mx[d] = max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
     }
     const int w = threadIdx.x >> 5;
@@ -168,24 +182,30 @@ __global__ void bbox_chunks_kernel(const int *__restrict__ chunk_beg, const uint
     __syncthreads();
     if (threadIdx.x < 6) {
         const int d = threadIdx.x;
-        double v = d < 3 ? 1e300 : -1e300;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) v = d < 3 ? fmin(v, sh[d][k]) : fmax(v, sh[d][k]);
-        red[blockIdx.x * 6 + d] = v;
+        long long v = sh[d][0];
+        for (int k = 1; k < W; k++) v = d < 3 ? min(v, sh[d][k]) : max(v, sh[d][k]);
+        red[blockIdx.x * 6 + d] = __longlong_as_double(ordered_bits(v));
     }
 }
 
-// Root record per plume: origin = bbox min, side = smallest power of two
-// above the largest extent, bbox max, empty flag.
+// Root record per plume, one warp each: origin = bbox min, side = smallest power
+// of two above the largest extent, bbox max, empty flag.
 __global__ void plume_roots_kernel(int np, const int *__restrict__ pid_chunk, const double *__restrict__ red,
                                    double *__restrict__ roots) {
-    const int pid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int pid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (pid >= np) return;
     double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300};
-    for (int k = pid_chunk[pid]; k < pid_chunk[pid + 1]; k++)
+    for (int k = pid_chunk[pid] + lane; k < pid_chunk[pid + 1]; k += 32)
         for (int d = 0; d < 3; d++) {
             mn[d] = fmin(mn[d], red[6 * k + d]);
             mx[d] = fmax(mx[d], red[6 * k + 3 + d]);
         }
+    for (int d = 0; d < 3; d++)
+        for (int o = 16; o > 0; o >>= 1) {
+            mn[d] = fmin(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
+            mx[d] = fmax(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+        }
+    if (lane) return;
     const bool empty = mn[0] > mx[0];
     double ext = 0.0;
     if (empty) {
@@ -208,6 +228,7 @@ __global__ void plume_roots_kernel(int np, const int *__restrict__ pid_chunk, co
     r[5] = mx[1];
     r[6] = mx[2];
     r[7] = empty ? 1.0 : 0.0;
+    roots[8 * np + pid] = (double)(1u << kBatchBits) / S;
 }
 
 __device__ __forceinline__ uint64_t spread3_18(uint32_t v) {
@@ -220,7 +241,11 @@ __device__ __forceinline__ uint64_t spread3_18(uint32_t v) {
     return x;
 }
 
-__global__ void batch_keys_kernel(int64_t nv, const uint32_t *__restrict__ vsrc, const uint32_t *__restrict__ vtag,
+// Nine FP64 operations per slot (GB300 issues two per clock and SM): the cells per
+// length come with the roots and the cell from one round-down conversion
+// (saturating) and integer clamps; a division, floor, fmax and fmin per slot took
+// 73 us for 1,313,906 slots.
+__global__ void batch_keys_kernel(int np, int64_t nv, const uint32_t *__restrict__ vsrc, const uint32_t *__restrict__ vtag,
                                   const double *__restrict__ x, const double *__restrict__ y,
                                   const double *__restrict__ z, const int32_t *__restrict__ st,
                                   const double *__restrict__ roots, uint64_t *__restrict__ keys,
@@ -232,13 +257,12 @@ __global__ void batch_keys_kernel(int64_t nv, const uint32_t *__restrict__ vsrc,
     bool src;
     slot_pos(i, tag, x, y, z, st, roots, p[0], p[1], p[2], src);
     const double *r = roots + 8 * (tag >> 2);
-    const double inv = (double)(1u << kBatchBits) / r[3];
+    const double inv = roots[8 * np + (tag >> 2)];
     uint32_t cc[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        double f = floor((p[d] - r[d]) * inv);
-        f = fmin(fmax(f, 0.0), (double)((1u << kBatchBits) - 1));
-        cc[d] = (uint32_t)f;
+        const int f = __double2int_rd((p[d] - r[d]) * inv);
+        cc[d] = (uint32_t)min(max(f, 0), (int)((1u << kBatchBits) - 1));
     }
     keys[v] = ((uint64_t)(tag >> 2) << kPidShift) | spread3_18(cc[0]) | (spread3_18(cc[1]) << 1) |
               (spread3_18(cc[2]) << 2);
@@ -316,23 +340,27 @@ __global__ void __launch_bounds__(256) plume_levels_kernel(const uint64_t *__res
 // with the occupied boxes' growth ratio g_k = boxes(k) / boxes(k-1) giving the
 // dimension d_k = log2(g_k) in which the plume is resolved at level k (1 for a
 // thin filament, 3 for a bulk), near boxes (2ws+1)^d and M2L boxes
-// (4ws+2)^d - (2ws+1)^d per box, pairs = n * occupancy * near.  W is the cost
-// of one M2L in pair units (tuned).  Levels below an occupancy of 2 are not
-// considered.
-__host__ __device__ inline int pick_level(double np_slots, const long long *boxes, double w, int ws) {
+// (4ws+2)^d - (2ws+1)^d per box, pairs = targets * occupancy * near (an image
+// slot is no target).  W is the cost of one M2L in pair units (tuned).  Levels
+// below an occupancy of 2 are not considered.
+__host__ __device__ inline void level_boxes_near_far(double nb, double nb_parent, int ws, double &near, double &far) {
     const double a = 2.0 * ws + 1.0, b = 4.0 * ws + 2.0;
+    double g = nb / nb_parent;
+    g = g < 1.0 ? 1.0 : (g > 8.0 ? 8.0 : g);
+    const double d = log2(g);
+    near = pow(a, d);
+    far = pow(b, d) - near;
+}
+inline int pick_level(double slots, int per_particle, const long long *boxes, double w, int ws) {
     int best = 2;
     double bestc = 1e300, m2l = 0.0;
     for (int l = 2; l <= kBatchBits; l++) {
-        const double nb = (double)boxes[l];
-        double g = nb / (double)boxes[l - 1];
-        g = g < 1.0 ? 1.0 : (g > 8.0 ? 8.0 : g);
-        const double d = log2(g);
-        const double near = pow(a, d), far = pow(b, d) - near;
+        const double nb = (double)boxes[l], occ = slots / nb;
+        double near, far;
+        level_boxes_near_far(nb, (double)boxes[l - 1], ws, near, far);
         m2l += nb * far;
-        const double occ = np_slots / nb;
         if (occ < 2.0 && l > 2) break;
-        const double cost = np_slots * occ * near + w * m2l;
+        const double cost = slots / per_particle * occ * near + w * m2l;
         if (cost < bestc) {
             bestc = cost;
             best = l;
@@ -341,17 +369,44 @@ __host__ __device__ inline int pick_level(double np_slots, const long long *boxe
     return best;
 }
 
-// Per FMM plume: its own leaf level Lp, delta = L - Lp, and the root side
-// scaled by 2^delta.
-__global__ void choose_delta_kernel(int nfp, const int *__restrict__ hist, const int *__restrict__ vbeg, int L,
-                                    double w, int ws, int *__restrict__ delta, double *__restrict__ roots) {
-    const int pid = blockIdx.x * blockDim.x + threadIdx.x;
+// Per FMM plume: its own leaf level Lp, delta = L - Lp, and the root side scaled
+// by 2^delta.  One warp per plume, one lane per level: the powers and logarithms
+// (FP64) of a level are independent of the other levels' (a thread per plume
+// took 74 us, whatever the number of plumes).  Only levels up to `top`, which the
+// keys are sorted to, are considered.
+__global__ void choose_delta_kernel(int np, int nfp, const int *__restrict__ hist, const int *__restrict__ vbeg, int L,
+                                    int top, double w, int ws, int *__restrict__ delta,
+                                    double *__restrict__ roots) {
+    const int pid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (pid >= nfp) return;
-    const double np_slots = (double)(vbeg[pid + 1] - vbeg[pid]);
-    long long boxes[kBatchBits + 1];
-    boxes[0] = 1;
-    for (int l = 1; l <= kBatchBits; l++) boxes[l] = boxes[l - 1] + hist[pid * kBLevels + l];
-    const int lp = pick_level(np_slots, boxes, w, ws);
+    const double slots = (double)(vbeg[pid + 1] - vbeg[pid]);
+    int boxes = l == 0 ? 1 : l <= kBatchBits ? hist[pid * kBLevels + l] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, boxes, o);
+        if (l >= o) boxes += t;
+    }
+    const int parent = __shfl_up_sync(0xffffffffu, boxes, 1);
+    const double nb = (double)boxes, occ = slots / nb;
+    double near, far;
+    level_boxes_near_far(nb, (double)max(parent, 1), ws, near, far);
+    double m2l = 0.0;
+    for (int k = 2; k <= kBatchBits; k++) {
+        const double v = __shfl_sync(0xffffffffu, nb * far, k);
+        if (k <= l) m2l += v;
+    }
+    double cost = 1e300;
+    if (l == 2 || (l > 2 && l <= top && occ >= 2.0)) cost = slots / vbeg[np + 1 + pid] * occ * near + w * m2l;
+    int lp = l;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double oc = __shfl_xor_sync(0xffffffffu, cost, o);
+        const int ol = __shfl_xor_sync(0xffffffffu, lp, o);
+        if (oc < cost || (oc == cost && ol < lp)) {
+            cost = oc;
+            lp = ol;
+        }
+    }
+    if (l) return;
+    if (!(cost < 1e300)) lp = 2;
     const int d = L > lp ? L - lp : 0;
     delta[pid] = d;
     roots[8 * pid + 3] = ldexp(roots[8 * pid + 3], d);
@@ -496,6 +551,12 @@ sv_status build_items(sv_ctx *c, Batch &B) {
     return SV_OK;
 }
 
+// view slots per particle of an FMM plume: its quadrants' images are slots too
+int slots_per_particle(const Batch &B, int pid) {
+    const int p = B.plume_of[pid];
+    return B.method[p] == SV_METHOD_FMM && B.sym[p] == SV_SYM_ROTATIONAL ? 4 : 1;
+}
+
 // bbox, roots, keys, sort, (adapt: per-plume depth), gather (launches only)
 sv_status sort_batch(sv_ctx *c, Batch &B, bool adapt) {
     Sorted &S = c->S;
@@ -503,22 +564,30 @@ sv_status sort_batch(sv_ctx *c, Batch &B, bool adapt) {
     bbox_chunks_kernel<<<B.nchunks, 256, 0, c->stream>>>(B.chunk_beg, B.vsrc, B.vtag, c->x, c->y, c->z, force_status(c),
                                                          B.chunk_red);
     SV_LAUNCHED(c);
-    plume_roots_kernel<<<div_up(B.np, 128), 128, 0, c->stream>>>(B.np, B.pid_chunk, B.chunk_red, B.roots);
+    plume_roots_kernel<<<div_up(B.np, 4), 128, 0, c->stream>>>(B.np, B.pid_chunk, B.chunk_red, B.roots);
     SV_LAUNCHED(c);
-    batch_keys_kernel<<<div_up(nv, 256), 256, 0, c->stream>>>(nv, B.vsrc, B.vtag, c->x, c->y, c->z, force_status(c),
+    batch_keys_kernel<<<div_up(nv, 256), 256, 0, c->stream>>>(B.np, nv, B.vsrc, B.vtag, c->x, c->y, c->z, force_status(c),
                                                               B.roots, S.keys_alt, S.idx_alt);
     SV_LAUNCHED(c);
+    // An evaluation uses the boxes of levels up to L in each plume's own cube, and one
+    // level more for its choice of level; order below that and bits no plume id
+    // has take no sort pass (24 plumes, L = 9: 35 of 63 bits, five passes of 19 us
+    // instead of eight).
+    const int top = adapt && B.fa.spec.L > 0 ? std::min(kBatchBits, B.fa.spec.L + 1) : kBatchBits;
+    const int bit0 = 3 * (kBatchBits - top);
+    int bit1 = kPidShift;
+    while ((1 << (bit1 - kPidShift)) < B.np) bit1++;
     size_t bytes = B.cub_bytes;
-    SV_CK(c, cub::DeviceRadixSort::SortPairs(B.cub_tmp, bytes, S.keys_alt, S.keys, S.idx_alt, S.idx, (int)nv, 0,
-                                             kPidShift + 9, c->stream));
-    c->launches += 2 * ((kPidShift + 9 + 7) / 8);
+    SV_CK(c, cub::DeviceRadixSort::SortPairs(B.cub_tmp, bytes, S.keys_alt, S.keys, S.idx_alt, S.idx, (int)nv, bit0,
+                                             bit1, c->stream));
+    c->launches += 2 * ((bit1 - bit0 + 7) / 8);
     if (adapt && B.nfp > 0 && B.nf > 0) {
         SV_CK(c, cudaMemsetAsync(B.d_hist, 0, sizeof(int) * kBLevels * B.nfp, c->stream));
         plume_levels_kernel<<<div_up(B.nf, 256), 256, 0, c->stream>>>(S.keys, B.nf, B.d_hist);
         SV_LAUNCHED(c);
-        choose_delta_kernel<<<div_up(B.nfp, 128), 128, 0, c->stream>>>(B.nfp, B.d_hist, B.d_vbeg, B.fa.spec.L,
-                                                                       (double)B.m2l_weight, c->P.fmm_ws, B.delta,
-                                                                       B.roots);
+        choose_delta_kernel<<<div_up(B.nfp, 4), 128, 0, c->stream>>>(B.np, B.nfp, B.d_hist, B.d_vbeg, B.fa.spec.L, top,
+                                                                     (double)B.m2l_weight, c->P.fmm_ws, B.delta,
+                                                                     B.roots);
         SV_LAUNCHED(c);
         shift_keys_kernel<<<div_up(B.nf, 256), 256, 0, c->stream>>>(S.keys, B.nf, B.delta);
         SV_LAUNCHED(c);
@@ -582,8 +651,8 @@ sv_status plan_forest(sv_ctx *c, Batch &B, int cap_scale) {
             if (l > 0) acc += hist[(size_t)pid * kBLevels + l];
             boxes[pid][l] = acc;
         }
-        Lp[pid] = pick_level((double)(B.vbeg[pid + 1] - B.vbeg[pid]), boxes[pid].data(), (double)B.m2l_weight,
-                             c->P.fmm_ws);
+        Lp[pid] = pick_level((double)(B.vbeg[pid + 1] - B.vbeg[pid]), slots_per_particle(B, pid), boxes[pid].data(),
+                             (double)B.m2l_weight, c->P.fmm_ws);
     }
     // one level of headroom: a plume that contracts can still deepen
     int L = 2;
@@ -611,7 +680,7 @@ sv_status plan_forest(sv_ctx *c, Batch &B, int cap_scale) {
     B.fa.ws = c->P.fmm_ws;
     B.fa.nroots = B.nfp;
     B.fa.images = false;
-    for (int pid = 0; pid < B.nfp; pid++) B.fa.images |= B.sym[B.plume_of[pid]] == SV_SYM_ROTATIONAL;
+    for (int pid = 0; pid < B.nfp; pid++) B.fa.images |= slots_per_particle(B, pid) > 1;
     B.fa.roots = B.roots;
     B.fa.d_nbox = B.d_nbox;
     B.fa.d_err = B.d_err;
@@ -760,7 +829,7 @@ sv_status batch_plan(sv_ctx *c, int32_t np, const int64_t *counts, const int32_t
     B.vbeg.assign(np + 1, 0);
     for (int pid = 0; pid < np; pid++) {
         const int p = B.plume_of[pid];
-        const int nimg = (method[p] == SV_METHOD_FMM && sym[p] == SV_SYM_ROTATIONAL) ? 4 : 1;
+        const int nimg = slots_per_particle(B, pid);
         B.vbeg[pid + 1] = B.vbeg[pid] + counts[p] * nimg;
     }
     B.nv = B.vbeg[np];
@@ -790,14 +859,15 @@ sv_status batch_plan(sv_ctx *c, int32_t np, const int64_t *counts, const int32_t
     const size_t nvb = (size_t)std::max<int64_t>(B.nv, 1);
     SV_CK(c, cudaMalloc(&B.vsrc, sizeof(uint32_t) * nvb));
     SV_CK(c, cudaMalloc(&B.vtag, sizeof(uint32_t) * nvb));
-    SV_CK(c, cudaMalloc(&B.roots, sizeof(double) * 8 * np));
+    SV_CK(c, cudaMalloc(&B.roots, sizeof(double) * 9 * np));
     SV_CK(c, cudaMalloc(&B.delta, sizeof(int) * np));
     SV_CK(c, cudaMemset(B.delta, 0, sizeof(int) * np));
     SV_CK(c, cudaMalloc(&B.d_hist, sizeof(int) * kBLevels * std::max(B.nfp, 1)));
-    SV_CK(c, cudaMalloc(&B.d_vbeg, sizeof(int) * (np + 1)));
+    SV_CK(c, cudaMalloc(&B.d_vbeg, sizeof(int) * (2 * np + 1)));
     {
         std::vector<int> vb(B.vbeg.begin(), B.vbeg.end());
-        SV_CK(c, cudaMemcpy(B.d_vbeg, vb.data(), sizeof(int) * (np + 1), cudaMemcpyHostToDevice));
+        for (int pid = 0; pid < np; pid++) vb.push_back(slots_per_particle(B, pid));
+        SV_CK(c, cudaMemcpy(B.d_vbeg, vb.data(), sizeof(int) * vb.size(), cudaMemcpyHostToDevice));
     }
     SV_CK(c, cudaMalloc(&B.chunk_beg, sizeof(int) * cbeg.size()));
     SV_CK(c, cudaMalloc(&B.pid_chunk, sizeof(int) * (np + 1)));

@@ -1068,6 +1068,7 @@ l2p_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ bpid, 
            double *__restrict__ ay, double *__restrict__ az, const int *__restrict__ has_tgt, int accumulate) {
     constexpr int NC = ncoef(P);
     __shared__ float2 lam[kWarps][NC];
+    __shared__ int wait[kWarps][64];
     SV_WARP_BOXES(kWarps) {
     const double *root = box_root(roots, bpid, b);
     if (!has_tgt[b]) {
@@ -1087,8 +1088,37 @@ l2p_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ bpid, 
     // pipe (1/64 of its rate on this GPU) sees only the stores' conversions.
     const double h = root[3] / (double)(1 << level);
     const float ihf = (float)(1.0 / h), mih2 = (float)(-1.0 / (h * h));
+    // Rounds of 32 particles; where the box holds more than targets (image copies), of
+    // 32 targets gathered first.
     const int s1 = start[b + 1];
-    for (int i = start[b] + lane; i < s1; i += 32) {
+    const bool some = has_tgt[b] < s1 - start[b];
+    int have = 0;
+    for (int next = start[b];;) {
+        int i = next + lane;
+        bool live = i < s1;
+        if (some) {
+            while (have < 32 && next < s1) {
+                const int k = next + lane;
+                const bool f = k < s1 && qm[k] != 0.0;
+                const unsigned bal = __ballot_sync(0xffffffffu, f);
+                if (f) wait[wid][have + __popc(bal & ((1u << lane) - 1u))] = k;
+                have += __popc(bal);
+                next += 32;
+                __syncwarp();
+            }
+            if (have == 0) break;
+            live = lane < have;
+            i = wait[wid][lane];
+            const int left = lane + 32 < have ? wait[wid][lane + 32] : 0;
+            __syncwarp();
+            wait[wid][lane] = left;
+            have = max(have - 32, 0);
+            __syncwarp();
+        } else {
+            if (next >= s1) break;
+            next += 32;
+        }
+        if (!live) continue;
         float2 R[ncoef(P - 1) > 0 ? ncoef(P - 1) : 1];
         const float4 r = rel[i];
         solid_harmonics<P - 1>(r.x * ihf, r.y * ihf, r.z * ihf, R);

@@ -20,16 +20,6 @@ constexpr int kRedThreads = 256;
 
 __device__ __forceinline__ bool is_source(int32_t s) { return s == 1 || s == 2; }
 
-// A double's bits as a signed integer whose order is the double's order
-// (non-NaN values); the map is its own inverse.  Min / max on these run on
-// the integer pipe: GB300's FP64 pipe issues ~2 operations per clock per SM,
-// which made the FP64 fmin / fmax the bound of this reduction.
-__device__ __forceinline__ long long ordered_bits(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
-
-__device__ __forceinline__ bool ordered_nan(long long v) {
-    return (ordered_bits(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
-}
-
 constexpr double kBig = 1e300;  // bounds of an empty set
 
 // Reduce (mn, mx) over a CTA of NT threads into threads 0..5 of the first

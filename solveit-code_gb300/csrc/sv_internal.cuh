@@ -304,6 +304,16 @@ void direct_sort_wants(sv_ctx *c);
 cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, int n, float eps2, double *ax, double *ay,
                                        double *az, const int *charges_differ, cudaStream_t stream);
 
+// A double's bits as a signed integer whose order is the double's order
+// (non-NaN values); the map is its own inverse.  Min / max on these run on
+// the integer pipe: GB300's FP64 pipe issues ~2 operations per clock per SM,
+// which made the FP64 fmin / fmax the bound of the bounding-box reductions.
+__device__ __forceinline__ long long ordered_bits(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
+
+__device__ __forceinline__ bool ordered_nan(long long v) {
+    return (ordered_bits(v) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+
 // a double as FP32 hi + lo parts (48 bits)
 __device__ __forceinline__ void split_hilo(double v, float &hi, float &lo) {
     hi = (float)v;
