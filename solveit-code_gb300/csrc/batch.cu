@@ -679,8 +679,6 @@ sv_status plan_forest(sv_ctx *c, Batch &B, int cap_scale) {
     B.fa.p = c->P.fmm_order;
     B.fa.ws = c->P.fmm_ws;
     B.fa.nroots = B.nfp;
-    B.fa.images = false;
-    for (int pid = 0; pid < B.nfp; pid++) B.fa.images |= slots_per_particle(B, pid) > 1;
     B.fa.roots = B.roots;
     B.fa.d_nbox = B.d_nbox;
     B.fa.d_err = B.d_err;

@@ -43,6 +43,9 @@
 
 namespace sv {
 
+constexpr int kItemClasses = 32;           // near-field work items by log2 of their estimated pairs
+constexpr int kCounts = 6 + kItemClasses;  // words of Fmm::d_counts
+
 struct Fmm {
     int p = 0, ws = 0;
     int trim = 0;  // trimmed near field (sv_params.fmm_near = 2 at ws = 2) for the next evaluation
@@ -57,7 +60,8 @@ struct Fmm {
     void *arena = nullptr;
     size_t arena_bytes = 0;
     unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue,
-                                             // [4] finished target-flag CTAs
+                                             // [4] finished target-flag CTAs, [5] P2P work items, then per size
+                                             // class of them (ints) their number and the number placed
     unsigned long long *h_counts = nullptr;
     // caller particles followed by their source-only symmetry images
     double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr;
@@ -79,6 +83,7 @@ struct Fmm {
     int2 *flst[kMortonBits + 1] = {};
     int *ffd = nullptr, *ffd_cnt = nullptr;  // far-direct lists of the forest's leaf boxes
     float4 *frel = nullptr;
+    int2 *fitems = nullptr;  // near field's work items (box, chunk), largest first
     int64_t frel_cap = 0;
     // the near field runs on its own stream beside the upward and downward passes
     cudaStream_t side = nullptr;
@@ -393,16 +398,6 @@ __global__ void expand_images_kernel(const double *__restrict__ x, const double 
 // box holds at least one target (K q/m != 0).  Forest: leaf level from particles,
 // coarser levels from children, a launch each (its box counts are only known on
 // the device, and its launches are cheap graph nodes)
-__global__ void leaf_targets_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ start,
-                                    const double *__restrict__ qm, int *__restrict__ flag) {
-    SV_WARP_BOXES(kWarps) {
-        int f = 0;
-        for (int j = start[b] + lane; j < start[b + 1]; j += 32) f += qm[j] != 0.0;
-        f = __reduce_add_sync(0xffffffffu, f);
-        if (lane == 0) flag[b] = f;
-    }
-}
-
 __global__ void parent_targets_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ child0,
                                       const int *__restrict__ cflag, int *__restrict__ flag) {
     const int nb = level_boxes(nbox, nbd);
@@ -1418,7 +1413,7 @@ __device__ __forceinline__ int p2p_chunks(int nt, int parts) {
 
 template <int WS, bool CLAMP, bool UQ, bool SOME>
 __device__ __forceinline__ void
-p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, const int *__restrict__ bpid, const int *__restrict__ start,
+p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, int stride, const int *__restrict__ bpid, const int *__restrict__ start,
          const int4 *__restrict__ coord, const int *__restrict__ nbr, const double *__restrict__ qm,
          const double *__restrict__ roots, int level, float eps2, double *__restrict__ ax, double *__restrict__ ay,
          double *__restrict__ az, unsigned long long *__restrict__ counts, const float4 *__restrict__ rel,
@@ -1479,7 +1474,7 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, const int *__r
     if (SOME && part == 0 && tid == 0)
         atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)(start[b + 1] - t0));
     const int csize = (nt_all + nchunk - 1) / nchunk;
-    for (int ch = part; ch < nchunk; ch += parts) {
+    for (int ch = part; ch < nchunk; ch += stride) {
         const int tb = t0 + ch * csize, nt = min(csize, t0 + nt_all - tb);
         // The chunk's targets by index, where the box holds other particles too: in the copy
         // buffer that is first written after the first tile's barrier.
@@ -1627,41 +1622,114 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, const int *__r
     }
 }
 
-// Items are (box, part): part p of `parts` takes the box's target chunks p,
-// p + parts, ...  A single tree launches one CTA per item; a forest (box count
-// on the device) launches resident CTAs that pull items from *queue.  IMG: the
-// tree holds image copies, which are sources only: a box's targets are gathered
-// first, so that the lanes hold no image (three of four particles of a plume on
-// the rotation axis: 24 plumes, every other one rotational, 5.19 -> 3.2 ms a
-// step).  Without images nearly every particle is a target and the kernel is 2 %
-// faster without the second form (one million ions, 7.63 against 7.83 ms).
+// The forest's work items (box, chunk of its targets), largest first by class:
+// a plume's densest boxes hold twenty times the mean, and one of their chunks
+// started last keeps a few CTAs running after all others (24 plumes 6.09 -> 5.30 ms
+// per two steps, 256 plumes 41.7 -> 39.1 ms a step, against boxes in order).  An item's size is
+// estimated by targets x particles of its box, for its near boxes are as dense.
+// Targets and items per class are counted in one launch; in the next each CTA
+// reserves its places in every class.
+constexpr int kItemThreads = 256;
+// the most items: a box's targets are cut into ceil(targets / 8) chunks at most (p2p_chunks)
+inline size_t near_items_room(int n, int boxes) { return (size_t)n / 8 + (size_t)boxes; }
+__device__ __forceinline__ int near_item_class(int nt, int np, int chunks) {
+    return 31 - __clz((int)min(1ll + (long long)((nt + chunks - 1) / chunks) * np, 0x7fffffffll));
+}
+__global__ void __launch_bounds__(kWarps * 32)
+leaf_targets_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ start,
+                    const double *__restrict__ qm, int *__restrict__ ntgt, int *__restrict__ classes) {
+    __shared__ int cnt[kItemClasses];
+    if (threadIdx.x < kItemClasses) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    SV_WARP_BOXES(kWarps) {
+        const int s0 = start[b], s1 = start[b + 1];
+        int f = 0;
+        for (int j = s0 + lane; j < s1; j += 32) f += qm[j] != 0.0;
+        f = __reduce_add_sync(0xffffffffu, f);
+        const int c = p2p_chunks(f, 1);
+        if (lane == 0) {
+            ntgt[b] = f;
+            if (c) atomicAdd(&cnt[near_item_class(f, s1 - s0, c)], c);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kItemClasses && cnt[threadIdx.x]) atomicAdd(&classes[threadIdx.x], cnt[threadIdx.x]);
+}
+__global__ void __launch_bounds__(kItemThreads)
+near_items_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__ start,
+                  const int *__restrict__ ntgt, const int *__restrict__ classes, int *__restrict__ placed,
+                  int *__restrict__ total, int2 *__restrict__ items, int room) {
+    __shared__ int cnt[kItemClasses], at[kItemClasses];
+    const int tid = threadIdx.x;
+    if (tid < kItemClasses) cnt[tid] = 0;
+    __syncthreads();
+    const int nb = level_boxes(nbox, nbd);
+    const int b = blockIdx.x * kItemThreads + tid;  // one box per thread
+    const int nt = b < nb ? ntgt[b] : 0, c = p2p_chunks(nt, 1);
+    int cls = 0, mine = 0;
+    if (c) {
+        cls = near_item_class(nt, start[b + 1] - start[b], c);
+        mine = atomicAdd(&cnt[cls], c);
+    }
+    __syncthreads();
+    if (tid < kItemClasses) {
+        // classes in falling order: those above this one come first
+        int before = 0, all = 0;
+        for (int k = 0; k < kItemClasses; k++) {
+            const int n = classes[k];
+            all += n;
+            if (k > tid) before += n;
+        }
+        at[tid] = before + (cnt[tid] ? atomicAdd(&placed[tid], cnt[tid]) : 0);
+        if (blockIdx.x == 0 && tid == 0) *total = min(all, room);
+    }
+    __syncthreads();
+    for (int k = 0; k < c; k++) {
+        const int o = at[cls] + mine + k;
+        if (o < room) items[o] = make_int2(b, k);
+    }
+}
+
+// A single tree launches one CTA per item (box, part): part p of `parts` takes the
+// box's target chunks p, p + parts, ...  LIST: trees with image copies, and the
+// forest (list set), whose resident CTAs pull items (box, chunk) from the list.
+// Image copies are sources only: a box's targets are gathered first, so that the
+// lanes hold no image (three of four particles of a plume on the rotation axis: 24
+// plumes, every other one rotational, 5.19 -> 3.2 ms a step).  Without images
+// nearly every particle is a target and the kernel is 2 % faster without the
+// second form (one million ions, 7.63 against 7.83 ms).
 // counts[2] != 0: box_relative_kernel met two different charges.
-template <int WS, bool CLAMP, bool IMG>
+template <int WS, bool CLAMP, bool LIST>
 __global__ void __launch_bounds__(kP2PThreads, 6)
-p2p_kernel(int nbox, const int *__restrict__ nbd, int parts, int *__restrict__ queue, const int *__restrict__ bpid,
+p2p_kernel(int nbox, int parts, const int2 *__restrict__ list, const int *__restrict__ bpid,
            const int *__restrict__ start, const int4 *__restrict__ coord, const int *__restrict__ nbr,
            const double *__restrict__ qm, const double *__restrict__ roots, int level, float eps2,
            double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
            unsigned long long *__restrict__ counts, const int *__restrict__ has_tgt, const float4 *__restrict__ rel,
            const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap) {
     __shared__ __align__(16) P2PShared<WS> sh;
-    const int items = level_boxes(nbox, nbd) * parts;
+    const int items = LIST && list ? (int)counts[5] : nbox * parts;
+    const int stride = LIST && list ? 1 << 20 : parts;
     const bool uq = counts[2] == 0;
     int it = blockIdx.x;
     while (true) {
-        if (queue) {
+        if (LIST && list) {
             __syncthreads();
-            if (threadIdx.x == 0) sh.item = atomicAdd(queue, 1);
+            if (threadIdx.x == 0) sh.item = (int)atomicAdd(&counts[3], 1ull);
             __syncthreads();
             it = sh.item;
         }
         if (it >= items) return;
-        const int b = it / parts, part = it - b * parts;
+        int b = it / parts, part = it - b * parts;
+        if (LIST && list) {
+            b = list[it].x;
+            part = list[it].y;
+        }
         const int ntgt = has_tgt[b];
         if (ntgt) {
-#define SV_ITEM(U, S) p2p_item<WS, CLAMP, U, S>(sh, b, ntgt, part, parts, bpid, start, coord, nbr, qm, roots, level, \
-                                                eps2, ax, ay, az, counts, rel, fd, fd_cnt, fd_cap)
-            if (IMG && ntgt < start[b + 1] - start[b]) {
+#define SV_ITEM(U, S) p2p_item<WS, CLAMP, U, S>(sh, b, ntgt, part, parts, stride, bpid, start, coord, nbr, qm, roots, \
+                                                level, eps2, ax, ay, az, counts, rel, fd, fd_cnt, fd_cap)
+            if (LIST && ntgt < start[b + 1] - start[b]) {
                 if (uq) SV_ITEM(true, true);
                 else SV_ITEM(false, true);
             } else {
@@ -1670,26 +1738,27 @@ p2p_kernel(int nbox, const int *__restrict__ nbd, int parts, int *__restrict__ q
             }
 #undef SV_ITEM
         }
-        if (!queue) return;
+        if (!(LIST && list)) return;
     }
 }
 
-// P2P launch: well-separation and whether r^2 needs the kMinR2 floor
-inline void launch_p2p(int ws, bool images, float eps2, int grid, cudaStream_t st, int nbox, const int *nbd, int parts, int *queue,
-                       const int *bpid, const int *start, const int4 *coord, const int *nbr, const double *qm,
-                       const double *roots, int level, double *ax, double *ay, double *az, unsigned long long *counts,
-                       const int *has_tgt, const float4 *rel, const int *fd = nullptr,
+// P2P launch: well-separation, whether r^2 needs the kMinR2 floor, and whether the tree holds images or comes
+// with a list of items
+inline void launch_p2p(int ws, bool images, float eps2, int grid, cudaStream_t st, int nbox, int parts,
+                       const int2 *list, const int *bpid, const int *start, const int4 *coord, const int *nbr,
+                       const double *qm, const double *roots, int level, double *ax, double *ay, double *az,
+                       unsigned long long *counts, const int *has_tgt, const float4 *rel, const int *fd = nullptr,
                        const int *fd_cnt = nullptr, int fd_cap = 0) {
-    const bool clamp = !(eps2 >= kMinR2);
-#define SV_P2P(W, C, I) p2p_kernel<W, C, I><<<grid, kP2PThreads, 0, st>>>(nbox, nbd, parts, queue, bpid, start, coord, nbr, \
-                                                                   qm, roots, level, eps2, ax, ay, az, counts,       \
-                                                                   has_tgt, rel, fd, fd_cnt, fd_cap)
+    const bool clamp = !(eps2 >= kMinR2), gather = images || list;
+#define SV_P2P(W, C, G) p2p_kernel<W, C, G><<<grid, kP2PThreads, 0, st>>>(nbox, parts, list, bpid, start, coord, nbr,  \
+                                                                      qm, roots, level, eps2, ax, ay, az, counts, \
+                                                                      has_tgt, rel, fd, fd_cnt, fd_cap)
     if (ws == 1) {
-        if (clamp) images ? SV_P2P(1, true, true) : SV_P2P(1, true, false);
-        else images ? SV_P2P(1, false, true) : SV_P2P(1, false, false);
+        if (clamp) gather ? SV_P2P(1, true, true) : SV_P2P(1, true, false);
+        else gather ? SV_P2P(1, false, true) : SV_P2P(1, false, false);
     } else {
-        if (clamp) images ? SV_P2P(2, true, true) : SV_P2P(2, true, false);
-        else images ? SV_P2P(2, false, true) : SV_P2P(2, false, false);
+        if (clamp) gather ? SV_P2P(2, true, true) : SV_P2P(2, true, false);
+        else gather ? SV_P2P(2, false, true) : SV_P2P(2, false, false);
     }
 #undef SV_P2P
 }
@@ -1789,7 +1858,7 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         la.lv[L].fd_cnt = (int *)carve((size_t)T.lv[L].nbox * sizeof(int));
     }
     phase_mark(c, 2);
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 5 * sizeof(unsigned long long), c->stream));
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, kCounts * sizeof(unsigned long long), c->stream));
     if (F.rel_cap < c->S.n) {
         cudaFree(F.rel);
         cudaFree(F.far);
@@ -1834,7 +1903,7 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         if (c->P.profile_phases) SV_CK(c, cudaEventRecord(F.ev_near[0], F.side));
         // few boxes: their target chunks to several CTAs, two waves of the CTAs that fit at once
         const int parts = std::max(1, std::min(8, div_up(2 * 6 * device_sms(), V.nbox)));
-        launch_p2p(ws, c->P.symmetry != SV_SYM_NONE, (float)c->P.softening2, V.nbox * parts, F.side, V.nbox, nullptr, parts, nullptr, nullptr, V.start,
+        launch_p2p(ws, c->P.symmetry != SV_SYM_NONE, (float)c->P.softening2, V.nbox * parts, F.side, V.nbox, parts, nullptr, nullptr, V.start,
                    V.coord, nbr[L], S.qm, S.root, L, S.ax, S.ay, S.az, F.d_counts, tgt[L], F.rel, la.lv[L].fd,
                    la.lv[L].fd_cnt, kFarDirectCap);
         SV_LAUNCHED(c);
@@ -2053,7 +2122,6 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
 
 
 // ------------------------------------------------------------------ forest --
-constexpr int kForestParts = 2;  // work items per leaf box of the forest's near field
 
 inline int forest_grid(int cap, int per_cta) {
     const int g = div_up(cap > 0 ? cap : 1, per_cta);
@@ -2072,7 +2140,7 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
     Tree &T = *F.ftree;
     int *nbd = fa.d_nbox;
     SV_TRY(tree_build_forest(c, T, f, nbd, fa.d_err));
-    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, 5 * sizeof(unsigned long long), c->stream));
+    SV_CK(c, cudaMemsetAsync(F.d_counts, 0, kCounts * sizeof(unsigned long long), c->stream));
     // Two streams, as in run_fmm: target flags, lists and the near field on the
     // second (the forest's slots only: the direct plumes' slots belong to
     // another stream), the upward and downward passes on the main one.
@@ -2081,8 +2149,9 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
     SV_CK(c, cudaStreamWaitEvent(sd, F.ev_fork, 0));
     root_nbr_kernel<<<forest_grid(f.cap[0] * ns, 256), 256, 0, sd>>>(F.fnbr[0], ns, f.cap[0], nbd);
     SV_LAUNCHED(c);
+    int *classes = reinterpret_cast<int *>(F.d_counts + 6);
     leaf_targets_kernel<<<forest_grid(f.cap[L], kWarps), kWarps * 32, 0, sd>>>(f.cap[L], nbd + L, T.lv[L].start, S.qm,
-                                                                  F.ftgt[L]);
+                                                                             F.ftgt[L], classes);
     SV_LAUNCHED(c);
     for (int l = L - 1; l >= 0; l--) {
         parent_targets_kernel<<<forest_grid(f.cap[l], 256), 256, 0, sd>>>(f.cap[l], nbd + l, T.lv[l].child0,
@@ -2115,11 +2184,13 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
         box_relative_kernel<<<g, kWarps * 32, 0, sd>>>(f.cap[L], nbd + L, V.pid, V.start, V.coord, S.x, S.y, S.z,
                                                        S.q, fa.roots, L, F.frel, F.d_counts + 2);
         SV_LAUNCHED(c);
-        launch_p2p(ws, fa.images, (float)c->P.softening2, std::min(kForestParts * f.cap[L], 6 * device_sms()), sd, f.cap[L],
-                   nbd + L, kForestParts,
-                   reinterpret_cast<int *>(F.d_counts + 3), V.pid, V.start, V.coord, F.fnbr[L], S.qm,
-                   fa.roots, L, S.ax, S.ay, S.az, F.d_counts, F.ftgt[L], F.frel, fd_thresh > 0 ? F.ffd : nullptr,
-                   F.ffd_cnt, kFarDirectCap);
+        near_items_kernel<<<std::max(1, div_up(f.cap[L], kItemThreads)), kItemThreads, 0, sd>>>(
+            f.cap[L], nbd + L, V.start, F.ftgt[L], classes, classes + kItemClasses,
+            reinterpret_cast<int *>(F.d_counts + 5), F.fitems, (int)near_items_room(f.n, f.cap[L]));
+        SV_LAUNCHED(c);
+        launch_p2p(ws, true, (float)c->P.softening2, 6 * device_sms(), sd, f.cap[L], 1, F.fitems, V.pid,
+                   V.start, V.coord, F.fnbr[L], S.qm, fa.roots, L, S.ax, S.ay, S.az, F.d_counts, F.ftgt[L], F.frel,
+                   fd_thresh > 0 ? F.ffd : nullptr, F.ffd_cnt, kFarDirectCap);
         SV_LAUNCHED(c);
         SV_CK(c, cudaEventRecord(F.ev_join, sd));
     }
@@ -2291,7 +2362,7 @@ static sv_status fmm_state(sv_ctx *c) {
     if (!c->fmm) {
         c->fmm = new Fmm();
         Fmm &F = *c->fmm;
-        SV_CK(c, cudaMalloc(&F.d_counts, 5 * sizeof(unsigned long long)));
+        SV_CK(c, cudaMalloc(&F.d_counts, kCounts * sizeof(unsigned long long)));
         SV_CK(c, cudaMallocHost(&F.h_counts, 2 * sizeof(unsigned long long)));
         SV_CK(c, cudaStreamCreateWithFlags(&F.side, cudaStreamNonBlocking));
         SV_CK(c, cudaEventCreateWithFlags(&F.ev_fork, cudaEventDisableTiming));
@@ -2406,6 +2477,8 @@ sv_status fmm_forest_reserve(sv_ctx *c, const ForestArgs &fa) {
         if (F.fchunks[l] > 1) bytes += rounded(nb * F.fchunks[l] * NC * sizeof(float2));
     }
     bytes += rounded((size_t)f.cap[f.L] * kFarDirectCap * sizeof(int)) + rounded((size_t)f.cap[f.L] * sizeof(int));
+    const size_t item_bytes = near_items_room(f.n, f.cap[f.L]) * sizeof(int2);
+    bytes += rounded(item_bytes);
     if (F.farena_bytes < bytes) {
         cudaFree(F.farena);
         F.farena = nullptr;
@@ -2436,6 +2509,7 @@ sv_status fmm_forest_reserve(sv_ctx *c, const ForestArgs &fa) {
     }
     F.ffd = (int *)carve((size_t)f.cap[f.L] * kFarDirectCap * sizeof(int));
     F.ffd_cnt = (int *)carve((size_t)f.cap[f.L] * sizeof(int));
+    F.fitems = (int2 *)carve(item_bytes);
     if (c->P.fmm_m2l_tc >= 0 && f.L >= 2) {
         // room of the tensor-core M2L: the last run's translations with a
         // margin, at least 32 per box of the M2L levels (a graph keeps the

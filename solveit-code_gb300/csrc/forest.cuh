@@ -16,7 +16,6 @@ struct ForestArgs {
     ForestSpec spec;                 // slots, leaf level, Morton bits, box capacities
     int p = 6, ws = 2;               // expansion order and well-separation
     int nroots = 0;                  // plumes in the forest
-    bool images = false;             // some plumes carry image slots, which are sources only
     const double *roots = nullptr;   // device [8 * nroots]
     int *d_nbox = nullptr;           // device [3 * (kMortonBits + 1)]: counts, capacities, largest counts
     int *d_err = nullptr;            // device: bit l = level l overflowed its capacity

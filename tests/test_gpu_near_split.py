@@ -87,3 +87,26 @@ def test_images_leave_the_targets_lanes(n, ws, mixed):
     assert s.cell_interactions == 0
     assert rel_l2(a, ref, st["status"]) < 2e-6
     assert not np.any(a[st["status"] != 1])
+
+
+@pytest.mark.parametrize("sizes", [(8200, 30, 12000), (9001,), (20011, 8193)])
+def test_forest_work_list(sizes):
+    """The forest's list of work items, largest first: plumes of very different density, every
+    other one with image copies, source-only particles among them.  Order 10 keeps the far field
+    below the bound wherever the levels fall."""
+    states = []
+    for k, n in enumerate(sizes):
+        st = plume.make_plume(n, (0.4e-6, 3e-6)[k % 2], 40 + n)
+        st["status"][3::7] = 2
+        states.append(st)
+    syms = [(sv.SYM_ROTATIONAL, sv.SYM_NONE)[k % 2] for k in range(len(sizes))]
+    with sv.ForceMethod(softening2=EPS20, fmm_order=10, fmm_ws=2) as fm:
+        fm.upload_batch(states, [sv.FMM if n > 1000 else sv.DIRECT for n in sizes], syms)
+        a = fm.accel()
+    o = 0
+    for st, sym in zip(states, syms):
+        n = st["q"].size
+        ref = O.direct_f64(st, EPS20, sym=1 if sym == sv.SYM_ROTATIONAL else 0)
+        assert rel_l2(a[o:o + n], ref, st["status"]) < 1e-5
+        assert not np.any(a[o:o + n][st["status"] != 1])
+        o += n
