@@ -95,7 +95,12 @@ struct Batch {
     int8_t *pfold = nullptr;          // n: 1 for the particles of rotational plumes (folding)
     double step_dt = 0;               // dt baked into g_step
     // tuning
-    int m2l_weight = 400, direct_chunk = 2048;  // tuned: M2L cost in pair units, direct work-item size
+    // Tuned: M2L cost in pair units, direct work-item size.  The weight before tuning:
+    // 200 against 400 on batches of 3 to 24 plumes at orders 4, 6 and 8 is 0 to 3 % faster
+    // (24 plumes at order 6: 5.25 against 5.40 ms per two steps) and at order 4 up to 34 %
+    // (1.21 against 1.63 ms); 100 costs 7 %.  256 large plumes, which the tuner is for:
+    // 41.2 against 39.1 ms a step.
+    int m2l_weight = 200, direct_chunk = 2048;
     double tuned_ms = 0;
     int regrows = 0;
 };
