@@ -44,7 +44,7 @@
 namespace sv {
 
 constexpr int kItemClasses = 32;           // near-field work items by log2 of their estimated pairs
-constexpr int kCounts = 6 + kItemClasses;  // words of Fmm::d_counts
+constexpr int kCounts = 5 + kItemClasses;  // words of Fmm::d_counts
 
 struct Fmm {
     int p = 0, ws = 0;
@@ -59,9 +59,9 @@ struct Fmm {
     float *otab = nullptr;   // rotation-based M2M / L2L tables (oct_layout)
     void *arena = nullptr;
     size_t arena_bytes = 0;
-    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work queue,
-                                             // [4] finished target-flag CTAs, [5] P2P work items, then per size
-                                             // class of them (ints) their number and the number placed
+    unsigned long long *d_counts = nullptr;  // [0] M2L translations, [1] P2P pairs, [2] charges differ, [3] P2P work
+                                             // items, [4] finished target-flag CTAs, then per size class of
+                                             // the items (ints) their number and the number placed
     unsigned long long *h_counts = nullptr;
     // caller particles followed by their source-only symmetry images
     double *ex = nullptr, *ey = nullptr, *ez = nullptr, *eq = nullptr, *em = nullptr;
@@ -1385,7 +1385,6 @@ struct P2PShared {
     float4 nb_off[p2p_nsp<WS>()];  // source box centre - target box centre (exact in FP32)
     int2 nb_rng[p2p_nsp<WS>()];    // (first source, running source count at the box's end)
     int scan[2][kP2PThreads / 32], nz[2][kP2PThreads / 32];  // per warp and list: sources, non-empty boxes
-    int item;
 };
 
 // Chunks a box's nt targets are cut into.  A chunk's time per source is that
@@ -1471,8 +1470,6 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, int stride, co
     add_boxes(nbr + (size_t)b * NS, NS, 0);
     if (fd) add_boxes(fd + (size_t)b * fd_cap, fd_cnt[b], 1);
     __syncthreads();
-    if (SOME && part == 0 && tid == 0)
-        atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)(start[b + 1] - t0));
     const int csize = (nt_all + nchunk - 1) / nchunk;
     for (int ch = part; ch < nchunk; ch += stride) {
         const int tb = t0 + ch * csize, nt = min(csize, t0 + nt_all - tb);
@@ -1509,7 +1506,7 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, int stride, co
         const bool vb = active && lt + h < nt;
         const int ia = SOME ? tix[active ? lt : 0] : tb + lt, ib = SOME ? tix[vb ? lt + h : 0] : ia + h;
         const float4 ta = rel[SOME || active ? ia : tb], tbv = rel[SOME || vb ? ib : tb];
-        if (!SOME && tid == 0) atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)nt);
+        if (tid == 0) atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)nt);
         const float2 AX = make_float2(ta.x, ta.x), AY = make_float2(ta.y, ta.y), AZ = make_float2(ta.z, ta.z);
         const float2 BX = make_float2(tbv.x, tbv.x), BY = make_float2(tbv.y, tbv.y), BZ = make_float2(tbv.z, tbv.z);
         float sax = 0.f, say = 0.f, saz = 0.f, eax = 0.f, eay = 0.f, eaz = 0.f;
@@ -1692,7 +1689,12 @@ near_items_kernel(int nbox, const int *__restrict__ nbd, const int *__restrict__
 
 // A single tree launches one CTA per item (box, part): part p of `parts` takes the
 // box's target chunks p, p + parts, ...  LIST: trees with image copies, and the
-// forest (list set), whose resident CTAs pull items (box, chunk) from the list.
+// forest (list set), one CTA per item (box, chunk) of the list and as many as the
+// boxes have room, items past that shared out: a CTA that ends after its item lets
+// the far field's kernels in between.  (As many as fit at once, pulling items from a
+// queue, held every SM until the list was done and ran the two in turn on small
+// batches: 0.71 to 1.0 ms against 0.64 to 0.66 for three balls of 9,000 to 20,000
+// ions; 24 and 256 plumes the same within 1 %.)
 // Image copies are sources only: a box's targets are gathered first, so that the
 // lanes hold no image (three of four particles of a plume on the rotation axis: 24
 // plumes, every other one rotational, 5.19 -> 3.2 ms a step).  Without images
@@ -1708,18 +1710,10 @@ p2p_kernel(int nbox, int parts, const int2 *__restrict__ list, const int *__rest
            unsigned long long *__restrict__ counts, const int *__restrict__ has_tgt, const float4 *__restrict__ rel,
            const int *__restrict__ fd, const int *__restrict__ fd_cnt, int fd_cap) {
     __shared__ __align__(16) P2PShared<WS> sh;
-    const int items = LIST && list ? (int)counts[5] : nbox * parts;
+    const int items = LIST && list ? (int)counts[3] : nbox * parts;
     const int stride = LIST && list ? 1 << 20 : parts;
     const bool uq = counts[2] == 0;
-    int it = blockIdx.x;
-    while (true) {
-        if (LIST && list) {
-            __syncthreads();
-            if (threadIdx.x == 0) sh.item = (int)atomicAdd(&counts[3], 1ull);
-            __syncthreads();
-            it = sh.item;
-        }
-        if (it >= items) return;
+    for (int it = blockIdx.x; it < items; it += gridDim.x) {
         int b = it / parts, part = it - b * parts;
         if (LIST && list) {
             b = list[it].x;
@@ -1738,7 +1732,8 @@ p2p_kernel(int nbox, int parts, const int2 *__restrict__ list, const int *__rest
             }
 #undef SV_ITEM
         }
-        if (!(LIST && list)) return;
+        if (!LIST) return;
+        __syncthreads();
     }
 }
 
@@ -2149,7 +2144,7 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
     SV_CK(c, cudaStreamWaitEvent(sd, F.ev_fork, 0));
     root_nbr_kernel<<<forest_grid(f.cap[0] * ns, 256), 256, 0, sd>>>(F.fnbr[0], ns, f.cap[0], nbd);
     SV_LAUNCHED(c);
-    int *classes = reinterpret_cast<int *>(F.d_counts + 6);
+    int *classes = reinterpret_cast<int *>(F.d_counts + 5);
     leaf_targets_kernel<<<forest_grid(f.cap[L], kWarps), kWarps * 32, 0, sd>>>(f.cap[L], nbd + L, T.lv[L].start, S.qm,
                                                                              F.ftgt[L], classes);
     SV_LAUNCHED(c);
@@ -2186,9 +2181,9 @@ sv_status run_fmm_forest(sv_ctx *c, Fmm &F, const ForestArgs &fa) {
         SV_LAUNCHED(c);
         near_items_kernel<<<std::max(1, div_up(f.cap[L], kItemThreads)), kItemThreads, 0, sd>>>(
             f.cap[L], nbd + L, V.start, F.ftgt[L], classes, classes + kItemClasses,
-            reinterpret_cast<int *>(F.d_counts + 5), F.fitems, (int)near_items_room(f.n, f.cap[L]));
+            reinterpret_cast<int *>(F.d_counts + 3), F.fitems, (int)near_items_room(f.n, f.cap[L]));
         SV_LAUNCHED(c);
-        launch_p2p(ws, true, (float)c->P.softening2, 6 * device_sms(), sd, f.cap[L], 1, F.fitems, V.pid,
+        launch_p2p(ws, true, (float)c->P.softening2, f.cap[L], sd, f.cap[L], 1, F.fitems, V.pid,
                    V.start, V.coord, F.fnbr[L], S.qm, fa.roots, L, S.ax, S.ay, S.az, F.d_counts, F.ftgt[L], F.frel,
                    fd_thresh > 0 ? F.ffd : nullptr, F.ffd_cnt, kFarDirectCap);
         SV_LAUNCHED(c);
