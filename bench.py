@@ -56,7 +56,7 @@ WORKLOADS = {
                     desc="FMM p=8 ws=2, N=1048576 ions, plume r=20nm z=50um, eps=1e-10m, "
                          "leapfrog DKD dt=1e-13s, E_z=1e8V/m"),
     "bh_n65536": dict(n=65536, length=10e-6, method="bh", theta=0.5, leaf=16, seed=1,
-                      desc="Barnes-Hut theta=0.5 leaf 16 (stackless warp walk, FP32 forces, FP64 integration), "
+                      desc="Barnes-Hut theta=0.5 leaf 16 (warp walk over batches of cells, FP32 forces, FP64 integration), "
                            "N=65536 ions, plume r=20nm z=10um, eps=1e-10m, leapfrog DKD dt=1e-13s, E_z=1e8V/m"),
     "direct_n4096": dict(n=4096, length=1e-6, method="direct", precision="fp64", seed=0,
                          desc="FP64 direct sum, N=4096 ions, plume r=20nm z=1um, eps=1e-10m, "

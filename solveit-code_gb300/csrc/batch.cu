@@ -8,7 +8,7 @@
 //  * view: one slot per (particle, image).  FMM plumes come first (plume ids
 //    0..nfp-1), each particle followed by its source-only rotated copies for
 //    the 4-fold rotational variant; direct plumes follow (their images are
-//    formed on the fly by the pair kernel, as in direct.cu).
+//    formed on the fly by the pair kernel).
 //  * one radix sort of all slots by key = plume id << 54 | 18-bit-per-axis
 //    Morton code relative to the plume's own root cube, so each plume's slots
 //    stay contiguous and spatially ordered.
@@ -432,9 +432,8 @@ constexpr int kDTPB = 128;  // threads per CTA of the direct batch kernel
 constexpr int kDTPT = 2;    // targets per thread
 constexpr int kDTile = 256; // sources per shared-memory tile
 
-// Persistent all-pairs kernel over the direct plumes' work items.  Same
-// arithmetic as direct_mixed_kernel (direct.cu): FP32 pairs on offsets from the
-// item's first target, FP64 accumulation across tiles, atomics into the
+// Persistent all-pairs kernel over the direct plumes' work items, one-sided:
+// FP32 pairs on offsets from the item's first target, FP64 accumulation across tiles, atomics into the
 // sorted acceleration (zeroed beforehand).
 __global__ void __launch_bounds__(kDTPB)
 direct_batch_kernel(const DirectItem *__restrict__ items, int nitems, int *__restrict__ queue,
@@ -1084,8 +1083,8 @@ sv_status time_accel(sv_ctx *c, Batch &B, int reps, double *ms) {
 // Leaf occupancy of the FMM plumes: the M2L weight of the depth model.
 // Among the weights within 3 % of the fastest, the largest is kept: it
 // chooses shallower trees, and as the plumes expand their M2L translations
-// grow faster than their pairs (batch256 over 10 steps from a tie at the
-// start: weight 400 95 ms per step, weight 200 107 ms).
+// grow faster than their pairs (256 plumes over 10 steps: weight 400 39.1 ms
+// per step, weight 200 41.2 ms).
 sv_status sweep_weights(sv_ctx *c, Batch &B, int *best_lt, double *best_ms) {
     const int weights[6] = {100, 200, 400, 800, 1600, 3200};
     double t[6], best = 1e30;

@@ -9,19 +9,19 @@
 //   P2M   leaf boxes, one warp per box, lanes over particles, then over
 //         coefficients (shared-memory transpose).
 //   M2M   one warp per parent, lanes over the parent's coefficients, children
-//         added in turn (no mutex: one writer per parent).
-//   lists per level, one thread per box: the children of the parent's
-//         neighbours split into near boxes (|offset| <= ws) and the M2L list
-//         (offset class = integer offset target - source).
+//         added in turn (no mutex: one writer per parent); coarse levels in one
+//         launch of one CTA.
+//   lists near boxes (|offset| <= ws) and the M2L list (offset class = integer
+//         offset target - source): every level in two launches; the forest's
+//         per level from the parents' near lists.
 //   down  one warp per box and level: L2L from the parent, then every M2L of
 //         the box's list (phase, folded y-rotation, z-translation, inverse
 //         rotation, inverse phase), accumulated in registers, written once.
 //   L2P   leaf boxes, lanes over particles: gradient of the local expansion.
-//   P2P   leaf boxes, lanes over targets, source chunks staged in shared
-//         memory as FP32 offsets from the target box centre (FP64 subtraction
-//         once per staged source); a box's short tail chunk of targets spreads
-//         each target over a group of lanes that split the sources; per-source-
-//         box FP32 partial sums are accumulated with Kahan compensation.
+//   P2P   leaf boxes, a CTA per box or chunk of its targets; groups of
+//         threads, two targets each, share the sources staged in shared memory
+//         as FP32 offsets from the target box centre; FP32 partial sums of at
+//         most 64 sources are accumulated with Kahan compensation.
 //
 // Expansions are kept in box units (coordinates divided by the box side h),
 // so the M2L tables depend on the integer offset only; the softened M2L
