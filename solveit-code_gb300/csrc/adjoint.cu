@@ -517,12 +517,13 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
                                                               c->t_inj, c->status, nn, ts, A.dt, c->P.e_over_amu,
                                                               c->P.k_const, A.lE, umax});
     SV_LAUNCHED(c);
-    // the particles of the step's window in Morton order
+    // the particles of the step's window in Morton order (a small window: sources first)
     const bool fp64 = c->P.precision == SV_PREC_FP64;
     c->fstatus = c->wstatus;
     c->S.want_zero = true;
     c->S.want_hilo = !fp64;
     c->S.hl_abs = false;
+    c->S.any_order = true;
     const sv_status st = sort_state(c, 0, nn);
     c->fstatus = nullptr;
     SV_TRY(st);

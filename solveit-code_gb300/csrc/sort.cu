@@ -189,8 +189,9 @@ __device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
     return tgt ? a.kconst * (a.qom ? a.qom[i] : a.q[i] / a.m[i]) : 0.0;
 }
 
-// particle i into sorted slot s (every load before the first store)
-__device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s, uint32_t i) {
+// particle i into sorted slot s (every load before the first store); with ph, whether its source
+// charge differs from particle 0's
+__device__ __forceinline__ bool gather_one(const GatherArgs &a, const double *root, int64_t s, uint32_t i) {
     const double x = a.x[i], y = a.y[i], z = a.z[i], k = sorted_qm(a, i);
     const float q = sorted_charge(a, i);
     a.xs[s] = x;
@@ -201,20 +202,21 @@ __device__ __forceinline__ void gather_one(const GatherArgs &a, int64_t s, uint3
     if (a.zax) a.zax[s] = a.zay[s] = a.zaz[s] = 0.0;
     if (a.ph) {
         float4 h, l;
-        split_hilo(x - (a.abs_xy ? 0.0 : a.root[0]), h.x, l.x);
-        split_hilo(y - (a.abs_xy ? 0.0 : a.root[1]), h.y, l.y);
-        split_hilo(z - a.root[2], h.z, l.z);
+        split_hilo(x - (a.abs_xy ? 0.0 : root[0]), h.x, l.x);
+        split_hilo(y - (a.abs_xy ? 0.0 : root[1]), h.y, l.y);
+        split_hilo(z - root[2], h.z, l.z);
         h.w = q;
         l.w = k != 0.0 ? 1.f : 0.f;
         a.ph[s] = h;
         a.pl[s] = l;
-        if (h.w != sorted_charge(a, 0)) *a.differ = 1;
+        return h.w != sorted_charge(a, 0);
     }
+    return false;
 }
 
 __global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, GatherArgs a) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s < n) gather_one(a, s, idx[s]);
+    if (s < n && gather_one(a, a.root, s, idx[s])) *a.differ = 1;
 }
 
 // ------------------------------------------------------------- rank sort --
@@ -231,6 +233,12 @@ __global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, Gathe
 // 54 of the six passes a tree needs, so the radix passes stay above
 // kRankSortMax.
 constexpr int64_t kRankSortMax = 32768;
+// Up to this many particles the direct sum and the adjoint take their sources in the
+// caller's order: the sort's launches take longer than the pairs' close form on
+// every tile.  A step of the direct sum at 8,192 particles 89 -> 79 us, at 2,048 62 ->
+// 48; above, the close form costs more: four adjoint steps at 16,384 2.73 -> 2.81 ms,
+// the sum at 30,011 565 -> 618 us.
+constexpr int64_t kAnyOrderMax = 8192;
 constexpr int64_t kSmallChunkMax = 8192;  // chunks of 256 up to here, of 1024 above
 constexpr int kOneChunk = 1024;           // one CTA sorts a plume of up to this many
 
@@ -313,7 +321,7 @@ sort_one_chunk(int n, int sh, double scale, double *__restrict__ root, uint64_t 
     if (i < n) {
         keys[pos] = key;
         idx[pos] = (uint32_t)i;
-        gather_one(a, pos, (uint32_t)i);
+        if (gather_one(a, root, pos, (uint32_t)i)) *a.differ = 1;
     }
 }
 
@@ -329,6 +337,64 @@ sort_chunks(int n, int sh, const double *__restrict__ root, uint64_t *__restrict
     if (i < n) {
         ckeys[pos] = key;
         cidx[pos] = (uint32_t)i;
+    }
+}
+
+// Sources first, otherwise in the caller's order, and the gather, in one launch:
+// for the pair-once sums, which need no order among the sources (blocks that
+// spread over the plume take the path that keeps the coordinates' parts below FP32
+// for every tile).  Latency bound: one launch where the bounding box, the chunk sort
+// and the ranks took three (25 us of 58 per evaluation at 4,096).  Every CTA counts the sources before its own particles itself,
+// and takes the first source's position as the origin of the FP32 parts.
+__global__ void __launch_bounds__(256)
+sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restrict__ done, int *__restrict__ mixed) {
+    __shared__ int wsum[8], tot[3];  // sources before this CTA, in all; first source
+    __shared__ double org[3];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    if (tid < 3) tot[tid] = tid == 2 ? n : 0;
+    __syncthreads();
+    int before = 0, all = 0, first = n;
+#pragma unroll 4
+    for (int c = 0; c < (int)gridDim.x; c++) {
+        const int k = c * 256 + tid;
+        if (k < n && is_source(a.st[k])) {
+            all++;
+            if (c < (int)blockIdx.x) before++;
+            first = min(first, k);
+        }
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    first = __reduce_min_sync(0xffffffffu, first);
+    const int i = blockIdx.x * 256 + tid;
+    const bool src = i < n && is_source(a.st[i]);
+    const unsigned bal = __ballot_sync(0xffffffffu, src);
+    if (lane == 0) {
+        atomicAdd(&tot[0], before);
+        atomicAdd(&tot[1], all);
+        atomicMin(&tot[2], first);
+        wsum[wid] = __popc(bal);
+    }
+    __syncthreads();
+    if (tid < 3) org[tid] = tot[2] < n ? (tid == 0 ? a.x : tid == 1 ? a.y : a.z)[tot[2]] : 0.0;
+    __syncthreads();
+    bool differ = false;
+    if (i < n) {
+        int s = tot[0] + __popc(bal & ((1u << lane) - 1u));  // sources before this particle
+        for (int w = 0; w < wid; w++) s += wsum[w];
+        const int pos = src ? s : tot[1] + (i - s);
+        idx[pos] = (uint32_t)i;
+        differ = gather_one(a, org, pos, (uint32_t)i);
+    }
+    // the mark of differing charges, from the last CTA to finish
+    differ = __syncthreads_or(differ);
+    if (tid == 0) {
+        if (differ) atomicOr(mixed, 1);
+        __threadfence();
+        if (atomicAdd(done, 1u) == gridDim.x - 1) {
+            *a.differ = atomicExch(mixed, 0);
+            *done = 0;
+        }
     }
 }
 
@@ -496,7 +562,8 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     const bool zero = c->S.want_zero, hilo = c->S.want_hilo, hl_abs = c->S.hl_abs;
     SV_TRY(ensure_sorted_capacity(c, n));
     Sorted &S = c->S;
-    S.want_zero = S.want_hilo = S.raw = false;
+    const bool any_order = S.any_order && n <= kAnyOrderMax;
+    S.want_zero = S.want_hilo = S.any_order = S.raw = false;
     S.hl_abs = hl_abs;
     if (hilo && S.hl_cap < n) {
         cudaFree(S.ph);
@@ -521,6 +588,12 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
         ga.zax = S.ax;
         ga.zay = S.ay;
         ga.zaz = S.az;
+    }
+    if (any_order && n > 0) {
+        sources_first<<<div_up(n, 256), 256, 0, c->stream>>>((int)n, S.idx, ga, reinterpret_cast<unsigned *>(S.root + 15),
+                                                           reinterpret_cast<int *>(S.root + 13));
+        SV_LAUNCHED(c);
+        return SV_OK;
     }
     if (n <= kOneChunk) {
         if (n <= 256)

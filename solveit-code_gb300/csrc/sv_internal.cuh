@@ -55,6 +55,7 @@ struct Sorted {
     int want_levels = kMortonBits, key_levels = kMortonBits;
     bool want_zero = false;  // the next sort also clears ax, ay, az (a method that adds into them)
     bool want_hilo = false, hl_abs = false;  // the next sort also writes ph, pl
+    bool any_order = false;  // the next sort need only put the sources first
     bool resort = false;  // the FMM found its leaf level below key_levels: sort again, fully
     int64_t n = 0;       // sorted entries (caller particles plus any image copies)
     int64_t n_orig = 0;  // caller particles; sorted idx >= n_orig are image copies

@@ -84,3 +84,18 @@ def test_fp64_tiles_of_equal_charges(n):
     st["status"][7::19] = 0
     a = accel(st, softening2=EPS20, precision=sv.FP64)
     assert rel_l2(a, O.direct_f64(st, EPS20), st["status"]) < BOUND[sv.FP64]
+
+
+@pytest.mark.parametrize("prec", [sv.MIXED, sv.FP64], ids=["mixed", "fp64"])
+@pytest.mark.parametrize("n", [3, 255, 257, 8191, 8192, 8193])
+def test_sources_first(n, prec):
+    """Around the size up to which the sources are only put before the other particles: the first
+    particles and others in between are none, the plume lies far from the origin, and its blocks
+    spread over all of it."""
+    st = state(n, True, 600 + n)
+    st["status"][: n // 3] = 0
+    st["status"][n // 2] = 1
+    st["x"] += np.array([1e-3, -2e-3, 5e-3])
+    a = accel(st, softening2=EPS20, precision=prec)
+    assert rel_l2(a, O.direct_f64(st, EPS20), st["status"]) < BOUND[prec]
+    assert not np.any(a[st["status"] != 1])
