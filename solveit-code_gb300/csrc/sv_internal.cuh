@@ -45,7 +45,8 @@ struct Sorted {
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
     double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S;
-                               // [14] int: 1 when the sorted source charges differ (want_hilo)
+                               // [14] int: 1 when the sorted source charges differ (want_hilo); [13], [15]
+                               // int: words of the kernels whose last CTA finishes, zero between launches
     long long *red = nullptr;  // device reduction scratch
     int red_blocks = 0;
     int64_t cap = 0;
