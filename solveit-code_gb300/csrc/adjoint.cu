@@ -523,7 +523,7 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
     c->S.want_zero = true;
     c->S.want_hilo = !fp64;
     c->S.hl_abs = false;
-    c->S.any_order = true;
+    c->S.any_order = nn <= kAnyOrderMax;
     const sv_status st = sort_state(c, 0, nn);
     c->fstatus = nullptr;
     SV_TRY(st);

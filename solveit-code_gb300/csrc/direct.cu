@@ -7,8 +7,8 @@
 // for inbound targets i and sources j with status 1 or 2 (j != i for the plain
 // sum; the symmetric variants keep the self image, which contributes 0).
 //
-// Targets and sources are the Morton-sorted copy (sort.cu), or without symmetry
-// images, up to 8,192 particles, the copy with the sources first.
+// Targets and sources are the Morton-sorted copy (sort.cu), or for few pairs
+// the copy with the sources first.
 //
 // MIXED: every unordered pair once.  The particles form blocks of 32 R; a warp
 // holds a block's coordinates and sums in registers (R particles per lane) and
@@ -469,7 +469,10 @@ void direct_sort_wants(sv_ctx *c) {
     c->S.want_zero = true;
     c->S.want_hilo = c->P.precision == SV_PREC_MIXED;
     c->S.hl_abs = c->P.symmetry == SV_SYM_ROTATIONAL;
-    c->S.any_order = c->P.symmetry == SV_SYM_NONE;
+    const ImageSet *I = nullptr;
+    int64_t images = c->P.symmetry == SV_SYM_ROTATIONAL ? 4 : 1;
+    if (c->P.symmetry == SV_SYM_TRANSLATIONAL) images = image_set(c, &I) == SV_OK ? I->count : INT32_MAX;
+    c->S.any_order = c->n * c->n <= kAnyOrderMax * kAnyOrderMax / images;
 }
 
 sv_status direct_accel(sv_ctx *c) {

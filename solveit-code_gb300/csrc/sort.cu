@@ -233,12 +233,6 @@ __global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, Gathe
 // 54 of the six passes a tree needs, so the radix passes stay above
 // kRankSortMax.
 constexpr int64_t kRankSortMax = 32768;
-// Up to this many particles the direct sum and the adjoint take their sources in the
-// caller's order: the sort's launches take longer than the pairs' close form on
-// every tile.  A step of the direct sum at 8,192 particles 89 -> 79 us, at 2,048 62 ->
-// 48; above, the close form costs more: four adjoint steps at 16,384 2.73 -> 2.81 ms,
-// the sum at 30,011 565 -> 618 us.
-constexpr int64_t kAnyOrderMax = 8192;
 constexpr int64_t kSmallChunkMax = 8192;  // chunks of 256 up to here, of 1024 above
 constexpr int kOneChunk = 1024;           // one CTA sorts a plume of up to this many
 
@@ -562,7 +556,7 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     const bool zero = c->S.want_zero, hilo = c->S.want_hilo, hl_abs = c->S.hl_abs;
     SV_TRY(ensure_sorted_capacity(c, n));
     Sorted &S = c->S;
-    const bool any_order = S.any_order && n <= kAnyOrderMax;
+    const bool any_order = S.any_order;
     S.want_zero = S.want_hilo = S.any_order = S.raw = false;
     S.hl_abs = hl_abs;
     if (hilo && S.hl_cap < n) {

@@ -298,6 +298,13 @@ sv_status unsort_accel(sv_ctx *c);
 
 // direct.cu
 sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; raw sums in mixed precision)
+// Up to the pairs of this many particles (images counted) the direct sum and the
+// adjoint take their sources in the caller's order: the sort's launches take longer
+// than the pairs' close form on every tile.  A step of the direct sum at 8,192
+// particles 89 -> 79 us, at 2,048 62 -> 48, with four quadrants at 4,096 85 -> 76 and
+// at 900 58 -> 43; above, the close form costs more: four adjoint steps at 16,384
+// 2.73 -> 2.81 ms, the sum at 30,011 565 -> 618 us, four quadrants at 8,000 153 -> 161.
+constexpr int64_t kAnyOrderMax = 8192;
 // what the direct sum of this context needs of its sort (want_zero, want_hilo)
 void direct_sort_wants(sv_ctx *c);
 // the mixed-precision all-pairs sums (no symmetry images) of n sorted

@@ -99,3 +99,12 @@ def test_sources_first(n, prec):
     a = accel(st, softening2=EPS20, precision=prec)
     assert rel_l2(a, O.direct_f64(st, EPS20), st["status"]) < BOUND[prec]
     assert not np.any(a[st["status"] != 1])
+
+
+@pytest.mark.parametrize("n", [4096, 4097])
+def test_sources_first_with_images(n):
+    """The same at the size of the four quadrants (an image counts as a particle's pairs do)."""
+    st = state(n, True, 700 + n)
+    st["status"][:5] = 0
+    a = accel(st, softening2=EPS20, precision=sv.MIXED, symmetry=sv.SYM_ROTATIONAL)
+    assert rel_l2(a, O.direct_f64(st, EPS20, sym=1), st["status"]) < BOUND[sv.MIXED]
