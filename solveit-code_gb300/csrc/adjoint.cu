@@ -520,10 +520,9 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
     // the particles of the step's window in Morton order (a small window: sources first)
     const bool fp64 = c->P.precision == SV_PREC_FP64;
     c->fstatus = c->wstatus;
-    c->S.want_zero = true;
-    c->S.want_hilo = !fp64;
-    c->S.hl_abs = false;
-    c->S.any_order = nn <= kAnyOrderMax;
+    c->S.want.zero = true;
+    c->S.want.hilo = !fp64;
+    c->S.want.any_order = nn <= kAnyOrderMax;
     const sv_status st = sort_state(c, 0, nn);
     c->fstatus = nullptr;
     SV_TRY(st);

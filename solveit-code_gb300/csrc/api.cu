@@ -1090,7 +1090,7 @@ sv_status sv::compute_accel_device(sv_ctx *c, int64_t first, int64_t last) {
         const int32_t *st2 = nullptr;
         if (outliers) SV_TRY(outliers_detect(c, &st2));  // outliers leave the tree; summed directly below
         auto sort_all = [&](int levels) -> sv_status {
-            c->S.want_levels = levels;
+            c->S.want.levels = levels;
             if (c->P.method == SV_METHOD_DIRECT) direct_sort_wants(c);
             else if (c->P.method == SV_METHOD_BARNES_HUT) bh_sort_wants(c);
             if (outliers) {

@@ -547,9 +547,8 @@ sv_status bh_accel(sv_ctx *c) {
 }
 
 void bh_sort_wants(sv_ctx *c) {
-    c->S.want_hilo = true;
-    c->S.hl_abs = false;
-    c->S.want_zero = c->P.symmetry != SV_SYM_NONE;  // the images' forces are added up
+    c->S.want.hilo = true;
+    c->S.want.zero = c->P.symmetry != SV_SYM_NONE;  // the images' forces are added up
 }
 
 int bh_sort_levels(const sv_ctx *c) {

@@ -466,13 +466,13 @@ direct_fp64_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
 }  // namespace
 
 void direct_sort_wants(sv_ctx *c) {
-    c->S.want_zero = true;
-    c->S.want_hilo = c->P.precision == SV_PREC_MIXED;
-    c->S.hl_abs = c->P.symmetry == SV_SYM_ROTATIONAL;
+    c->S.want.zero = true;
+    c->S.want.hilo = c->P.precision == SV_PREC_MIXED;
+    c->S.want.hl_abs = c->P.symmetry == SV_SYM_ROTATIONAL;
     const ImageSet *I = nullptr;
     int64_t images = c->P.symmetry == SV_SYM_ROTATIONAL ? 4 : 1;
     if (c->P.symmetry == SV_SYM_TRANSLATIONAL) images = image_set(c, &I) == SV_OK ? I->count : INT32_MAX;
-    c->S.any_order = c->n * c->n <= kAnyOrderMax * kAnyOrderMax / images;
+    c->S.want.any_order = c->n * c->n <= kAnyOrderMax * kAnyOrderMax / images;
 }
 
 sv_status direct_accel(sv_ctx *c) {

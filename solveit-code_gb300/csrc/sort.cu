@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <utility>
 
 #include "sv_internal.cuh"
 
@@ -553,13 +554,11 @@ static double root_scale(const sv_ctx *c) {
 
 sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t last) {
     const int64_t n = v.n;
-    const bool zero = c->S.want_zero, hilo = c->S.want_hilo, hl_abs = c->S.hl_abs;
+    const SortWants want = std::exchange(c->S.want, SortWants());  // before the buffers are replaced
     SV_TRY(ensure_sorted_capacity(c, n));
     Sorted &S = c->S;
-    const bool any_order = S.any_order;
-    S.want_zero = S.want_hilo = S.any_order = S.raw = false;
-    S.hl_abs = hl_abs;
-    if (hilo && S.hl_cap < n) {
+    S.raw = false;
+    if (want.hilo && S.hl_cap < n) {
         cudaFree(S.ph);
         cudaFree(S.pl);
         S.ph = S.pl = nullptr;
@@ -570,20 +569,19 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     }
     S.n = n;
     S.n_orig = v.n_orig;
-    // levels 1 .. want_levels occupy bits >= 3 (kMortonBits - want_levels); bit 63 marks inactive keys
-    const int levels = std::max(1, std::min(kMortonBits, S.want_levels));
-    S.want_levels = kMortonBits;
+    // levels 1 .. levels occupy bits >= 3 (kMortonBits - levels); bit 63 marks inactive keys
+    const int levels = std::max(1, std::min(kMortonBits, want.levels));
     S.key_levels = levels;
     const int sh = 3 * (kMortonBits - levels);
     GatherArgs ga{v.x, v.y, v.z, v.q, v.m, v.qom, v.status, first, std::min(last, v.n_orig), c->P.k_const,
-                  S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr, hilo ? S.ph : nullptr,
-                  hilo ? S.pl : nullptr, hl_abs ? 1 : 0, S.root, reinterpret_cast<int *>(S.root + 14)};
-    if (zero) {
+                  S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr, want.hilo ? S.ph : nullptr,
+                  want.hilo ? S.pl : nullptr, want.hl_abs ? 1 : 0, S.root, reinterpret_cast<int *>(S.root + 14)};
+    if (want.zero) {
         ga.zax = S.ax;
         ga.zay = S.ay;
         ga.zaz = S.az;
     }
-    if (any_order && n > 0) {
+    if (want.any_order && n > 0) {
         sources_first<<<div_up(n, 256), 256, 0, c->stream>>>((int)n, S.idx, ga, reinterpret_cast<unsigned *>(S.root + 15),
                                                            reinterpret_cast<int *>(S.root + 13));
         SV_LAUNCHED(c);

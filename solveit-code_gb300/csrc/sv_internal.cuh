@@ -20,6 +20,15 @@ constexpr uint64_t kInactiveKey = ~0ull;
 // closer than 1 pm.
 constexpr float kMinR2 = 1e-24f;
 
+// What a method needs of the next sort: a one-shot request, taken by the sort.
+struct SortWants {
+    int levels = kMortonBits;  // Morton levels to order: a tree needs its keys ordered down to its leaf level only
+    bool zero = false;         // also clear ax, ay, az (a method that adds into them)
+    bool hilo = false;         // also write ph, pl
+    bool hl_abs = false;       // ... relative to the z axis in x and y
+    bool any_order = false;    // only put the sources first
+};
+
 // Morton-sorted working copy of the plume, rebuilt at every force evaluation.
 // Sorting makes every block of consecutive targets spatially compact, which is
 // what lets the mixed-precision kernels take FP32 coordinates relative to an
@@ -35,7 +44,7 @@ struct Sorted {
     bool raw = false;  // ax, ay, az lack the factor K q/m (the scatter multiplies; cleared by it)
     // positions as FP32 hi + lo parts relative to `root`'s origin (hl_abs: to the
     // z axis in x and y), hi.w the source charge, lo.w 1 for targets; written by
-    // the sort when want_hilo
+    // the sort when want.hilo
     float4 *ph = nullptr, *pl = nullptr;
     int64_t hl_cap = 0;
     // a second field to add in the scatter (the FMM's far field: x, y, z at
@@ -45,18 +54,13 @@ struct Sorted {
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
     double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S;
-                               // [14] int: 1 when the sorted source charges differ (want_hilo); [13], [15]
+                               // [14] int: 1 when the sorted source charges differ (want.hilo); [13], [15]
                                // int: words of the kernels whose last CTA finishes, zero between launches
     long long *red = nullptr;  // device reduction scratch
     int red_blocks = 0;
     int64_t cap = 0;
-    // Morton levels the next sort must order (a one-shot request, reset to all
-    // of them by the sort) and the levels the last sort ordered: an FMM tree
-    // needs its keys ordered down to its leaf level only
-    int want_levels = kMortonBits, key_levels = kMortonBits;
-    bool want_zero = false;  // the next sort also clears ax, ay, az (a method that adds into them)
-    bool want_hilo = false, hl_abs = false;  // the next sort also writes ph, pl
-    bool any_order = false;  // the next sort need only put the sources first
+    SortWants want;                // of the next sort
+    int key_levels = kMortonBits;  // Morton levels the last sort ordered
     bool resort = false;  // the FMM found its leaf level below key_levels: sort again, fully
     int64_t n = 0;       // sorted entries (caller particles plus any image copies)
     int64_t n_orig = 0;  // caller particles; sorted idx >= n_orig are image copies
@@ -305,7 +309,7 @@ sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; r
 // at 900 58 -> 43; above, the close form costs more: four adjoint steps at 16,384
 // 2.73 -> 2.81 ms, the sum at 30,011 565 -> 618 us, four quadrants at 8,000 153 -> 161.
 constexpr int64_t kAnyOrderMax = 8192;
-// what the direct sum of this context needs of its sort (want_zero, want_hilo)
+// what the direct sum of this context needs of its sort
 void direct_sort_wants(sv_ctx *c);
 // the mixed-precision all-pairs sums (no symmetry images) of n sorted
 // particles given as FP32 hi + lo parts (Sorted::ph, pl), without the targets'
@@ -336,7 +340,7 @@ sv_status bh_accel(sv_ctx *c);
 sv_status sampled_error_range(sv_ctx *c, int64_t first, int64_t count, int k_max, double *err);
 // Morton levels the Barnes-Hut's next sort needs (its last tree's depth + 2, or all)
 int bh_sort_levels(const sv_ctx *c);
-void bh_sort_wants(sv_ctx *c);  // what the walk needs of its sort (want_hilo, want_zero)
+void bh_sort_wants(sv_ctx *c);  // what the walk needs of its sort
 // the last Barnes-Hut evaluation's cell and pair interaction counts (waits for the stream)
 sv_status bh_counts(sv_ctx *c, double *cells, double *pairs);
 sv_status fmm_accel(sv_ctx *c);
