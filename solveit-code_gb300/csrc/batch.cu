@@ -9,9 +9,9 @@
 //    0..nfp-1), each particle followed by its source-only rotated copies for
 //    the 4-fold rotational variant; direct plumes follow (their images are
 //    formed on the fly by the pair kernel).
-//  * one radix sort of all slots by key = plume id << 54 | 18-bit-per-axis
-//    Morton code relative to the plume's own root cube, so each plume's slots
-//    stay contiguous and spatially ordered.
+//  * radix sorts of the FMM plumes' and of the direct plumes' slots by key =
+//    plume id << 54 | 18-bit-per-axis Morton code relative to the plume's own
+//    root cube, so each plume's slots stay contiguous and spatially ordered.
 //  * FMM plumes: one forest of octrees (forest.cuh).  Each plume's cube is
 //    enlarged by 2^delta so that a single leaf level L is, for every plume,
 //    the level its cost model picks.  delta is chosen on the device at every
@@ -52,6 +52,11 @@ struct DirectItem {
     int t0, t1, j0, j1, nimg, pad0, pad1, pad2;
 };
 
+struct SortRoom {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+
 struct Batch {
     int np = 0, nfp = 0;
     std::vector<int64_t> count, off;  // caller order: plume p owns [off[p], off[p] + count[p])
@@ -75,8 +80,7 @@ struct Batch {
     int nitems = 0;
     double direct_pairs = 0;          // pair interactions of the direct plumes per evaluation
     int *queue = nullptr;
-    void *cub_tmp = nullptr;
-    size_t cub_bytes = 0;
+    SortRoom cub, cub_side;           // of the forest's slots, of the direct plumes' (side stream)
     // forest
     ForestArgs fa;
     bool planned = false;
@@ -561,8 +565,40 @@ int slots_per_particle(const Batch &B, int pid) {
     return B.method[p] == SV_METHOD_FMM && B.sym[p] == SV_SYM_ROTATIONAL ? 4 : 1;
 }
 
-// bbox, roots, keys, sort, (adapt: per-plume depth), gather (launches only)
-sv_status sort_batch(sv_ctx *c, Batch &B, bool adapt) {
+// room for the sort of n slots by any of their key bits
+sv_status sort_room(sv_ctx *c, int64_t n, SortRoom &r) {
+    SV_CK(c, cub::DeviceRadixSort::SortPairs(nullptr, r.bytes, c->S.keys_alt, c->S.keys, c->S.idx_alt, c->S.idx,
+                                             (int)std::max<int64_t>(n, 1), 0, kPidShift + 9, c->stream));
+    SV_CK(c, cudaMalloc(&r.p, r.bytes));
+    return SV_OK;
+}
+
+// view slots [v0, v1) in the order of their key bits bit0 and up
+sv_status order_slots(sv_ctx *c, Batch &B, int64_t v0, int64_t v1, int bit0, const SortRoom &room,
+                      cudaStream_t st) {
+    Sorted &S = c->S;
+    int bit1 = kPidShift;  // bits that no plume id has take no sort pass
+    while ((1 << (bit1 - kPidShift)) < B.np) bit1++;
+    size_t bytes = room.bytes;
+    SV_CK(c, cub::DeviceRadixSort::SortPairs(room.p, bytes, S.keys_alt + v0, S.keys + v0, S.idx_alt + v0, S.idx + v0,
+                                             (int)(v1 - v0), bit0, bit1, st));
+    c->launches += 2 * ((bit1 - bit0 + 7) / 8);
+    return SV_OK;
+}
+
+sv_status gather_slots(sv_ctx *c, Batch &B, int64_t v0, int64_t v1, cudaStream_t st) {
+    Sorted &S = c->S;
+    batch_gather_kernel<<<div_up(v1 - v0, 256), 256, 0, st>>>(v1 - v0, S.idx + v0, B.vsrc, B.vtag, c->x, c->y, c->z,
+                                                              c->q, c->m, c->qom, force_status(c), B.roots,
+                                                              c->P.k_const, S.x + v0, S.y + v0, S.z + v0, S.q + v0,
+                                                              S.qm + v0);
+    SV_LAUNCHED(c);
+    return SV_OK;
+}
+
+// bbox, roots and keys of every slot; the forest's slots in order, (adapt:
+// per-plume depth), gathered (launches only)
+sv_status keys_batch(sv_ctx *c, Batch &B) {
     Sorted &S = c->S;
     const int64_t nv = B.nv;
     bbox_chunks_kernel<<<B.nchunks, 256, 0, c->stream>>>(B.chunk_beg, B.vsrc, B.vtag, c->x, c->y, c->z, force_status(c),
@@ -573,19 +609,18 @@ sv_status sort_batch(sv_ctx *c, Batch &B, bool adapt) {
     batch_keys_kernel<<<div_up(nv, 256), 256, 0, c->stream>>>(B.np, nv, B.vsrc, B.vtag, c->x, c->y, c->z, force_status(c),
                                                               B.roots, S.keys_alt, S.idx_alt);
     SV_LAUNCHED(c);
+    return SV_OK;
+}
+
+sv_status sort_forest(sv_ctx *c, Batch &B, bool adapt) {
+    Sorted &S = c->S;
+    if (B.nf == 0) return SV_OK;
     // An evaluation uses the boxes of levels up to L in each plume's own cube, and one
-    // level more for its choice of level; order below that and bits no plume id
-    // has take no sort pass (24 plumes, L = 9: 35 of 63 bits, five passes of 19 us
-    // instead of eight).
+    // level more for its choice of level; order below that takes no sort pass (24
+    // plumes, L = 9: 35 of 63 bits, five passes of 19 us instead of eight).
     const int top = adapt && B.fa.spec.L > 0 ? std::min(kBatchBits, B.fa.spec.L + 1) : kBatchBits;
-    const int bit0 = 3 * (kBatchBits - top);
-    int bit1 = kPidShift;
-    while ((1 << (bit1 - kPidShift)) < B.np) bit1++;
-    size_t bytes = B.cub_bytes;
-    SV_CK(c, cub::DeviceRadixSort::SortPairs(B.cub_tmp, bytes, S.keys_alt, S.keys, S.idx_alt, S.idx, (int)nv, bit0,
-                                             bit1, c->stream));
-    c->launches += 2 * ((bit1 - bit0 + 7) / 8);
-    if (adapt && B.nfp > 0 && B.nf > 0) {
+    SV_TRY(order_slots(c, B, 0, B.nf, 3 * (kBatchBits - top), B.cub, c->stream));
+    if (adapt && B.nfp > 0) {
         SV_CK(c, cudaMemsetAsync(B.d_hist, 0, sizeof(int) * kBLevels * B.nfp, c->stream));
         plume_levels_kernel<<<div_up(B.nf, 256), 256, 0, c->stream>>>(S.keys, B.nf, B.d_hist);
         SV_LAUNCHED(c);
@@ -596,33 +631,37 @@ sv_status sort_batch(sv_ctx *c, Batch &B, bool adapt) {
         shift_keys_kernel<<<div_up(B.nf, 256), 256, 0, c->stream>>>(S.keys, B.nf, B.delta);
         SV_LAUNCHED(c);
     }
-    batch_gather_kernel<<<div_up(nv, 256), 256, 0, c->stream>>>(nv, S.idx, B.vsrc, B.vtag, c->x, c->y, c->z, c->q,
-                                                                c->m, c->qom, force_status(c), B.roots, c->P.k_const,
-                                                                S.x, S.y, S.z, S.q, S.qm);
-    SV_LAUNCHED(c);
-    return SV_OK;
+    return gather_slots(c, B, 0, B.nf, c->stream);
 }
 
 // one force evaluation of every plume into c->a{x,y,z} (launches only)
 sv_status batch_force(sv_ctx *c, Batch &B) {
     Sorted &S = c->S;
-    SV_TRY(sort_batch(c, B, true));
+    SV_TRY(keys_batch(c, B));
     const int64_t nd = B.nv - B.nf;
-    if (B.nitems > 0) {
-        SV_CK(c, cudaMemsetAsync(S.ax + B.nf, 0, sizeof(double) * nd, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.ay + B.nf, 0, sizeof(double) * nd, c->stream));
-        SV_CK(c, cudaMemsetAsync(S.az + B.nf, 0, sizeof(double) * nd, c->stream));
-        SV_CK(c, cudaMemsetAsync(B.queue, 0, sizeof(int), c->stream));
+    if (nd > 0) {
+        // The direct plumes on their own stream, beside the forest.  All Morton levels are
+        // ordered: the pair kernel's FP32 offsets are as precise as 256 consecutive
+        // slots are compact, and an order as shallow as the forest's loses up to a
+        // factor of ten there (8,000 ions, one of them 0.1 mm ahead: 4e-6 -> 7e-5).
         SV_CK(c, cudaEventRecord(B.fork, c->stream));
         SV_CK(c, cudaStreamWaitEvent(B.side, B.fork, 0));
-        const int dev_sms = device_sms();
-        direct_batch_kernel<<<std::min(B.nitems, 8 * dev_sms), kDTPB, 0, B.side>>>(
-            B.items, B.nitems, B.queue, S.x, S.y, S.z, S.q, S.qm, (float)c->P.softening2, S.ax, S.ay, S.az);
-        SV_LAUNCHED(c);
+        SV_TRY(order_slots(c, B, B.nf, B.nv, 0, B.cub_side, B.side));
+        SV_TRY(gather_slots(c, B, B.nf, B.nv, B.side));
+        SV_CK(c, cudaMemsetAsync(S.ax + B.nf, 0, sizeof(double) * nd, B.side));
+        SV_CK(c, cudaMemsetAsync(S.ay + B.nf, 0, sizeof(double) * nd, B.side));
+        SV_CK(c, cudaMemsetAsync(S.az + B.nf, 0, sizeof(double) * nd, B.side));
+        if (B.nitems > 0) {
+            SV_CK(c, cudaMemsetAsync(B.queue, 0, sizeof(int), B.side));
+            direct_batch_kernel<<<std::min(B.nitems, 8 * device_sms()), kDTPB, 0, B.side>>>(
+                B.items, B.nitems, B.queue, S.x, S.y, S.z, S.q, S.qm, (float)c->P.softening2, S.ax, S.ay, S.az);
+            SV_LAUNCHED(c);
+        }
         SV_CK(c, cudaEventRecord(B.join, B.side));
     }
+    SV_TRY(sort_forest(c, B, true));
     if (B.nf > 0) SV_TRY(fmm_forest_run(c, B.fa));
-    if (B.nitems > 0) SV_CK(c, cudaStreamWaitEvent(c->stream, B.join, 0));
+    if (nd > 0) SV_CK(c, cudaStreamWaitEvent(c->stream, B.join, 0));
     batch_scatter_kernel<<<div_up(B.nv, 256), 256, 0, c->stream>>>(B.nv, S.idx, B.vsrc, B.vtag, S.ax, S.ay, S.az,
                                                                    c->ax, c->ay, c->az);
     SV_LAUNCHED(c);
@@ -633,7 +672,8 @@ sv_status batch_force(sv_ctx *c, Batch &B) {
 // the box capacities from the current state (blocking; not captured).
 sv_status plan_forest(sv_ctx *c, Batch &B, int cap_scale) {
     drop_graphs(B);
-    SV_TRY(sort_batch(c, B, false));
+    SV_TRY(keys_batch(c, B));
+    SV_TRY(sort_forest(c, B, false));
     B.fa.spec.n = (int)B.nf;
     if (B.nfp == 0 || B.nf == 0) {
         SV_CK(c, cudaStreamSynchronize(c->stream));
@@ -757,7 +797,7 @@ void batch_free(sv_ctx *c) {
     cudaFree(B.vsrc); cudaFree(B.vtag); cudaFree(B.roots); cudaFree(B.delta); cudaFree(B.d_hist);
     cudaFree(B.d_vbeg);
     cudaFree(B.chunk_beg); cudaFree(B.pid_chunk); cudaFree(B.chunk_red); cudaFree(B.items);
-    cudaFree(B.queue); cudaFree(B.cub_tmp); cudaFree(B.d_nbox); cudaFree(B.d_err); cudaFree(B.d_time);
+    cudaFree(B.queue); cudaFree(B.cub.p); cudaFree(B.cub_side.p); cudaFree(B.d_nbox); cudaFree(B.d_err); cudaFree(B.d_time);
     cudaFree(B.backup);
     cudaFree(B.backup_st);
     cudaFree(B.ev_count0);
@@ -901,11 +941,8 @@ sv_status batch_plan(sv_ctx *c, int32_t np, const int64_t *counts, const int32_t
     SV_CK(c, cudaEventCreateWithFlags(&B.fork, cudaEventDisableTiming));
     SV_CK(c, cudaEventCreateWithFlags(&B.join, cudaEventDisableTiming));
     SV_TRY(ensure_sorted_capacity(c, std::max<int64_t>(B.nv, 1)));
-    size_t bytes = 0;
-    SV_CK(c, cub::DeviceRadixSort::SortPairs(nullptr, bytes, c->S.keys_alt, c->S.keys, c->S.idx_alt, c->S.idx,
-                                             (int)std::max<int64_t>(B.nv, 1), 0, kPidShift + 9, c->stream));
-    SV_CK(c, cudaMalloc(&B.cub_tmp, bytes));
-    B.cub_bytes = bytes;
+    SV_TRY(sort_room(c, B.nf, B.cub));
+    SV_TRY(sort_room(c, B.nv - B.nf, B.cub_side));
     c->S.n = B.nv;
     c->S.n_orig = c->n;
     SV_TRY(build_items(c, B));
