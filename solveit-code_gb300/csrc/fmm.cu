@@ -21,7 +21,7 @@
 //   P2P   leaf boxes, a CTA per box or chunk of its targets; groups of
 //         threads, two targets each, share the sources staged in shared memory
 //         as FP32 offsets from the target box centre; FP32 partial sums of at
-//         most 64 sources are accumulated with Kahan compensation.
+//         most 32 sources are accumulated with Kahan compensation.
 //
 // Expansions are kept in box units (coordinates divided by the box side h),
 // so the M2L tables depend on the integer offset only; the softened M2L
@@ -1358,8 +1358,8 @@ __device__ __forceinline__ void kahan_add(float &s, float &e, float v) {
 // two targets each, and s = kP2PThreads / h such groups (32 at most) that share
 // the staged sources run by run, so the lanes stay busy whatever the box
 // holds (h s / kP2PThreads, ~0.9 on average) and a box with many targets and
-// sources occupies four warps instead of one.  Up to 64 sources per group are
-// summed in FP32 (32 per half of the packed pair), then added with Kahan
+// sources occupies four warps instead of one.  Up to 32 sources per group are
+// summed in FP32 (16 per half of the packed pair), then added with Kahan
 // compensation; the groups' sums are added in group order at the end, so the
 // result does not depend on scheduling.  FP32-pipe bound: 11 FMA-pipe operations and one reciprocal
 // square root per pair.
@@ -1569,8 +1569,9 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, int stride, co
                         pair2<CLAMP, UQ>(X, Y, Z, Q, BX, BY, BZ, E2, gbx, gby, gbz);
                     }
                 }
-                // at most 64 sources' FP32 sums (two tiles) per compensated addition
-                if (buf || c0 + tile >= total) {
+                // 32 sources' FP32 sums per compensated addition (two tiles of a shorter run); 64
+                // take 0.4 to 1.3 % less of a step and lose twice as much to each uncompensated sum
+                if (run == 32 || buf || c0 + tile >= total) {
                     kahan_add(sax, eax, gax.x + gax.y);
                     kahan_add(say, eay, gay.x + gay.y);
                     kahan_add(saz, eaz, gaz.x + gaz.y);
