@@ -158,12 +158,14 @@ __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double 
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = idx[s];
-    float4 h, l;
-    split_hilo(x3[3 * i] - root[0], h.x, l.x);
-    split_hilo(x3[3 * i + 1] - root[1], h.y, l.y);
-    split_hilo(x3[3 * i + 2] - root[2], h.z, l.z);
     const int32_t w = st[i];
-    h.w = is_src(w) ? (float)q[i] : 0.0f;
+    // a particle that is no source sits at the origin: its own position may be anywhere
+    const bool src = is_src(w);
+    float4 h, l;
+    split_hilo(src ? x3[3 * i] - root[0] : 0.0, h.x, l.x);
+    split_hilo(src ? x3[3 * i + 1] - root[1] : 0.0, h.y, l.y);
+    split_hilo(src ? x3[3 * i + 2] - root[2] : 0.0, h.z, l.z);
+    h.w = src ? (float)q[i] : 0.0f;
     const double k = (w == 1 && m[i] > 0.0) ? kconst * q[i] / m[i] : 0.0;
     l.w = k != 0.0 ? 1.f : 0.f;
     ph[s] = h;

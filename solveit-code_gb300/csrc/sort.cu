@@ -190,10 +190,15 @@ __device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
     return tgt ? a.kconst * (a.qom ? a.qom[i] : a.q[i] / a.m[i]) : 0.0;
 }
 
-// particle i into sorted slot s (every load before the first store); with ph, whether its source
-// charge differs from particle 0's
+// Particle i into sorted slot s (every load before the first store); with ph, whether its source
+// charge differs from particle 0's.  A particle that is no source takes no part in any sum; it
+// is put at the root's origin, for its own position may be anywhere and could become the
+// origin of a block's FP32 coordinates (300 ions among as many lost ones within 100 m:
+// 7.7e-7 against 1.2e-4 force error).
 __device__ __forceinline__ bool gather_one(const GatherArgs &a, const double *root, int64_t s, uint32_t i) {
-    const double x = a.x[i], y = a.y[i], z = a.z[i], k = sorted_qm(a, i);
+    const bool src = is_source(a.st[i]);
+    const double x = src ? a.x[i] : root[0], y = src ? a.y[i] : root[1], z = src ? a.z[i] : root[2];
+    const double k = sorted_qm(a, i);
     const float q = sorted_charge(a, i);
     a.xs[s] = x;
     a.ys[s] = y;
@@ -444,7 +449,7 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
     if (!live) return;
     const uint32_t i = cidx[s];
     if (part < 3) {
-        const double v = (part == 0 ? a.x : part == 1 ? a.y : a.z)[i];
+        const double v = is_source(a.st[i]) ? (part == 0 ? a.x : part == 1 ? a.y : a.z)[i] : a.root[part];  // as gather_one
         (part == 0 ? a.xs : part == 1 ? a.ys : a.zs)[rank] = v;
         if (a.ph) {
             float h, l;
