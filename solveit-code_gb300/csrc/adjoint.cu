@@ -252,13 +252,16 @@ __global__ void __launch_bounds__(32 * kPairWarps) jtv_pairs64_kernel(JPair64Arg
 // The reciprocal square root is refined by one Newton step.  FP32-pipe bound:
 // 45 operations per pair (39 when all charges are equal), two targets per packed
 // instruction, each pair once: 16,384 particles 532 -> 211 us per launch, 4,096
-// 54 -> 21 us, against the one-sided scalar kernel.
+// 54 -> 21 us, against the one-sided scalar kernel.  Wide plumes (kWide) take their
+// coordinates from the FP64 positions in the same code (1 % of a gradient; a form of its
+// own costs as much inlined, 2 to 3 % out of line).
 struct JPairArgs {
     const float4 *ph, *pl, *uh, *ul;
+    const double *x, *y, *z;  // wide plumes
     int n, nb, ct, nch;
     float e2;
     double *ox, *oy, *oz;
-    const int *differ;
+    const int *marks;
 };
 
 constexpr int kJR = 4, kJH = kJR / 2;  // particles (packed pairs) of the block per lane
@@ -269,17 +272,18 @@ struct JBlock {
 };
 struct JLow {
     float2 x[kJH][32], y[kJH][32], z[kJH][32];
+    float2 rx[kJH][32], ry[kJH][32], rz[kJH][32];
 };
-// the travelling particle: negated coordinates, their parts below FP32, charge,
-// negated u (hi, lo), and its sums
+// the travelling particle: negated coordinates, charge, negated u (hi, lo), and its sums
 struct JTravel {
-    float x, y, z, mx, my, mz, q, ux, uy, uz, vx, vy, vz, sx, sy, sz;
+    Parts x, y, z;
+    float q = 0.f, ux = 0.f, uy = 0.f, uz = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
 };
 
 __device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float turn(float v) { return __shfl_sync(0xffffffffu, v, ((threadIdx.x & 31) + 1) & 31); }
 
-template <bool UQ, bool SYM, bool NEAR>
+template <bool UQ, bool SYM, int MODE>
 __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, float min_r2, JTravel &t) {
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -287,12 +291,19 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
         float2 jx, jy, jz;
 #pragma unroll
         for (int p = 0; p < kJH; p++) {
-            float2 dx = __fadd2_rn(b.X[p], dup(t.x)), dy = __fadd2_rn(b.Y[p], dup(t.y)),
-                   dz = __fadd2_rn(b.Z[p], dup(t.z));
-            if (NEAR) {
-                dx = __fadd2_rn(dx, __fadd2_rn(low.x[p][lane], dup(t.mx)));
-                dy = __fadd2_rn(dy, __fadd2_rn(low.y[p][lane], dup(t.my)));
-                dz = __fadd2_rn(dz, __fadd2_rn(low.z[p][lane], dup(t.mz)));
+            float2 dx = __fadd2_rn(b.X[p], dup(t.x.v)), dy = __fadd2_rn(b.Y[p], dup(t.y.v)),
+                   dz = __fadd2_rn(b.Z[p], dup(t.z.v));
+            if (MODE != kTileFar) {
+                float2 ex = __fadd2_rn(low.x[p][lane], dup(t.x.low)), ey = __fadd2_rn(low.y[p][lane], dup(t.y.low)),
+                       ez = __fadd2_rn(low.z[p][lane], dup(t.z.low));
+                if (MODE == kTileWide) {
+                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(t.x.rest)));
+                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(t.y.rest)));
+                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(t.z.rest)));
+                }
+                dx = __fadd2_rn(dx, ex);
+                dy = __fadd2_rn(dy, ey);
+                dz = __fadd2_rn(dz, ez);
             }
             float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, E2)));
             r2 = make_float2(fmaxf(r2.x, min_r2), fmaxf(r2.y, min_r2));
@@ -320,13 +331,18 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
                 jz = p == 0 ? vz : __fadd2_rn(jz, vz);
             }
         }
-        t.x = turn(t.x);
-        t.y = turn(t.y);
-        t.z = turn(t.z);
-        if (NEAR) {
-            t.mx = turn(t.mx);
-            t.my = turn(t.my);
-            t.mz = turn(t.mz);
+        t.x.v = turn(t.x.v);
+        t.y.v = turn(t.y.v);
+        t.z.v = turn(t.z.v);
+        if (MODE != kTileFar) {
+            t.x.low = turn(t.x.low);
+            t.y.low = turn(t.y.low);
+            t.z.low = turn(t.z.low);
+        }
+        if (MODE == kTileWide) {
+            t.x.rest = turn(t.x.rest);
+            t.y.rest = turn(t.y.rest);
+            t.z.rest = turn(t.z.rest);
         }
         if (!UQ) t.q = turn(t.q);
         t.ux = turn(t.ux);
@@ -344,52 +360,78 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
 }
 
 template <bool UQ, bool SYM>
-__device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, int B, int k0, int k1) {
+__device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, bool wide, int A, int B, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     const float sc = (float)kLen;
     const int i0 = A * 32 * kJR, io = min(i0 + 16 * kJR, a.n - 1);
     const float4 oh = a.ph[io], ol = a.pl[io];
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+    if (wide) {
+        ox = a.x[io];
+        oy = a.y[io];
+        oz = a.z[io];
+    }
+    // particle i's coordinates from the block's origin, in 2^-30 m
+    auto coordinates = [&](int i, const float4 &h, Parts &x, Parts &y, Parts &z) {
+        if (wide) {
+            x = parts_of((a.x[i] - ox) * kLen);
+            y = parts_of((a.y[i] - oy) * kLen);
+            z = parts_of((a.z[i] - oz) * kLen);
+            return;
+        }
+        const float4 l = a.pl[i];
+        x.v = hilo_diff(h.x, l.x, oh.x, ol.x, x.low) * sc;
+        y.v = hilo_diff(h.y, l.y, oh.y, ol.y, y.low) * sc;
+        z.v = hilo_diff(h.z, l.z, oh.z, ol.z, z.low) * sc;
+        x.low *= sc;
+        y.low *= sc;
+        z.low *= sc;
+    };
     JBlock b;
     float ext = 0.f;
     __syncwarp();  // the previous unit's reads of `low`
 #pragma unroll
     for (int p = 0; p < kJH; p++) {
-        float c[2][13];
+        Parts x[2], y[2], z[2];
+        float c[2][7];  // charge, u (hi, lo)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int i = i0 + 32 * (2 * p + u) + lane;
 #pragma unroll
-            for (int e = 0; e < 13; e++) c[u][e] = 0.f;
-            c[u][0] = -kFar;
+            for (int e = 0; e < 7; e++) c[u][e] = 0.f;
+            x[u].v = -kFar;
             if (i < a.n) {
-                const float4 h = a.ph[i], l = a.pl[i], uh = a.uh[i], ul = a.ul[i];
-                c[u][0] = hilo_diff(h.x, l.x, oh.x, ol.x, c[u][4]) * sc;
-                c[u][1] = hilo_diff(h.y, l.y, oh.y, ol.y, c[u][5]) * sc;
-                c[u][2] = hilo_diff(h.z, l.z, oh.z, ol.z, c[u][6]) * sc;
-                c[u][3] = h.w;
-                c[u][7] = uh.x;
-                c[u][8] = uh.y;
-                c[u][9] = uh.z;
-                c[u][10] = ul.x;
-                c[u][11] = ul.y;
-                c[u][12] = ul.z;
-                ext = fmaxf(ext, fmaxf(fabsf(c[u][0]), fmaxf(fabsf(c[u][1]), fabsf(c[u][2]))));
+                const float4 h = a.ph[i], uh = a.uh[i], ul = a.ul[i];
+                coordinates(i, h, x[u], y[u], z[u]);
+                c[u][0] = h.w;
+                c[u][1] = uh.x;
+                c[u][2] = uh.y;
+                c[u][3] = uh.z;
+                c[u][4] = ul.x;
+                c[u][5] = ul.y;
+                c[u][6] = ul.z;
+                ext = fmaxf(ext, fmaxf(fabsf(x[u].v), fmaxf(fabsf(y[u].v), fabsf(z[u].v))));
             }
         }
         auto both = [&](int e) { return make_float2(c[0][e], c[1][e]); };
-        b.X[p] = both(0);
-        b.Y[p] = both(1);
-        b.Z[p] = both(2);
-        b.Q[p] = both(3);
-        low.x[p][lane] = make_float2(c[0][4] * sc, c[1][4] * sc);
-        low.y[p][lane] = make_float2(c[0][5] * sc, c[1][5] * sc);
-        low.z[p][lane] = make_float2(c[0][6] * sc, c[1][6] * sc);
-        b.ux[p] = both(7);
-        b.uy[p] = both(8);
-        b.uz[p] = both(9);
-        b.vx[p] = both(10);
-        b.vy[p] = both(11);
-        b.vz[p] = both(12);
+        b.X[p] = make_float2(x[0].v, x[1].v);
+        b.Y[p] = make_float2(y[0].v, y[1].v);
+        b.Z[p] = make_float2(z[0].v, z[1].v);
+        low.x[p][lane] = make_float2(x[0].low, x[1].low);
+        low.y[p][lane] = make_float2(y[0].low, y[1].low);
+        low.z[p][lane] = make_float2(z[0].low, z[1].low);
+        if (wide) {
+            low.rx[p][lane] = make_float2(x[0].rest, x[1].rest);
+            low.ry[p][lane] = make_float2(y[0].rest, y[1].rest);
+            low.rz[p][lane] = make_float2(z[0].rest, z[1].rest);
+        }
+        b.Q[p] = both(0);
+        b.ux[p] = both(1);
+        b.uy[p] = both(2);
+        b.uz[p] = both(3);
+        b.vx[p] = both(4);
+        b.vy[p] = both(5);
+        b.vz[p] = both(6);
         b.fx[p] = b.fy[p] = b.fz[p] = make_float2(0.f, 0.f);
     }
     __syncwarp();
@@ -400,17 +442,11 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, i
     const float min_r2 = kMinR2 * sc * sc;
     for (int k = k0; k < k1; k++) {
         const int j = B * 32 * kJR + 32 * k + lane;
-        JTravel t{};
-        t.x = -kFar;
-        bool near = false;
+        JTravel t;
+        Parts x{kFar}, y, z;
         if (j < a.n) {
-            const float4 h = a.ph[j], l = a.pl[j], uh = a.uh[j], ul = a.ul[j];
-            t.x = -sc * hilo_diff(h.x, l.x, oh.x, ol.x, t.mx);
-            t.y = -sc * hilo_diff(h.y, l.y, oh.y, ol.y, t.my);
-            t.z = -sc * hilo_diff(h.z, l.z, oh.z, ol.z, t.mz);
-            t.mx *= -sc;
-            t.my *= -sc;
-            t.mz *= -sc;
+            const float4 h = a.ph[j], uh = a.uh[j], ul = a.ul[j];
+            coordinates(j, h, x, y, z);
             t.q = h.w;
             t.ux = -uh.x;
             t.uy = -uh.y;
@@ -418,10 +454,17 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, i
             t.vx = -ul.x;
             t.vy = -ul.y;
             t.vz = -ul.z;
-            near = fmaxf(fabsf(t.x), fmaxf(fabsf(t.y), fabsf(t.z))) <= 2.f * ext;
         }
-        if (!SYM || __any_sync(0xffffffffu, near)) jtv_tile<UQ, SYM, true>(b, low, E2, min_r2, t);
-        else jtv_tile<UQ, SYM, false>(b, low, E2, min_r2, t);
+        const bool near = j < a.n && fmaxf(fabsf(x.v), fmaxf(fabsf(y.v), fabsf(z.v))) <= 2.f * ext;
+        t.x = negated(x);
+        t.y = negated(y);
+        t.z = negated(z);
+        if (!SYM || __any_sync(0xffffffffu, near)) {
+            if (wide) jtv_tile<UQ, SYM, kTileWide>(b, low, E2, min_r2, t);
+            else jtv_tile<UQ, SYM, kTileNear>(b, low, E2, min_r2, t);
+        } else {
+            jtv_tile<UQ, SYM, kTileFar>(b, low, E2, min_r2, t);
+        }
         if (SYM && j < a.n) {
             atomicAdd(&a.ox[j], widen(t.sx * q0));
             atomicAdd(&a.oy[j], widen(t.sy * q0));
@@ -442,17 +485,17 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) jtv_pairs_kernel(JPairArgs
     __shared__ JLow lows[kPairWarps];
     JLow &low = lows[threadIdx.x >> 5];
     const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
-    const bool differ = *a.differ != 0;
+    const bool differ = a.marks[0] != 0, wide = a.marks[1] != 0;
     for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
         int A, B, ch;
         if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;
         const int k0 = ch * a.ct, k1 = min(k0 + a.ct, kJR);
         if (differ) {
-            if (A != B) jtv_unit<false, true>(a, low, A, B, k0, k1);
-            else jtv_unit<false, false>(a, low, A, B, k0, k1);
+            if (A != B) jtv_unit<false, true>(a, low, wide, A, B, k0, k1);
+            else jtv_unit<false, false>(a, low, wide, A, B, k0, k1);
         } else {
-            if (A != B) jtv_unit<true, true>(a, low, A, B, k0, k1);
-            else jtv_unit<true, false>(a, low, A, B, k0, k1);
+            if (A != B) jtv_unit<true, true>(a, low, wide, A, B, k0, k1);
+            else jtv_unit<true, false>(a, low, wide, A, B, k0, k1);
         }
     }
 }
@@ -536,7 +579,7 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
         const JPair64Args a{S.x, S.y, S.z, u, S.q, n, div_up(n, 32), c->P.softening2, S.ax, S.ay, S.az};
         jtv_pairs64_kernel<<<pair_grid(a.nb, 1), 32 * kPairWarps, 0, c->stream>>>(a);
     } else {
-        JPairArgs a{S.ph, S.pl, uh, ul, n, div_up(n, 32 * kJR), 0, 0, (float)(c->P.softening2 * kLen * kLen),
+        JPairArgs a{S.ph, S.pl, uh, ul, S.x, S.y, S.z, n, div_up(n, 32 * kJR), 0, 0, (float)(c->P.softening2 * kLen * kLen),
                     S.ax, S.ay, S.az, reinterpret_cast<const int *>(S.root + 14)};
         // about 16 units per SM sub-partition
         const int64_t tiles = (int64_t)a.nb * (a.nb + 1) / 2 * kJR;

@@ -22,7 +22,8 @@
 // rounding; where a tile comes within the block's extent, the parts that rounding
 // left out are kept too and added to each difference (six operations more, in a
 // few tiles per block), so that every pair's offset is rounded relative to its own
-// length and not to the block's.  The force error against FP64 is 1.2e-7 to 3e-7
+// length and not to the block's; a wide plume (kWide) takes its coordinates from the FP64
+// positions and keeps all their bits.  The force error against FP64 is 1.2e-7 to 3e-7
 // (relative L2 over plumes of 256 to 30,011 ions); coordinates rounded relative to
 // a CTA's first target gave 3e-7 to 5.6e-6, set by each plume's closest pairs.
 // The loop has no FP64 instruction (GB300 issues one FP64 warp instruction in 64
@@ -90,12 +91,14 @@ struct PairArgs {
     float eps2;
     int kind, images;        // symmetry images, as Images
     const float4 *off;       // translational offsets: hi (xyz) and lo (xyz) per image
+    const double *x, *y, *z, *off64;  // sorted positions and translational offsets, metres
     double *ax, *ay, *az;    // sums, added into
-    const int *differ;       // nonzero: source charges differ
+    const int *marks;        // nonzero: [0] source charges differ, [1] the plume is wide (kWide)
 };
 
 // A block's particles in registers (two per packed value) and the travelling
-// particle; the parts of the block's coordinates below FP32 in shared memory.
+// particle; the parts of the block's coordinates below FP32 in shared memory (wide
+// plumes: two of them).
 template <int R>
 struct PairBlock {
     float2 X[R / 2], Y[R / 2], Z[R / 2], Q[R / 2];   // coordinates, charges
@@ -104,29 +107,35 @@ struct PairBlock {
 template <int R>
 struct PairLow {
     float2 x[R / 2][32], y[R / 2][32], z[R / 2][32];
+    float2 rx[R / 2][32], ry[R / 2][32], rz[R / 2][32];
 };
 
-// 32 steps of a travelling tile: negated coordinates (nx, ny, nz), charge q, and
-// with NEAR the parts below FP32 (mx, my, mz); (sx, sy, sz) return the sums on
-// the travelling particle (SYM).
-template <int R, bool UQ, bool CLAMP, bool SYM, bool NEAR>
-__device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low, float2 E2, float nx, float ny,
-                                          float nz, float q, float mx, float my, float mz, float &sx, float &sy,
-                                          float &sz) {
+// 32 steps of a travelling tile: negated coordinates nx, ny, nz and charge q; (sx, sy,
+// sz) return the sums on the travelling particle (SYM).
+template <int R, bool UQ, bool CLAMP, bool SYM, int MODE>
+__device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low, float2 E2, Parts nx, Parts ny,
+                                          Parts nz, float q, float &sx, float &sy, float &sz) {
+    auto dup = [](float v) { return make_float2(v, v); };
     constexpr int H = R / 2;
     const int lane = threadIdx.x & 31, from = (lane + 1) & 31;
 #pragma unroll 1
     for (int step = 0; step < 32; step++) {
-        const float2 NX = make_float2(nx, nx), NY = make_float2(ny, ny), NZ = make_float2(nz, nz);
-        const float2 QJ = make_float2(q, q);
+        const float2 NX = dup(nx.v), NY = dup(ny.v), NZ = dup(nz.v), QJ = dup(q);
         float2 jx, jy, jz;
 #pragma unroll
         for (int p = 0; p < H; p++) {
             float2 dx = __fadd2_rn(b.X[p], NX), dy = __fadd2_rn(b.Y[p], NY), dz = __fadd2_rn(b.Z[p], NZ);
-            if (NEAR) {
-                dx = __fadd2_rn(dx, __fadd2_rn(low.x[p][lane], make_float2(mx, mx)));
-                dy = __fadd2_rn(dy, __fadd2_rn(low.y[p][lane], make_float2(my, my)));
-                dz = __fadd2_rn(dz, __fadd2_rn(low.z[p][lane], make_float2(mz, mz)));
+            if (MODE != kTileFar) {
+                float2 ex = __fadd2_rn(low.x[p][lane], dup(nx.low)), ey = __fadd2_rn(low.y[p][lane], dup(ny.low)),
+                       ez = __fadd2_rn(low.z[p][lane], dup(nz.low));
+                if (MODE == kTileWide) {
+                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(nx.rest)));
+                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(ny.rest)));
+                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(nz.rest)));
+                }
+                dx = __fadd2_rn(dx, ex);
+                dy = __fadd2_rn(dy, ey);
+                dz = __fadd2_rn(dz, ez);
             }
             float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, E2)));
             if (CLAMP) r2 = make_float2(fmaxf(r2.x, kMinR2), fmaxf(r2.y, kMinR2));
@@ -143,13 +152,18 @@ __device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low
                 jz = p == 0 ? __fmul2_rn(dz, wj) : __ffma2_rn(dz, wj, jz);
             }
         }
-        nx = __shfl_sync(0xffffffffu, nx, from);
-        ny = __shfl_sync(0xffffffffu, ny, from);
-        nz = __shfl_sync(0xffffffffu, nz, from);
-        if (NEAR) {
-            mx = __shfl_sync(0xffffffffu, mx, from);
-            my = __shfl_sync(0xffffffffu, my, from);
-            mz = __shfl_sync(0xffffffffu, mz, from);
+        nx.v = __shfl_sync(0xffffffffu, nx.v, from);
+        ny.v = __shfl_sync(0xffffffffu, ny.v, from);
+        nz.v = __shfl_sync(0xffffffffu, nz.v, from);
+        if (MODE != kTileFar) {
+            nx.low = __shfl_sync(0xffffffffu, nx.low, from);
+            ny.low = __shfl_sync(0xffffffffu, ny.low, from);
+            nz.low = __shfl_sync(0xffffffffu, nz.low, from);
+        }
+        if (MODE == kTileWide) {
+            nx.rest = __shfl_sync(0xffffffffu, nx.rest, from);
+            ny.rest = __shfl_sync(0xffffffffu, ny.rest, from);
+            nz.rest = __shfl_sync(0xffffffffu, nz.rest, from);
         }
         if (!UQ) q = __shfl_sync(0xffffffffu, q, from);
         if (SYM) {
@@ -164,41 +178,58 @@ __device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low
 // sides' sums (A != B); otherwise the sums of A only (A == B, every ordered
 // pair).  UQ: all charges equal, applied once at the end.
 template <int R, bool UQ, bool CLAMP, bool SYM>
-__device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, int A, int B, int k0, int k1) {
+__device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bool wide, int A, int B, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     const int i0 = A * 32 * R;
     const int io = min(i0 + 16 * R, a.n - 1);  // the block's middle particle: offsets half as long as from its first
     const float4 oh = a.ph[io], ol = a.pl[io];
+    double ox = 0.0, oy = 0.0, oz = 0.0;
+    if (wide) {
+        ox = a.x[io];
+        oy = a.y[io];
+        oz = a.z[io];
+    }
     PairBlock<R> b;
     int tgt = 0;     // bit r: this lane's particle r of the block is a target
     float ext = 0.f;  // the block's largest offset on any axis
     __syncwarp();    // the previous unit's reads of `low`
 #pragma unroll
     for (int p = 0; p < R / 2; p++) {
-        float c[2][7];
+        Parts x[2], y[2], z[2];
+        float c[2] = {0.f, 0.f};
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const int i = i0 + 32 * (2 * p + u) + lane;
             if (i < a.n) {
                 const float4 h = a.ph[i], l = a.pl[i];
-                c[u][0] = hilo_diff(h.x, l.x, oh.x, ol.x, c[u][4]);
-                c[u][1] = hilo_diff(h.y, l.y, oh.y, ol.y, c[u][5]);
-                c[u][2] = hilo_diff(h.z, l.z, oh.z, ol.z, c[u][6]);
-                c[u][3] = h.w;
+                if (wide) {
+                    x[u] = parts_of(a.x[i] - ox);
+                    y[u] = parts_of(a.y[i] - oy);
+                    z[u] = parts_of(a.z[i] - oz);
+                } else {
+                    x[u].v = hilo_diff(h.x, l.x, oh.x, ol.x, x[u].low);
+                    y[u].v = hilo_diff(h.y, l.y, oh.y, ol.y, y[u].low);
+                    z[u].v = hilo_diff(h.z, l.z, oh.z, ol.z, z[u].low);
+                }
+                c[u] = h.w;
                 tgt |= l.w != 0.f ? 1 << (2 * p + u) : 0;
-                ext = fmaxf(ext, fmaxf(fabsf(c[u][0]), fmaxf(fabsf(c[u][1]), fabsf(c[u][2]))));
+                ext = fmaxf(ext, fmaxf(fabsf(x[u].v), fmaxf(fabsf(y[u].v), fabsf(z[u].v))));
             } else {
-                c[u][0] = -kFar;
-                c[u][1] = c[u][2] = c[u][3] = c[u][4] = c[u][5] = c[u][6] = 0.f;
+                x[u].v = -kFar;
             }
         }
-        b.X[p] = make_float2(c[0][0], c[1][0]);
-        b.Y[p] = make_float2(c[0][1], c[1][1]);
-        b.Z[p] = make_float2(c[0][2], c[1][2]);
-        b.Q[p] = make_float2(c[0][3], c[1][3]);
-        low.x[p][lane] = make_float2(c[0][4], c[1][4]);
-        low.y[p][lane] = make_float2(c[0][5], c[1][5]);
-        low.z[p][lane] = make_float2(c[0][6], c[1][6]);
+        b.X[p] = make_float2(x[0].v, x[1].v);
+        b.Y[p] = make_float2(y[0].v, y[1].v);
+        b.Z[p] = make_float2(z[0].v, z[1].v);
+        b.Q[p] = make_float2(c[0], c[1]);
+        low.x[p][lane] = make_float2(x[0].low, x[1].low);
+        low.y[p][lane] = make_float2(y[0].low, y[1].low);
+        low.z[p][lane] = make_float2(z[0].low, z[1].low);
+        if (wide) {
+            low.rx[p][lane] = make_float2(x[0].rest, x[1].rest);
+            low.ry[p][lane] = make_float2(y[0].rest, y[1].rest);
+            low.rz[p][lane] = make_float2(z[0].rest, z[1].rest);
+        }
         b.gx[p] = b.gy[p] = b.gz[p] = make_float2(0.f, 0.f);
     }
     __syncwarp();
@@ -209,9 +240,18 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, in
     const float2 E2 = make_float2(a.eps2, a.eps2);
     for (int k = k0; k < k1; k++) {
         const int g = k / R, j = B * 32 * R + 32 * (k - g * R) + lane;
-        float nx = -kFar, ny = 0.f, nz = 0.f, q = 0.f, mx = 0.f, my = 0.f, mz = 0.f;  // negated coordinates
-        bool jt = false, near = false;
-        if (j < a.n) {
+        Parts x{kFar}, y, z;
+        float q = 0.f;
+        bool jt = false;
+        if (j < a.n && wide) {
+            double px = a.x[j], py = a.y[j], pz = a.z[j];
+            image_of(Images{a.kind, a.images, a.off64}, g, px, py, pz);
+            x = parts_of(px - ox);
+            y = parts_of(py - oy);
+            z = parts_of(pz - oz);
+            jt = a.pl[j].w != 0.f;
+            q = a.ph[j].w;
+        } else if (j < a.n) {
             float4 h = a.ph[j], l = a.pl[j];
             jt = l.w != 0.f;
             q = h.w;
@@ -240,23 +280,21 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, in
                 back(ohy, oly, fh.y, fl.y);
                 back(ohz, olz, fh.z, fl.z);
             }
-            nx = -hilo_diff(h.x, l.x, ohx, olx, mx);
-            ny = -hilo_diff(h.y, l.y, ohy, oly, my);
-            nz = -hilo_diff(h.z, l.z, ohz, olz, mz);
-            mx = -mx;
-            my = -my;
-            mz = -mz;
-            // within twice the block's extent of its origin (a pair may be closer
-            // than the coordinates' rounding allows for)
-            near = fmaxf(fabsf(nx), fmaxf(fabsf(ny), fabsf(nz))) <= 2.f * ext;
+            x.v = hilo_diff(h.x, l.x, ohx, olx, x.low);
+            y.v = hilo_diff(h.y, l.y, ohy, oly, y.low);
+            z.v = hilo_diff(h.z, l.z, ohz, olz, z.low);
         }
+        // within twice the block's extent of its origin (a pair may be closer than
+        // the coordinates' rounding allows for)
+        const bool near = j < a.n && fmaxf(fabsf(x.v), fmaxf(fabsf(y.v), fabsf(z.v))) <= 2.f * ext;
         const bool anyB = SYM && __any_sync(0xffffffffu, jt);
         if (!anyA && !anyB) continue;
         float sx = 0.f, sy = 0.f, sz = 0.f;  // the travelling particle's sums
-        if (!SYM || __any_sync(0xffffffffu, near))
-            pair_tile<R, UQ, CLAMP, SYM, true>(b, low, E2, nx, ny, nz, q, mx, my, mz, sx, sy, sz);
-        else
-            pair_tile<R, UQ, CLAMP, SYM, false>(b, low, E2, nx, ny, nz, q, mx, my, mz, sx, sy, sz);
+        const Parts nx = negated(x), ny = negated(y), nz = negated(z);
+        if (!SYM || __any_sync(0xffffffffu, near)) {
+            if (wide) pair_tile<R, UQ, CLAMP, SYM, kTileWide>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
+            else pair_tile<R, UQ, CLAMP, SYM, kTileNear>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
+        } else pair_tile<R, UQ, CLAMP, SYM, kTileFar>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
         if (SYM && jt) {
             if (a.kind == 1 && g) {  // the sum on the unrotated particle: turned back by -g*pi/2
                 const float tx = sx, ty = sy;
@@ -289,17 +327,17 @@ __global__ void __launch_bounds__(32 * kPairWarps, 3) direct_pairs_kernel(PairAr
     __shared__ PairLow<R> lows[kPairWarps];
     PairLow<R> &low = lows[threadIdx.x >> 5];
     const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
-    const bool differ = *a.differ != 0;
+    const bool differ = a.marks[0] != 0, wide = a.marks[1] != 0;
     for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
         int A, B, ch;
         if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;  // also for every larger distance
         const int k0 = ch * a.ct, k1 = min(k0 + a.ct, R * a.images);
         if (differ) {
-            if (A != B) pair_unit<R, false, CLAMP, true>(a, low, A, B, k0, k1);
-            else pair_unit<R, false, CLAMP, false>(a, low, A, B, k0, k1);
+            if (A != B) pair_unit<R, false, CLAMP, true>(a, low, wide, A, B, k0, k1);
+            else pair_unit<R, false, CLAMP, false>(a, low, wide, A, B, k0, k1);
         } else {
-            if (A != B) pair_unit<R, true, CLAMP, true>(a, low, A, B, k0, k1);
-            else pair_unit<R, true, CLAMP, false>(a, low, A, B, k0, k1);
+            if (A != B) pair_unit<R, true, CLAMP, true>(a, low, wide, A, B, k0, k1);
+            else pair_unit<R, true, CLAMP, false>(a, low, wide, A, B, k0, k1);
         }
     }
 }
@@ -513,10 +551,14 @@ sv_status direct_accel(sv_ctx *c) {
         a.kind = im.kind;
         a.images = im.count;
         a.off = off_hl;
+        a.x = S.x;
+        a.y = S.y;
+        a.z = S.z;
+        a.off64 = im.off;
         a.ax = S.ax;
         a.ay = S.ay;
         a.az = S.az;
-        a.differ = reinterpret_cast<const int *>(S.root + 14);
+        a.marks = reinterpret_cast<const int *>(S.root + 14);
         SV_CK(c, launch_pairs(a, c->stream));
     }
     SV_LAUNCHED(c);
@@ -527,18 +569,22 @@ sv_status direct_accel(sv_ctx *c) {
     return SV_OK;
 }
 
-cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, int n, float eps2, double *ax, double *ay,
-                                       double *az, const int *charges_differ, cudaStream_t stream) {
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const double *x, const double *y,
+                                       const double *z, int n, float eps2, double *ax, double *ay, double *az,
+                                       const int *marks, cudaStream_t stream) {
     PairArgs a{};
     a.ph = ph;
     a.pl = pl;
+    a.x = x;
+    a.y = y;
+    a.z = z;
     a.n = n;
     a.eps2 = eps2;
     a.images = 1;
     a.ax = ax;
     a.ay = ay;
     a.az = az;
-    a.differ = charges_differ;
+    a.marks = marks;
     return launch_pairs(a, stream);
 }
 

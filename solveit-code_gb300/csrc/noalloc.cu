@@ -112,7 +112,7 @@ __global__ void na_bbox_final(const double *__restrict__ part, int nb, double *_
         root[1] = sh[0] > sh[3] ? 0.0 : sh[1];
         root[2] = sh[0] > sh[3] ? 0.0 : sh[2];
         root[3] = S;
-        reinterpret_cast<int *>(root + 7)[0] = 0;
+        root[7] = 0.0;  // both marks
     }
 }
 
@@ -152,9 +152,10 @@ __global__ void na_keys(const double *__restrict__ x3, const int32_t *__restrict
 __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double *__restrict__ x3,
                           const double *__restrict__ q, const double *__restrict__ m,
                           const int32_t *__restrict__ st, double kconst, const double *__restrict__ root,
-                          float4 *__restrict__ ph, float4 *__restrict__ pl, double *__restrict__ qm,
+                          float4 *__restrict__ ph, float4 *__restrict__ pl, double *__restrict__ xs,
+                          double *__restrict__ ys, double *__restrict__ zs, double *__restrict__ qm,
                           double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
-                          int *__restrict__ differ) {
+                          int *__restrict__ marks) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const uint32_t i = idx[s];
@@ -162,9 +163,13 @@ __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double 
     // a particle that is no source sits at the origin: its own position may be anywhere
     const bool src = is_src(w);
     float4 h, l;
-    split_hilo(src ? x3[3 * i] - root[0] : 0.0, h.x, l.x);
-    split_hilo(src ? x3[3 * i + 1] - root[1] : 0.0, h.y, l.y);
-    split_hilo(src ? x3[3 * i + 2] - root[2] : 0.0, h.z, l.z);
+    const double x = src ? x3[3 * i] : root[0], y = src ? x3[3 * i + 1] : root[1], z = src ? x3[3 * i + 2] : root[2];
+    split_hilo(x - root[0], h.x, l.x);
+    split_hilo(y - root[1], h.y, l.y);
+    split_hilo(z - root[2], h.z, l.z);
+    xs[s] = x;
+    ys[s] = y;
+    zs[s] = z;
     h.w = src ? (float)q[i] : 0.0f;
     const double k = (w == 1 && m[i] > 0.0) ? kconst * q[i] / m[i] : 0.0;
     l.w = k != 0.0 ? 1.f : 0.f;
@@ -172,7 +177,8 @@ __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double 
     pl[s] = l;
     qm[s] = k;
     ax[s] = ay[s] = az[s] = 0.0;
-    if (h.w != (is_src(st[0]) ? (float)q[0] : 0.0f)) *differ = 1;
+    if (h.w != (is_src(st[0]) ? (float)q[0] : 0.0f)) marks[0] = 1;
+    if (fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z))) > kWide) marks[1] = 1;
 }
 
 // every output entry is written: targets get their acceleration, everything else 0
@@ -224,14 +230,17 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     uint32_t *idx_alt = (uint32_t *)carve(sizeof(uint32_t) * ni);
     float4 *ph = (float4 *)carve(sizeof(float4) * ni);
     float4 *pl = (float4 *)carve(sizeof(float4) * ni);
+    double *xs = (double *)carve(sizeof(double) * ni);
+    double *ys = (double *)carve(sizeof(double) * ni);
+    double *zs = (double *)carve(sizeof(double) * ni);
     double *qm = (double *)carve(sizeof(double) * ni);
     double *ax = (double *)carve(sizeof(double) * ni);
     double *ay = (double *)carve(sizeof(double) * ni);
     double *az = (double *)carve(sizeof(double) * ni);
     const int red_blocks = 2 * device_sms();
     double *part = (double *)carve(sizeof(double) * 6 * red_blocks);
-    double *root = (double *)carve(sizeof(double) * 8);  // [7] int: source charges differ
-    int *differ = reinterpret_cast<int *>(root + 7);
+    double *root = (double *)carve(sizeof(double) * 8);  // [7] two ints: marks, as the sort's
+    int *marks = reinterpret_cast<int *>(root + 7);
     cub::DoubleBuffer<uint64_t> kb(keys, keys_alt);
     cub::DoubleBuffer<uint32_t> vb(idx, idx_alt);
     size_t tmp_bytes = 0;
@@ -248,10 +257,10 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     if (cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, ni, 0, 3 * kMortonBits + 1, s) != cudaSuccess)
         return SV_ERR_CUDA;
     const uint32_t *sidx = vb.Current();
-    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, root, ph, pl, qm, ax, ay, az,
-                                  differ);
+    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, root, ph, pl, xs, ys, zs,
+                                 qm, ax, ay, az, marks);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;
-    if (launch_direct_mixed_sorted(ph, pl, ni, (float)softening2, ax, ay, az, differ, s) != cudaSuccess)
+    if (launch_direct_mixed_sorted(ph, pl, xs, ys, zs, ni, (float)softening2, ax, ay, az, marks, s) != cudaSuccess)
         return SV_ERR_CUDA;
     na_scatter<<<nb, 256, 0, s>>>(sidx, ni, qm, ax, ay, az, a3);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;

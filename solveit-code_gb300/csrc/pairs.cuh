@@ -43,6 +43,25 @@ __device__ __forceinline__ void split_hilo_bits(double v, float &hi, float &lo) 
     lo = (float)(v - widen(hi));
 }
 
+// A coordinate as FP32 parts: the value rounded once, what that left out, and (wide
+// plumes) what both left out.
+struct Parts {
+    float v = 0.f, low = 0.f, rest = 0.f;
+};
+__device__ __forceinline__ Parts negated(const Parts &p) { return Parts{-p.v, -p.low, -p.rest}; }
+__device__ __forceinline__ Parts parts_of(double d) {
+    Parts p;
+    p.v = (float)d;
+    d -= (double)p.v;
+    p.low = (float)d;
+    p.rest = (float)(d - (double)p.low);
+    return p;
+}
+
+// Tiles by distance: far from the block, near it (the second parts added to each
+// difference), of a wide plume (all three: the FP64 difference, rounded to FP32)
+enum { kTileFar, kTileNear, kTileWide };
+
 constexpr int kPairWarps = 4;    // warps (units) per CTA
 constexpr int kMaxTiles = 4;     // tiles per unit: 128 sources per FP32 sum of a target
 constexpr float kFar = 1e18f;    // coordinate of absent particles: r^-3 underflows to zero

@@ -128,7 +128,7 @@ bbox_kernel(const double *__restrict__ x, const double *__restrict__ y, const do
     __syncthreads();
     if (threadIdx.x == 0) {
         write_root(bounds, scale, root);
-        reinterpret_cast<int *>(root + 14)[0] = 0;
+        root[14] = 0.0;  // both marks
         *done = 0;
     }
 }
@@ -178,7 +178,8 @@ struct GatherArgs {
     float4 *ph, *pl;          // FP32 hi + lo positions to write, or null
     int abs_xy;               // ... relative to the z axis in x and y, not to the root's origin
     const double *root;
-    int *differ;              // set when a source charge differs from particle 0's (with ph)
+    int *marks;               // set with ph: [0] a source charge differs from particle 0's, [1] a source lies
+                              // further than kWide from the origin of ph
 };
 
 // source charge of particle i (0: no source), and its K q / m (0: no target)
@@ -190,12 +191,12 @@ __device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
     return tgt ? a.kconst * (a.qom ? a.qom[i] : a.q[i] / a.m[i]) : 0.0;
 }
 
-// Particle i into sorted slot s (every load before the first store); with ph, whether its source
-// charge differs from particle 0's.  A particle that is no source takes no part in any sum; it
+// Particle i into sorted slot s (every load before the first store); with ph, its marks as bits.
+// A particle that is no source takes no part in any sum; it
 // is put at the root's origin, for its own position may be anywhere and could become the
 // origin of a block's FP32 coordinates (300 ions among as many lost ones within 100 m:
 // 7.7e-7 against 1.2e-4 force error).
-__device__ __forceinline__ bool gather_one(const GatherArgs &a, const double *root, int64_t s, uint32_t i) {
+__device__ __forceinline__ int gather_one(const GatherArgs &a, const double *root, int64_t s, uint32_t i) {
     const bool src = is_source(a.st[i]);
     const double x = src ? a.x[i] : root[0], y = src ? a.y[i] : root[1], z = src ? a.z[i] : root[2];
     const double k = sorted_qm(a, i);
@@ -215,14 +216,19 @@ __device__ __forceinline__ bool gather_one(const GatherArgs &a, const double *ro
         l.w = k != 0.0 ? 1.f : 0.f;
         a.ph[s] = h;
         a.pl[s] = l;
-        return h.w != sorted_charge(a, 0);
+        const bool wide = fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z))) > kWide;
+        return (h.w != sorted_charge(a, 0) ? 1 : 0) | (wide ? 2 : 0);
     }
-    return false;
+    return 0;
+}
+__device__ __forceinline__ void set_marks(const GatherArgs &a, int bits) {
+    if (bits & 1) a.marks[0] = 1;
+    if (bits & 2) a.marks[1] = 1;
 }
 
 __global__ void gather_sorted(const uint32_t *__restrict__ idx, int64_t n, GatherArgs a) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s < n && gather_one(a, a.root, s, idx[s])) *a.differ = 1;
+    if (s < n) set_marks(a, gather_one(a, a.root, s, idx[s]));
 }
 
 // ------------------------------------------------------------- rank sort --
@@ -313,7 +319,7 @@ sort_one_chunk(int n, int sh, double scale, double *__restrict__ root, uint64_t 
     __syncthreads();
     if (i == 0) {
         write_root(bounds, scale, root);
-        reinterpret_cast<int *>(root + 14)[0] = 0;
+        root[14] = 0.0;  // both marks
     }
     __syncthreads();
     const uint64_t key = i < n ? morton_key(p[0], p[1], p[2], st, root) : kInactiveKey;
@@ -321,7 +327,7 @@ sort_one_chunk(int n, int sh, double scale, double *__restrict__ root, uint64_t 
     if (i < n) {
         keys[pos] = key;
         idx[pos] = (uint32_t)i;
-        if (gather_one(a, root, pos, (uint32_t)i)) *a.differ = 1;
+        set_marks(a, gather_one(a, root, pos, (uint32_t)i));
     }
 }
 
@@ -347,7 +353,7 @@ sort_chunks(int n, int sh, const double *__restrict__ root, uint64_t *__restrict
 // and the ranks took three (25 us of 58 per evaluation at 4,096).  Every CTA counts the sources before its own particles itself,
 // and takes the first source's position as the origin of the FP32 parts.
 __global__ void __launch_bounds__(256)
-sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restrict__ done, int *__restrict__ mixed) {
+sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restrict__ done, int *__restrict__ bits) {
     __shared__ int wsum[8], tot[3];  // sources before this CTA, in all; first source
     __shared__ double org[3];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -378,21 +384,23 @@ sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restr
     __syncthreads();
     if (tid < 3) org[tid] = tot[2] < n ? (tid == 0 ? a.x : tid == 1 ? a.y : a.z)[tot[2]] : 0.0;
     __syncthreads();
-    bool differ = false;
+    int marks = 0;
     if (i < n) {
         int s = tot[0] + __popc(bal & ((1u << lane) - 1u));  // sources before this particle
         for (int w = 0; w < wid; w++) s += wsum[w];
         const int pos = src ? s : tot[1] + (i - s);
         idx[pos] = (uint32_t)i;
-        differ = gather_one(a, org, pos, (uint32_t)i);
+        marks = gather_one(a, org, pos, (uint32_t)i);
     }
-    // the mark of differing charges, from the last CTA to finish
-    differ = __syncthreads_or(differ);
+    // the marks, from the last CTA to finish
+    const int differ = __syncthreads_or(marks & 1), wide = __syncthreads_or(marks & 2);
     if (tid == 0) {
-        if (differ) atomicOr(mixed, 1);
+        if (differ || wide) atomicOr(bits, (differ ? 1 : 0) | (wide ? 2 : 0));
         __threadfence();
         if (atomicAdd(done, 1u) == gridDim.x - 1) {
-            *a.differ = atomicExch(mixed, 0);
+            const int b = atomicExch(bits, 0);
+            a.marks[0] = b & 1;
+            a.marks[1] = b >> 1;
             *done = 0;
         }
     }
@@ -456,6 +464,7 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
             split_hilo(v - (a.abs_xy && part < 2 ? 0.0 : a.root[part]), h, l);
             reinterpret_cast<float *>(a.ph + rank)[part] = h;
             reinterpret_cast<float *>(a.pl + rank)[part] = l;
+            if (fabsf(h) > kWide) a.marks[1] = 1;
         }
         return;
     }
@@ -465,7 +474,7 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
         a.qs[rank] = q;
         if (a.ph) {
             a.ph[rank].w = q;
-            if (q != sorted_charge(a, 0)) *a.differ = 1;
+            if (q != sorted_charge(a, 0)) a.marks[0] = 1;
         }
         break;
     }

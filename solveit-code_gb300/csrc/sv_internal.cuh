@@ -54,8 +54,8 @@ struct Sorted {
     void *cub_tmp = nullptr;
     size_t cub_bytes = 0;
     double *root = nullptr;    // device [16]: origin xyz, cube side S, bbox max xyz, empty flag, 2^21/S;
-                               // [14] int: 1 when the sorted source charges differ (want.hilo); [13], [15]
-                               // int: words of the kernels whose last CTA finishes, zero between launches
+                               // [14] two ints, the marks of GatherArgs (want.hilo); [13], [15] int: words of
+                               // the kernels whose last CTA finishes, zero between launches
     long long *red = nullptr;  // device reduction scratch
     int red_blocks = 0;
     int64_t cap = 0;
@@ -311,11 +311,20 @@ sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; r
 constexpr int64_t kAnyOrderMax = 8192;
 // what the direct sum of this context needs of its sort
 void direct_sort_wants(sv_ctx *c);
+// Extent of a plume, from its sort's origin, past which the mixed pair sums take their
+// coordinates from the FP64 positions.  FP32 hi + lo parts resolve 2^-49 of the distance
+// to the origin, 5.5e-17 m at this one: FP32's own rounding of a nanometre.  Clusters
+// of 10 nm spread over 10 m: 5.6e-5 force error from the parts, 9e-7 from offsets
+// to each block, 2e-7 so.
+constexpr float kWide = 0.03125f;
+
 // the mixed-precision all-pairs sums (no symmetry images) of n sorted
-// particles given as FP32 hi + lo parts (Sorted::ph, pl), without the targets'
-// factor K q / m, added into the cleared ax, ay, az; launches only, allocates nothing
-cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, int n, float eps2, double *ax, double *ay,
-                                       double *az, const int *charges_differ, cudaStream_t stream);
+// particles given as FP32 hi + lo parts (Sorted::ph, pl) and FP64 positions, without
+// the targets' factor K q / m, added into the cleared ax, ay, az; marks: the sort's two;
+// launches only, allocates nothing
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const double *x, const double *y,
+                                       const double *z, int n, float eps2, double *ax, double *ay, double *az,
+                                       const int *marks, cudaStream_t stream);
 
 // A double's bits as a signed integer whose order is the double's order
 // (non-NaN values); the map is its own inverse.  Min / max on these run on
