@@ -1506,8 +1506,7 @@ p2p_item(P2PShared<WS> &sh, int b, int ntgt, int part, int parts, int stride, co
         const bool vb = active && lt + h < nt;
         const int ia = SOME ? tix[active ? lt : 0] : tb + lt, ib = SOME ? tix[vb ? lt + h : 0] : ia + h;
         const float4 ta = rel[SOME || active ? ia : tb], tbv = rel[SOME || vb ? ib : tb];
-        // pairs on targets, whichever particles the lanes hold beside them
-        if (tid == 0 && ch == 0) atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)ntgt);
+        if (tid == 0) atomicAdd(&counts[1], (unsigned long long)total * (unsigned long long)nt);
         const float2 AX = make_float2(ta.x, ta.x), AY = make_float2(ta.y, ta.y), AZ = make_float2(ta.z, ta.z);
         const float2 BX = make_float2(tbv.x, tbv.x), BY = make_float2(tbv.y, tbv.y), BZ = make_float2(tbv.z, tbv.z);
         float sax = 0.f, say = 0.f, saz = 0.f, eax = 0.f, eay = 0.f, eaz = 0.f;
