@@ -121,7 +121,9 @@ typedef struct {
 
 /* Per-call statistics of the last force evaluation. */
 typedef struct {
-    double pair_interactions;     /* particle-particle pairs evaluated */
+    double pair_interactions;     /* particle-particle pairs evaluated; the FMM's near field evaluates every
+                                     particle of a box that holds targets, with symmetry images the
+                                     targets alone */
     double cell_interactions;     /* BH accepted cells / FMM M2L translations */
     double flops_algorithmic;     /* 20 flop/pair + expansion flops (method's count) */
     double ms_total;              /* device time of the whole evaluation */
@@ -497,7 +499,7 @@ typedef struct {
     double tuned_ms;                /* force-evaluation time measured by sv_batch_tune */
     double direct_pairs;            /* pair interactions of the direct plumes per evaluation */
     double fmm_m2l;                 /* M2L translations of the last FMM forest evaluation */
-    double fmm_pairs;               /* P2P pair interactions of the last FMM forest evaluation */
+    double fmm_pairs;               /* P2P pairs (on targets) evaluated by the last FMM forest evaluation */
     int32_t regrows;                /* times a box capacity overflowed and the work was redone */
     int32_t overflow_mask;          /* bit l: forest level l overflowed at the last regrow */
     int32_t level_boxes[22];        /* forest boxes per level at the last evaluation */
