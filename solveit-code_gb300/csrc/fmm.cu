@@ -1911,12 +1911,16 @@ sv_status run_fmm(sv_ctx *c, Fmm &F, Tree &T) {
         SV_CK(c, cudaEventRecord(F.ev_join, F.side));
     }
     phase_mark(c, 3);
-    // Upward pass.  Where its blocks fill the SMs it starts after the lists: beside
-    // them it would hold the SMs that the lists, and the near field behind them
-    // (the longest kernel of an evaluation), are waiting for.  131,101 ions in a
-    // ball, 728 leaf boxes: 3,820 against 3,896 us for three steps; 20,011 ions,
-    // 272 boxes: 420 against 405 us, so fewer boxes start at once.
-    if (T.lv[L].nbox >= kWarps * device_sms()) SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_lists, 0));
+    // Upward pass.  Beside the lists it holds SMs that the lists, and behind them the near
+    // field, the longest kernel of an evaluation, are waiting for; after them it
+    // starts late.  It waits where the near field is long: in trees of four boxes per
+    // level or more (balls of 8,000 to a million ions, orders 6 and 8: 0.97 to 1.03 of the
+    // time at once, 0.99 on average), and in columns of 64 leaf boxes per SM or more
+    // (0.99 to 1.04 at 350,000 and 420,000 ions, 0.97 to 1.00 from 500,000 to a million).
+    // Smaller columns start at once: waiting takes 1.03 to 1.10 of the time up to
+    // 65,000 ions, 0.99 to 1.05 up to 300,000.
+    if (T.lv[L].nbox >= 64 * device_sms() || (int64_t)T.lv[L].nbox >= int64_t(1) << 2 * L)
+        SV_CK(c, cudaStreamWaitEvent(c->stream, F.ev_lists, 0));
     {
         const Level &V = T.lv[L];
         p2m_kernel<P><<<div_up(V.nbox, p2m_warps<P>()), p2m_warps<P>() * 32, 0, c->stream>>>(
