@@ -98,13 +98,8 @@ struct Batch {
     unsigned long long *ev_count0 = nullptr;  // event count at the start of a leapfrog call
     int8_t *pfold = nullptr;          // n: 1 for the particles of rotational plumes (folding)
     double step_dt = 0;               // dt baked into g_step
-    // tuning
-    // Tuned: M2L cost in pair units, direct work-item size.  The weight before tuning:
-    // 200 against 400 on batches of 3 to 24 plumes at orders 4, 6 and 8 is 0 to 3 % faster
-    // (24 plumes at order 6: 5.25 against 5.40 ms per two steps) and at order 4 up to 34 %
-    // (1.21 against 1.63 ms); 100 costs 7 %.  256 large plumes, which the tuner is for:
-    // 41.2 against 39.1 ms a step.
-    int m2l_weight = 200, direct_chunk = 2048;
+    int m2l_weight = 200, direct_chunk = 2048;  // tuned: M2L cost in pair units, direct work-item size
+    bool weight_given = false;        // by the tuner, its file or the caller; else every plan sets it (untuned_weight)
     double tuned_ms = 0;
     int regrows = 0;
 };
@@ -378,6 +373,30 @@ inline int pick_level(double slots, int per_particle, const long long *boxes, do
     return best;
 }
 
+// view slots per particle of an FMM plume: its quadrants' images are slots too
+int slots_per_particle(const Batch &B, int pid) {
+    const int p = B.plume_of[pid];
+    return B.method[p] == SV_METHOD_FMM && B.sym[p] == SV_SYM_ROTATIONAL ? 4 : 1;
+}
+
+// The M2L's weight before tuning, by the shape of the plumes that hold most of the slots:
+// 200 where they are columns, 800 where they fill their cubes (four boxes per level or
+// more, up to the level that 200 picks).  Times of an evaluation of 24 plumes of 9,000
+// to 60,000 ions at orders 4, 6 and 8, of the best weight of 50 to 800 (mean, worst):
+// columns 200 1.00, 1.06; 400 1.03, 1.39; 800 1.11, 1.82; balls 200 1.18, 1.64; 400
+// 1.07, 1.42; 800 1.00, 1.01; with four quadrants columns the same, balls 1.00 with any of
+// 100 to 800.
+int untuned_weight(const Batch &B, const std::vector<std::vector<long long>> &boxes, int ws) {
+    double filled = 0.0, all = 0.0;
+    for (int pid = 0; pid < B.nfp; pid++) {
+        const double slots = (double)(B.vbeg[pid + 1] - B.vbeg[pid]);
+        const int l = pick_level(slots, slots_per_particle(B, pid), boxes[pid].data(), 200.0, ws);
+        all += slots;
+        if ((double)boxes[pid][l] >= std::ldexp(1.0, 2 * l)) filled += slots;
+    }
+    return 2.0 * filled > all ? 800 : 200;
+}
+
 // Per FMM plume: its own leaf level Lp, delta = L - Lp, and the root side scaled
 // by 2^delta.  One warp per plume, one lane per level: the powers and logarithms
 // (FP64) of a level are independent of the other levels' (a thread per plume
@@ -559,12 +578,6 @@ sv_status build_items(sv_ctx *c, Batch &B) {
     return SV_OK;
 }
 
-// view slots per particle of an FMM plume: its quadrants' images are slots too
-int slots_per_particle(const Batch &B, int pid) {
-    const int p = B.plume_of[pid];
-    return B.method[p] == SV_METHOD_FMM && B.sym[p] == SV_SYM_ROTATIONAL ? 4 : 1;
-}
-
 // room for the sort of n slots by any of their key bits
 sv_status sort_room(sv_ctx *c, int64_t n, SortRoom &r) {
     SV_CK(c, cub::DeviceRadixSort::SortPairs(nullptr, r.bytes, c->S.keys_alt, c->S.keys, c->S.idx_alt, c->S.idx,
@@ -695,6 +708,9 @@ sv_status plan_forest(sv_ctx *c, Batch &B, int cap_scale) {
             if (l > 0) acc += hist[(size_t)pid * kBLevels + l];
             boxes[pid][l] = acc;
         }
+    }
+    if (!B.weight_given) B.m2l_weight = untuned_weight(B, boxes, c->P.fmm_ws);
+    for (int pid = 0; pid < B.nfp; pid++) {
         Lp[pid] = pick_level((double)(B.vbeg[pid + 1] - B.vbeg[pid]), slots_per_particle(B, pid), boxes[pid].data(),
                              (double)B.m2l_weight, c->P.fmm_ws);
     }
@@ -1125,6 +1141,7 @@ sv_status time_accel(sv_ctx *c, Batch &B, int reps, double *ms) {
 sv_status sweep_weights(sv_ctx *c, Batch &B, int *best_lt, double *best_ms) {
     const int weights[6] = {100, 200, 400, 800, 1600, 3200};
     double t[6], best = 1e30;
+    B.weight_given = true;
     for (int k = 0; k < 6; k++) {
         B.m2l_weight = weights[k];
         SV_TRY(plan_forest(c, B, 1));
@@ -1175,6 +1192,7 @@ sv_status batch_tune(sv_ctx *c, const char *cache_path, double *best_ms) {
             batch_invalidate(c);
         }
         B.m2l_weight = t.lt;
+        B.weight_given = true;
         B.direct_chunk = t.dc;
         SV_TRY(build_items(c, B));
         drop_graphs(B);
@@ -1268,6 +1286,7 @@ sv_status batch_set_tuning(sv_ctx *c, int m2l_weight, int direct_chunk) {
     if (m2l_weight < 1 || direct_chunk < kDTile)
         return set_error(c, SV_ERR_INVALID, "M2L weight >= 1 and direct chunk >= %d required", kDTile);
     B.m2l_weight = m2l_weight;
+    B.weight_given = true;
     B.direct_chunk = direct_chunk;
     SV_TRY(build_items(c, B));
     drop_graphs(B);
