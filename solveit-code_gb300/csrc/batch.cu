@@ -380,12 +380,16 @@ int slots_per_particle(const Batch &B, int pid) {
 }
 
 // The M2L's weight before tuning, by the shape of the plumes that hold most of the slots:
-// 200 where they are columns, 800 where they fill their cubes (four boxes per level or
-// more, up to the level that 200 picks).  Times of an evaluation of 24 plumes of 9,000
-// to 60,000 ions at orders 4, 6 and 8, of the best weight of 50 to 800 (mean, worst):
-// columns 200 1.00, 1.06; 400 1.03, 1.39; 800 1.11, 1.82; balls 200 1.18, 1.64; 400
-// 1.07, 1.42; 800 1.00, 1.01; with four quadrants columns the same, balls 1.00 with any of
-// 100 to 800.
+// 200 where they are columns, 400 from kLargeColumn slots per plume on, 800 where they
+// fill their cubes (four boxes per level or more, up to the level that 200 picks).  Times
+// of an evaluation of 24 plumes of 9,000 to 60,000 ions at orders 4, 6 and 8, of the best
+// weight of 50 to 800 (mean, worst): columns 200 1.00, 1.06; 400 1.03, 1.39; 800 1.11,
+// 1.82; balls 200 1.18, 1.64; 400 1.07, 1.42; 800 1.00, 1.01; with four quadrants columns
+// the same, balls 1.00 with any of 100 to 800.  The time with 200 of that with 400, 24 to
+// 256 columns of 1,024 to 65,536 ions, every other one with quadrants (90,000 to 96,000
+// slots per plume): 0.98 to 1.02 at order 4, 0.99 to 1.03 at 6, 1.05 to 1.11 at 8; 24 of up
+// to 24,000 ions (41,000 slots): 1.02, 0.98 and 1.00; 8 of up to 20,000 (37,000): 0.78 to 0.89.
+constexpr int64_t kLargeColumn = 85000;
 int untuned_weight(const Batch &B, const std::vector<std::vector<long long>> &boxes, int ws) {
     double filled = 0.0, all = 0.0;
     for (int pid = 0; pid < B.nfp; pid++) {
@@ -394,7 +398,7 @@ int untuned_weight(const Batch &B, const std::vector<std::vector<long long>> &bo
         all += slots;
         if ((double)boxes[pid][l] >= std::ldexp(1.0, 2 * l)) filled += slots;
     }
-    return 2.0 * filled > all ? 800 : 200;
+    return 2.0 * filled > all ? 800 : B.nf > kLargeColumn * B.nfp ? 400 : 200;
 }
 
 // Per FMM plume: its own leaf level Lp, delta = L - Lp, and the root side scaled

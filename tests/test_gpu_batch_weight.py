@@ -1,7 +1,7 @@
 """The M2L's weight that a batch takes before tuning: by the shape of its plumes.
 
-Plumes that fill their cubes take 800, columns 200 (both measured beside the rule); a
-weight that the caller sets stays, over re-planning and further evaluations.
+Plumes that fill their cubes take 800, columns 200, large columns 400 (measured beside
+the rule); a weight that the caller sets stays, over re-planning and further evaluations.
 Accelerations meet the batch's order-6 bound either way.
 """
 import numpy as np
@@ -41,3 +41,11 @@ def test_untuned_weight(kinds, weight):
         for _ in range(2):
             fm.accel(out=False)
             assert fm.batch_info().m2l_weight == 400
+
+
+def test_large_columns():
+    states = [column(22000, 50 + i) for i in range(2)]
+    with sv.ForceMethod(softening2=EPS20, fmm_order=4, fmm_ws=2) as fm:
+        fm.upload_batch(states, [sv.FMM] * 2, [sv.SYM_ROTATIONAL] * 2)
+        fm.accel(out=False)
+        assert fm.batch_info().m2l_weight == 400
