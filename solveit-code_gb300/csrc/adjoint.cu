@@ -252,12 +252,11 @@ __global__ void __launch_bounds__(32 * kPairWarps) jtv_pairs64_kernel(JPair64Arg
 // The reciprocal square root is refined by one Newton step.  FP32-pipe bound:
 // 45 operations per pair (39 when all charges are equal), two targets per packed
 // instruction, each pair once: 16,384 particles 532 -> 211 us per launch, 4,096
-// 54 -> 21 us, against the one-sided scalar kernel.  Wide plumes (kWide) take their
-// coordinates from the FP64 positions in the same code (1 % of a gradient; a form of its
-// own costs as much inlined, 2 to 3 % out of line).
+// 54 -> 21 us, against the one-sided scalar kernel.  Wide plumes (kWide) keep a third
+// part of their coordinates.
 struct JPairArgs {
     const float4 *ph, *pl, *uh, *ul;
-    const double *x, *y, *z;  // wide plumes
+    const float4 *pr;  // wide plumes
     int n, nb, ct, nch;
     float e2;
     double *ox, *oy, *oz;
@@ -359,37 +358,32 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
     }
 }
 
-template <bool UQ, bool SYM>
-__device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, bool wide, int A, int B, int k0, int k1) {
+template <bool UQ, bool SYM, bool WIDE>
+__device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, int B, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     const float sc = (float)kLen;
     const int i0 = A * 32 * kJR, io = min(i0 + 16 * kJR, a.n - 1);
     const float4 oh = a.ph[io], ol = a.pl[io];
-    double ox = 0.0, oy = 0.0, oz = 0.0;
-    if (wide) {
-        ox = a.x[io];
-        oy = a.y[io];
-        oz = a.z[io];
-    }
+    Parts ox{oh.x, ol.x}, oy{oh.y, ol.y}, oz{oh.z, ol.z};
     // particle i's coordinates from the block's origin, in 2^-30 m
     auto coordinates = [&](int i, const float4 &h, Parts &x, Parts &y, Parts &z) {
-        if (wide) {
-            x = parts_of((a.x[i] - ox) * kLen);
-            y = parts_of((a.y[i] - oy) * kLen);
-            z = parts_of((a.z[i] - oz) * kLen);
-            return;
-        }
-        const float4 l = a.pl[i];
-        x.v = hilo_diff(h.x, l.x, oh.x, ol.x, x.low) * sc;
-        y.v = hilo_diff(h.y, l.y, oh.y, ol.y, y.low) * sc;
-        z.v = hilo_diff(h.z, l.z, oh.z, ol.z, z.low) * sc;
-        x.low *= sc;
-        y.low *= sc;
-        z.low *= sc;
+        const float4 l = a.pl[i], r = WIDE ? a.pr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        x = parts_diff<WIDE>(Parts{h.x, l.x, r.x}, ox);
+        y = parts_diff<WIDE>(Parts{h.y, l.y, r.y}, oy);
+        z = parts_diff<WIDE>(Parts{h.z, l.z, r.z}, oz);
+        x = Parts{x.v * sc, x.low * sc, x.rest * sc};
+        y = Parts{y.v * sc, y.low * sc, y.rest * sc};
+        z = Parts{z.v * sc, z.low * sc, z.rest * sc};
     };
     JBlock b;
     float ext = 0.f;
     __syncwarp();  // the previous unit's reads of `low`
+    if (WIDE) {
+        const float4 r = a.pr[io];
+        ox.rest = r.x;
+        oy.rest = r.y;
+        oz.rest = r.z;
+    }
 #pragma unroll
     for (int p = 0; p < kJH; p++) {
         Parts x[2], y[2], z[2];
@@ -420,7 +414,7 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, bool wid
         low.x[p][lane] = make_float2(x[0].low, x[1].low);
         low.y[p][lane] = make_float2(y[0].low, y[1].low);
         low.z[p][lane] = make_float2(z[0].low, z[1].low);
-        if (wide) {
+        if (WIDE) {
             low.rx[p][lane] = make_float2(x[0].rest, x[1].rest);
             low.ry[p][lane] = make_float2(y[0].rest, y[1].rest);
             low.rz[p][lane] = make_float2(z[0].rest, z[1].rest);
@@ -460,8 +454,7 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, bool wid
         t.y = negated(y);
         t.z = negated(z);
         if (!SYM || __any_sync(0xffffffffu, near)) {
-            if (wide) jtv_tile<UQ, SYM, kTileWide>(b, low, E2, min_r2, t);
-            else jtv_tile<UQ, SYM, kTileNear>(b, low, E2, min_r2, t);
+            jtv_tile<UQ, SYM, WIDE ? kTileWide : kTileNear>(b, low, E2, min_r2, t);
         } else {
             jtv_tile<UQ, SYM, kTileFar>(b, low, E2, min_r2, t);
         }
@@ -481,21 +474,37 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, bool wid
     }
 }
 
+// all units of a warp of a wide plume, with any charges (out of line, as the direct sum's:
+// 16,384 particles 211 without it, 217 us so, 229 in line)
+__device__ __noinline__ void jtv_wide(JPairArgs a, JLow &low, int64_t v) {
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;
+        const int k0 = ch * a.ct, k1 = min(k0 + a.ct, kJR);
+        if (A != B) jtv_unit<false, true, true>(a, low, A, B, k0, k1);
+        else jtv_unit<false, false, true>(a, low, A, B, k0, k1);
+    }
+}
+
 __global__ void __launch_bounds__(32 * kPairWarps, 3) jtv_pairs_kernel(JPairArgs a) {
     __shared__ JLow lows[kPairWarps];
     JLow &low = lows[threadIdx.x >> 5];
     const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
-    const bool differ = a.marks[0] != 0, wide = a.marks[1] != 0;
+    if (a.marks[1] != 0) {
+        jtv_wide(a, low, v);
+        return;
+    }
+    const bool differ = a.marks[0] != 0;
     for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
         int A, B, ch;
         if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;
         const int k0 = ch * a.ct, k1 = min(k0 + a.ct, kJR);
         if (differ) {
-            if (A != B) jtv_unit<false, true>(a, low, wide, A, B, k0, k1);
-            else jtv_unit<false, false>(a, low, wide, A, B, k0, k1);
+            if (A != B) jtv_unit<false, true, false>(a, low, A, B, k0, k1);
+            else jtv_unit<false, false, false>(a, low, A, B, k0, k1);
         } else {
-            if (A != B) jtv_unit<true, true>(a, low, wide, A, B, k0, k1);
-            else jtv_unit<true, false>(a, low, wide, A, B, k0, k1);
+            if (A != B) jtv_unit<true, true, false>(a, low, A, B, k0, k1);
+            else jtv_unit<true, false, false>(a, low, A, B, k0, k1);
         }
     }
 }
@@ -564,7 +573,7 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
     const bool fp64 = c->P.precision == SV_PREC_FP64;
     c->fstatus = c->wstatus;
     c->S.want.zero = true;
-    c->S.want.hilo = !fp64;
+    c->S.want.hilo = c->S.want.rest = !fp64;
     c->S.want.any_order = nn <= kAnyOrderMax;
     const sv_status st = sort_state(c, 0, nn);
     c->fstatus = nullptr;
@@ -579,7 +588,7 @@ sv_status reverse_step(sv_ctx *c, const double *xh, double ts) {
         const JPair64Args a{S.x, S.y, S.z, u, S.q, n, div_up(n, 32), c->P.softening2, S.ax, S.ay, S.az};
         jtv_pairs64_kernel<<<pair_grid(a.nb, 1), 32 * kPairWarps, 0, c->stream>>>(a);
     } else {
-        JPairArgs a{S.ph, S.pl, uh, ul, S.x, S.y, S.z, n, div_up(n, 32 * kJR), 0, 0, (float)(c->P.softening2 * kLen * kLen),
+        JPairArgs a{S.ph, S.pl, uh, ul, S.pr, n, div_up(n, 32 * kJR), 0, 0, (float)(c->P.softening2 * kLen * kLen),
                     S.ax, S.ay, S.az, reinterpret_cast<const int *>(S.root + 14)};
         // about 16 units per SM sub-partition
         const int64_t tiles = (int64_t)a.nb * (a.nb + 1) / 2 * kJR;

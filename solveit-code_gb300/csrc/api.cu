@@ -142,17 +142,21 @@ sv_status image_set(sv_ctx *c, const ImageSet **out) {
     std::vector<double> m(3 * kMaxImages);
     const int cnt = trans_images(P, m.data(), kMaxImages);
     if (cnt <= 0 || cnt > kMaxImages) return set_error(c, SV_ERR_INVALID, "bad translational image set (%d)", cnt);
-    // metres; FP32 hi and lo parts; metres with the zero offset (the particles themselves) first
-    std::vector<double> buf(14 * (size_t)cnt);
+    // metres; FP32 parts; metres with the zero offset (the particles themselves) first
+    std::vector<double> buf(16 * (size_t)cnt);
     float4 *hl = reinterpret_cast<float4 *>(buf.data() + 4 * (size_t)cnt);
-    double *zf = buf.data() + 8 * (size_t)cnt;
+    double *zf = buf.data() + 10 * (size_t)cnt;
     int zero = -1, k = 0;
     for (int g = 0; g < cnt; g++) {
         const double *v = &m[3 * (size_t)g];
-        const float hi[3] = {(float)v[0], (float)v[1], (float)v[2]};
-        for (int d = 0; d < 3; d++) buf[3 * (size_t)g + d] = v[d];
-        hl[2 * g] = make_float4(hi[0], hi[1], hi[2], 0.f);
-        hl[2 * g + 1] = make_float4((float)(v[0] - hi[0]), (float)(v[1] - hi[1]), (float)(v[2] - hi[2]), 0.f);
+        float part[3][3];  // hi, lo and what they leave out
+        for (int d = 0; d < 3; d++) {
+            buf[3 * (size_t)g + d] = v[d];
+            part[0][d] = (float)v[d];
+            part[1][d] = (float)(v[d] - part[0][d]);
+            part[2][d] = (float)((v[d] - part[0][d]) - part[1][d]);
+        }
+        for (int p = 0; p < 3; p++) hl[3 * g + p] = make_float4(part[p][0], part[p][1], part[p][2], 0.f);
         if (v[0] == 0.0 && v[1] == 0.0 && v[2] == 0.0) zero = g;
     }
     if (zero < 0) return set_error(c, SV_ERR_INVALID, "image set without the zero offset");
@@ -169,7 +173,7 @@ sv_status image_set(sv_ctx *c, const ImageSet **out) {
     SV_CK(c, cudaMemcpy(I.buf, buf.data(), sizeof(double) * buf.size(), cudaMemcpyHostToDevice));
     I.m = I.buf;
     I.hl = reinterpret_cast<const float4 *>(I.buf + 4 * (size_t)cnt);
-    I.zero_first = I.buf + 8 * (size_t)cnt;
+    I.zero_first = I.buf + 10 * (size_t)cnt;
     I.levels = P.sym_levels;
     for (int d = 0; d < 3; d++) {
         I.axes[d] = P.sym_axes[d];
@@ -819,7 +823,7 @@ void sv_destroy(sv_ctx *c) {
     cudaFree(S.x); cudaFree(S.y); cudaFree(S.z); cudaFree(S.q); cudaFree(S.qm);
     cudaFree(S.idx); cudaFree(S.keys); cudaFree(S.keys_alt); cudaFree(S.idx_alt);
     cudaFree(S.ax); cudaFree(S.ay); cudaFree(S.az); cudaFree(S.cub_tmp);
-    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl);
+    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl); cudaFree(S.pr);
     cudaFree(c->d_stage);
     cudaFree(c->d_scalar);
     if (c->h_scalar) cudaFreeHost(c->h_scalar);

@@ -22,8 +22,8 @@
 // rounding; where a tile comes within the block's extent, the parts that rounding
 // left out are kept too and added to each difference (six operations more, in a
 // few tiles per block), so that every pair's offset is rounded relative to its own
-// length and not to the block's; a wide plume (kWide) takes its coordinates from the FP64
-// positions and keeps all their bits.  The force error against FP64 is 1.2e-7 to 3e-7
+// length and not to the block's; a wide plume (kWide) keeps all bits of the FP64 positions in
+// a third part.  The force error against FP64 is 1.2e-7 to 3e-7
 // (relative L2 over plumes of 256 to 30,011 ions); coordinates rounded relative to
 // a CTA's first target gave 3e-7 to 5.6e-6, set by each plume's closest pairs.
 // The loop has no FP64 instruction (GB300 issues one FP64 warp instruction in 64
@@ -86,12 +86,12 @@ __device__ __forceinline__ bool block_has_target(const double *__restrict__ qm, 
 // ------------------------------------------------------------------ mixed --
 struct PairArgs {
     const float4 *ph, *pl;   // sorted positions hi (w: charge) and lo (w: 1 = target)
+    const float4 *pr;        // what hi and lo leave out (wide plumes)
     int n, nb;               // particles, blocks of 32 R of them
     int ct, nch;             // tiles per unit (of the R x images of a block pair), units per block pair
     float eps2;
     int kind, images;        // symmetry images, as Images
-    const float4 *off;       // translational offsets: hi (xyz) and lo (xyz) per image
-    const double *x, *y, *z, *off64;  // sorted positions and translational offsets, metres
+    const float4 *off;       // translational offsets: hi, lo and what they leave out (xyz) per image
     double *ax, *ay, *az;    // sums, added into
     const int *marks;        // nonzero: [0] source charges differ, [1] the plume is wide (kWide)
 };
@@ -177,22 +177,23 @@ __device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low
 // One unit: block A (registers) against tiles [k0, k1) of block B.  SYM: both
 // sides' sums (A != B); otherwise the sums of A only (A == B, every ordered
 // pair).  UQ: all charges equal, applied once at the end.
-template <int R, bool UQ, bool CLAMP, bool SYM>
-__device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bool wide, int A, int B, int k0, int k1) {
+template <int R, bool UQ, bool CLAMP, bool SYM, bool WIDE>
+__device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, int A, int B, int k0, int k1) {
     const int lane = threadIdx.x & 31;
     const int i0 = A * 32 * R;
     const int io = min(i0 + 16 * R, a.n - 1);  // the block's middle particle: offsets half as long as from its first
     const float4 oh = a.ph[io], ol = a.pl[io];
-    double ox = 0.0, oy = 0.0, oz = 0.0;
-    if (wide) {
-        ox = a.x[io];
-        oy = a.y[io];
-        oz = a.z[io];
-    }
+    Parts ox{oh.x, ol.x}, oy{oh.y, ol.y}, oz{oh.z, ol.z};
     PairBlock<R> b;
     int tgt = 0;     // bit r: this lane's particle r of the block is a target
     float ext = 0.f;  // the block's largest offset on any axis
     __syncwarp();    // the previous unit's reads of `low`
+    if (WIDE) {
+        const float4 r = a.pr[io];
+        ox.rest = r.x;
+        oy.rest = r.y;
+        oz.rest = r.z;
+    }
 #pragma unroll
     for (int p = 0; p < R / 2; p++) {
         Parts x[2], y[2], z[2];
@@ -201,16 +202,10 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bo
         for (int u = 0; u < 2; u++) {
             const int i = i0 + 32 * (2 * p + u) + lane;
             if (i < a.n) {
-                const float4 h = a.ph[i], l = a.pl[i];
-                if (wide) {
-                    x[u] = parts_of(a.x[i] - ox);
-                    y[u] = parts_of(a.y[i] - oy);
-                    z[u] = parts_of(a.z[i] - oz);
-                } else {
-                    x[u].v = hilo_diff(h.x, l.x, oh.x, ol.x, x[u].low);
-                    y[u].v = hilo_diff(h.y, l.y, oh.y, ol.y, y[u].low);
-                    z[u].v = hilo_diff(h.z, l.z, oh.z, ol.z, z[u].low);
-                }
+                const float4 h = a.ph[i], l = a.pl[i], r = WIDE ? a.pr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                x[u] = parts_diff<WIDE>(Parts{h.x, l.x, r.x}, ox);
+                y[u] = parts_diff<WIDE>(Parts{h.y, l.y, r.y}, oy);
+                z[u] = parts_diff<WIDE>(Parts{h.z, l.z, r.z}, oz);
                 c[u] = h.w;
                 tgt |= l.w != 0.f ? 1 << (2 * p + u) : 0;
                 ext = fmaxf(ext, fmaxf(fabsf(x[u].v), fmaxf(fabsf(y[u].v), fabsf(z[u].v))));
@@ -225,7 +220,7 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bo
         low.x[p][lane] = make_float2(x[0].low, x[1].low);
         low.y[p][lane] = make_float2(y[0].low, y[1].low);
         low.z[p][lane] = make_float2(z[0].low, z[1].low);
-        if (wide) {
+        if (WIDE) {
             low.rx[p][lane] = make_float2(x[0].rest, x[1].rest);
             low.ry[p][lane] = make_float2(y[0].rest, y[1].rest);
             low.rz[p][lane] = make_float2(z[0].rest, z[1].rest);
@@ -243,46 +238,26 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bo
         Parts x{kFar}, y, z;
         float q = 0.f;
         bool jt = false;
-        if (j < a.n && wide) {
-            double px = a.x[j], py = a.y[j], pz = a.z[j];
-            image_of(Images{a.kind, a.images, a.off64}, g, px, py, pz);
-            x = parts_of(px - ox);
-            y = parts_of(py - oy);
-            z = parts_of(pz - oz);
-            jt = a.pl[j].w != 0.f;
-            q = a.ph[j].w;
-        } else if (j < a.n) {
-            float4 h = a.ph[j], l = a.pl[j];
+        if (j < a.n) {
+            const float4 h = a.ph[j], l = a.pl[j], r = WIDE ? a.pr[j] : make_float4(0.f, 0.f, 0.f, 0.f);
             jt = l.w != 0.f;
             q = h.w;
-            float ohx = oh.x, ohy = oh.y, ohz = oh.z, olx = ol.x, oly = ol.y, olz = ol.z;
+            Parts px{h.x, l.x, r.x}, py{h.y, l.y, r.y}, pz{h.z, l.z, r.z}, cx = ox, cy = oy, cz = oz;
             if (a.kind == 1 && g) {
                 // source rotated by g*pi/2 about z (quadrantRotationFunction, auxiliary_functions.h:55-57)
-                const float hx = h.x, lx = l.x, sgx = g == 3 ? 1.f : -1.f, sgy = g == 1 ? 1.f : -1.f;
-                if (g == 2) {
-                    h.x = -hx; l.x = -lx;
-                    h.y = -h.y; l.y = -l.y;
-                } else {
-                    h.x = sgx * h.y; l.x = sgx * l.y;
-                    h.y = sgy * hx; l.y = sgy * lx;
-                }
+                const Parts x0 = px, y0 = py;
+                px = g == 1 ? negated(y0) : g == 2 ? negated(x0) : y0;
+                py = g == 1 ? x0 : g == 2 ? negated(y0) : negated(x0);
             } else if (a.kind == 2) {
                 // source shifted by the image offset: the origin shifted back
-                const float4 fh = a.off[2 * g], fl = a.off[2 * g + 1];
-                auto back = [](float &hi, float &lo, float fhi, float flo) {
-                    const float s = hi - fhi, bb = s - hi;
-                    const float e = ((hi - (s - bb)) - (fhi + bb)) + (lo - flo);
-                    const float r = s + e;
-                    lo = e - (r - s);
-                    hi = r;
-                };
-                back(ohx, olx, fh.x, fl.x);
-                back(ohy, oly, fh.y, fl.y);
-                back(ohz, olz, fh.z, fl.z);
+                const float4 fh = a.off[3 * g], fl = a.off[3 * g + 1], fr = a.off[3 * g + 2];
+                cx = parts_diff<WIDE>(cx, Parts{fh.x, fl.x, fr.x});
+                cy = parts_diff<WIDE>(cy, Parts{fh.y, fl.y, fr.y});
+                cz = parts_diff<WIDE>(cz, Parts{fh.z, fl.z, fr.z});
             }
-            x.v = hilo_diff(h.x, l.x, ohx, olx, x.low);
-            y.v = hilo_diff(h.y, l.y, ohy, oly, y.low);
-            z.v = hilo_diff(h.z, l.z, ohz, olz, z.low);
+            x = parts_diff<WIDE>(px, cx);
+            y = parts_diff<WIDE>(py, cy);
+            z = parts_diff<WIDE>(pz, cz);
         }
         // within twice the block's extent of its origin (a pair may be closer than
         // the coordinates' rounding allows for)
@@ -292,8 +267,7 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bo
         float sx = 0.f, sy = 0.f, sz = 0.f;  // the travelling particle's sums
         const Parts nx = negated(x), ny = negated(y), nz = negated(z);
         if (!SYM || __any_sync(0xffffffffu, near)) {
-            if (wide) pair_tile<R, UQ, CLAMP, SYM, kTileWide>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
-            else pair_tile<R, UQ, CLAMP, SYM, kTileNear>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
+            pair_tile<R, UQ, CLAMP, SYM, WIDE ? kTileWide : kTileNear>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
         } else pair_tile<R, UQ, CLAMP, SYM, kTileFar>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
         if (SYM && jt) {
             if (a.kind == 1 && g) {  // the sum on the unrotated particle: turned back by -g*pi/2
@@ -322,22 +296,40 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, bo
     }
 }
 
+// All units of a warp of a wide plume, with any charges: out of line and called once, for
+// its code beside the other's costs the other plumes (per launch, without it / so / in
+// line: 4,096 particles 15.5 / 15.8 / 18.2 us, 16,384 97 / 99 / 102).
+template <int R, bool CLAMP>
+__device__ __noinline__ void pairs_wide(PairArgs a, PairLow<R> &low, int64_t v) {
+    for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
+        int A, B, ch;
+        if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;
+        const int k0 = ch * a.ct, k1 = min(k0 + a.ct, R * a.images);
+        if (A != B) pair_unit<R, false, CLAMP, true, true>(a, low, A, B, k0, k1);
+        else pair_unit<R, false, CLAMP, false, true>(a, low, A, B, k0, k1);
+    }
+}
+
 template <int R, bool CLAMP>
 __global__ void __launch_bounds__(32 * kPairWarps, 3) direct_pairs_kernel(PairArgs a) {
     __shared__ PairLow<R> lows[kPairWarps];
     PairLow<R> &low = lows[threadIdx.x >> 5];
     const int64_t v = (int64_t)blockIdx.x * kPairWarps + (threadIdx.x >> 5);
-    const bool differ = a.marks[0] != 0, wide = a.marks[1] != 0;
+    if (a.marks[1] != 0) {
+        pairs_wide<R, CLAMP>(a, low, v);
+        return;
+    }
+    const bool differ = a.marks[0] != 0;
     for (int d = blockIdx.y; d <= a.nb / 2; d += gridDim.y) {
         int A, B, ch;
         if (!unit_blocks(v, d, a.nb, a.nch, A, B, ch)) return;  // also for every larger distance
         const int k0 = ch * a.ct, k1 = min(k0 + a.ct, R * a.images);
         if (differ) {
-            if (A != B) pair_unit<R, false, CLAMP, true>(a, low, wide, A, B, k0, k1);
-            else pair_unit<R, false, CLAMP, false>(a, low, wide, A, B, k0, k1);
+            if (A != B) pair_unit<R, false, CLAMP, true, false>(a, low, A, B, k0, k1);
+            else pair_unit<R, false, CLAMP, false, false>(a, low, A, B, k0, k1);
         } else {
-            if (A != B) pair_unit<R, true, CLAMP, true>(a, low, wide, A, B, k0, k1);
-            else pair_unit<R, true, CLAMP, false>(a, low, wide, A, B, k0, k1);
+            if (A != B) pair_unit<R, true, CLAMP, true, false>(a, low, A, B, k0, k1);
+            else pair_unit<R, true, CLAMP, false, false>(a, low, A, B, k0, k1);
         }
     }
 }
@@ -506,6 +498,7 @@ direct_fp64_kernel(const double *__restrict__ xs, const double *__restrict__ ys,
 void direct_sort_wants(sv_ctx *c) {
     c->S.want.zero = true;
     c->S.want.hilo = c->P.precision == SV_PREC_MIXED;
+    c->S.want.rest = c->S.want.hilo;
     c->S.want.hl_abs = c->P.symmetry == SV_SYM_ROTATIONAL;
     const ImageSet *I = nullptr;
     int64_t images = c->P.symmetry == SV_SYM_ROTATIONAL ? 4 : 1;
@@ -551,10 +544,7 @@ sv_status direct_accel(sv_ctx *c) {
         a.kind = im.kind;
         a.images = im.count;
         a.off = off_hl;
-        a.x = S.x;
-        a.y = S.y;
-        a.z = S.z;
-        a.off64 = im.off;
+        a.pr = S.pr;
         a.ax = S.ax;
         a.ay = S.ay;
         a.az = S.az;
@@ -569,15 +559,12 @@ sv_status direct_accel(sv_ctx *c) {
     return SV_OK;
 }
 
-cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const double *x, const double *y,
-                                       const double *z, int n, float eps2, double *ax, double *ay, double *az,
-                                       const int *marks, cudaStream_t stream) {
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const float4 *pr, int n, float eps2,
+                                       double *ax, double *ay, double *az, const int *marks, cudaStream_t stream) {
     PairArgs a{};
     a.ph = ph;
     a.pl = pl;
-    a.x = x;
-    a.y = y;
-    a.z = z;
+    a.pr = pr;
     a.n = n;
     a.eps2 = eps2;
     a.images = 1;

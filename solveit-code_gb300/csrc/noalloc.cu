@@ -146,14 +146,14 @@ __global__ void na_keys(const double *__restrict__ x3, const int32_t *__restrict
     keys[i] = na_spread3(c[0]) | (na_spread3(c[1]) << 1) | (na_spread3(c[2]) << 2);
 }
 
-// the sorted particles as the pair kernel takes them (FP32 hi + lo positions
+// the sorted particles as the pair kernel takes them (positions in FP32 parts
 // relative to the root's origin, source charge, target mark), K q / m, the sums
 // cleared, and a mark when the source charges differ
 __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double *__restrict__ x3,
                           const double *__restrict__ q, const double *__restrict__ m,
                           const int32_t *__restrict__ st, double kconst, const double *__restrict__ root,
-                          float4 *__restrict__ ph, float4 *__restrict__ pl, double *__restrict__ xs,
-                          double *__restrict__ ys, double *__restrict__ zs, double *__restrict__ qm,
+                          float4 *__restrict__ ph, float4 *__restrict__ pl, float4 *__restrict__ pr,
+                          double *__restrict__ qm,
                           double *__restrict__ ax, double *__restrict__ ay, double *__restrict__ az,
                           int *__restrict__ marks) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -167,9 +167,12 @@ __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double 
     split_hilo(x - root[0], h.x, l.x);
     split_hilo(y - root[1], h.y, l.y);
     split_hilo(z - root[2], h.z, l.z);
-    xs[s] = x;
-    ys[s] = y;
-    zs[s] = z;
+    const bool wide = fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z))) > kWide;
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (wide)
+        r = make_float4(split_rest(x, root[0], h.x, l.x), split_rest(y, root[1], h.y, l.y),
+                        split_rest(z, root[2], h.z, l.z), 0.f);
+    pr[s] = r;
     h.w = src ? (float)q[i] : 0.0f;
     const double k = (w == 1 && m[i] > 0.0) ? kconst * q[i] / m[i] : 0.0;
     l.w = k != 0.0 ? 1.f : 0.f;
@@ -178,7 +181,7 @@ __global__ void na_gather(const uint32_t *__restrict__ idx, int n, const double 
     qm[s] = k;
     ax[s] = ay[s] = az[s] = 0.0;
     if (h.w != (is_src(st[0]) ? (float)q[0] : 0.0f)) marks[0] = 1;
-    if (fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z))) > kWide) marks[1] = 1;
+    if (wide) marks[1] = 1;
 }
 
 // every output entry is written: targets get their acceleration, everything else 0
@@ -230,9 +233,7 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     uint32_t *idx_alt = (uint32_t *)carve(sizeof(uint32_t) * ni);
     float4 *ph = (float4 *)carve(sizeof(float4) * ni);
     float4 *pl = (float4 *)carve(sizeof(float4) * ni);
-    double *xs = (double *)carve(sizeof(double) * ni);
-    double *ys = (double *)carve(sizeof(double) * ni);
-    double *zs = (double *)carve(sizeof(double) * ni);
+    float4 *pr = (float4 *)carve(sizeof(float4) * ni);
     double *qm = (double *)carve(sizeof(double) * ni);
     double *ax = (double *)carve(sizeof(double) * ni);
     double *ay = (double *)carve(sizeof(double) * ni);
@@ -257,10 +258,10 @@ extern "C" sv_status sv_direct_accel_noalloc(int64_t n, const double *x3, const 
     if (cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, kb, vb, ni, 0, 3 * kMortonBits + 1, s) != cudaSuccess)
         return SV_ERR_CUDA;
     const uint32_t *sidx = vb.Current();
-    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, root, ph, pl, xs, ys, zs,
-                                 qm, ax, ay, az, marks);
+    na_gather<<<nb, 256, 0, s>>>(sidx, ni, x3, q, m_amu, status, k_const, root, ph, pl, pr, qm,
+                                 ax, ay, az, marks);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;
-    if (launch_direct_mixed_sorted(ph, pl, xs, ys, zs, ni, (float)softening2, ax, ay, az, marks, s) != cudaSuccess)
+    if (launch_direct_mixed_sorted(ph, pl, pr, ni, (float)softening2, ax, ay, az, marks, s) != cudaSuccess)
         return SV_ERR_CUDA;
     na_scatter<<<nb, 256, 0, s>>>(sidx, ni, qm, ax, ay, az, a3);
     if (cudaGetLastError() != cudaSuccess) return SV_ERR_CUDA;

@@ -49,13 +49,31 @@ struct Parts {
     float v = 0.f, low = 0.f, rest = 0.f;
 };
 __device__ __forceinline__ Parts negated(const Parts &p) { return Parts{-p.v, -p.low, -p.rest}; }
-__device__ __forceinline__ Parts parts_of(double d) {
-    Parts p;
-    p.v = (float)d;
-    d -= (double)p.v;
-    p.low = (float)d;
-    p.rest = (float)(d - (double)p.low);
-    return p;
+
+// a + b as its rounded value and the exact rest (Knuth)
+__device__ __forceinline__ float two_sum(float a, float b, float &err) {
+    const float s = a + b, bb = s - a;
+    err = (a - (s - bb)) + (b - bb);
+    return s;
+}
+
+// The difference a - o of two coordinates as parts that do not overlap: of the first
+// two parts with hilo_diff, or (wide) of all three, exact to their last bits.
+template <bool WIDE>
+__device__ __forceinline__ Parts parts_diff(const Parts &a, const Parts &o) {
+    Parts d;
+    if (!WIDE) {
+        d.v = hilo_diff(a.v, a.low, o.v, o.low, d.low);
+        return d;
+    }
+    float e, f, g, h;
+    const float s = two_sum(a.v, -o.v, e), t = two_sum(a.low, -o.low, f);
+    const float u = two_sum(e, t, g);
+    d.v = two_sum(s, u, h);
+    const float r = g + (f + (a.rest - o.rest));
+    d.low = h + r;
+    d.rest = r - (d.low - h);
+    return d;
 }
 
 // Tiles by distance: far from the block, near it (the second parts added to each

@@ -175,7 +175,7 @@ struct GatherArgs {
     float *qs;
     double *qm;
     double *zax, *zay, *zaz;  // sorted accelerations to clear, or null
-    float4 *ph, *pl;          // FP32 hi + lo positions to write, or null
+    float4 *ph, *pl, *pr;     // FP32 hi and lo positions and what they leave out to write, or null
     int abs_xy;               // ... relative to the z axis in x and y, not to the root's origin
     const double *root;
     int *marks;               // set with ph: [0] a source charge differs from particle 0's, [1] a source lies
@@ -198,8 +198,8 @@ __device__ __forceinline__ double sorted_qm(const GatherArgs &a, uint32_t i) {
 // 7.7e-7 against 1.2e-4 force error).
 __device__ __forceinline__ int gather_one(const GatherArgs &a, const double *root, int64_t s, uint32_t i) {
     const bool src = is_source(a.st[i]);
-    const double x = src ? a.x[i] : root[0], y = src ? a.y[i] : root[1], z = src ? a.z[i] : root[2];
-    const double k = sorted_qm(a, i);
+    const double px = a.x[i], py = a.y[i], pz = a.z[i], k = sorted_qm(a, i);
+    const double x = src ? px : root[0], y = src ? py : root[1], z = src ? pz : root[2];
     const float q = sorted_charge(a, i);
     a.xs[s] = x;
     a.ys[s] = y;
@@ -217,6 +217,11 @@ __device__ __forceinline__ int gather_one(const GatherArgs &a, const double *roo
         a.ph[s] = h;
         a.pl[s] = l;
         const bool wide = fmaxf(fabsf(h.x), fmaxf(fabsf(h.y), fabsf(h.z))) > kWide;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (wide)
+            r = make_float4(split_rest(x, a.abs_xy ? 0.0 : root[0], h.x, l.x),
+                            split_rest(y, a.abs_xy ? 0.0 : root[1], h.y, l.y), split_rest(z, root[2], h.z, l.z), 0.f);
+        if (a.pr) a.pr[s] = r;
         return (h.w != sorted_charge(a, 0) ? 1 : 0) | (wide ? 2 : 0);
     }
     return 0;
@@ -354,10 +359,10 @@ sort_chunks(int n, int sh, const double *__restrict__ root, uint64_t *__restrict
 // and takes the first source's position as the origin of the FP32 parts.
 __global__ void __launch_bounds__(256)
 sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restrict__ done, int *__restrict__ bits) {
-    __shared__ int wsum[8], tot[3];  // sources before this CTA, in all; first source
+    __shared__ int wsum[8], tot[4];  // sources before this CTA, in all; first source; marks
     __shared__ double org[3];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    if (tid < 3) tot[tid] = tid == 2 ? n : 0;
+    if (tid < 4) tot[tid] = tid == 2 ? n : 0;
     __syncthreads();
     int before = 0, all = 0, first = n;
 #pragma unroll 4
@@ -393,9 +398,11 @@ sources_first(int n, uint32_t *__restrict__ idx, GatherArgs a, unsigned *__restr
         marks = gather_one(a, org, pos, (uint32_t)i);
     }
     // the marks, from the last CTA to finish
-    const int differ = __syncthreads_or(marks & 1), wide = __syncthreads_or(marks & 2);
+    marks = __reduce_or_sync(0xffffffffu, marks);
+    if (lane == 0 && marks) atomicOr(&tot[3], marks);
+    __syncthreads();
     if (tid == 0) {
-        if (differ || wide) atomicOr(bits, (differ ? 1 : 0) | (wide ? 2 : 0));
+        if (tot[3]) atomicOr(bits, tot[3]);
         __threadfence();
         if (atomicAdd(done, 1u) == gridDim.x - 1) {
             const int b = atomicExch(bits, 0);
@@ -457,11 +464,14 @@ rank_gather(int n, int sh, const uint64_t *__restrict__ ckeys, const uint32_t *_
     if (!live) return;
     const uint32_t i = cidx[s];
     if (part < 3) {
-        const double v = is_source(a.st[i]) ? (part == 0 ? a.x : part == 1 ? a.y : a.z)[i] : a.root[part];  // as gather_one
+        const double own = (part == 0 ? a.x : part == 1 ? a.y : a.z)[i];
+        const double v = is_source(a.st[i]) ? own : a.root[part];  // as gather_one
         (part == 0 ? a.xs : part == 1 ? a.ys : a.zs)[rank] = v;
         if (a.ph) {
             float h, l;
-            split_hilo(v - (a.abs_xy && part < 2 ? 0.0 : a.root[part]), h, l);
+            const double o = a.abs_xy && part < 2 ? 0.0 : a.root[part];
+            split_hilo(v - o, h, l);
+            if (a.pr) reinterpret_cast<float *>(a.pr + rank)[part] = fabsf(h) > kWide ? split_rest(v, o, h, l) : 0.f;
             reinterpret_cast<float *>(a.ph + rank)[part] = h;
             reinterpret_cast<float *>(a.pl + rank)[part] = l;
             if (fabsf(h) > kWide) a.marks[1] = 1;
@@ -530,7 +540,7 @@ sv_status ensure_sorted_capacity(sv_ctx *c, int64_t n) {
     cudaFree(S.x); cudaFree(S.y); cudaFree(S.z); cudaFree(S.q); cudaFree(S.qm);
     cudaFree(S.idx); cudaFree(S.keys); cudaFree(S.keys_alt); cudaFree(S.idx_alt);
     cudaFree(S.ax); cudaFree(S.ay); cudaFree(S.az); cudaFree(S.cub_tmp);
-    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl);
+    cudaFree(S.root); cudaFree(S.red); cudaFree(S.ph); cudaFree(S.pl); cudaFree(S.pr);
     S = Sorted();
     const int64_t cap = n < 1024 ? 1024 : n;
     SV_CK(c, cudaMalloc(&S.x, cap * sizeof(double)));
@@ -581,6 +591,13 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
         SV_CK(c, cudaMalloc(&S.pl, sizeof(float4) * S.cap));
         S.hl_cap = S.cap;
     }
+    if (want.rest && S.pr_cap < n) {
+        cudaFree(S.pr);
+        S.pr = nullptr;
+        S.pr_cap = 0;
+        SV_CK(c, cudaMalloc(&S.pr, sizeof(float4) * S.cap));
+        S.pr_cap = S.cap;
+    }
     S.n = n;
     S.n_orig = v.n_orig;
     // levels 1 .. levels occupy bits >= 3 (kMortonBits - levels); bit 63 marks inactive keys
@@ -589,7 +606,7 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
     const int sh = 3 * (kMortonBits - levels);
     GatherArgs ga{v.x, v.y, v.z, v.q, v.m, v.qom, v.status, first, std::min(last, v.n_orig), c->P.k_const,
                   S.x, S.y, S.z, S.q, S.qm, nullptr, nullptr, nullptr, want.hilo ? S.ph : nullptr,
-                  want.hilo ? S.pl : nullptr, want.hl_abs ? 1 : 0, S.root, reinterpret_cast<int *>(S.root + 14)};
+                  want.hilo ? S.pl : nullptr, want.rest ? S.pr : nullptr, want.hl_abs ? 1 : 0, S.root, reinterpret_cast<int *>(S.root + 14)};
     if (want.zero) {
         ga.zax = S.ax;
         ga.zay = S.ay;

@@ -25,6 +25,7 @@ struct SortWants {
     int levels = kMortonBits;  // Morton levels to order: a tree needs its keys ordered down to its leaf level only
     bool zero = false;         // also clear ax, ay, az (a method that adds into them)
     bool hilo = false;         // also write ph, pl
+    bool rest = false;         // ... and pr
     bool hl_abs = false;       // ... relative to the z axis in x and y
     bool any_order = false;    // only put the sources first
 };
@@ -46,7 +47,8 @@ struct Sorted {
     // z axis in x and y), hi.w the source charge, lo.w 1 for targets; written by
     // the sort when want.hilo
     float4 *ph = nullptr, *pl = nullptr;
-    int64_t hl_cap = 0;
+    float4 *pr = nullptr;  // what hi and lo leave of the FP64 position (want.rest)
+    int64_t hl_cap = 0, pr_cap = 0;
     // a second field to add in the scatter (the FMM's far field: x, y, z at
     // far, far + far_stride, far + 2 far_stride), or null; cleared by it
     const double *far = nullptr;
@@ -106,7 +108,7 @@ struct ImageSet {
     double domain[3] = {};
     double *buf = nullptr;
     const double *m = nullptr;           // 3 per image: metres, in the reference's summation order
-    const float4 *hl = nullptr;          // the same as FP32 hi and lo parts, two per image
+    const float4 *hl = nullptr;          // the same as FP32 parts: hi, lo and what they leave out, per image
     const double *zero_first = nullptr;  // metres, the zero offset first
 };
 
@@ -311,20 +313,19 @@ sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; r
 constexpr int64_t kAnyOrderMax = 8192;
 // what the direct sum of this context needs of its sort
 void direct_sort_wants(sv_ctx *c);
-// Extent of a plume, from its sort's origin, past which the mixed pair sums take their
-// coordinates from the FP64 positions.  FP32 hi + lo parts resolve 2^-49 of the distance
-// to the origin, 5.5e-17 m at this one: FP32's own rounding of a nanometre.  Clusters
-// of 10 nm spread over 10 m: 5.6e-5 force error from the parts, 9e-7 from offsets
-// to each block, 2e-7 so.
+// Extent of a plume, from its sort's origin, past which the mixed pair sums keep a third
+// part of every coordinate.  FP32 hi + lo parts resolve 2^-49 of the distance to the
+// origin, 5.5e-17 m at this one: FP32's own rounding of a nanometre.  Force error of
+// clusters of 10 nm spread over 10 m: 5.6e-5 with two parts, 9e-7 with FP64 offsets to
+// each block rounded to FP32, 7e-8 so.
 constexpr float kWide = 0.03125f;
 
 // the mixed-precision all-pairs sums (no symmetry images) of n sorted
-// particles given as FP32 hi + lo parts (Sorted::ph, pl) and FP64 positions, without
-// the targets' factor K q / m, added into the cleared ax, ay, az; marks: the sort's two;
-// launches only, allocates nothing
-cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const double *x, const double *y,
-                                       const double *z, int n, float eps2, double *ax, double *ay, double *az,
-                                       const int *marks, cudaStream_t stream);
+// particles given as FP32 parts (Sorted::ph, pl, pr), without the targets' factor
+// K q / m, added into the cleared ax, ay, az; marks: the sort's two; launches only,
+// allocates nothing
+cudaError_t launch_direct_mixed_sorted(const float4 *ph, const float4 *pl, const float4 *pr, int n, float eps2,
+                                       double *ax, double *ay, double *az, const int *marks, cudaStream_t stream);
 
 // A double's bits as a signed integer whose order is the double's order
 // (non-NaN values); the map is its own inverse.  Min / max on these run on
@@ -340,6 +341,12 @@ __device__ __forceinline__ bool ordered_nan(long long v) {
 __device__ __forceinline__ void split_hilo(double v, float &hi, float &lo) {
     hi = (float)v;
     lo = (float)(v - (double)hi);
+}
+// what they leave out of v - o, its own rounding included (kept for particles further than
+// kWide from the origin: up to there two parts are enough)
+__device__ __forceinline__ float split_rest(double v, double o, float hi, float lo) {
+    const double d = v - o, b = d - v, e = (v - (d - b)) - (o + b);
+    return (float)(((d - (double)hi) - (double)lo) + e);
 }
 
 // tree.cu / bh.cu / fmm.cu

@@ -1,7 +1,7 @@
 """Plumes of tight clusters over metres: the mixed pair sums keep the FP64 positions' differences.
 
 FP32 hi + lo parts resolve 2^-49 of a particle's distance from the plume's origin; from
-1/32 m on the pair kernels take FP64 offsets and keep all their bits, in the caller's
+1/32 m on the pair kernels keep a third part, all bits of the position, in the caller's
 order (up to 8,192 particles) as in the Morton order, for clusters that fill whole
 blocks and for clusters that alternate in the caller's order.  What is left is
 the FP32 pair arithmetic: 2e-6 relative L2 per particle, the mixed direct sum's bound;
@@ -36,7 +36,7 @@ def clusters(n, k, size, d, alternate, seed=3):
 @pytest.mark.parametrize("alternate", [False, True], ids=["grouped", "alternating"])
 @pytest.mark.parametrize("n,k,size,d", [(300, 3, 1e-8, 10.0), (2048, 4, 1e-8, 10.0), (2500, 5, 1e-7, 10.0),
                                         (2048, 4, 1e-8, 0.012), (2048, 4, 1e-8, 0.05), (16384, 8, 1e-8, 1.0),
-                                        (16384, 64, 1e-8, 10.0)])
+                                        (16384, 8, 1e-8, 10.0), (16384, 64, 1e-8, 10.0), (40000, 8, 1e-8, 10.0)])
 def test_forces(n, k, size, d, alternate, charges):
     st = clusters(n, k, size, d, alternate)
     if charges == "mixed":
