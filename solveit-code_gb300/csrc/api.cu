@@ -492,12 +492,12 @@ sv_status stage_bytes(sv_ctx *c, size_t bytes, void **p) {
 
 // Page-locked, mapped staging for small uploads: the host copies the caller's
 // arrays there and the unpacking kernel reads them in place, one launch instead
-// of a copy per array.  A force call with it, of the same with copies: 0.77 to 0.93 of the
-// time up to 8,000 ions, 0.93 to 0.96 at 16,000, 1.00 to 1.01 at 20,000, 1.04 to 1.05
-// at 24,000 and 1.09 to 1.11 at 32,000, where the host's own copy is the slower one
-// (direct sum and Barnes-Hut).
+// of a copy per array.  A force call with it, of the same with copies (direct sum,
+// Barnes-Hut, FMM): 0.84 to 0.95 of the time at 12,000 ions, 0.92 to 0.98 at 16,000, 0.97
+// to 1.00 at 20,000, 0.99 to 1.02 at 22,000, 1.01 to 1.05 at 24,000 and 1.06 to 1.11 at
+// 32,000, where the host's own copy is the slower one.
 // Waits until the last kernel that read it is done.
-constexpr int64_t kPinnedMax = 20000;
+constexpr int64_t kPinnedMax = 22000;
 
 sv_status pinned_stage(sv_ctx *c, size_t bytes, void **dev) {
     if (!c->h_stage_read) SV_CK(c, cudaEventCreateWithFlags(&c->h_stage_read, cudaEventDisableTiming));

@@ -303,7 +303,7 @@ sv_status sort_view(sv_ctx *c, const ParticleView &v, int64_t first, int64_t las
 sv_status unsort_accel(sv_ctx *c);
 
 // direct.cu
-sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; raw sums in mixed precision)
+sv_status direct_accel(sv_ctx *c);  // sorted -> c->S.a* (cleared by the sort; raw sums)
 // Up to the pairs of this many particles (images counted) the direct sum and the
 // adjoint take their sources in the caller's order: the sort's launches take longer
 // than the pairs' close form on every tile.  A step of the direct sum at 8,192
