@@ -273,9 +273,9 @@ struct JLow {
     float2 x[kJH][32], y[kJH][32], z[kJH][32];
     float2 rx[kJH][32], ry[kJH][32], rz[kJH][32];
 };
-// the travelling particle: negated coordinates, charge, negated u (hi, lo), and its sums
+// the travelling particle: negated coordinates and what they leave out, charge, negated u (hi, lo), and its sums
 struct JTravel {
-    Parts x, y, z;
+    float x, y, z, mx, my, mz, kx, ky, kz;
     float q = 0.f, ux = 0.f, uy = 0.f, uz = 0.f, vx = 0.f, vy = 0.f, vz = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
 };
 
@@ -290,15 +290,15 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
         float2 jx, jy, jz;
 #pragma unroll
         for (int p = 0; p < kJH; p++) {
-            float2 dx = __fadd2_rn(b.X[p], dup(t.x.v)), dy = __fadd2_rn(b.Y[p], dup(t.y.v)),
-                   dz = __fadd2_rn(b.Z[p], dup(t.z.v));
+            float2 dx = __fadd2_rn(b.X[p], dup(t.x)), dy = __fadd2_rn(b.Y[p], dup(t.y)),
+                   dz = __fadd2_rn(b.Z[p], dup(t.z));
             if (MODE != kTileFar) {
-                float2 ex = __fadd2_rn(low.x[p][lane], dup(t.x.low)), ey = __fadd2_rn(low.y[p][lane], dup(t.y.low)),
-                       ez = __fadd2_rn(low.z[p][lane], dup(t.z.low));
+                float2 ex = __fadd2_rn(low.x[p][lane], dup(t.mx)), ey = __fadd2_rn(low.y[p][lane], dup(t.my)),
+                       ez = __fadd2_rn(low.z[p][lane], dup(t.mz));
                 if (MODE == kTileWide) {
-                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(t.x.rest)));
-                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(t.y.rest)));
-                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(t.z.rest)));
+                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(t.kx)));
+                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(t.ky)));
+                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(t.kz)));
                 }
                 dx = __fadd2_rn(dx, ex);
                 dy = __fadd2_rn(dy, ey);
@@ -330,18 +330,18 @@ __device__ __forceinline__ void jtv_tile(JBlock &b, const JLow &low, float2 E2, 
                 jz = p == 0 ? vz : __fadd2_rn(jz, vz);
             }
         }
-        t.x.v = turn(t.x.v);
-        t.y.v = turn(t.y.v);
-        t.z.v = turn(t.z.v);
+        t.x = turn(t.x);
+        t.y = turn(t.y);
+        t.z = turn(t.z);
         if (MODE != kTileFar) {
-            t.x.low = turn(t.x.low);
-            t.y.low = turn(t.y.low);
-            t.z.low = turn(t.z.low);
+            t.mx = turn(t.mx);
+            t.my = turn(t.my);
+            t.mz = turn(t.mz);
         }
         if (MODE == kTileWide) {
-            t.x.rest = turn(t.x.rest);
-            t.y.rest = turn(t.y.rest);
-            t.z.rest = turn(t.z.rest);
+            t.kx = turn(t.kx);
+            t.ky = turn(t.ky);
+            t.kz = turn(t.kz);
         }
         if (!UQ) t.q = turn(t.q);
         t.ux = turn(t.ux);
@@ -450,9 +450,15 @@ __device__ __forceinline__ void jtv_unit(const JPairArgs &a, JLow &low, int A, i
             t.vz = -ul.z;
         }
         const bool near = j < a.n && fmaxf(fabsf(x.v), fmaxf(fabsf(y.v), fabsf(z.v))) <= 2.f * ext;
-        t.x = negated(x);
-        t.y = negated(y);
-        t.z = negated(z);
+        t.x = -x.v;
+        t.y = -y.v;
+        t.z = -z.v;
+        t.mx = -x.low;
+        t.my = -y.low;
+        t.mz = -z.low;
+        t.kx = -x.rest;
+        t.ky = -y.rest;
+        t.kz = -z.rest;
         if (!SYM || __any_sync(0xffffffffu, near)) {
             jtv_tile<UQ, SYM, WIDE ? kTileWide : kTileNear>(b, low, E2, min_r2, t);
         } else {

@@ -110,28 +110,29 @@ struct PairLow {
     float2 rx[R / 2][32], ry[R / 2][32], rz[R / 2][32];
 };
 
-// 32 steps of a travelling tile: negated coordinates nx, ny, nz and charge q; (sx, sy,
-// sz) return the sums on the travelling particle (SYM).
+// 32 steps of a travelling tile: negated coordinates (nx, ny, nz; what they leave out: m, k)
+// and charge q; (sx, sy, sz) return the sums on the travelling particle (SYM).  (As three
+// Parts the loop takes a move more per step: 2,000 particles with 81 images 185 -> 191 us.)
 template <int R, bool UQ, bool CLAMP, bool SYM, int MODE>
-__device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low, float2 E2, Parts nx, Parts ny,
-                                          Parts nz, float q, float &sx, float &sy, float &sz) {
+__device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low, float2 E2, float nx, float ny, float nz, float q,
+                                          float mx, float my, float mz, float kx, float ky, float kz, float &sx, float &sy, float &sz) {
     auto dup = [](float v) { return make_float2(v, v); };
     constexpr int H = R / 2;
     const int lane = threadIdx.x & 31, from = (lane + 1) & 31;
 #pragma unroll 1
     for (int step = 0; step < 32; step++) {
-        const float2 NX = dup(nx.v), NY = dup(ny.v), NZ = dup(nz.v), QJ = dup(q);
+        const float2 NX = dup(nx), NY = dup(ny), NZ = dup(nz), QJ = dup(q);
         float2 jx, jy, jz;
 #pragma unroll
         for (int p = 0; p < H; p++) {
             float2 dx = __fadd2_rn(b.X[p], NX), dy = __fadd2_rn(b.Y[p], NY), dz = __fadd2_rn(b.Z[p], NZ);
             if (MODE != kTileFar) {
-                float2 ex = __fadd2_rn(low.x[p][lane], dup(nx.low)), ey = __fadd2_rn(low.y[p][lane], dup(ny.low)),
-                       ez = __fadd2_rn(low.z[p][lane], dup(nz.low));
+                float2 ex = __fadd2_rn(low.x[p][lane], dup(mx)), ey = __fadd2_rn(low.y[p][lane], dup(my)),
+                       ez = __fadd2_rn(low.z[p][lane], dup(mz));
                 if (MODE == kTileWide) {
-                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(nx.rest)));
-                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(ny.rest)));
-                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(nz.rest)));
+                    ex = __fadd2_rn(ex, __fadd2_rn(low.rx[p][lane], dup(kx)));
+                    ey = __fadd2_rn(ey, __fadd2_rn(low.ry[p][lane], dup(ky)));
+                    ez = __fadd2_rn(ez, __fadd2_rn(low.rz[p][lane], dup(kz)));
                 }
                 dx = __fadd2_rn(dx, ex);
                 dy = __fadd2_rn(dy, ey);
@@ -152,18 +153,18 @@ __device__ __forceinline__ void pair_tile(PairBlock<R> &b, const PairLow<R> &low
                 jz = p == 0 ? __fmul2_rn(dz, wj) : __ffma2_rn(dz, wj, jz);
             }
         }
-        nx.v = __shfl_sync(0xffffffffu, nx.v, from);
-        ny.v = __shfl_sync(0xffffffffu, ny.v, from);
-        nz.v = __shfl_sync(0xffffffffu, nz.v, from);
+        nx = __shfl_sync(0xffffffffu, nx, from);
+        ny = __shfl_sync(0xffffffffu, ny, from);
+        nz = __shfl_sync(0xffffffffu, nz, from);
         if (MODE != kTileFar) {
-            nx.low = __shfl_sync(0xffffffffu, nx.low, from);
-            ny.low = __shfl_sync(0xffffffffu, ny.low, from);
-            nz.low = __shfl_sync(0xffffffffu, nz.low, from);
+            mx = __shfl_sync(0xffffffffu, mx, from);
+            my = __shfl_sync(0xffffffffu, my, from);
+            mz = __shfl_sync(0xffffffffu, mz, from);
         }
         if (MODE == kTileWide) {
-            nx.rest = __shfl_sync(0xffffffffu, nx.rest, from);
-            ny.rest = __shfl_sync(0xffffffffu, ny.rest, from);
-            nz.rest = __shfl_sync(0xffffffffu, nz.rest, from);
+            kx = __shfl_sync(0xffffffffu, kx, from);
+            ky = __shfl_sync(0xffffffffu, ky, from);
+            kz = __shfl_sync(0xffffffffu, kz, from);
         }
         if (!UQ) q = __shfl_sync(0xffffffffu, q, from);
         if (SYM) {
@@ -250,10 +251,17 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, in
                 py = g == 1 ? x0 : g == 2 ? negated(y0) : negated(x0);
             } else if (a.kind == 2) {
                 // source shifted by the image offset: the origin shifted back
-                const float4 fh = a.off[3 * g], fl = a.off[3 * g + 1], fr = a.off[3 * g + 2];
-                cx = parts_diff<WIDE>(cx, Parts{fh.x, fl.x, fr.x});
-                cy = parts_diff<WIDE>(cy, Parts{fh.y, fl.y, fr.y});
-                cz = parts_diff<WIDE>(cz, Parts{fh.z, fl.z, fr.z});
+                const float4 fh = a.off[3 * g], fl = a.off[3 * g + 1],
+                             fr = WIDE ? a.off[3 * g + 2] : make_float4(0.f, 0.f, 0.f, 0.f);
+                auto back = [](const Parts &o, const Parts &f) {
+                    if (WIDE) return parts_diff<WIDE>(o, f);
+                    const float s = o.v - f.v, bb = s - o.v;
+                    const float e = ((o.v - (s - bb)) - (f.v + bb)) + (o.low - f.low), r = s + e;
+                    return Parts{r, e - (r - s)};
+                };
+                cx = back(cx, Parts{fh.x, fl.x, fr.x});
+                cy = back(cy, Parts{fh.y, fl.y, fr.y});
+                cz = back(cz, Parts{fh.z, fl.z, fr.z});
             }
             x = parts_diff<WIDE>(px, cx);
             y = parts_diff<WIDE>(py, cy);
@@ -265,10 +273,9 @@ __device__ __forceinline__ void pair_unit(const PairArgs &a, PairLow<R> &low, in
         const bool anyB = SYM && __any_sync(0xffffffffu, jt);
         if (!anyA && !anyB) continue;
         float sx = 0.f, sy = 0.f, sz = 0.f;  // the travelling particle's sums
-        const Parts nx = negated(x), ny = negated(y), nz = negated(z);
         if (!SYM || __any_sync(0xffffffffu, near)) {
-            pair_tile<R, UQ, CLAMP, SYM, WIDE ? kTileWide : kTileNear>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
-        } else pair_tile<R, UQ, CLAMP, SYM, kTileFar>(b, low, E2, nx, ny, nz, q, sx, sy, sz);
+            pair_tile<R, UQ, CLAMP, SYM, WIDE ? kTileWide : kTileNear>(b, low, E2, -x.v, -y.v, -z.v, q, -x.low, -y.low, -z.low, -x.rest, -y.rest, -z.rest, sx, sy, sz);
+        } else pair_tile<R, UQ, CLAMP, SYM, kTileFar>(b, low, E2, -x.v, -y.v, -z.v, q, -x.low, -y.low, -z.low, -x.rest, -y.rest, -z.rest, sx, sy, sz);
         if (SYM && jt) {
             if (a.kind == 1 && g) {  // the sum on the unrotated particle: turned back by -g*pi/2
                 const float tx = sx, ty = sy;
