@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(32 * kPairWarps) jtv_pairs64_kernel(JPair64Arg
 // a power of two from max|u|; both are exact and undone in FP64 at the end.
 // The reciprocal square root is refined by one Newton step.  FP32-pipe bound:
 // 45 operations per pair (39 when all charges are equal), two targets per packed
-// instruction, each pair once: 16,384 particles 532 -> 211 us per launch, 4,096
-// 54 -> 21 us, against the one-sided scalar kernel.  Wide plumes (kWide) keep a third
+// instruction, each pair once: 16,384 particles 532 -> 217 us per launch, 4,096
+// 54 -> 22 us, against the one-sided scalar kernel.  Wide plumes (kWide) keep a third
 // part of their coordinates.
 struct JPairArgs {
     const float4 *ph, *pl, *uh, *ul;

@@ -36,8 +36,8 @@
 // correction in FP64.
 //
 // Measured per launch (serialised), against the one-sided kernels they
-// replaced: mixed, 30,011 particles of two charges 381 -> 303 us, 16,384 of one
-// charge 123 -> 99 us, 3,001 with 81 images 652 -> 235 us (144 CTAs before: the
+// replaced: mixed, 30,011 particles of two charges 381 -> 289 us, 16,384 of one
+// charge 123 -> 99 us, 3,001 with 81 images 652 -> 232 us (144 CTAs before: the
 // images were not split); FP64, 4,096 particles 773 -> 285 us.
 #include <algorithm>
 
